@@ -16,8 +16,9 @@ Operations (`op`):
 Potentials are the seeded synthetic ones of vhci_b200/pes.py (the first admissible draw of each
 workload, restricted to its first `modes` modes); a case's seed scales every force constant by about
 2 % and every frequency by about 0.5 %, so each seed is another molecule of the same kind.  Bases
-are the n product states of lowest harmonic energy, in the order heat-bath iterations would append
-them: a few growing shells, ascending keys within each.
+are like the ones that heat-bath selection leaves: half of the n product states are a core of low
+harmonic energy, the others are reached from it through the stronger force constants in two more
+rounds; each round is appended in ascending key order, as the library does.
 """
 import functools
 import itertools
@@ -108,24 +109,35 @@ def _molecule(case, seed):
     return [float("%.6f" % x) for x in f], [(ms, float("%.10f" % x)) for (ms, _), x in zip(fcs, v)]
 
 
-def _basis(freq, n, cap=12):
-    """The n states of lowest harmonic energy (quanta, energies above the zero point), in shells."""
-    step = 5.0
-    emax = step * 64
-    while True:  # an energy bound that holds at least n states, by counting on a grid
+@functools.lru_cache(maxsize=None)
+def _changes(kind, modes):
+    """(quanta changes, cumulated share of each) of a potential, shares by size of force constant."""
+    found = _patterns(_potential(kind, modes)[1])
+    found.pop((), None)
+    delta = np.zeros((len(found), modes), np.int8)
+    for i, d in enumerate(found):
+        for m, x in d:
+            delta[i, m] = x
+    size = np.array([sum(abs(c) for c, _ in terms) for terms in found.values()])
+    return delta, np.cumsum(size / size.sum())
+
+
+def _core(freq, n, cap):
+    """The n states of lowest harmonic energy."""
+    step, emax = 5.0, 320.0
+    while True:  # an energy bound that holds them, by counting on a grid
         count = np.zeros(int(emax / step) + 1)
         count[0] = 1
         for w in freq:
             s = max(1, int(w / step))
             for e in range(s, len(count)):
                 count[e] += count[e - s]
-        if count.sum() >= 1.3 * n + 10:
+        if count.sum() >= 1.2 * n + 10:
             break
         emax *= 1.3
-    emax = step * (np.searchsorted(np.cumsum(count), 1.3 * n + 10) + 1) + step * 8
-    q = np.zeros((1, len(freq)), np.uint8)
-    e = np.zeros(1)
+    emax = step * (np.searchsorted(np.cumsum(count), 1.2 * n + 10) + 8)
     while True:
+        q, e = np.zeros((1, len(freq)), np.uint8), np.zeros(1)
         for i, w in enumerate(freq):
             reps = np.minimum(cap, np.floor((emax - e) / w)).astype(np.int64) + 1
             at = np.repeat(np.arange(len(e)), reps)
@@ -133,24 +145,45 @@ def _basis(freq, n, cap=12):
             q, e = q[at], e[at] + j * w
             q[:, i] = j
         if len(e) >= n:
-            break
-        q, e, emax = np.zeros((1, len(freq)), np.uint8), np.zeros(1), emax * 1.1
-    low = np.argsort(e, kind="stable")[:n]
-    q, e = q[low], e[low]
-    words = -(-len(freq) // 16)
-    key = np.zeros((words, n), np.uint64)
-    for m in range(len(freq)):
-        key[m // 16] |= q[:, m].astype(np.uint64) << np.uint64(4 * (m % 16))
-    order, cuts = [], [0, max(1, n // 20), max(1, n // 2), n]
-    for a, b in zip(cuts, cuts[1:]):
-        order.append(a + np.lexsort(key[:, a:b]))
-    order = np.concatenate(order)
-    return np.ascontiguousarray(q[order]), e[order]
+            return q[np.argsort(e, kind="stable")[:n]]
+        emax *= 1.1
+
+
+def _basis(case, freq, seed, cap=12):
+    """n states (quanta, harmonic energies above the zero point): a core and two rounds of growth."""
+    n, modes = case["n"], len(freq)
+    rng = np.random.Generator(np.random.PCG64([seed, 14]))
+    delta, share = _changes(case["pes"], modes)
+    mult = np.random.Generator(np.random.PCG64(5)).integers(-2**62, 2**62, modes)
+    q = _core(freq, -(-n // 2), cap)
+    parts = [q]
+    for want in (n // 4, n - len(q) - n // 4):
+        have = np.sort(q.astype(np.int64) @ mult)  # a linear hash tells states apart
+        new, keys = np.zeros((0, modes), np.uint8), np.zeros(0, np.int64)
+        while len(new) < want:
+            m = 2 * (want - len(new)) + 1000
+            t = q[rng.integers(0, len(q), m)].astype(np.int8) + delta[np.searchsorted(share, rng.random(m)).clip(max=len(delta) - 1)]
+            t = t[((t >= 0) & (t <= cap)).all(1)].astype(np.uint8)
+            new = np.concatenate([new, t])
+            keys = np.concatenate([keys, t.astype(np.int64) @ mult])
+            at = np.searchsorted(have, keys).clip(max=len(have) - 1)
+            first = np.zeros(len(keys), bool)
+            first[np.unique(keys, return_index=True)[1]] = True
+            new, keys = new[first & (have[at] != keys)], keys[first & (have[at] != keys)]
+        parts.append(new[:want])
+        q = np.concatenate([q, new[:want]])
+    for i, part in enumerate(parts):
+        key = np.zeros((-(-modes // 16), len(part)), np.uint64)
+        for m in range(modes):
+            key[m // 16] |= part[:, m].astype(np.uint64) << np.uint64(4 * (m % 16))
+        parts[i] = part[np.lexsort(key)]
+    q = np.ascontiguousarray(np.concatenate(parts))
+    return q, q @ np.array(freq)
 
 
 def _context(case, seed):
     freq, fcs = _molecule(case, seed)
-    q, e = _basis(freq, case["n"])
+    q, e = _basis(case, freq, seed)
     v = VHCI(problem=dict(freq=freq, cap=[8] * len(freq), ntot=1, fcs=fcs, eps1=0.0, nstate=case.get("k", 1), pt2=1, eps2=case.get("eps", 0.0)),
              precision=case["precision"])
     return v, freq, q, e
@@ -325,7 +358,7 @@ def exact(case, seed):
     if case["op"] in ("solve", "pt2") or (case["op"] == "eigs" and case["n"] > 2000):
         return None
     freq, fcs = _molecule(case, seed)
-    q, e = _basis(freq, case["n"])
+    q, e = _basis(case, freq, seed)
     if case["op"] == "eigs":
         h = _apply(freq, fcs, q, np.eye(case["n"]))
         return None if h is None else torch.linalg.eigvalsh((0.5 * (h + h.T)).cpu())[: case["k"]]
