@@ -61,7 +61,7 @@ def bench_config(workload: int, batch: int) -> dict:
 
 # Basis size after each heat-bath iteration and |P| of the workload-1 solve (FP64 path).
 WORKLOAD_COUNTS = {"sizes": [38934, 215006, 336950, 372333, 380418], "n_pert": 6583465}
-# DRAM traffic of one k_spmm_pairs launch over its algorithmic bytes, from an ncu capture
+# DRAM traffic of one product over its algorithmic bytes, from an ncu capture of its earlier form
 # (dram__bytes_read.sum + dram__bytes_write.sum = 4.186e9 + 0.051e9 bytes) of a 16-column product
 # on the final workload-1 basis (380,418 rows, 255,052,558 entries; algorithmic 3.164e9 bytes) by
 # `python bench.py --spmm-sweep --sweep-eigs --sweep-reps 2 --checkpoint <file>` on B200.  The
@@ -322,7 +322,7 @@ def run_ours(args):
     en_gbs = (st["pt2_reduce_bytes"] / (st["ms_pt2_reduce"] / 1e3) / 1e9
               if st["ms_pt2_reduce"] else None)
     alg_per_launch = st["spmm_bytes"] / st["spmm_calls"] if st["spmm_calls"] else None
-    roof = {"bound": "hbm", "kernel": "k_spmm_pairs (eigensolver H*X)", "achieved": spmm_gbs,
+    roof = {"bound": "hbm", "kernel": "k_spmm (eigensolver H*X)", "achieved": spmm_gbs,
             "peak": hbm, "unit": "GB/s", "frac": (spmm_gbs / hbm) if spmm_gbs else None,
             "traffic": (args.traffic if args.traffic else
                         NCU_SPMM_TRAFFIC_RATIO * alg_per_launch if alg_per_launch else None),

@@ -7,6 +7,7 @@
 
 #include "conn.cuh"
 #include "ops.h"
+#include "rowprod.cuh"
 
 namespace vhci {
 
@@ -86,155 +87,46 @@ void hbuild_fill_launch(const uint64_t* keys, int64_t row0, int64_t n, KeyLayout
       keys, row0, n, L, basis, cd, nullptr, rowptr, col, val, valf, diag);
 }
 
-// Row-group SpMM, Y[:, 0:bp] = (D + H_off) X[:, 0:bp] for bp <= BP columns: a warp holds
-// G = 32/BP rows, each handled by a group of BP lanes that own one column each and walk the row's
-// entries together (the entry loads are broadcasts within the group and L1 hits across
-// consecutive entries), eight entries per iteration so each lane keeps eight vector-row gathers in
-// flight.  Entry loads are 16-byte (four columns, two or four values) after a scalar prologue to
-// 4-entry alignment.  The diagonal term reads X row xrow0 + i (a rank's row block of a sharded
-// matrix multiplies the gathered whole block); accum != 0 adds into Y instead (a later column
-// panel).
-template <int BP, typename VT>
-__global__ void __launch_bounds__(256) k_spmm_rows(int64_t n, const int64_t* __restrict__ rowptr,
-                                                   const int32_t* __restrict__ col,
-                                                   const VT* __restrict__ val,
-                                                   const double* __restrict__ diag,
-                                                   const double* __restrict__ X, int ldx, int bp,
-                                                   double* __restrict__ Y, int ldy, int accum,
-                                                   int64_t xrow0) {
-  constexpr int G = 32 / BP;
-  const int lane = threadIdx.x & 31;
-  const int grp = lane / BP, cc = lane % BP;
-  const bool active = cc < bp;
-  const int64_t stride = (int64_t)gridDim.x * (blockDim.x >> 5) * G;
-  for (int64_t i = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * G + grp;
-       i < n; i += stride) {
-    const int64_t beg = __ldg(rowptr + i), end = __ldg(rowptr + i + 1);
-    double acc = 0.0;
-    if (active && (!accum || end > beg)) {
-      auto gx = [&](int j) { return __ldg(X + (int64_t)j * ldx + cc); };
-      int64_t e = beg;
-      for (; e < end && (e & 3); ++e) acc = fma((double)__ldg(val + e), gx(__ldg(col + e)), acc);
-      for (; e + 8 <= end; e += 8) {
-        const int4 ja = __ldg(reinterpret_cast<const int4*>(col + e));
-        const int4 jb = __ldg(reinterpret_cast<const int4*>(col + e + 4));
-        double v[8];
-        if constexpr (sizeof(VT) == 8) {
-          const double2 v01 = __ldg(reinterpret_cast<const double2*>(val + e));
-          const double2 v23 = __ldg(reinterpret_cast<const double2*>(val + e + 2));
-          const double2 v45 = __ldg(reinterpret_cast<const double2*>(val + e + 4));
-          const double2 v67 = __ldg(reinterpret_cast<const double2*>(val + e + 6));
-          v[0] = v01.x; v[1] = v01.y; v[2] = v23.x; v[3] = v23.y;
-          v[4] = v45.x; v[5] = v45.y; v[6] = v67.x; v[7] = v67.y;
-        } else {
-          const float4 va = __ldg(reinterpret_cast<const float4*>(val + e));
-          const float4 vb = __ldg(reinterpret_cast<const float4*>(val + e + 4));
-          v[0] = va.x; v[1] = va.y; v[2] = va.z; v[3] = va.w;
-          v[4] = vb.x; v[5] = vb.y; v[6] = vb.z; v[7] = vb.w;
-        }
-        const double x0 = gx(ja.x), x1 = gx(ja.y), x2 = gx(ja.z), x3 = gx(ja.w);
-        const double x4 = gx(jb.x), x5 = gx(jb.y), x6 = gx(jb.z), x7 = gx(jb.w);
-        acc = fma(v[0], x0, acc);
-        acc = fma(v[1], x1, acc);
-        acc = fma(v[2], x2, acc);
-        acc = fma(v[3], x3, acc);
-        acc = fma(v[4], x4, acc);
-        acc = fma(v[5], x5, acc);
-        acc = fma(v[6], x6, acc);
-        acc = fma(v[7], x7, acc);
-      }
-#pragma unroll 4
-      for (; e < end; ++e) acc = fma((double)__ldg(val + e), gx(__ldg(col + e)), acc);
-      if (accum) Y[i * ldy + cc] += acc;
-      else Y[i * ldy + cc] = fma(diag[i], X[(xrow0 + i) * ldx + cc], acc);
-    }
-  }
-}
+// Y[:, 0:VEC bq] = (D + H_off) X, FP64 vectors, one warp per row (rowprod.cuh).  The diagonal term
+// reads X row xrow0 + i (a rank's row block of a sharded matrix multiplies the gathered whole
+// block); accum != 0 adds into Y instead (a later column panel).  Eight gathers in flight per lane at
+// five blocks per SM (51 registers): against sixteen at four blocks 0.375 : 0.401 ms at 120,011 rows
+// and 0.056 : 0.058 ms at 24,000; sixteen win by 3 % only at 300,000 rows.  One warp per row with no
+// loop over rows: the hardware evens out the rows' lengths (0.375 : 0.395 ms against 2368 blocks).
+constexpr int kSpmmUnroll = 8, kSpmmUnrollF = 16;
 
-// Column-pair form of the row-group SpMM: each lane owns two adjacent columns and gathers them as
-// one 16-byte load, so a 16-column block row (128 bytes) takes 8 lanes and a warp holds 4 rows;
-// sixteen entries per iteration keep sixteen 16-byte gathers in flight per lane.  The product is
-// bound by the latency of those gathers (L2 at under half its throughput), so the register budget
-// is set for four resident blocks per SM (64 registers): the compiler then keeps all sixteen
-// gathers in flight, where at its own choice (40 registers, six blocks) it kept fewer.  Measured on
-// the 380k-state workload-1 matrix (b = 16): 2.62 ms, against 2.96 ms at 40 registers and 3.35 ms
-// for one column per lane.  Needs X and Y 16-byte aligned with even strides (the launcher checks).
-template <int BQ, typename VT>
-__global__ void __launch_bounds__(256, 4) k_spmm_pairs(int64_t n, const int64_t* __restrict__ rowptr,
-                                                    const int32_t* __restrict__ col,
-                                                    const VT* __restrict__ val,
-                                                    const double* __restrict__ diag,
-                                                    const double* __restrict__ X, int ldx, int bq,
-                                                    double* __restrict__ Y, int ldy, int accum,
-                                                    int64_t xrow0) {
-  constexpr int G = 32 / BQ, U = 16;
-  const int lane = threadIdx.x & 31;
-  const int grp = lane / BQ, cc = lane % BQ;
-  const bool active = cc < bq;
-  const double2* __restrict__ X2 = reinterpret_cast<const double2*>(X);
-  const int ldx2 = ldx >> 1, ldy2 = ldy >> 1;
-  const int64_t stride = (int64_t)gridDim.x * (blockDim.x >> 5) * G;
-  for (int64_t i = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * G + grp;
-       i < n; i += stride) {
-    const int64_t beg = __ldg(rowptr + i), end = __ldg(rowptr + i + 1);
-    if (!active || (accum && end == beg)) continue;
-    double ax = 0.0, ay = 0.0;
-    auto gx = [&](int j) { return __ldg(X2 + (int64_t)j * ldx2 + cc); };
-    int64_t e = beg;
-    for (; e < end && (e & 3); ++e) {
-      const double v = (double)__ldg(val + e);
-      const double2 x = gx(__ldg(col + e));
-      ax = fma(v, x.x, ax);
-      ay = fma(v, x.y, ay);
-    }
-    for (; e + U <= end; e += U) {
-      int j[U];
-      double v[U];
+template <int BQ, int VEC, typename VT>
+__global__ void __launch_bounds__(256, 5) k_spmm(int64_t n, const int64_t* __restrict__ rowptr,
+                                                 const int32_t* __restrict__ col,
+                                                 const VT* __restrict__ val,
+                                                 const double* __restrict__ diag,
+                                                 const double* __restrict__ X, int ldx, int bq,
+                                                 double* __restrict__ Y, int ldy, int accum,
+                                                 int64_t xrow0) {
+  const int lane = threadIdx.x & 31, cc = lane % BQ;
+  const bool on = cc < bq;
+  const int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (i >= n) return;
+  const int64_t beg = __ldg(rowptr + i), end = __ldg(rowptr + i + 1);
+  if (accum && end == beg) return;
+  double a[VEC];
+  row_product<kSpmmUnroll, BQ, VEC>(beg, end, col, val, X, ldx / VEC, cc, on, a);
+  if (!on || lane >= BQ) return;
+  double* y = Y + i * ldy + cc * VEC;
+  const double* xi = X + (xrow0 + i) * ldx + cc * VEC;
+  const double d = diag[i];
+  double o[VEC];
 #pragma unroll
-      for (int u = 0; u < U; u += 4) {
-        const int4 jj = __ldg(reinterpret_cast<const int4*>(col + e + u));
-        j[u] = jj.x; j[u + 1] = jj.y; j[u + 2] = jj.z; j[u + 3] = jj.w;
-        if constexpr (sizeof(VT) == 8) {
-          const double2 va = __ldg(reinterpret_cast<const double2*>(val + e + u));
-          const double2 vb = __ldg(reinterpret_cast<const double2*>(val + e + u + 2));
-          v[u] = va.x; v[u + 1] = va.y; v[u + 2] = vb.x; v[u + 3] = vb.y;
-        } else {
-          const float4 vf = __ldg(reinterpret_cast<const float4*>(val + e + u));
-          v[u] = vf.x; v[u + 1] = vf.y; v[u + 2] = vf.z; v[u + 3] = vf.w;
-        }
-      }
-      double2 x[U];
+  for (int c = 0; c < VEC; ++c) o[c] = accum ? y[c] + a[c] : fma(d, xi[c], a[c]);
 #pragma unroll
-      for (int u = 0; u < U; ++u) x[u] = gx(j[u]);
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        ax = fma(v[u], x[u].x, ax);
-        ay = fma(v[u], x[u].y, ay);
-      }
-    }
-#pragma unroll 4
-    for (; e < end; ++e) {
-      const double v = (double)__ldg(val + e);
-      const double2 x = gx(__ldg(col + e));
-      ax = fma(v, x.x, ax);
-      ay = fma(v, x.y, ay);
-    }
-    double2* y = reinterpret_cast<double2*>(Y) + i * ldy2 + cc;
-    if (accum) {
-      const double2 o = *y;
-      *y = make_double2(o.x + ax, o.y + ay);
-    } else {
-      const double d = diag[i];
-      const double2 xi = X2[(xrow0 + i) * ldx2 + cc];
-      *y = make_double2(fma(d, xi.x, ax), fma(d, xi.y, ay));
-    }
-  }
+  for (int c = 0; c < VEC; ++c) y[c] = o[c];
 }
 
 // Mixed-precision form: the gathered vector block is FP32 (each lane owns four adjacent columns,
-// one 16-byte float4 gather), the matrix values FP32, the accumulation FP64, and the diagonal term
+// one 16-byte gather), the matrix values FP32, the accumulation FP64, and the diagonal term
 // multiplies the FP64 block Xd (row i of the rows held, stride ldd).  A 16-column FP32 block row
-// is 64 bytes, half the gathered bytes of the FP64 form.  Register budget as for k_spmm_pairs.
+// is 64 bytes, half the gathered bytes of the FP64 form.  Measured (16 columns, four rows per warp
+// -> one): 120,011 rows 0.391 -> 0.314 ms, 60,011 rows of the 48-mode basis 0.141 -> 0.053 ms.
 template <int BQ>
 __global__ void __launch_bounds__(256, 4) k_spmm_f32x(int64_t n, const int64_t* __restrict__ rowptr,
                                                    const int32_t* __restrict__ col,
@@ -243,55 +135,26 @@ __global__ void __launch_bounds__(256, 4) k_spmm_f32x(int64_t n, const int64_t* 
                                                    const float* __restrict__ X, int ldx, int bq,
                                                    const double* __restrict__ Xd, int ldd,
                                                    double* __restrict__ Y, int ldy) {
-  constexpr int G = 32 / BQ, U = 16;
-  const int lane = threadIdx.x & 31;
-  const int grp = lane / BQ, cc = lane % BQ;
-  const bool active = cc < bq;
-  const float4* __restrict__ X4 = reinterpret_cast<const float4*>(X);
-  const int ldx4 = ldx >> 2;
-  const int64_t stride = (int64_t)gridDim.x * (blockDim.x >> 5) * G;
-  for (int64_t i = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * G + grp;
-       i < n; i += stride) {
-    if (!active) continue;
-    const int64_t beg = __ldg(rowptr + i), end = __ldg(rowptr + i + 1);
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-    auto acc = [&](double v, float4 x) {
-      a0 = fma(v, (double)x.x, a0);
-      a1 = fma(v, (double)x.y, a1);
-      a2 = fma(v, (double)x.z, a2);
-      a3 = fma(v, (double)x.w, a3);
-    };
-    auto gx = [&](int j) { return __ldg(X4 + (int64_t)j * ldx4 + cc); };
-    int64_t e = beg;
-    for (; e < end && (e & 3); ++e) acc((double)__ldg(val + e), gx(__ldg(col + e)));
-    for (; e + U <= end; e += U) {
-      int j[U];
-      float v[U];
-#pragma unroll
-      for (int u = 0; u < U; u += 4) {
-        const int4 jj = __ldg(reinterpret_cast<const int4*>(col + e + u));
-        j[u] = jj.x; j[u + 1] = jj.y; j[u + 2] = jj.z; j[u + 3] = jj.w;
-        const float4 vf = __ldg(reinterpret_cast<const float4*>(val + e + u));
-        v[u] = vf.x; v[u + 1] = vf.y; v[u + 2] = vf.z; v[u + 3] = vf.w;
-      }
-      float4 x[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) x[u] = gx(j[u]);
-#pragma unroll
-      for (int u = 0; u < U; ++u) acc((double)v[u], x[u]);
-    }
-#pragma unroll 4
-    for (; e < end; ++e) acc((double)__ldg(val + e), gx(__ldg(col + e)));
+  const int lane = threadIdx.x & 31, cc = lane % BQ;
+  const bool on = cc < bq;
+  const int64_t stride = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += stride) {
+    double a[4];
+    row_product<kSpmmUnrollF, BQ, 4>(__ldg(rowptr + i), __ldg(rowptr + i + 1), col, val, X,
+                                     ldx / 4, cc, on, a);
+    if (!on || lane >= BQ) continue;
     const double d = diag[i];
     const double* xd = Xd + i * ldd + 4 * cc;
     double* y = Y + i * ldy + 4 * cc;
-    y[0] = fma(d, xd[0], a0);
-    y[1] = fma(d, xd[1], a1);
-    y[2] = fma(d, xd[2], a2);
-    y[3] = fma(d, xd[3], a3);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) y[c] = fma(d, xd[c], a[c]);
   }
 }
 
+// Lanes per row group and columns per lane by the block's width: pairs of columns (16-byte gathers)
+// when the width, the strides and the addresses allow, else single columns; the widest launch covers
+// 32 columns.  Narrow blocks spread a row's entries over the lanes that columns leave free (one
+// column, 120,011 rows: 0.546 -> 0.177 ms; two 0.350 -> 0.208; four 0.339 -> 0.230).
 template <typename VT>
 void spmm_rows_launch(int64_t n, const int64_t* rowptr, const int32_t* col, const VT* val,
                       const double* diag, const double* X, int ldx, int b, double* Y, int ldy,
@@ -299,32 +162,27 @@ void spmm_rows_launch(int64_t n, const int64_t* rowptr, const int32_t* col, cons
   const bool pairs = (b % 2 == 0) && (ldx % 2 == 0) && (ldy % 2 == 0) &&
                      (reinterpret_cast<uintptr_t>(X) % 16 == 0) &&
                      (reinterpret_cast<uintptr_t>(Y) % 16 == 0);
-  if (pairs) {
-    const int BQ = b <= 8 ? 4 : (b <= 16 ? 8 : 16);  // lanes per row; columns per launch 2 BQ
-    const int gr = grid_for(n * BQ, 256, 148 * 16);
-    for (int c0 = 0; c0 < b; c0 += 2 * BQ) {
-      const int bq = std::min(BQ, (b - c0) / 2);
-      note_launch();
-      if (BQ == 16)
-        k_spmm_pairs<16, VT><<<gr, 256, 0, s>>>(n, rowptr, col, val, diag, X + c0, ldx, bq, Y + c0, ldy, accum, xrow0);
-      else if (BQ == 8)
-        k_spmm_pairs<8, VT><<<gr, 256, 0, s>>>(n, rowptr, col, val, diag, X + c0, ldx, bq, Y + c0, ldy, accum, xrow0);
-      else
-        k_spmm_pairs<4, VT><<<gr, 256, 0, s>>>(n, rowptr, col, val, diag, X + c0, ldx, bq, Y + c0, ldy, accum, xrow0);
-    }
-    return;
-  }
-  const int BP = b <= 8 ? 8 : (b <= 16 ? 16 : 32);
-  const int gr = grid_for(n * BP, 256, 148 * 16);
-  for (int c0 = 0; c0 < b; c0 += BP) {
-    const int bp = std::min(BP, b - c0);
+  const int64_t gr = (n + 7) / 8;
+  for (int c0 = 0; c0 < b; c0 += 32) {
+    const int w = std::min(32, b - c0), q = pairs ? w / 2 : w;
     note_launch();
-    if (BP == 32)
-      k_spmm_rows<32, VT><<<gr, 256, 0, s>>>(n, rowptr, col, val, diag, X + c0, ldx, bp, Y + c0, ldy, accum, xrow0);
-    else if (BP == 16)
-      k_spmm_rows<16, VT><<<gr, 256, 0, s>>>(n, rowptr, col, val, diag, X + c0, ldx, bp, Y + c0, ldy, accum, xrow0);
-    else
-      k_spmm_rows<8, VT><<<gr, 256, 0, s>>>(n, rowptr, col, val, diag, X + c0, ldx, bp, Y + c0, ldy, accum, xrow0);
+#define VHCI_SPMM(BQ, VEC)                                                                        \
+  k_spmm<BQ, VEC, VT><<<(unsigned)gr, 256, 0, s>>>(n, rowptr, col, val, diag, X + c0, ldx, q,       \
+                                                   Y + c0, ldy, accum, xrow0)
+    if (pairs) {
+      if (q == 1) VHCI_SPMM(1, 2);
+      else if (q == 2) VHCI_SPMM(2, 2);
+      else if (q <= 4) VHCI_SPMM(4, 2);
+      else if (q <= 8) VHCI_SPMM(8, 2);
+      else VHCI_SPMM(16, 2);
+    } else {
+      if (q == 1) VHCI_SPMM(1, 1);
+      else if (q <= 4) VHCI_SPMM(4, 1);
+      else if (q <= 8) VHCI_SPMM(8, 1);
+      else if (q <= 16) VHCI_SPMM(16, 1);
+      else VHCI_SPMM(32, 1);
+    }
+#undef VHCI_SPMM
   }
 }
 
@@ -493,7 +351,7 @@ bool spmm_f32x(int64_t n, const int64_t* rowptr, const int32_t* col, const float
   if (n <= 0 || b <= 0) return true;
   if (b % 4 || ldx % 4 || reinterpret_cast<uintptr_t>(X) % 16) return false;
   const int BQ = b <= 16 ? 4 : 8;  // lanes per row; 4 BQ columns per launch
-  const int gr = grid_for(n * BQ, 256, 148 * 16);
+  const int gr = grid_for(n * 32, 256, 148 * 16);
   for (int c0 = 0; c0 < b; c0 += 4 * BQ) {
     const int bq = std::min(BQ, (b - c0) / 4);
     note_launch();

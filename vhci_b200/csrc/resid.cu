@@ -1,82 +1,114 @@
 // Residual norms of caller-supplied eigenpairs with the context's Hamiltonian:
 // rnorm[j] = || H x_j - theta_j x_j ||, the quantity the reference's eigensolver tests against its
-// tolerance (Ham.cpp:363).  One fused pass: row groups form (H x)_i for a panel of up to 32 columns
-// (the SpMM of k_ham.cu), subtract theta x_i, square, and add into per-block partial sums kept in
-// scratch memory; a second kernel sums the partials in a fixed order.
+// tolerance (Ham.cpp:363).  One fused pass: each warp forms (H x)_i for a panel of up to 32 columns
+// (the row product of the SpMM), subtracts theta x_i, squares, and adds into per-block partial sums
+// kept in scratch memory; a second kernel sums the partials in a fixed order.
 #include <algorithm>
 #include <mutex>
 #include <vector>
 
 #include "internal.h"
+#include "rowprod.cuh"
 
 namespace vhci {
 
 namespace {
 
-constexpr int kResidThreads = 256;
+// Two blocks of 20 warps per SM (51 registers, the budget of k_spmm): the scratch holds one row of
+// partial sums per block, so the blocks are few and wide.
+constexpr int kResidThreads = 640, kResidWarps = kResidThreads / 32;
 constexpr int kResidBlocks = 148 * 2;  // partial-sum rows (one per block)
+constexpr int kResidUnroll = 8;
 
-template <int BP, typename VT>
-__global__ void __launch_bounds__(kResidThreads) k_resid_fused(
+// One warp per row forms (H x)_i for up to 32 columns (rowprod.cuh) and keeps the running sums of
+// the squared residuals; bound by the gathers from L2 as the product is.  Measured against rows
+// shared by 8-byte gathers four at a time: 150,001 rows, 51M entries, 200 vectors 27.1 -> 7.9
+// ms; 3,001 rows, 10 vectors 93 -> 29 us a call (both kernels).
+template <int BQ, int VEC, typename VT>
+__global__ void __launch_bounds__(kResidThreads, 2) k_resid_fused(
     int64_t n, const int64_t* __restrict__ rowptr, const int32_t* __restrict__ col,
     const VT* __restrict__ val, const double* __restrict__ diag, const double* __restrict__ X,
-    int ldx, int bp, const double* __restrict__ theta, double* __restrict__ part, int ldp) {
-  constexpr int G = 32 / BP;
-  __shared__ double red[kResidThreads / BP][BP];
-  const int lane = threadIdx.x & 31;
-  const int grp = lane / BP, cc = lane % BP;
-  const bool active = cc < bp;
-  const double th = active ? theta[cc] : 0.0;
-  double s = 0.0;
-  const int64_t stride = (int64_t)gridDim.x * (blockDim.x >> 5) * G;
-  for (int64_t i = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * G + grp;
-       i < n; i += stride) {
-    if (!active) continue;
-    const int64_t beg = __ldg(rowptr + i), end = __ldg(rowptr + i + 1);
-    double acc = 0.0;
-#pragma unroll 4
-    for (int64_t e = beg; e < end; ++e) {
-      const int j = __ldg(col + e);
-      const double v = (double)__ldg(val + e);
-      acc = fma(v, __ldg(X + (int64_t)j * ldx + cc), acc);
+    int ldx, int bq, const double* __restrict__ theta, double* __restrict__ part, int ldp) {
+  __shared__ double red[kResidWarps][BQ * VEC];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, cc = lane % BQ;
+  const bool on = cc < bq;
+  double th[VEC], s[VEC];
+#pragma unroll
+  for (int c = 0; c < VEC; ++c) {
+    th[c] = on ? theta[cc * VEC + c] : 0.0;
+    s[c] = 0.0;
+  }
+  for (int64_t i = (int64_t)blockIdx.x * kResidWarps + wid; i < n;
+       i += (int64_t)gridDim.x * kResidWarps) {
+    double a[VEC];
+    row_product<kResidUnroll, BQ, VEC>(__ldg(rowptr + i), __ldg(rowptr + i + 1), col, val, X,
+                                       ldx / VEC, cc, on, a);
+    if (on && lane < BQ) {
+      const double d = diag[i];
+#pragma unroll
+      for (int c = 0; c < VEC; ++c) {
+        const double xi = X[i * ldx + cc * VEC + c];
+        const double r = fma(d, xi, a[c]) - th[c] * xi;
+        s[c] = fma(r, r, s[c]);
+      }
     }
-    const double xi = X[i * ldx + cc];
-    const double r = fma(diag[i], xi, acc) - th * xi;
-    s = fma(r, r, s);
   }
   // block reduction per column, in a fixed order
-  red[threadIdx.x / BP][cc] = active ? s : 0.0;
+  if (lane < BQ) {
+#pragma unroll
+    for (int c = 0; c < VEC; ++c) red[wid][cc * VEC + c] = s[c];
+  }
   __syncthreads();
-  if (threadIdx.x < BP) {
+  if (threadIdx.x < VEC * bq) {
     double t = 0.0;
-    for (int q = 0; q < kResidThreads / BP; ++q) t += red[q][threadIdx.x];
-    if (threadIdx.x < bp) part[(int64_t)blockIdx.x * ldp + threadIdx.x] = t;
+    for (int q = 0; q < kResidWarps; ++q) t += red[q][threadIdx.x];
+    part[(int64_t)blockIdx.x * ldp + threadIdx.x] = t;
   }
 }
 
-__global__ void k_resid_finish(const double* __restrict__ part, int nblk, int ldp, int k,
-                               double* __restrict__ rnorm) {
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < k; c += gridDim.x * blockDim.x) {
-    double t = 0.0;
-    for (int q = 0; q < nblk; ++q) t += part[(int64_t)q * ldp + c];
-    rnorm[c] = sqrt(t);
-  }
+// One warp per column adds the blocks' partial sums (lane l those of blocks l, l + 32, ...) and the
+// lanes' sums in a fixed tree (one thread per column took 34 us of a small call).
+__global__ void __launch_bounds__(256) k_resid_finish(const double* __restrict__ part, int nblk,
+                                                      int ldp, int k, double* __restrict__ rnorm) {
+  const int lane = threadIdx.x & 31;
+  const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (c >= k) return;
+  double t = 0.0;
+#pragma unroll 4
+  for (int q = lane; q < nblk; q += 32) t += part[(int64_t)q * ldp + c];
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) t += __shfl_xor_sync(0xffffffffu, t, d);
+  if (lane == 0) rnorm[c] = sqrt(t);
 }
 
+// Column pairs (16-byte gathers) when the vectors' width and address allow, else single columns.
 template <typename VT>
 void resid_launch(int64_t n, const int64_t* rowptr, const int32_t* col, const VT* val,
                   const double* diag, const double* X, int ldx, int k, const double* theta,
                   double* part, double* rnorm, cudaStream_t s) {
+  const bool pairs = k % 2 == 0 && ldx % 2 == 0 && reinterpret_cast<uintptr_t>(X) % 16 == 0;
   for (int c0 = 0; c0 < k; c0 += 32) {
-    const int bp = std::min(32, k - c0);
-    const int BP = bp <= 8 ? 8 : (bp <= 16 ? 16 : 32);
-    double* pp = part + c0;
-    if (BP == 8) { note_launch(); k_resid_fused<8, VT><<<kResidBlocks, kResidThreads, 0, s>>>(n, rowptr, col, val, diag, X + c0, ldx, bp, theta + c0, pp, k); }
-    else if (BP == 16) { note_launch(); k_resid_fused<16, VT><<<kResidBlocks, kResidThreads, 0, s>>>(n, rowptr, col, val, diag, X + c0, ldx, bp, theta + c0, pp, k); }
-    else { note_launch(); k_resid_fused<32, VT><<<kResidBlocks, kResidThreads, 0, s>>>(n, rowptr, col, val, diag, X + c0, ldx, bp, theta + c0, pp, k); }
+    const int w = std::min(32, k - c0), q = pairs ? w / 2 : w;
+    note_launch();
+#define VHCI_RESID(BQ, VEC)                                                                       \
+  k_resid_fused<BQ, VEC, VT><<<kResidBlocks, kResidThreads, 0, s>>>(                                \
+      n, rowptr, col, val, diag, X + c0, ldx, q, theta + c0, part + c0, k)
+    if (pairs) {
+      if (q <= 2) VHCI_RESID(2, 2);
+      else if (q <= 4) VHCI_RESID(4, 2);
+      else if (q <= 8) VHCI_RESID(8, 2);
+      else VHCI_RESID(16, 2);
+    } else {
+      if (q <= 1) VHCI_RESID(1, 1);
+      else if (q <= 4) VHCI_RESID(4, 1);
+      else if (q <= 8) VHCI_RESID(8, 1);
+      else if (q <= 16) VHCI_RESID(16, 1);
+      else VHCI_RESID(32, 1);
+    }
+#undef VHCI_RESID
   }
   note_launch();
-  k_resid_finish<<<(k + 127) / 128, 128, 0, s>>>(part, kResidBlocks, k, k, rnorm);
+  k_resid_finish<<<(k + 7) / 8, 256, 0, s>>>(part, kResidBlocks, k, k, rnorm);
 }
 
 }  // namespace
