@@ -27,21 +27,26 @@ int blas_fail(vhci_ctx* c, int st, const char* where) {
 
 HashView basis_view(vhci_ctx* c) { return HashView{c->hslots.p, c->hmask, c->keys.p}; }
 
+static void set_groups(ConnDev& d, const DevGroups& g) {
+  d.groups = g.groups.p;
+  d.wdelta = g.wdelta.p;
+  d.hdelta = g.hdelta.p;
+  d.ngroups = g.ngroups;
+  d.lkey = g.lkey.p;
+  d.lseg = g.lseg.p;
+  d.lmask = g.lmask;
+  d.maxl = g.maxl;
+}
+
 ConnDev conn_view(vhci_ctx* c) {
   ConnDev d;
-  d.groups = c->groups.p;
-  d.wdelta = c->wdelta.p;
-  d.ngroups = (int64_t)c->conn.groups.size();
+  set_groups(d, c->conn_dev);
   d.terms = c->terms.p;
   d.dterms = c->dterms.p;
   d.ndterms = (int)c->conn.diag_terms.size();
   d.T = c->T.p;
   d.freq = c->freq.p;
   d.nm = c->M.nm;
-  d.lkey = c->lkey.p;
-  d.lseg = c->lseg.p;
-  d.lmask = c->lmask;
-  d.maxl = c->maxl;
   return d;
 }
 
@@ -93,6 +98,7 @@ struct HandleSet {
   cudaStream_t st;
   cublasHandle_t blas;
   cusolverDnHandle_t sol;
+  double dev_bytes;  // the device's memory
 };
 std::mutex g_handle_mu;
 std::vector<HandleSet> g_handle_pool;
@@ -116,6 +122,7 @@ static int acquire_handles(vhci_ctx* c) {
         c->st = g_handle_pool[i].st;
         c->blas = g_handle_pool[i].blas;
         c->sol = g_handle_pool[i].sol;
+        c->dev_bytes = g_handle_pool[i].dev_bytes;
         g_handle_pool.erase(g_handle_pool.begin() + i);
         return VHCI_OK;
       }
@@ -125,6 +132,9 @@ static int acquire_handles(vhci_ctx* c) {
   VBL(cublasSetStream(c->blas, c->st));
   VBL(cusolverDnCreate(&c->sol));
   VBL(cusolverDnSetStream(c->sol, c->st));
+  size_t freeb = 0, totb = 0;
+  VCK(cudaMemGetInfo(&freeb, &totb));
+  c->dev_bytes = (double)totb;
   return VHCI_OK;
 }
 
@@ -137,7 +147,7 @@ static void release_handles(vhci_ctx* c) {
   }
   cudaStreamSynchronize(c->st);
   std::lock_guard<std::mutex> lk(g_handle_mu);
-  g_handle_pool.push_back(HandleSet{c->o.device, c->o.stream_priority, c->st, c->blas, c->sol});
+  g_handle_pool.push_back(HandleSet{c->o.device, c->o.stream_priority, c->st, c->blas, c->sol, c->dev_bytes});
 }
 
 // Layout-dependent tables (packed key deltas, ladder factors) and the layout-free ones.
@@ -147,6 +157,7 @@ static int upload_groups(vhci_ctx* c, const ConnTables& t, DevGroups& dg) {
   const KeyLayout& L = c->L;
   std::vector<GroupDev> g(t.groups.size());
   std::vector<int64_t> wd(t.groups.size() * L.W, 0);
+  std::vector<uint64_t> hd(t.groups.size(), 0);
   for (size_t u = 0; u < g.size(); ++u) {
     const Group& s = t.groups[u];
     GroupDev d{};
@@ -160,9 +171,11 @@ static int upload_groups(vhci_ctx* c, const ConnTables& t, DevGroups& dg) {
       wd[u * L.W + w] += (int64_t)((uint64_t)(int64_t)s.delta[k] << ((s.mode[k] % L.mpw) * L.bits));
     }
     g[u] = d;
+    for (int w = 0; w < L.W; ++w) hd[u] += hash_word((uint64_t)wd[u * L.W + w], w);
   }
   VTRY(upload(c, dg.groups, g));
   VTRY(upload(c, dg.wdelta, wd));
+  VTRY(upload(c, dg.hdelta, hd));
   const size_t nseg = t.seg_key.size();
   size_t P = 64;
   while (P < 2 * nseg) P <<= 1;
@@ -187,22 +200,7 @@ static int upload_groups(vhci_ctx* c, const ConnTables& t, DevGroups& dg) {
 int upload_tables(vhci_ctx* c) {
   const KeyLayout& L = c->L;
   if (c->gate_built) VTRY(upload_groups(c, c->gate, c->gate_dev));  // re-packed for the layout
-  std::vector<GroupDev> g(c->conn.groups.size());
-  std::vector<int64_t> wd(c->conn.groups.size() * L.W, 0);
-  for (size_t u = 0; u < g.size(); ++u) {
-    const Group& s = c->conn.groups[u];
-    GroupDev d{};
-    d.tb = s.term_begin;
-    d.te = s.term_end;
-    d.nchg = (uint8_t)s.nchg;
-    for (int k = 0; k < s.nchg; ++k) {
-      d.mode[k] = (uint8_t)s.mode[k];
-      d.delta[k] = (int8_t)s.delta[k];
-      const int w = s.mode[k] / L.mpw;
-      wd[u * L.W + w] += (int64_t)((uint64_t)(int64_t)s.delta[k] << ((s.mode[k] % L.mpw) * L.bits));
-    }
-    g[u] = d;
-  }
+  VTRY(upload_groups(c, c->conn, c->conn_dev));
   auto conv = [](const std::vector<Term>& in) {
     std::vector<TermDev> out(in.size());
     for (size_t i = 0; i < in.size(); ++i) {
@@ -232,29 +230,6 @@ int upload_tables(vhci_ctx* c) {
     }
     hb[i] = d;
     habs[i] = c->hbe[i].absfc;
-  }
-  VTRY(upload(c, c->groups, g));
-  VTRY(upload(c, c->wdelta, wd));
-  // lowered-mode segment index: open addressing on the segment keys, load <= 1/2
-  {
-    const ConnTables& t = c->conn;
-    const size_t nseg = t.seg_key.size();
-    size_t P = 64;
-    while (P < 2 * nseg) P <<= 1;
-    std::vector<uint64_t> lk(P, 0);
-    std::vector<int32_t> ls(2 * P, 0);
-    for (size_t q = 0; q < nseg; ++q) {
-      size_t h = mix64(t.seg_key[q]) & (P - 1);
-      while (lk[h] != 0) h = (h + 1) & (P - 1);
-      lk[h] = t.seg_key[q];
-      ls[2 * h] = t.seg_begin[q];
-      ls[2 * h + 1] = t.seg_begin[q + 1] - t.seg_begin[q];
-    }
-    VTRY(upload(c, c->lkey, lk));
-    VTRY(upload(c, c->lseg, ls));
-    c->lmask = (uint32_t)(P - 1);
-    // the index covers up to 126 modes and 6 lowered modes (the key packs 7 bits per mode)
-    c->maxl = (c->M.nm <= 126 && t.max_lowered <= 6 && nseg > 0) ? t.max_lowered : -1;
   }
   VTRY(upload(c, c->terms, conv(c->conn.terms)));
   VTRY(upload(c, c->dterms, conv(c->conn.diag_terms)));
@@ -494,18 +469,12 @@ int structural_count(vhci_ctx* c, int64_t* out) {
     return fail(c, VHCI_E_LIMIT, "the pair gates admit more than " +
                                      std::to_string(kMaxGatePatterns) + " change patterns");
   ConnDev d = conn_view(c);
-  d.groups = c->gate_dev.groups.p;
-  d.wdelta = c->gate_dev.wdelta.p;
-  d.ngroups = c->gate_dev.ngroups;
-  d.lkey = c->gate_dev.lkey.p;
-  d.lseg = c->gate_dev.lseg.p;
-  d.lmask = c->gate_dev.lmask;
-  d.maxl = c->gate_dev.maxl;
+  set_groups(d, c->gate_dev);
   DBuf<int64_t> sum;
   VCK(c->rowcnt.reserve(n, c->st));
   VCK(sum.reserve(n + 1, c->st));
   VCK(c->scan_tmp.reserve(std::max<int64_t>(scan_tmp_elems(n), 1), c->st));
-  hbuild_count(c->keys.p, 0, n, c->L, basis_view(c), d, c->rowcnt.p, c->st);
+  hbuild_count(c->keys.p, 0, 1, n, c->L, basis_view(c), d, c->rowcnt.p, StageView{}, c->st);
   exclusive_scan_i32(c->rowcnt.p, sum.p, n, c->scan_tmp.p, c->st);
   int64_t pairs = 0;
   VCK(d2h(c, &pairs, sum.p + n, sizeof(int64_t)));
@@ -552,6 +521,74 @@ bool dense_path(int64_t n, int k) {
   return n <= 2000 || n <= 3 * kk + 64;
 }
 
+// A sample of at least 256 and about one row in 64 counts the connections (the walks that the sample
+// costs are 1.5 % of the one it saves); 25 % and two batches per row of slack cover its spread and
+// the part-filled last batches.  Small row sets skip the sample for 8 batches (256 connections) a
+// row.  The room is limited to a quarter of the device, and a failed allocation is no error.
+int stage_reserve(vhci_ctx* c, Stage& st, HashView table, int64_t row0, int64_t n) {
+  cudaStream_t s = c->st;
+  st.view = StageView{};
+  if (n <= 0 || n >= 0xFFFFFFFFll) return VHCI_OK;
+  double batches = 8.0 * (double)n;
+  VCK(st.cursor.reserve(1, s));
+  if (n > 4096) {
+    const int64_t stride = std::max<int64_t>(1, std::min<int64_t>(64, n / 256)), ns = n / stride;
+    VCK(c->rowcnt.reserve(n, s));
+    VCK(c->scan_tmp.reserve(std::max<int64_t>(scan_tmp_elems(n), 1), s));
+    DBuf<int64_t> sum;
+    VCK(sum.reserve(ns + 1, s));
+    hbuild_count(c->keys.p, row0, stride, ns, c->L, table, conn_view(c), c->rowcnt.p, StageView{}, s);
+    exclusive_scan_i32(c->rowcnt.p, sum.p, ns, c->scan_tmp.p, s);
+    int64_t found = 0;
+    VCK(d2h(c, &found, sum.p + ns, sizeof(int64_t)));
+    VCK(cudaStreamSynchronize(s));
+    sum.release(s);
+    batches = 1.25 * (double)found / (double)ns * (double)n / 32.0 + 2.0 * (double)n;
+  }
+  if (batches * 264.0 > 0.25 * (double)c->dev_bytes) return VHCI_OK;
+  const int64_t cap = (int64_t)batches;
+  if (st.batch.reserve(cap, s) != cudaSuccess || st.pair.reserve(32 * (size_t)cap, s) != cudaSuccess) {
+    cudaGetLastError();
+    st.batch.release(s);
+    st.pair.release(s);
+    return VHCI_OK;
+  }
+  VCK(cudaMemsetAsync(st.cursor.p, 0, sizeof(unsigned long long), s));
+  st.view = StageView{st.batch.p, st.pair.p, st.cursor.p, cap};
+  return VHCI_OK;
+}
+
+// Counts rows row0 .. row0 + n - 1 into rowptr (scanned) with their connections kept where there is
+// room; *nnz: all entries, *nbatch: the batches kept, 0 when some were lost (st is then empty).
+static int count_rows(vhci_ctx* c, Stage& st, int64_t row0, int64_t n, int32_t* cnt, int64_t* rowptr,
+                      int64_t* nnz, int64_t* nbatch) {
+  cudaStream_t s = c->st;
+  VTRY(stage_reserve(c, st, basis_view(c), row0, n));
+  hbuild_count(c->keys.p, row0, 1, n, c->L, basis_view(c), conn_view(c), cnt, st.view, s);
+  exclusive_scan_i32(cnt, rowptr, n, c->scan_tmp.p, s);
+  unsigned long long nb = 0;
+  VCK(d2h(c, nnz, rowptr + n, sizeof(int64_t)));
+  if (st.view.cap > 0) VCK(d2h(c, &nb, st.cursor.p, sizeof(nb)));
+  VCK(cudaStreamSynchronize(s));
+  if ((int64_t)nb > st.view.cap) {
+    st.release(s);
+    nb = 0;
+  }
+  *nbatch = (int64_t)nb;
+  return VHCI_OK;
+}
+
+// The rows' entries and diagonal, from the kept batches or by a second walk.
+static void fill_rows(vhci_ctx* c, Stage& st, int64_t nbatch, int64_t row0, int64_t n,
+                      const int64_t* rowptr, int32_t* col, double* val, float* valf, double* diag) {
+  if (nbatch > 0)
+    hbuild_fill_staged(c->keys.p, row0, c->L, conn_view(c), st.view, nbatch, rowptr, col, val, valf, c->st);
+  else
+    hbuild_fill(c->keys.p, row0, n, c->L, basis_view(c), conn_view(c), rowptr, col, val, valf, c->st);
+  diag_energies(c->keys.p, row0, n, c->L, conn_view(c), diag, c->st);
+  st.release(c->st);
+}
+
 // Incremental build: rows of the states appended since the stored matrix was built (states
 // h_prefix .. n - 1), their entries in old columns transposed into the tails of the old rows
 // (H is symmetric to the bit: each element's ladder factors come from the lower state), merged
@@ -572,20 +609,18 @@ static int build_h_incremental(vhci_ctx* c) {
   DBuf<float> tvalf, valf_all;
   DBuf<uint64_t> keys, alt;
   DBuf<unsigned long long> kc;
+  Stage stage;
   auto release_all = [&] {
     cnt_new.release(s); tcol.release(s); add.release(s); erow.release(s); len.release(s);
     col_all.release(s); rp_new.release(s); xoff.release(s); rp_all.release(s); hist.release(s);
     tval.release(s); tdiag.release(s); val_all.release(s); diag_all.release(s); tvalf.release(s);
-    valf_all.release(s); keys.release(s); alt.release(s); kc.release(s);
+    valf_all.release(s); keys.release(s); alt.release(s); kc.release(s); stage.release(s);
   };
   VCK(cnt_new.reserve(nn, s));
   VCK(rp_new.reserve(nn + 1, s));
   VCK(c->scan_tmp.reserve(std::max<int64_t>(scan_tmp_elems(n), 1), s));
-  hbuild_count(c->keys.p, n_old, nn, c->L, basis_view(c), conn_view(c), cnt_new.p, s);
-  exclusive_scan_i32(cnt_new.p, rp_new.p, nn, c->scan_tmp.p, s);
-  int64_t nnz_new = 0;
-  VCK(d2h(c, &nnz_new, rp_new.p + nn, sizeof(int64_t)));
-  VCK(cudaStreamSynchronize(s));
+  int64_t nnz_new = 0, nbatch = 0;
+  VTRY(count_rows(c, stage, n_old, nn, cnt_new.p, rp_new.p, &nnz_new, &nbatch));
   // working set: the new rows, their transposed keys (sorted through a second buffer), the entry
   // rows, and the merged matrix (at most nnz_old + 2 nnz_new entries) beside the stored one
   const double nnz_all_max = (double)c->nnz + 2.0 * (double)nnz_new;
@@ -593,8 +628,15 @@ static int build_h_incremental(vhci_ctx* c) {
                       (double)n * 40.0 + 8.0 * radix_hist_elems(nnz_new);
   const double eig = lanczos_min_bytes(c, c->M.nstate);
   const double old_bytes = (double)c->nnz * (4.0 + vb) + 16.0 * (double)n_old;
-  const double avail = device_available(c);
-  if (nnz_new >= 0xFFFFFFFFll || need > 0.9 * avail || nnz_all_max * (4.0 + vb) + eig > avail + old_bytes) {
+  // the kept connections give way when the matrix needs their room
+  double avail = device_available(c);
+  auto fits = [&] { return need <= 0.9 * avail && nnz_all_max * (4.0 + vb) + eig <= avail + old_bytes; };
+  if (nbatch > 0 && !fits()) {
+    avail += 264.0 * (double)stage.view.cap;
+    stage.release(s);
+    nbatch = 0;
+  }
+  if (nnz_new >= 0xFFFFFFFFll || !fits()) {
     release_all();
     return 1;
   }
@@ -602,8 +644,8 @@ static int build_h_incremental(vhci_ctx* c) {
   if (f) VCK(tvalf.reserve(std::max<int64_t>(nnz_new, 1), s));
   else VCK(tval.reserve(std::max<int64_t>(nnz_new, 1), s));
   VCK(tdiag.reserve(nn, s));
-  hbuild_fill(c->keys.p, n_old, nn, c->L, basis_view(c), conn_view(c), rp_new.p, tcol.p,
-              f ? nullptr : tval.p, f ? tvalf.p : nullptr, tdiag.p, s);
+  fill_rows(c, stage, nbatch, n_old, nn, rp_new.p, tcol.p, f ? nullptr : tval.p,
+            f ? tvalf.p : nullptr, tdiag.p);
   // transposed entries: per old column counts and (column, entry) keys, sorted
   VCK(add.reserve(n_old, s));
   VCK(cudaMemsetAsync(add.p, 0, n_old * sizeof(int32_t), s));
@@ -696,11 +738,9 @@ int build_h(vhci_ctx* c, bool all_rows) {
   VCK(c->rowcnt.reserve(std::max<int64_t>(nr, 1), c->st));
   VCK(c->rowptr.reserve(nr + 1, c->st));
   VCK(c->scan_tmp.reserve(std::max<int64_t>(scan_tmp_elems(nr), 1), c->st));
-  hbuild_count(c->keys.p, r0, nr, c->L, basis_view(c), conn_view(c), c->rowcnt.p, c->st);
-  exclusive_scan_i32(c->rowcnt.p, c->rowptr.p, nr, c->scan_tmp.p, c->st);
-  int64_t nnz = 0;
-  VCK(d2h(c, &nnz, c->rowptr.p + nr, sizeof(int64_t)));
-  VCK(cudaStreamSynchronize(c->st));
+  Stage stage;
+  int64_t nnz = 0, nbatch = 0;
+  VTRY(count_rows(c, stage, r0, nr, c->rowcnt.p, c->rowptr.p, &nnz, &nbatch));
   // the previous matrix's arrays are replaced, not grown in place: release them first so the old
   // and new matrix never coexist
   if ((int64_t)c->col.cap < nnz) c->col.release(c->st);
@@ -708,9 +748,15 @@ int build_h(vhci_ctx* c, bool all_rows) {
   if ((int64_t)c->valf.cap < nnz) c->valf.release(c->st);
   {  // admission: the matrix and the eigensolver's smallest working set must fit together
     const double hbytes = (double)nnz * (4.0 + (c->o.precision == 1 ? 4.0 : 8.0)) + 8.0 * nr;
-    const double avail = device_available(c) + 8.0 * (double)c->x_rows * c->ldx;
+    double avail = device_available(c) + 8.0 * (double)c->x_rows * c->ldx;
     const double eig = lanczos_min_bytes(c, c->M.nstate);
+    if (nbatch > 0 && hbytes + eig > avail) {  // the kept connections give way
+      avail += 264.0 * (double)stage.view.cap;
+      stage.release(c->st);
+      nbatch = 0;
+    }
     if (hbytes + eig > avail) {
+      stage.release(c->st);
       char msg[320];
       std::snprintf(msg, sizeof msg,
                     "Hamiltonian rows of %lld states and %lld off-diagonal entries need %.1f GB "
@@ -726,9 +772,8 @@ int build_h(vhci_ctx* c, bool all_rows) {
     VCK(c->val.reserve(std::max<int64_t>(nnz, 1), c->st));
   }
   VCK(c->diag.reserve(std::max<int64_t>(nr, 1), c->st));
-  hbuild_fill(c->keys.p, r0, nr, c->L, basis_view(c), conn_view(c), c->rowptr.p, c->col.p,
-              c->o.precision == 1 ? nullptr : c->val.p, c->o.precision == 1 ? c->valf.p : nullptr,
-              c->diag.p, c->st);
+  fill_rows(c, stage, nbatch, r0, nr, c->rowptr.p, c->col.p, c->o.precision == 1 ? nullptr : c->val.p,
+            c->o.precision == 1 ? c->valf.p : nullptr, c->diag.p);
   c->nnz = nnz;
   VTRY(build_panels(c));
   VCK(cudaEventRecord(c->ev_b, c->st));
@@ -839,7 +884,7 @@ vhci_status vhci_destroy(vhci_ctx* c) {
   if (c->st) {
     cudaStreamSynchronize(c->st);
     c->keys.release(c->st); c->hslots.release(c->st);
-    c->groups.release(c->st); c->wdelta.release(c->st); c->terms.release(c->st);
+    c->conn_dev.release(c->st); c->terms.release(c->st);
     c->dterms.release(c->st); c->T.release(c->st); c->freq.release(c->st);
     c->hbdev.release(c->st); c->hbabs.release(c->st); c->hbcumd.release(c->st);
     c->rowcnt.release(c->st); c->rowptr.release(c->st); c->col.release(c->st);
@@ -849,7 +894,6 @@ vhci_status vhci_destroy(vhci_ctx* c) {
     c->d64a.release(c->st); c->u64a.release(c->st); c->u64b.release(c->st);
     c->u8a.release(c->st); c->ull.release(c->st); c->solver_work.release(c->st);
     c->solver_info.release(c->st);
-    c->lkey.release(c->st); c->lseg.release(c->st);
     c->prow.release(c->st); c->pcol.release(c->st); c->pval.release(c->st);
     c->pvalf.release(c->st); c->gate_dev.release(c->st);
     cudaStreamSynchronize(c->st);

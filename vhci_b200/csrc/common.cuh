@@ -31,21 +31,22 @@ __host__ __device__ inline int key_word(int m, int mpw) { return m / mpw; }
 __host__ __device__ inline int key_shift(int m, int mpw, int bits) { return (m % mpw) * bits; }
 
 // Quanta of mode m from a key held in registers (W words); the word is picked without dynamic
-// register indexing.
+// register indexing.  mpw is a power of two (8 or 16): shifts and masks, no division (a division by
+// a run-time mpw per field took most of the instructions of the connection walk).
 template <int W>
 __device__ __forceinline__ int key_q(const uint64_t (&k)[W], int m, int mpw, int bits) {
-  const int w = m / mpw;
+  const int w = m >> (31 - __clz(mpw));
   uint64_t v = k[0];
 #pragma unroll
   for (int i = 1; i < W; ++i)
     if (w == i) v = k[i];
-  return (int)((v >> ((m % mpw) * bits)) & ((1u << bits) - 1u));
+  return (int)((v >> ((m & (mpw - 1)) * bits)) & ((1u << bits) - 1u));
 }
 
 template <int W>
 __device__ __forceinline__ void key_add(uint64_t (&k)[W], int m, int mpw, int bits, int d) {
-  const int w = m / mpw;
-  const uint64_t add = (uint64_t)((int64_t)d << ((m % mpw) * bits));
+  const int w = m >> (31 - __clz(mpw));
+  const uint64_t add = (uint64_t)((int64_t)d << ((m & (mpw - 1)) * bits));
 #pragma unroll
   for (int i = 0; i < W; ++i)
     if (w == i) k[i] += add;
@@ -61,12 +62,30 @@ __host__ __device__ __forceinline__ uint64_t mix64(uint64_t x) {
   return x;
 }
 
+// Key hash in two parts: a sum that is linear in the key words (mod 2^64), so the sum of a target
+// key k + delta is that of k plus a constant of delta (stored per connection group), and a
+// finaliser.
+constexpr int kMaxKeyWords = 8;
+__host__ __device__ __forceinline__ uint64_t hash_word(uint64_t k, int w) {
+  // odd multipliers, spaced by an odd constant
+  return k * (0x9E3779B97F4A7C15ull + 0xA24BAED4963EE406ull * (uint64_t)w);
+}
+__host__ __device__ __forceinline__ uint64_t hash_final(uint64_t x) {
+  x ^= x >> 32;
+  x *= 0xD6E8FEB86659FD93ull;
+  x ^= x >> 32;
+  return x;
+}
+template <int W>
+__device__ __forceinline__ uint64_t hash_lin(const uint64_t (&k)[W]) {
+  uint64_t h = 0;
+#pragma unroll
+  for (int i = 0; i < W; ++i) h += hash_word(k[i], i);
+  return h;
+}
 template <int W>
 __device__ __forceinline__ uint64_t key_hash(const uint64_t (&k)[W]) {
-  uint64_t h = mix64(k[0] ^ 0x9E3779B97F4A7C15ull);
-#pragma unroll
-  for (int i = 1; i < W; ++i) h = mix64(h ^ (k[i] + 0x632BE59BD9B4E019ull * (uint64_t)i));
-  return h;
+  return hash_final(hash_lin<W>(k));
 }
 
 template <int W>
@@ -85,19 +104,49 @@ __device__ __forceinline__ bool key_eq(const uint64_t* __restrict__ keys, int64_
   return eq;
 }
 
-// Read-only view of a unique-key hash: slot = (fingerprint << 32) | index into `keys`.
+// Read-only view of a unique-key hash: slot = (31-bit fingerprint << 32) | index into `keys`.
+// Linear probing from a home slot that is a multiple of four: a lookup reads the four slots of its
+// home as one 32-byte sector, and since nothing is ever removed they fill from the first on, so a
+// miss usually ends with that one read (an empty fourth slot).
 struct HashView {
   const uint64_t* __restrict__ slots;
   uint64_t mask;
   const uint64_t* __restrict__ keys;
 };
 
-// Returns the key's index or -1.  Linear probing; at load <= 1/2 a miss ends after ~2.5 slots.
+__device__ __forceinline__ uint64_t hash_home(uint64_t h, uint64_t mask) { return h & mask & ~3ull; }
+// never the fingerprint field of an empty slot
+__device__ __forceinline__ uint32_t hash_fp(uint64_t h) { return (uint32_t)(h >> 33); }
+
+// The four slots at s: index of the first whose fingerprint is fp (kNoIndex if none), and whether
+// the probe sequence goes on (no match and no empty slot).
+struct SlotHit {
+  uint32_t idx;
+  bool more;
+};
+__device__ __forceinline__ SlotHit match_slots(const ulonglong2& a, const ulonglong2& b, uint32_t fp) {
+  SlotHit r{kNoIndex, b.y != kEmptySlot};
+  if ((uint32_t)(b.y >> 32) == fp) r.idx = (uint32_t)b.y;
+  if ((uint32_t)(b.x >> 32) == fp) r.idx = (uint32_t)b.x;
+  if ((uint32_t)(a.y >> 32) == fp) r.idx = (uint32_t)a.y;
+  if ((uint32_t)(a.x >> 32) == fp) r.idx = (uint32_t)a.x;
+  r.more = r.more && r.idx == kNoIndex;
+  return r;
+}
+// One 32-byte load: as two 16-byte loads the L1 tag stage, which takes a scattered access lane by
+// lane, was the walk's limit.
+__device__ __forceinline__ void load_slots(const uint64_t* p, ulonglong2& a, ulonglong2& b) {
+  asm("ld.global.nc.v4.u64 {%0,%1,%2,%3}, [%4];"
+      : "=l"(a.x), "=l"(a.y), "=l"(b.x), "=l"(b.y)
+      : "l"(p));
+}
+
+// Returns the key's index or -1.
 template <int W>
 __device__ __forceinline__ int64_t hash_find(const HashView& t, const uint64_t (&k)[W],
                                              uint64_t h) {
-  uint64_t s = h & t.mask;
-  const uint32_t fp = (uint32_t)(h >> 32);
+  uint64_t s = hash_home(h, t.mask);
+  const uint32_t fp = hash_fp(h);
   for (uint64_t it = 0; it <= t.mask; ++it) {
     const uint64_t v = __ldg(t.slots + s);
     if (v == kEmptySlot) return -1;
@@ -115,8 +164,8 @@ template <int W>
 __device__ __forceinline__ void hash_insert_unique(uint64_t* slots, uint64_t mask,
                                                    const uint64_t* keys, const uint64_t (&k)[W],
                                                    uint64_t h, uint32_t idx, int* flags) {
-  uint64_t s = h & mask;
-  const uint64_t val = ((uint64_t)(uint32_t)(h >> 32) << 32) | idx;
+  uint64_t s = hash_home(h, mask);
+  const uint64_t val = ((uint64_t)hash_fp(h) << 32) | idx;
   for (uint64_t it = 0; it <= mask; ++it) {
     const uint64_t old = atomicCAS((unsigned long long*)(slots + s), kEmptySlot, val);
     if (old == kEmptySlot) return;

@@ -47,13 +47,14 @@ struct DBuf {
 struct DevGroups {
   DBuf<GroupDev> groups;
   DBuf<int64_t> wdelta;
+  DBuf<uint64_t> hdelta;
   DBuf<uint64_t> lkey;
   DBuf<int32_t> lseg;
   uint32_t lmask = 0;
   int maxl = -1;
   int64_t ngroups = 0;
   void release(cudaStream_t s) {
-    groups.release(s); wdelta.release(s); lkey.release(s); lseg.release(s);
+    groups.release(s); wdelta.release(s); hdelta.release(s); lkey.release(s); lseg.release(s);
   }
 };
 
@@ -76,6 +77,7 @@ struct vhci_ctx {
   cublasHandle_t blas = nullptr;
   cusolverDnHandle_t sol = nullptr;
   cudaEvent_t ev_a = nullptr, ev_b = nullptr;
+  double dev_bytes = 0;  // the device's memory
 
   vhci::KeyLayout L{};
 
@@ -86,16 +88,11 @@ struct vhci_ctx {
   uint64_t hmask = 0;
 
   // tables on device
-  vhci::DBuf<vhci::GroupDev> groups;
-  vhci::DBuf<int64_t> wdelta;
+  vhci::DevGroups conn_dev;        // the connection groups
   // the reference's pair-gate patterns, for the structural entry count (built on first use)
   bool gate_built = false, gate_over = false;
   vhci::ConnTables gate;
   vhci::DevGroups gate_dev;
-  vhci::DBuf<uint64_t> lkey;       // lowered-mode segment index (see ConnDev)
-  vhci::DBuf<int32_t> lseg;
-  uint32_t lmask = 0;
-  int maxl = -1;
   vhci::DBuf<vhci::TermDev> terms, dterms;
   vhci::DBuf<double> T, freq;
   vhci::DBuf<vhci::HBDev> hbdev;

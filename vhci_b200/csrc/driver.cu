@@ -61,18 +61,32 @@ int pt2(vhci_ctx* c, double eps2, double* dE_out, int64_t* n_pert) {
     VCK(arow.reserve(NA + 1, s));
     VCK(tmp.reserve(std::max<int64_t>(scan_tmp_elems(NA), 1), s));
     VCK(cudaMemsetAsync(acount.p, 0, std::max<int64_t>(NA, 1) * sizeof(int32_t), s));
-    pt2_count(c->keys.p, n, L, pv, conn_view(c), A0, A1, acount.p, s);
+    Stage stage;
+    VTRY(stage_reserve(c, stage, pv, 0, n));
+    pt2_count(c->keys.p, n, L, pv, conn_view(c), A0, A1, acount.p, stage.view, s);
     exclusive_scan_i32(acount.p, arow.p, NA, tmp.p, s);
     int64_t total = 0;
+    unsigned long long nbatch = 0;
     VCK(d2h(c, &total, arow.p + NA, sizeof(int64_t)));
+    if (stage.view.cap > 0) VCK(d2h(c, &nbatch, stage.cursor.p, sizeof(nbatch)));
     VCK(cudaStreamSynchronize(s));
+    if ((int64_t)nbatch > stage.view.cap) {  // some connections were not kept: walk again per chunk
+      stage.release(s);
+      nbatch = 0;
+    }
     c->stats.pt2_entries += total;
     // chunk the perturber range so one chunk's entries fit the budget
-    size_t freeb = 0, totb = 0;
-    cudaMemGetInfo(&freeb, &totb);
     // entries (12 bytes) plus, in the worst case, the same again as scratch for long-row ordering
-    int64_t budget = c->o.pt2_chunk > 0 ? c->o.pt2_chunk : (int64_t)(freeb * 0.4 / 12.0);
-    budget = std::max<int64_t>(budget, 1 << 20);
+    auto chunk_budget = [&] {
+      const int64_t e = c->o.pt2_chunk > 0 ? c->o.pt2_chunk : (int64_t)(device_available(c) * 0.4 / 12.0);
+      return std::max<int64_t>(e, 1 << 20);
+    };
+    int64_t budget = chunk_budget();
+    if (nbatch > 0 && total > budget && c->o.pt2_chunk <= 0) {  // the kept connections give way
+      stage.release(s);
+      nbatch = 0;
+      budget = chunk_budget();
+    }
     // chunk bounds in perturber indices (arow_h is indexed from A0); one chunk needs only the total,
     // several the host copy of the row offsets
     std::vector<int64_t> bounds{A0};
@@ -96,7 +110,7 @@ int pt2(vhci_ctx* c, double eps2, double* dE_out, int64_t* n_pert) {
       bounds.push_back(std::min(a1, A1));
     }
     DBuf<int32_t> ecol;
-    DBuf<double> eval, part, dEd, Ed;
+    DBuf<double> eval, part, dEd, Ed, ediag;
     const int64_t maxchunk = [&] {
       int64_t mx = 0;
       for (size_t q = 1; q < bounds.size(); ++q)
@@ -133,7 +147,12 @@ int pt2(vhci_ctx* c, double eps2, double* dE_out, int64_t* n_pert) {
       VCK(d2h(c, lc, lcnt.p, sizeof(lc)));
       VCK(cudaStreamSynchronize(s));
       VCK(cudaMemsetAsync(acount.p, 0, na * sizeof(int32_t), s));
-      pt2_fill(c->keys.p, n, L, pv, conn_view(c), a0, a1, crow.p, acount.p, ecol.p, eval.p, s);
+      if (nbatch > 0)
+        pt2_fill_staged(c->keys.p, L, conn_view(c), stage.view, (int64_t)nbatch, a0, a1, crow.p, acount.p,
+                        ecol.p, eval.p, s);
+      else
+        pt2_fill(c->keys.p, n, L, pv, conn_view(c), a0, a1, crow.p, acount.p, ecol.p, eval.p, s);
+      if (a1 == A1) stage.release(s);
       // fixed entry order per row (the fill's atomics leave it arbitrary): short rows by one warp
       // each, long rows by one block each
       pt2_sort_rows(crow.p, na, ecol.p, eval.p, s);
@@ -145,13 +164,14 @@ int pt2(vhci_ctx* c, double eps2, double* dE_out, int64_t* n_pert) {
                         (int)std::min<int64_t>(65535, (int64_t)lc[0] - q0), ecol.p, eval.p, lcol.p,
                         lval.p, s);
       }
+      VCK(ediag.reserve(std::max<int64_t>(na, 1), s));
+      diag_energies(pkeys.p, a0, na, L, conn_view(c), ediag.p, s);
       EventPair ev_r0r1;
       VCK(ev_r0r1.create());
       cudaEvent_t r0 = ev_r0r1.a, r1 = ev_r0r1.b;
       VCK(cudaEventRecord(r0, s));
-      if (!pt2_en(pkeys.p, a0, a1, L, conn_view(c), crow.p, ecol.p, eval.p, c->X.p, c->ldx, nopt,
-                  Ed.p, part.p, s))
-        return fail(c, VHCI_E_INPUT, "PT2: unsupported key width or state count");
+      if (!pt2_en(ediag.p, na, crow.p, ecol.p, eval.p, c->X.p, c->ldx, nopt, Ed.p, part.p, s))
+        return fail(c, VHCI_E_INPUT, "PT2: unsupported state count");
       VCK(cudaEventRecord(r1, s));
       reduce_parts(part.p, nblk, nopt, dEd.p, s);
       VCK(cudaEventSynchronize(r1));
@@ -170,6 +190,7 @@ int pt2(vhci_ctx* c, double eps2, double* dE_out, int64_t* n_pert) {
     if (fl & kFlagTableFull) return fail(c, VHCI_E_TABLE_FULL, "perturber hash full");
     pkeys.release(s); pslots.release(s); acount.release(s); arow.release(s); tmp.release(s);
     ecol.release(s); eval.release(s); part.release(s); dEd.release(s); Ed.release(s); crow.release(s);
+    ediag.release(s);
     lrow_d.release(s); loff_d.release(s); lcol.release(s); lval.release(s); lcnt.release(s);
   }
   for (int j = 0; j < nopt; ++j) {

@@ -69,6 +69,20 @@ struct EventPair {
   }
 };
 
+// Device buffers of a walk's kept connections.
+struct Stage {
+  DBuf<uint2> batch, pair;
+  DBuf<unsigned long long> cursor;
+  StageView view{};
+  void release(cudaStream_t s) {
+    batch.release(s); pair.release(s); cursor.release(s);
+    view = StageView{};
+  }
+};
+// Room for the connections that rows row0 .. row0 + n - 1 have in `table`, by a sample of the rows;
+// without it (a view of capacity 0) the walks that would use it run twice.
+int stage_reserve(vhci_ctx* c, Stage& st, HashView table, int64_t row0, int64_t n);
+
 // Entries of the reference's stored pattern (diagonal + gated pairs, structural zeros included).
 bool structural_available(vhci_ctx* c);
 int structural_count(vhci_ctx* c, int64_t* out);

@@ -24,67 +24,104 @@ inline int grid_for(int64_t n, int threads, int max_blocks = 148 * 16) {
 
 namespace {
 
-// One warp per row; lanes stride over the connection groups, probe the basis hash and compact
-// the hits with a ballot, so a row's entries land in group order (deterministic layout).  Rows
-// row0 .. row0 + n - 1 of the basis are built (all of them, or one rank's block of a sharded
-// matrix); rowcnt, rowptr and diag are indexed from row0, columns are basis indices.
+// One warp per row: the states that the row's state is connected to (conn.cuh), in the walk's fixed
+// order, counted (and kept in `stage` when it has room) or written with their matrix elements
+// (FILL).  Row i is basis state row0 + stride i; columns are basis indices.  Blocks of four rows, no
+// loop: rows differ in work by their excited modes, and the hardware evens that out.
 template <int W, bool FILL>
-__global__ void __launch_bounds__(256) k_hbuild(const uint64_t* __restrict__ keys, int64_t row0,
-                                                int64_t n, KeyLayout L, HashView basis, ConnDev cd,
-                                                int32_t* __restrict__ rowcnt,
-                                                const int64_t* __restrict__ rowptr,
-                                                int32_t* __restrict__ col,
-                                                double* __restrict__ val,
-                                                float* __restrict__ valf,
-                                                double* __restrict__ diag) {
+__global__ void __launch_bounds__(kWalkThreads) k_hbuild(
+    const uint64_t* __restrict__ keys, int64_t row0, int64_t stride, int64_t n, KeyLayout L,
+    HashView basis, ConnDev cd, int32_t* __restrict__ rowcnt, StageView stage,
+    const int64_t* __restrict__ rowptr, int32_t* __restrict__ col, double* __restrict__ val,
+    float* __restrict__ valf) {
   __shared__ uint32_t s_binom[kBinomElems];
-  __shared__ uint8_t s_exc[8][128];
+  __shared__ WalkScratch s_walk[kWalkWarps];
   fill_binom(s_binom);
   __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t i = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); i < n;
-       i += warps) {
-    uint64_t k[W];
-    load_key<W>(keys, row0 + i, k);
-    const int64_t pos = FILL ? rowptr[i] : 0;
-    int cnt = 0;
-    for_each_group<W>(cd, k, L, s_exc[threadIdx.x >> 5], s_binom, [&](int64_t u) {
-      int64_t j = -1;
-      GroupDev g;
-      if (u >= 0) {
-        g = cd.groups[u];
-        uint64_t t[W];
-        if (group_target<W>(cd, u, g, k, L, t)) j = hash_find<W>(basis, t, key_hash<W>(t));
-      }
-      const unsigned b = __ballot_sync(0xffffffffu, j >= 0);
-      if (FILL && j >= 0) {
+  const int64_t i = blockIdx.x * (int64_t)kWalkWarps + (threadIdx.x >> 5);
+  if (i >= n) return;
+  uint64_t k[W];
+  load_key<W>(keys, row0 + stride * i, k);
+  const int64_t pos = FILL ? rowptr[i] : 0;
+  int cnt = 0;
+  walk_connections<W>(cd, basis, k, L, s_walk[threadIdx.x >> 5], s_binom, [&](int64_t j, uint32_t u) {
+    const unsigned b = __ballot_sync(0xffffffffu, j >= 0);
+    if (FILL) {
+      if (j >= 0) {
         const int64_t p = pos + cnt + __popc(b & lanemask_lt());
+        const GroupDev g = cd.groups[u];
         col[p] = (int32_t)j;
         const double v = group_value<W>(cd, g.tb, g.te, k, L);
         if (valf) valf[p] = (float)v; else val[p] = v;
       }
-      cnt += __popc(b);
-    });
-    if (lane == 0) {
-      if (FILL) diag[i] = diag_value<W>(cd, k, L);
-      else rowcnt[i] = cnt;
+    } else if (stage.cap > 0) {
+      stage_hits(stage, (uint32_t)i, (uint32_t)cnt, j, u);
     }
-  }
+    cnt += __popc(b);
+  });
+  if (!FILL && (threadIdx.x & 31) == 0) rowcnt[i] = cnt;
+}
+
+// The entries from kept batches, one warp per batch: every lane has an element to form and the
+// writes are consecutive, where a second walk costs as much as the first (fill of 200,000 states of
+// 48 modes 15.0 -> 0.7 ms, of 150,001 of 15 modes 5.8 -> 2.1 ms).  Bound by the term sums: a group
+// that changes one or two quanta has up to 16 terms, and the batch waits for its longest.
+template <int W>
+__global__ void __launch_bounds__(256) k_hfill_staged(
+    const uint64_t* __restrict__ keys, int64_t row0, KeyLayout L, ConnDev cd, StageView stage,
+    int64_t nbatch, const int64_t* __restrict__ rowptr, int32_t* __restrict__ col,
+    double* __restrict__ val, float* __restrict__ valf) {
+  const int64_t b = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (b >= nbatch) return;
+  const int lane = threadIdx.x & 31;
+  const uint2 h = stage.batch[b];
+  const uint2 e = stage.pair[b * 32 + lane];
+  if (e.x == kNoIndex) return;
+  uint64_t k[W];
+  load_key<W>(keys, row0 + h.x, k);
+  const GroupDev g = cd.groups[e.y];
+  const double v = group_value<W>(cd, g.tb, g.te, k, L);
+  const int64_t p = rowptr[h.x] + h.y + lane;
+  col[p] = (int32_t)e.x;
+  if (valf) valf[p] = (float)v; else val[p] = v;
+}
+
+// One thread per state (the terms are the same for all, their loads broadcast).
+template <int W>
+__global__ void __launch_bounds__(128) k_diag(const uint64_t* __restrict__ keys, int64_t row0, int64_t n,
+                                              KeyLayout L, ConnDev cd, double* __restrict__ diag) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  uint64_t k[W];
+  load_key<W>(keys, row0 + i, k);
+  diag[i] = diag_value<W>(cd, k, L);
 }
 
 template <int W>
-void hbuild_count_launch(const uint64_t* keys, int64_t row0, int64_t n, KeyLayout L,
-                         HashView basis, ConnDev cd, int32_t* rowcnt, cudaStream_t s) {
-  note_launch(); k_hbuild<W, false><<<grid_for(n * 32, 256, 148 * 8), 256, 0, s>>>(
-      keys, row0, n, L, basis, cd, rowcnt, nullptr, nullptr, nullptr, nullptr, nullptr);
+void hbuild_count_launch(const uint64_t* keys, int64_t row0, int64_t stride, int64_t n, KeyLayout L,
+                         HashView basis, ConnDev cd, int32_t* rowcnt, StageView stage,
+                         cudaStream_t s) {
+  note_launch(); k_hbuild<W, false><<<(unsigned)((n + kWalkWarps - 1) / kWalkWarps), kWalkThreads, 0, s>>>(
+      keys, row0, stride, n, L, basis, cd, rowcnt, stage, nullptr, nullptr, nullptr, nullptr);
 }
 template <int W>
 void hbuild_fill_launch(const uint64_t* keys, int64_t row0, int64_t n, KeyLayout L,
                         HashView basis, ConnDev cd, const int64_t* rowptr, int32_t* col,
-                        double* val, float* valf, double* diag, cudaStream_t s) {
-  note_launch(); k_hbuild<W, true><<<grid_for(n * 32, 256, 148 * 8), 256, 0, s>>>(
-      keys, row0, n, L, basis, cd, nullptr, rowptr, col, val, valf, diag);
+                        double* val, float* valf, cudaStream_t s) {
+  note_launch(); k_hbuild<W, true><<<(unsigned)((n + kWalkWarps - 1) / kWalkWarps), kWalkThreads, 0, s>>>(
+      keys, row0, 1, n, L, basis, cd, nullptr, StageView{}, rowptr, col, val, valf);
+}
+template <int W>
+void hbuild_fill_staged_launch(const uint64_t* keys, int64_t row0, KeyLayout L, ConnDev cd,
+                               StageView stage, int64_t nbatch, const int64_t* rowptr, int32_t* col,
+                               double* val, float* valf, cudaStream_t s) {
+  note_launch(); k_hfill_staged<W><<<(unsigned)((nbatch + 7) / 8), 256, 0, s>>>(
+      keys, row0, L, cd, stage, nbatch, rowptr, col, val, valf);
+}
+template <int W>
+void diag_launch(const uint64_t* keys, int64_t row0, int64_t n, KeyLayout L, ConnDev cd, double* diag,
+                 cudaStream_t s) {
+  note_launch(); k_diag<W><<<(unsigned)((n + 127) / 128), 128, 0, s>>>(keys, row0, n, L, cd, diag);
 }
 
 // Y[:, 0:VEC bq] = (D + H_off) X, FP64 vectors, one warp per row (rowprod.cuh).  The diagonal term
@@ -240,18 +277,31 @@ __global__ void k_fill_zero(double* p, int64_t n) {
 
 }  // namespace
 
-void hbuild_count(const uint64_t* keys, int64_t row0, int64_t n, KeyLayout L, HashView basis,
-                  ConnDev cd, int32_t* rowcnt, cudaStream_t s) {
+void hbuild_count(const uint64_t* keys, int64_t row0, int64_t stride, int64_t n, KeyLayout L,
+                  HashView basis, ConnDev cd, int32_t* rowcnt, StageView stage, cudaStream_t s) {
   if (n <= 0) return;
-  VHCI_DISPATCH_W(L.W, hbuild_count_launch, keys, row0, n, L, basis, cd, rowcnt, s);
+  VHCI_DISPATCH_W(L.W, hbuild_count_launch, keys, row0, stride, n, L, basis, cd, rowcnt, stage, s);
 }
 
 void hbuild_fill(const uint64_t* keys, int64_t row0, int64_t n, KeyLayout L, HashView basis,
                  ConnDev cd, const int64_t* rowptr, int32_t* col, double* val, float* valf,
-                 double* diag, cudaStream_t s) {
+                 cudaStream_t s) {
   if (n <= 0) return;
-  VHCI_DISPATCH_W(L.W, hbuild_fill_launch, keys, row0, n, L, basis, cd, rowptr, col, val, valf,
-                  diag, s);
+  VHCI_DISPATCH_W(L.W, hbuild_fill_launch, keys, row0, n, L, basis, cd, rowptr, col, val, valf, s);
+}
+
+void hbuild_fill_staged(const uint64_t* keys, int64_t row0, KeyLayout L, ConnDev cd, StageView stage,
+                        int64_t nbatch, const int64_t* rowptr, int32_t* col, double* val,
+                        float* valf, cudaStream_t s) {
+  if (nbatch <= 0) return;
+  VHCI_DISPATCH_W(L.W, hbuild_fill_staged_launch, keys, row0, L, cd, stage, nbatch, rowptr, col, val,
+                  valf, s);
+}
+
+void diag_energies(const uint64_t* keys, int64_t row0, int64_t n, KeyLayout L, ConnDev cd,
+                   double* diag, cudaStream_t s) {
+  if (n <= 0) return;
+  VHCI_DISPATCH_W(L.W, diag_launch, keys, row0, n, L, cd, diag, s);
 }
 
 // ---- column panels: the off-diagonal entries regrouped by column range -----------------------

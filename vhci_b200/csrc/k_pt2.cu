@@ -24,62 +24,87 @@ inline int grid_for(int64_t n, int threads, int max_blocks = 148 * 16) {
 constexpr int kEnThreads = 256;
 constexpr int kEnBlocks = 148 * 4;
 
+// One warp per variational state: its connected perturbers (conn.cuh, over the perturber table)
+// with indices in [a_lo, a_hi), counted per perturber (and all of them kept in `stage` when it has
+// room) or written with their matrix elements.
 template <int W, bool FILL>
-__global__ void __launch_bounds__(256) k_pt2_gen(const uint64_t* __restrict__ keys, int64_t n,
-                                                 KeyLayout L, HashView pert, ConnDev cd,
-                                                 int64_t a_lo, int64_t a_hi,
-                                                 int32_t* __restrict__ acount,
-                                                 const int64_t* __restrict__ arowptr,
-                                                 int32_t* __restrict__ ecol,
-                                                 double* __restrict__ eval) {
+__global__ void __launch_bounds__(kWalkThreads) k_pt2_gen(
+    const uint64_t* __restrict__ keys, int64_t n, KeyLayout L, HashView pert, ConnDev cd,
+    int64_t a_lo, int64_t a_hi, int32_t* __restrict__ acount, StageView stage,
+    const int64_t* __restrict__ arowptr, int32_t* __restrict__ ecol, double* __restrict__ eval) {
   __shared__ uint32_t s_binom[kBinomElems];
-  __shared__ uint8_t s_exc[8][128];
+  __shared__ WalkScratch s_walk[kWalkWarps];
   fill_binom(s_binom);
   __syncthreads();
-  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t i = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); i < n;
-       i += warps) {
-    uint64_t k[W];
-    load_key<W>(keys, i, k);
-    for_each_group<W>(cd, k, L, s_exc[threadIdx.x >> 5], s_binom, [&](int64_t u) {
-      if (u < 0) return;
+  const int64_t i = blockIdx.x * (int64_t)kWalkWarps + (threadIdx.x >> 5);
+  if (i >= n) return;
+  uint64_t k[W];
+  load_key<W>(keys, i, k);
+  walk_connections<W>(cd, pert, k, L, s_walk[threadIdx.x >> 5], s_binom, [&](int64_t a, uint32_t u) {
+    if (a < a_lo || a >= a_hi) a = -1;
+    if (!FILL) {
+      if (a >= 0) atomicAdd(acount + (a - a_lo), 1);
+      if (stage.cap > 0) stage_hits(stage, (uint32_t)i, 0, a, u);
+    } else if (a >= 0) {
+      const int64_t p = arowptr[a - a_lo] + atomicAdd(acount + (a - a_lo), 1);
       const GroupDev g = cd.groups[u];
-      uint64_t t[W];
-      if (!group_target<W>(cd, u, g, k, L, t)) return;
-      const int64_t a = hash_find<W>(pert, t, key_hash<W>(t));
-      if (a < a_lo || a >= a_hi) return;
-      if (!FILL) {
-        atomicAdd(acount + (a - a_lo), 1);
-      } else {
-        const int64_t p = arowptr[a - a_lo] + atomicAdd(acount + (a - a_lo), 1);
-        ecol[p] = (int32_t)i;
-        eval[p] = group_value<W>(cd, g.tb, g.te, k, L);
-      }
-    });
-  }
+      ecol[p] = (int32_t)i;
+      eval[p] = group_value<W>(cd, g.tb, g.te, k, L);
+    }
+  });
+}
+
+// The entries of perturbers [a_lo, a_hi) from kept batches, one warp per batch (as k_hfill_staged):
+// 60,000 states of 15 modes, 66M entries, 13.2 ms by a walk before, 3.2 ms now; bound by the slot
+// atomics and the scattered 4- and 8-byte writes.
+template <int W>
+__global__ void __launch_bounds__(256) k_pt2_fill_staged(
+    const uint64_t* __restrict__ keys, KeyLayout L, ConnDev cd, StageView stage, int64_t nbatch,
+    int64_t a_lo, int64_t a_hi, int32_t* __restrict__ afill, const int64_t* __restrict__ arowptr,
+    int32_t* __restrict__ ecol, double* __restrict__ eval) {
+  const int64_t b = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (b >= nbatch) return;
+  const uint32_t i = stage.batch[b].x;
+  const uint2 e = stage.pair[b * 32 + (threadIdx.x & 31)];
+  const int64_t a = e.x;
+  if (e.x == kNoIndex || a < a_lo || a >= a_hi) return;
+  const int64_t p = arowptr[a - a_lo] + atomicAdd(afill + (a - a_lo), 1);
+  uint64_t k[W];
+  load_key<W>(keys, i, k);
+  const GroupDev g = cd.groups[e.y];
+  ecol[p] = (int32_t)i;
+  eval[p] = group_value<W>(cd, g.tb, g.te, k, L);
 }
 
 template <int W>
 void pt2_count_launch(const uint64_t* keys, int64_t n, KeyLayout L, HashView pert, ConnDev cd,
-                      int64_t a_lo, int64_t a_hi, int32_t* acount, cudaStream_t s) {
-  note_launch(); k_pt2_gen<W, false><<<grid_for(n * 32, 256, 148 * 8), 256, 0, s>>>(
-      keys, n, L, pert, cd, a_lo, a_hi, acount, nullptr, nullptr, nullptr);
+                      int64_t a_lo, int64_t a_hi, int32_t* acount, StageView stage, cudaStream_t s) {
+  note_launch(); k_pt2_gen<W, false><<<(unsigned)((n + kWalkWarps - 1) / kWalkWarps), kWalkThreads, 0, s>>>(
+      keys, n, L, pert, cd, a_lo, a_hi, acount, stage, nullptr, nullptr, nullptr);
 }
 template <int W>
 void pt2_fill_launch(const uint64_t* keys, int64_t n, KeyLayout L, HashView pert, ConnDev cd,
                      int64_t a_lo, int64_t a_hi, const int64_t* arowptr, int32_t* afill,
                      int32_t* ecol, double* eval, cudaStream_t s) {
-  note_launch(); k_pt2_gen<W, true><<<grid_for(n * 32, 256, 148 * 8), 256, 0, s>>>(
-      keys, n, L, pert, cd, a_lo, a_hi, afill, arowptr, ecol, eval);
+  note_launch(); k_pt2_gen<W, true><<<(unsigned)((n + kWalkWarps - 1) / kWalkWarps), kWalkThreads, 0, s>>>(
+      keys, n, L, pert, cd, a_lo, a_hi, afill, StageView{}, arowptr, ecol, eval);
+}
+template <int W>
+void pt2_fill_staged_launch(const uint64_t* keys, KeyLayout L, ConnDev cd, StageView stage,
+                            int64_t nbatch, int64_t a_lo, int64_t a_hi, const int64_t* arowptr,
+                            int32_t* afill, int32_t* ecol, double* eval, cudaStream_t s) {
+  note_launch(); k_pt2_fill_staged<W><<<(unsigned)((nbatch + 7) / 8), 256, 0, s>>>(
+      keys, L, cd, stage, nbatch, a_lo, a_hi, afill, arowptr, ecol, eval);
 }
 
-// One warp per perturber row.  Lanes own eigenvector columns n = lane + 32 r.  Each warp keeps
+// One warp per perturber row; the perturbers' diagonal elements come from diag_energies (one lane
+// forming them here held up its warp: 8.0 -> 4.2 ms on 832k perturbers, 66M entries, 100 columns).
+// Lanes own eigenvector columns n = lane + 32 r.  Each warp keeps
 // running sums of num^2/(E_n - E_a) over the rows it visits; the block reduces its warps in
 // fixed order into part[block][n].
-template <int W, int NR>
+template <int NR>
 __global__ void __launch_bounds__(kEnThreads) k_pt2_en(
-    const uint64_t* __restrict__ pkeys, int64_t a_lo, int64_t a_hi, KeyLayout L, ConnDev cd,
-    const int64_t* __restrict__ arowptr, const int32_t* __restrict__ ecol,
+    const double* __restrict__ ediag, int64_t na, const int64_t* __restrict__ arowptr, const int32_t* __restrict__ ecol,
     const double* __restrict__ eval, const double* __restrict__ X, int ldx, int nopt,
     const double* __restrict__ E, double* __restrict__ part, int ldp) {
   __shared__ double red[kEnThreads / 32][NR * 32];
@@ -92,11 +117,11 @@ __global__ void __launch_bounds__(kEnThreads) k_pt2_en(
     en[r] = c < nopt ? E[c] : 0.0;
     sum[r] = 0.0;
   }
-  for (int64_t a = a_lo + blockIdx.x * (int64_t)(blockDim.x >> 5) + wid; a < a_hi; a += warps) {
+  for (int64_t a = blockIdx.x * (int64_t)(blockDim.x >> 5) + wid; a < na; a += warps) {
     double num[NR];
 #pragma unroll
     for (int r = 0; r < NR; ++r) num[r] = 0.0;
-    const int64_t beg = arowptr[a - a_lo], end = arowptr[a - a_lo + 1];
+    const int64_t beg = arowptr[a], end = arowptr[a + 1];
     for (int64_t e0 = beg; e0 < end; e0 += 32) {
       const int64_t e = e0 + lane;
       int ii = 0;
@@ -115,13 +140,7 @@ __global__ void __launch_bounds__(kEnThreads) k_pt2_en(
         }
       }
     }
-    double ea = 0.0;
-    if (lane == 0) {
-      uint64_t k[W];
-      load_key<W>(pkeys, a, k);
-      ea = diag_value<W>(cd, k, L);
-    }
-    ea = __shfl_sync(0xffffffffu, ea, 0);
+    const double ea = __ldg(ediag + a);
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
       const int c = lane + 32 * r;
@@ -142,31 +161,6 @@ __global__ void __launch_bounds__(kEnThreads) k_pt2_en(
 // requests (Nstate > 256; the reference has no such limit, PT2.cpp:29-37) run as column tiles of
 // 256, each tile writing its own columns of `part` (leading dimension nopt).
 constexpr int kEnMaxCols = 8 * 32;
-
-template <int W>
-bool pt2_en_launch(const uint64_t* pkeys, int64_t a_lo, int64_t a_hi, KeyLayout L, ConnDev cd,
-                   const int64_t* arowptr, const int32_t* ecol, const double* eval,
-                   const double* X, int ldx, int nopt, const double* E, double* part,
-                   cudaStream_t s) {
-  for (int c0 = 0; c0 < nopt; c0 += kEnMaxCols) {
-    const int nc = nopt - c0 < kEnMaxCols ? nopt - c0 : kEnMaxCols;
-    switch ((nc + 31) / 32) {
-#define VHCI_EN_CASE(R)                                                                        \
-  case R:                                                                                      \
-    note_launch();                                                                             \
-    k_pt2_en<W, R><<<kEnBlocks, kEnThreads, 0, s>>>(pkeys, a_lo, a_hi, L, cd, arowptr, ecol,  \
-                                                    eval, X + c0, ldx, nc, E + c0, part + c0, \
-                                                    nopt);                                     \
-    break;
-      VHCI_EN_CASE(1) VHCI_EN_CASE(2) VHCI_EN_CASE(3) VHCI_EN_CASE(4)
-      VHCI_EN_CASE(5) VHCI_EN_CASE(6) VHCI_EN_CASE(7) VHCI_EN_CASE(8)
-#undef VHCI_EN_CASE
-      default:
-        return false;
-    }
-  }
-  return true;
-}
 
 // ---- fixed entry order within perturber rows --------------------------------------------------
 // The fill pass takes slots with atomics, so the order of a row's entries (and with it the FP64
@@ -327,9 +321,17 @@ void pt2_sort_long(const int64_t* arowptr, const int64_t* rows, const int64_t* s
 }
 
 void pt2_count(const uint64_t* keys, int64_t n, KeyLayout L, HashView pert, ConnDev cd,
-               int64_t a_lo, int64_t a_hi, int32_t* acount, cudaStream_t s) {
+               int64_t a_lo, int64_t a_hi, int32_t* acount, StageView stage, cudaStream_t s) {
   if (n <= 0) return;
-  VHCI_DISPATCH_W(L.W, pt2_count_launch, keys, n, L, pert, cd, a_lo, a_hi, acount, s);
+  VHCI_DISPATCH_W(L.W, pt2_count_launch, keys, n, L, pert, cd, a_lo, a_hi, acount, stage, s);
+}
+
+void pt2_fill_staged(const uint64_t* keys, KeyLayout L, ConnDev cd, StageView stage, int64_t nbatch,
+                     int64_t a_lo, int64_t a_hi, const int64_t* arowptr, int32_t* afill,
+                     int32_t* ecol, double* eval, cudaStream_t s) {
+  if (nbatch <= 0) return;
+  VHCI_DISPATCH_W(L.W, pt2_fill_staged_launch, keys, L, cd, stage, nbatch, a_lo, a_hi, arowptr, afill,
+                  ecol, eval, s);
 }
 
 void pt2_fill(const uint64_t* keys, int64_t n, KeyLayout L, HashView pert, ConnDev cd,
@@ -342,18 +344,27 @@ void pt2_fill(const uint64_t* keys, int64_t n, KeyLayout L, HashView pert, ConnD
 
 int pt2_en_blocks() { return kEnBlocks; }
 
-bool pt2_en(const uint64_t* pkeys, int64_t a_lo, int64_t a_hi, KeyLayout L, ConnDev cd,
-            const int64_t* arowptr, const int32_t* ecol, const double* eval, const double* X,
-            int ldx, int nopt, const double* E, double* part, cudaStream_t s) {
+bool pt2_en(const double* ediag, int64_t na, const int64_t* arowptr, const int32_t* ecol,
+            const double* eval, const double* X, int ldx, int nopt, const double* E, double* part,
+            cudaStream_t s) {
   if (nopt <= 0) return false;
-  switch (L.W) {
-#define VHCI_EN_W(WV) \
-  case WV: return pt2_en_launch<WV>(pkeys, a_lo, a_hi, L, cd, arowptr, ecol, eval, X, ldx, nopt, E, part, s);
-    VHCI_EN_W(1) VHCI_EN_W(2) VHCI_EN_W(3) VHCI_EN_W(4)
-    VHCI_EN_W(5) VHCI_EN_W(6) VHCI_EN_W(7) VHCI_EN_W(8)
-#undef VHCI_EN_W
-    default: return false;
+  for (int c0 = 0; c0 < nopt; c0 += kEnMaxCols) {
+    const int nc = nopt - c0 < kEnMaxCols ? nopt - c0 : kEnMaxCols;
+    switch ((nc + 31) / 32) {
+#define VHCI_EN_CASE(R)                                                                        \
+  case R:                                                                                      \
+    note_launch();                                                                             \
+    k_pt2_en<R><<<kEnBlocks, kEnThreads, 0, s>>>(ediag, na, arowptr, ecol, eval, X + c0, ldx,  \
+                                                 nc, E + c0, part + c0, nopt);                 \
+    break;
+      VHCI_EN_CASE(1) VHCI_EN_CASE(2) VHCI_EN_CASE(3) VHCI_EN_CASE(4)
+      VHCI_EN_CASE(5) VHCI_EN_CASE(6) VHCI_EN_CASE(7) VHCI_EN_CASE(8)
+#undef VHCI_EN_CASE
+      default:
+        return false;
+    }
   }
+  return true;
 }
 
 }  // namespace vhci

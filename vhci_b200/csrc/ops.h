@@ -42,6 +42,7 @@ static_assert(sizeof(HBDev) == 20, "HBDev layout");
 struct ConnDev {            // connection tables on device
   const GroupDev* groups;
   const int64_t* wdelta;    // [ngroups * W] packed key change per word
+  const uint64_t* hdelta;   // [ngroups] change of the linear hash
   int64_t ngroups;
   const TermDev* terms;
   const TermDev* dterms;    // Delta = 0 terms
@@ -55,6 +56,15 @@ struct ConnDev {            // connection tables on device
   const int32_t* lseg;      // [2 (lmask + 1)] first group and group count of the segment
   uint32_t lmask;
   int maxl;                 // most modes one group lowers; -1: no index, visit every group
+};
+
+// Connections kept by a count pass (conn.cuh): per batch its row and row offset, 32 (index, group)
+// pairs; cursor: batches found (also those beyond the capacity, which are not stored).
+struct StageView {
+  uint2* batch;
+  uint2* pair;
+  unsigned long long* cursor;
+  int64_t cap;  // batches; 0: nothing is kept
 };
 
 struct HBTable {
@@ -126,12 +136,20 @@ void hmerge_cross_scatter(const uint64_t* keys, int64_t ncross, const int64_t* x
                           const int64_t* rp_old, const int64_t* rp_all, const int32_t* erow,
                           const double* vnew, const float* vnewf, int64_t n_old, int32_t* cd,
                           double* vd, float* vdf, cudaStream_t s);
-// Rows row0 .. row0 + n - 1 of the Hamiltonian (rowcnt, rowptr, diag indexed from row0).
-void hbuild_count(const uint64_t* keys, int64_t row0, int64_t n, KeyLayout L, HashView basis,
-                  ConnDev cd, int32_t* rowcnt, cudaStream_t s);
+// Rows row0 + stride i, i < n, of the Hamiltonian (rowcnt, rowptr indexed by i): entry counts,
+// keeping the connections in `stage` on the way; the entries by a second walk (stride 1), or from
+// the nbatch kept batches when none was lost.
+void hbuild_count(const uint64_t* keys, int64_t row0, int64_t stride, int64_t n, KeyLayout L,
+                  HashView basis, ConnDev cd, int32_t* rowcnt, StageView stage, cudaStream_t s);
 void hbuild_fill(const uint64_t* keys, int64_t row0, int64_t n, KeyLayout L, HashView basis,
                  ConnDev cd, const int64_t* rowptr, int32_t* col, double* val, float* valf,
-                 double* diag, cudaStream_t s);
+                 cudaStream_t s);
+void hbuild_fill_staged(const uint64_t* keys, int64_t row0, KeyLayout L, ConnDev cd, StageView stage,
+                        int64_t nbatch, const int64_t* rowptr, int32_t* col, double* val,
+                        float* valf, cudaStream_t s);
+// diag[i] = diagonal element of state row0 + i, i < n
+void diag_energies(const uint64_t* keys, int64_t row0, int64_t n, KeyLayout L, ConnDev cd,
+                   double* diag, cudaStream_t s);
 // Column panels of the off-diagonal CSR (at most kMaxPanels): entries of panel p (columns
 // [p cw, (p+1) cw)) for row i at [prow[p n + i], prow[p n + i + 1]).
 constexpr int kMaxPanels = 64;
@@ -190,18 +208,21 @@ void svqb_factor(const double* S, int nb, double* M, int* rank_short, cudaStream
 
 // ---- PT2 (k_pt2.cu) ----
 void pt2_count(const uint64_t* keys, int64_t n, KeyLayout L, HashView pert, ConnDev cd,
-               int64_t a_lo, int64_t a_hi, int32_t* acount, cudaStream_t s);
+               int64_t a_lo, int64_t a_hi, int32_t* acount, StageView stage, cudaStream_t s);
+void pt2_fill_staged(const uint64_t* keys, KeyLayout L, ConnDev cd, StageView stage, int64_t nbatch,
+                     int64_t a_lo, int64_t a_hi, const int64_t* arowptr, int32_t* afill,
+                     int32_t* ecol, double* eval, cudaStream_t s);
 void pt2_fill(const uint64_t* keys, int64_t n, KeyLayout L, HashView pert, ConnDev cd,
               int64_t a_lo, int64_t a_hi, const int64_t* arowptr, int32_t* afill, int32_t* ecol,
               double* eval, cudaStream_t s);
-// Fused EN reduction over perturbers [a_lo, a_hi): num_a = sum_e eval_e X[ecol_e, :nopt];
-// E_a = harmonic + diagonal terms; part[blk][n] += num^2 / (E_n - E_a).
+// Fused EN reduction over na perturber rows: num_a = sum_e eval_e X[ecol_e, :nopt];
+// part[blk][n] += num_a^2 / (E_n - ediag_a) (ediag: the perturbers' diagonal elements).
 // Every block writes all nopt columns of its part row; any nopt >= 1 (column tiles of 256);
-// returns false for an unsupported key width or nopt < 1 (nothing launched).
+// returns false for nopt < 1 (nothing launched).
 int pt2_en_blocks();
-bool pt2_en(const uint64_t* pkeys, int64_t a_lo, int64_t a_hi, KeyLayout L, ConnDev cd,
-            const int64_t* arowptr, const int32_t* ecol, const double* eval, const double* X,
-            int ldx, int nopt, const double* E, double* part, cudaStream_t s);
+bool pt2_en(const double* ediag, int64_t na, const int64_t* arowptr, const int32_t* ecol,
+            const double* eval, const double* X, int ldx, int nopt, const double* E, double* part,
+            cudaStream_t s);
 // Orders the entries of each perturber row [arowptr[r], arowptr[r+1]) by ascending state index,
 // so the EN sums run in one fixed order.  pt2_sort_rows handles rows shorter than
 // pt2_sort_long_min() entries; pt2_sort_long the listed longer rows (rows[q], with scratch
