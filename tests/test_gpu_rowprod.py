@@ -63,3 +63,17 @@ def test_residual_norms_at_every_lane_split(ctx, k, shift):
     # entrywise bound on the residual, plus the rounding of theta x and of the sum of n squares
     err = np.linalg.norm(bound(H, m, X) + 4 * U * np.abs(X * th), axis=0) + (v.n + 4) * U * ref
     assert (np.abs(r.cpu().numpy() - ref) <= err).all()
+
+
+@pytest.mark.parametrize("n,k", [(1, 1), (33, 31), (91, 65), (20011, 420)])  # the last: two transfers
+def test_vectors_round_trip(n, k):
+    from vhci_b200 import api
+    rng = np.random.default_rng(k)
+    with api.VHCI(os.path.join(GOLDEN, "workload0", "input.inp")) as v:
+        q = np.unique(rng.binomial(6, 0.3, (2 * n + 50, v.info.nmodes)).astype(np.uint8), axis=0)[:n]
+        v.set_basis(q)
+        C, E = rng.standard_normal((n, k)), np.sort(rng.standard_normal(k))
+        v.set_vectors(C, E)
+        for m in {1, k - k // 3, k}:
+            got, e = v.vectors(m)
+            assert np.array_equal(got, C[:, :m]) and np.array_equal(e, E[:m])

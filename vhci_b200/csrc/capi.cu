@@ -942,6 +942,47 @@ vhci_status vhci_reset_stats(vhci_ctx* c) {
   return VHCI_OK;
 }
 
+}  // extern "C"
+
+namespace vhci {
+
+// Columns per transfer: at least 64 MB of them, at least 16 (whole 128-byte lines of the rows).
+static int transfer_cols(int64_t n, int k) {
+  const int64_t w = std::max<int64_t>(16, (int64_t)(64e6 / (8.0 * (double)std::max<int64_t>(n, 1))) + 1);
+  return (int)std::min<int64_t>(k, w);
+}
+
+int upload_cols(vhci_ctx* c, const double* host, int64_t n, int k, double* dev, int ldd) {
+  const int w = transfer_cols(n, k);
+  DBuf<double> t;
+  VCK(t.reserve((size_t)n * w, c->st));
+  for (int j = 0; j < k; j += w) {
+    const int m = std::min(w, k - j);
+    VCK(h2d(c, t.p, host + (size_t)j * n, (size_t)n * m * sizeof(double)));
+    cols_to_rows(t.p, n, m, dev + j, ldd, c->st);
+  }
+  t.release(c->st);
+  return VHCI_OK;
+}
+
+int download_cols(vhci_ctx* c, const double* dev, int lds, int64_t n, int k, double* host) {
+  const int w = transfer_cols(n, k);
+  DBuf<double> t;
+  VCK(t.reserve((size_t)n * w, c->st));
+  for (int j = 0; j < k; j += w) {
+    const int m = std::min(w, k - j);
+    rows_to_cols(dev + j, lds, n, m, t.p, c->st);
+    VCK(d2h(c, host + (size_t)j * n, t.p, (size_t)n * m * sizeof(double)));
+  }
+  t.release(c->st);
+  VCK(cudaStreamSynchronize(c->st));
+  return VHCI_OK;
+}
+
+}  // namespace vhci
+
+extern "C" {
+
 static void dump_fc(const std::vector<ForceConstant>& L, double* v, int32_t* m, int32_t* p) {
   for (size_t i = 0; i < L.size(); ++i) {
     v[i] = L[i].fc;
@@ -1017,11 +1058,8 @@ vhci_status vhci_get_basis(const vhci_ctx* c0, uint8_t* quanta, int64_t cap, int
 vhci_status vhci_set_vectors(vhci_ctx* c, const double* C, const double* E, int k) {
   if (!c || !C || !E || k <= 0) return VHCI_E_INPUT;
   const int64_t n = c->n;
-  std::vector<double> h((size_t)n * k);
-  for (int64_t i = 0; i < n; ++i)
-    for (int j = 0; j < k; ++j) h[(size_t)i * k + j] = C[(size_t)j * n + i];
   VCK(c->X.reserve((size_t)n * k, c->st));
-  VCK(h2d(c, c->X.p, h.data(), h.size() * sizeof(double)));
+  VTRY(upload_cols(c, C, n, k, c->X.p, k));
   VCK(cudaStreamSynchronize(c->st));
   c->ldx = k;
   c->nvec = k;
@@ -1035,13 +1073,7 @@ vhci_status vhci_get_vectors(const vhci_ctx* c0, double* C, double* E, int k) {
   if (!c) return VHCI_E_INPUT;
   if (k > c->nvec || c->x_rows != c->n) return fail(c, VHCI_E_STATE, "fewer vectors held than requested");
   const int64_t n = c->n;
-  if (C) {
-    std::vector<double> h((size_t)n * c->ldx);
-    VCK(d2h(c, h.data(), c->X.p, h.size() * sizeof(double)));
-    VCK(cudaStreamSynchronize(c->st));
-    for (int64_t i = 0; i < n; ++i)
-      for (int j = 0; j < k; ++j) C[(size_t)j * n + i] = h[(size_t)i * c->ldx + j];
-  }
+  if (C && k > 0) VTRY(download_cols(c, c->X.p, c->ldx, n, k, C));
   if (E)
     for (int j = 0; j < k; ++j) E[j] = c->E[j];
   return VHCI_OK;

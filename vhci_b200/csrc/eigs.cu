@@ -116,20 +116,14 @@ extern "C" vhci_status vhci_apply_h(vhci_ctx* c, const double* X, double* Y, int
   if (is_sharded(c)) return fail(c, VHCI_E_STATE, "vhci_apply_h on a sharded context");
   if (!c->h_valid || c->h_rows) VTRY(build_h(c, true));
   const int64_t n = c->n;
-  std::vector<double> h((size_t)n * b);
-  for (int64_t i = 0; i < n; ++i)
-    for (int j = 0; j < b; ++j) h[(size_t)i * b + j] = X[(size_t)j * n + i];
   DBuf<double> dx, dy;
-  VCK(dx.reserve(h.size(), c->st));
-  VCK(dy.reserve(h.size(), c->st));
-  VCK(h2d(c, dx.p, h.data(), h.size() * sizeof(double)));
+  VCK(dx.reserve((size_t)n * b, c->st));
+  VCK(dy.reserve((size_t)n * b, c->st));
+  VTRY(upload_cols(c, X, n, b, dx.p, b));
   VTRY(apply_h(c, dx.p, b, b, dy.p, b));
-  VCK(d2h(c, h.data(), dy.p, h.size() * sizeof(double)));
-  VCK(cudaStreamSynchronize(c->st));
+  VTRY(download_cols(c, dy.p, b, n, b, Y));
   dx.release(c->st);
   dy.release(c->st);
-  for (int64_t i = 0; i < n; ++i)
-    for (int j = 0; j < b; ++j) Y[(size_t)j * n + i] = h[(size_t)i * b + j];
   return VHCI_OK;
 }
 

@@ -69,6 +69,10 @@ struct EventPair {
   }
 };
 
+// Blocks of k column-major host vectors (n x k, leading dimension n) to a row-major device block and
+// back, a few columns at a time through a device buffer of limited size.
+int upload_cols(vhci_ctx* c, const double* host, int64_t n, int k, double* dev, int ldd);
+int download_cols(vhci_ctx* c, const double* dev, int lds, int64_t n, int k, double* host);
 // Device buffers of a walk's kept connections.
 struct Stage {
   DBuf<uint2> batch, pair;

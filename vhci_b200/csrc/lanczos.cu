@@ -318,19 +318,6 @@ int fp64_sweep(vhci_ctx* c, LWork& w, int kk, int nk, int keff, int ld, std::vec
   return VHCI_OK;
 }
 
-// Start vectors of the cold start: standard normal values drawn from the global (row, column)
-// index, so every rank draws the same values for its rows whatever the sharding.
-void random_rows(int64_t r0, int64_t rows, int b, std::vector<double>& out) {
-  out.resize((size_t)rows * b);
-  for (int64_t i = 0; i < rows; ++i)
-    for (int j = 0; j < b; ++j) {
-      const uint64_t key = ((uint64_t)(r0 + i) << 6) ^ (uint64_t)j;
-      const double u1 = ((mix64(2 * key + 0x9E3779B97F4A7C15ull) >> 11) + 0.5) * (1.0 / 9007199254740992.0);
-      const double u2 = ((mix64(2 * key + 1 + 0x9E3779B97F4A7C15ull) >> 11) + 0.5) * (1.0 / 9007199254740992.0);
-      out[(size_t)i * b + j] = std::sqrt(-2.0 * std::log(u1)) * std::cos(6.283185307179586 * u2);
-    }
-}
-
 // Hands the Ritz block (this rank's rows, ld kk) to the context as its whole vectors: swapped in
 // on an unsharded context, all-gathered from the ranks' row blocks (rblk rows each; the buffer
 // holds at least that many) on a sharded one.
@@ -484,8 +471,7 @@ int block_lanczos_impl(vhci_ctx* c, int k, bool dev_svqb) {
     R.release(s);
     if (p == 0) return fail(c, VHCI_E_NOT_CONVERGED, "empty start block");
   } else {
-    random_rows(r0, nl, b, rnd);
-    VCK(h2d(c, w.W.p, rnd.data(), rnd.size() * sizeof(double)));
+    random_rows(r0, nl, b, w.W.p, s);
     VTRY(svqb_small(c, w, nl, w.W.p, b, b, w.Q.p, ld, &p));
     if (p == 0) return fail(c, VHCI_E_NOT_CONVERGED, "empty start block");
   }
@@ -728,8 +714,7 @@ int block_lanczos_lean(vhci_ctx* c, int k) {
     VCK(cudaStreamSynchronize(s));
     R.release(s);
   } else {
-    random_rows(r0, nl, b, rnd);
-    VCK(h2d(c, w.W.p, rnd.data(), rnd.size() * sizeof(double)));
+    random_rows(r0, nl, b, w.W.p, s);
     VTRY(svqb_small(c, w, nl, w.W.p, b, b, w.Q.p, ld, &p));
   }
   if (p == 0) return fail(c, VHCI_E_NOT_CONVERGED, "empty start block");

@@ -182,6 +182,13 @@ void residual_norms(const double* X, const double* HX, int64_t n, int ld, int kk
 int residual_blocks(int64_t n);
 void copy_cols(const double* src, int lds, double* dst, int ldd, int64_t n, int ncol,
                cudaStream_t s);
+// dst (n x w row-major, ldd) = src (n x w column-major, leading dimension n), and back.
+void cols_to_rows(const double* src, int64_t n, int w, double* dst, int ldd, cudaStream_t s);
+void rows_to_cols(const double* src, int lds, int64_t n, int w, double* dst, cudaStream_t s);
+// Rows r0 .. r0 + n - 1 of the cold start's block (n x b row-major): standard normal values drawn from
+// the global (row, column) index, so every rank draws the same values for its rows whatever the
+// sharding.
+void random_rows(int64_t r0, int64_t n, int b, double* out, cudaStream_t s);
 void dense_from_csr(int64_t n, const int64_t* rowptr, const int32_t* col, const double* val,
                     const float* valf, const double* diag, double* A, cudaStream_t s);
 void fill_zero(double* p, int64_t n, cudaStream_t s);

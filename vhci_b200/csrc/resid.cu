@@ -137,15 +137,12 @@ extern "C" vhci_status vhci_residual_norms(vhci_ctx* c, const double* X, const d
   if (is_sharded(c)) return fail(c, VHCI_E_STATE, "vhci_residual_norms on a sharded context");
   if (!c->h_valid || c->h_rows) VTRY(build_h(c, true));
   const int64_t n = c->n;
-  std::vector<double> h((size_t)n * k);
-  for (int64_t i = 0; i < n; ++i)
-    for (int j = 0; j < k; ++j) h[(size_t)i * k + j] = X[(size_t)j * n + i];
   DBuf<double> dx, dth, part, dr;
-  VCK(dx.reserve(h.size(), c->st));
+  VCK(dx.reserve((size_t)n * k, c->st));
   VCK(dth.reserve(k, c->st));
   VCK(part.reserve(resid_scratch_elems(k), c->st));
   VCK(dr.reserve(k, c->st));
-  VCK(h2d(c, dx.p, h.data(), h.size() * sizeof(double)));
+  VTRY(upload_cols(c, X, n, k, dx.p, k));
   VCK(h2d(c, dth.p, theta, k * sizeof(double)));
   residual_norms_fused(c, dx.p, k, dth.p, part.p, dr.p);
   VCK(d2h(c, rnorm, dr.p, k * sizeof(double)));
