@@ -12,9 +12,13 @@
 //               the partial products of its 8-row tiles of C in registers; the blocks' partials
 //               go to scratch and a second kernel sums them in block order, so the result does not
 //               depend on scheduling.
-//   proj_rows:  Out = alpha * A S + beta * Out   A: n x M row-major, S: M x P col-major,
-//               Out: n x P row-major.  Each block holds a 16-column slab of S in shared memory
-//               and its warps stream 8-row tiles of A.
+//   proj_rows:  Out = alpha * A S + beta * In    A: n x M row-major, S: M x P col-major,
+//               Out: n x P row-major.  Each block holds a 16- or 32-column slab of S in shared memory
+//               and its warps stream 8-row tiles of A.  proj_rows_self also forms Out^T Out.
+//
+// A Lanczos step reads the basis twice (coefficients, update).  Three passes with the first two fused
+// over 128-row chunks took 240 + 110 us of projections at 120,011 rows and 512 columns on average,
+// 44 us at 24,000 rows and 150 columns; now 140 + 114 and 15 + 13 us.
 //
 // Fragment layouts of m8n8k4 (row.col): A[m][k] sits in lane 4 m + k, B[k][n] in lane 4 n + k,
 // D[m][n] in lane 4 m + n / 2 (element n % 2).
@@ -132,7 +136,8 @@ constexpr int kRedWarps = 32;
 __global__ void __launch_bounds__(kRedWarps * 32) k_gram_reduce(const double* __restrict__ part,
                                                                 int nblk, int M, int P, double alpha,
                                                                 double beta, double* __restrict__ C,
-                                                                int ldc) {
+                                                                int ldc, double* __restrict__ Acc,
+                                                                int ldacc) {
   __shared__ double ws[kRedWarps][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int x = blockIdx.x * 32 + lane;
@@ -148,7 +153,9 @@ __global__ void __launch_bounds__(kRedWarps * 32) k_gram_reduce(const double* __
     for (int v = 1; v < kRedWarps; ++v) t += ws[v][lane];
     const int a = x / P, c = x - a * P;
     double* o = C + a + (int64_t)c * ldc;
-    *o = beta == 0.0 ? alpha * t : alpha * t + beta * *o;
+    const double v = beta == 0.0 ? alpha * t : alpha * t + beta * *o;
+    *o = v;
+    if (Acc) Acc[a + (int64_t)c * ldacc] += v;
   }
 }
 
@@ -156,34 +163,52 @@ __global__ void __launch_bounds__(kRedWarps * 32) k_gram_reduce(const double* __
 // distinct 32-byte bank groups.
 constexpr int kRowsMaxM = 1280;     // rows of S held in shared memory per pass over A
 constexpr int kRowsMaxM4 = 768;     // the same for 32-column slabs
+constexpr int kRowsSelfMaxM = 960;  // the same beside the fused Gram product's reduction
 
 template <int NT>
 constexpr size_t rows_smem(int M) {
   return (size_t)M * (8 * NT + 4) * sizeof(double);
 }
 
-// Out[i][c] = alpha sum_a A[i][a] S[a + c lds] + beta Out[i][c] for the Mc rows of S starting
-// at a0 (accum: add this slab to Out, which already holds the earlier slabs' sum; the alpha/beta
-// update happens on the first slab).  Warps stream 8-row tiles of A over the whole grid.
-template <int NT>
+// What k_rows does beside its product.
+struct RowsTail {
+  const double* In;  // the beta term's block (ld ldi); Out itself unless given
+  int ldi;
+  double* Out2;      // second copy of the result (ld ldo2), or null
+  int ldo2;
+  double* part;      // partial Gram products Out^T Out, P x P per block, or null
+};
+
+// Out[i][c] = alpha sum_a A[i][a] S[a + c lds] + beta In[i][c] for Mc rows of S; warps stream 8-row
+// tiles of A over the whole grid.  SELF: the tile's new rows also go, as they are in the accumulators
+// (moved into operand layout by shuffles), into the warp's share of Out^T Out, so that the block
+// orthonormalisation that follows a Gram-Schmidt pass needs no pass of its own (114 us at 120,011 rows
+// and 512 columns on average, where the pass without it took 110 and the Gram product another 16).
+template <int NT, bool SELF>
 __global__ void __launch_bounds__(kThreads, 1) k_rows(const double* __restrict__ A, int lda,
                                                       const double* __restrict__ S, int lds,
                                                       int64_t n, int Mc, int P, double alpha,
-                                                      double beta, double* __restrict__ Out,
-                                                      int ldo) {
-  extern __shared__ double ss[];  // [Mc][8 NT + 4]
+                                                      double beta, double* Out, int ldo,
+                                                      RowsTail tail) {
+  extern __shared__ double ss[];  // [Mc][8 NT + 4]; SELF: then [warps][64 NT NT] for the reduction
   constexpr int SW = 8 * NT + 4;
   for (int x = threadIdx.x; x < Mc * 8 * NT; x += blockDim.x) {
-    const int a = x / (8 * NT), c = x - a * (8 * NT);
+    const int c = x / Mc, a = x - c * Mc;  // consecutive threads read one column of S
     ss[a * SW + c] = c < P ? S[a + (int64_t)c * lds] : 0.0;
   }
   __syncthreads();
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int kl = lane & 3;
   const int64_t tiles = (n + 7) / 8;
   const int64_t wstride = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t tile = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); tile < tiles;
-       tile += wstride) {
+  double g[SELF ? NT : 1][SELF ? NT : 1][2];
+  if constexpr (SELF) {
+#pragma unroll
+    for (int u = 0; u < NT; ++u)
+#pragma unroll
+      for (int v = 0; v < NT; ++v) g[u][v][0] = g[u][v][1] = 0.0;
+  }
+  for (int64_t tile = (int64_t)blockIdx.x * (blockDim.x >> 5) + wid; tile < tiles; tile += wstride) {
     const int64_t i = tile * 8 + (lane >> 2);
     const bool rin = i < n;
     const double* arow = A + (rin ? i : 0) * lda;
@@ -207,281 +232,157 @@ __global__ void __launch_bounds__(kThreads, 1) k_rows(const double* __restrict__
         }
       }
     }
-    if (rin) {
-#pragma unroll
-      for (int u = 0; u < NT; ++u)
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const int c = 8 * u + 2 * (lane & 3) + j;
-          if (c < P) {
-            double* o = Out + i * ldo + c;
-            *o = beta == 0.0 ? alpha * acc[u][j] : alpha * acc[u][j] + beta * *o;
-          }
-        }
-    }
-  }
-}
-
-// The second and third Gram-Schmidt passes over the same rows of A, fused:
-//   W <- W - A S1            (S1: M x P column-major)
-//   part[block] = A^T W      (with the updated W; this block's rows, M x P a-major)
-// A block walks chunks of 128 rows (16 8-row tiles): warps w and w + 16 each form the product of
-// tile w over one half of A's columns (A from global memory, S1 from shared memory), the second
-// hands its half to the first through shared memory, which updates the tile of W and leaves the
-// new rows in a shared copy; then every warp adds A_chunk^T W_chunk to its 8-row tiles of the
-// partial Gram product, re-reading the chunk's rows of A, which the first phase has just brought
-// into L2.  One pass over A from HBM instead of two: the chunks in flight over the whole GPU
-// (148 x 128 rows of A, 58 MB at M = 384, 97 MB at M = 640) stay within L2, which 256-row chunks
-// did not (measured: 31 % L2 hits on the re-read at M = 437 with 256-row chunks).
-constexpr int kFuseChunk = 128;
-constexpr int kFuseTiles = 3;       // Gram tiles per warp: M <= 32 x 3 x 8 = 768
-constexpr int kFuseMaxM = 32 * kFuseTiles * 8;
-
-template <int NT>
-constexpr size_t fuse_smem(int M) {
-  // S1 slab, chunk of W, and the second half-products of phase 1 (16 warps x 32 lanes x NT x 2)
-  return (size_t)(M + kFuseChunk) * (8 * NT + 4) * sizeof(double) +
-         (size_t)16 * 32 * NT * 2 * sizeof(double);
-}
-
-template <int NT>
-__global__ void __launch_bounds__(kThreads, 1) k_rows_gram(const double* __restrict__ A, int lda,
-                                                           const double* __restrict__ S1, int lds,
-                                                           double* __restrict__ W, int ldw,
-                                                           int64_t n, int M, int P,
-                                                           double* __restrict__ part) {
-  extern __shared__ double smf[];
-  constexpr int SW = 8 * NT + 4;
-  double* sS = smf;               // [M][SW]
-  double* sW = smf + M * SW;      // [kFuseChunk][SW]
-  double* sH = sW + kFuseChunk * SW;  // [16][32][NT][2]: phase-1 products of the upper warps
-  for (int x = threadIdx.x; x < M * 8 * NT; x += blockDim.x) {
-    const int a = x / (8 * NT), c = x - a * (8 * NT);
-    sS[a * SW + c] = c < P ? S1[a + (int64_t)c * lds] : 0.0;
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, kl = lane & 3;
-  const int64_t per = ((n + gridDim.x - 1) / gridDim.x + 3) & ~int64_t(3);
-  const int64_t r0 = (int64_t)blockIdx.x * per, r1 = min(n, r0 + per);
-  const int mt_total = (M + 7) / 8;
-  double g[kFuseTiles][NT][2];
-#pragma unroll
-  for (int t = 0; t < kFuseTiles; ++t)
-#pragma unroll
-    for (int u = 0; u < NT; ++u) g[t][u][0] = g[t][u][1] = 0.0;
-  for (int64_t c0 = r0; c0 < r1; c0 += kFuseChunk) {
-    // phase 1: tile wid % 16 of W - A S1; warps 0-15 take A's columns [0, kh), warps 16-31
-    // [kh, M), kh a multiple of the 4 kUnroll columns one step covers
-    const int tl = wid & 15, half = wid >> 4;
-    const int kh = ((M + 1) / 2 + 4 * kUnroll - 1) / (4 * kUnroll) * (4 * kUnroll);
-    const int kb = half ? kh : 0, ke = half ? M : min(kh, M);
-    const int64_t i = c0 + 8 * tl + (lane >> 2);
-    const bool rin = i < r1;
-    const double* arow = A + (rin ? i : 0) * lda;
-    double acc[NT][2];
-#pragma unroll
-    for (int u = 0; u < NT; ++u) acc[u][0] = acc[u][1] = 0.0;
-    for (int k0 = kb; k0 < ke; k0 += 4 * kUnroll) {
-      double a[kUnroll];
-#pragma unroll
-      for (int s = 0; s < kUnroll; ++s) {
-        const int k = k0 + 4 * s + kl;
-        a[s] = (rin && k < ke) ? __ldg(arow + k) : 0.0;
-      }
-#pragma unroll
-      for (int s = 0; s < kUnroll; ++s) {
-        const int k = k0 + 4 * s + kl;
-        if (k0 + 4 * s < ke) {
-#pragma unroll
-          for (int u = 0; u < NT; ++u)
-            dmma(acc[u], a[s], k < ke ? sS[k * SW + 8 * u + (lane >> 2)] : 0.0);
-        }
-      }
-    }
-    if (half) {
-#pragma unroll
-      for (int u = 0; u < NT; ++u)
-#pragma unroll
-        for (int j = 0; j < 2; ++j) sH[((tl * 32 + lane) * NT + u) * 2 + j] = acc[u][j];
-    }
-    __syncthreads();
-    const int rl = 8 * tl + (lane >> 2);
 #pragma unroll
     for (int u = 0; u < NT; ++u)
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         const int c = 8 * u + 2 * (lane & 3) + j;
-        if (half) continue;
-        double wv = 0.0;
+        double o = 0.0;
         if (rin && c < P) {
-          wv = W[i * ldw + c] - (acc[u][j] + sH[((tl * 32 + lane) * NT + u) * 2 + j]);
-          W[i * ldw + c] = wv;
+          o = beta == 0.0 ? alpha * acc[u][j] : alpha * acc[u][j] + beta * tail.In[i * tail.ldi + c];
+          Out[i * ldo + c] = o;
+          if (tail.Out2) tail.Out2[i * tail.ldo2 + c] = o;
         }
-        sW[rl * SW + c] = wv;
+        acc[u][j] = o;
       }
-    __syncthreads();
-    // phase 2: the partial Gram product of the chunk, this warp's tiles w, w + 32, w + 64
-    for (int kk = 0; kk < kFuseChunk; kk += 8) {
-      double a[2][kFuseTiles], b[2][NT];
+    if constexpr (SELF) {
+      // operand element (row 4 h + (lane & 3), column 8 u + lane / 4) sits in lane
+      // 4 row + (column % 8) / 2, place column % 2
 #pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        const int kr = kk + 4 * s + kl;
-        const int64_t ir = c0 + kr;
-        const bool in2 = ir < r1;
+      for (int h = 0; h < 2; ++h) {
+        double w[NT];
+        const int src = 4 * (4 * h + (lane & 3)) + (lane >> 3);
 #pragma unroll
-        for (int t = 0; t < kFuseTiles; ++t) {
-          const int col = 8 * (wid + 32 * t) + (lane >> 2);
-          a[s][t] = (in2 && col < M) ? __ldg(A + ir * lda + col) : 0.0;
+        for (int u = 0; u < NT; ++u) {
+          const double x0 = __shfl_sync(0xffffffffu, acc[u][0], src);
+          const double x1 = __shfl_sync(0xffffffffu, acc[u][1], src);
+          w[u] = (lane >> 2) & 1 ? x1 : x0;
         }
 #pragma unroll
-        for (int u = 0; u < NT; ++u) b[s][u] = sW[kr * SW + 8 * u + (lane >> 2)];
+        for (int u = 0; u < NT; ++u)
+#pragma unroll
+          for (int v = 0; v < NT; ++v) dmma(g[u][v], w[u], w[v]);
       }
-#pragma unroll
-      for (int s = 0; s < 2; ++s)
-#pragma unroll
-        for (int t = 0; t < kFuseTiles; ++t)
-          if (wid + 32 * t < mt_total)
-#pragma unroll
-            for (int u = 0; u < NT; ++u) dmma(g[t][u], a[s][t], b[s][u]);
     }
-    __syncthreads();
   }
-  double* out = part + (int64_t)blockIdx.x * M * P;
-#pragma unroll
-  for (int t = 0; t < kFuseTiles; ++t) {
-    const int mt = wid + 32 * t;
-    if (mt >= mt_total) continue;
-    const int r = 8 * mt + (lane >> 2);
-    if (r >= M) continue;
+  if constexpr (SELF) {
+    // the warps' shares, added in warp order
+    double* sg = ss + Mc * SW;
 #pragma unroll
     for (int u = 0; u < NT; ++u)
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const int c = 8 * u + 2 * (lane & 3) + j;
-        if (c < P) out[(int64_t)r * P + c] = g[t][u][j];
-      }
+      for (int v = 0; v < NT; ++v)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+          sg[wid * 64 * NT * NT + (8 * u + (lane >> 2)) * 8 * NT + 8 * v + 2 * (lane & 3) + j] = g[u][v][j];
+    __syncthreads();
+    for (int x = threadIdx.x; x < 64 * NT * NT; x += blockDim.x) {
+      const int r = x / (8 * NT), c = x - r * (8 * NT);
+      if (r >= P || c >= P) continue;
+      double t = 0.0;
+      for (int q = 0; q < (int)(blockDim.x >> 5); ++q) t += sg[q * 64 * NT * NT + x];
+      tail.part[(int64_t)blockIdx.x * P * P + r * P + c] = t;
+    }
   }
 }
 
-// SVQB factor of a small Gram matrix on the device (one block of 128 threads), so that a Lanczos
-// step needs no host round trip.  S (nb x nb, column-major, nb <= 16) = W^T W.  With
-// D = diag(S)^(-1/2) (zero for a diagonal at or below 1e-28 of the largest), D S D = U L U^T by
-// cyclic Jacobi in the parallel round-robin order (nb/2 disjoint rotations per round, Golub-Van
-// Loan's symmetric 2 x 2 Schur step; one thread per (rotation, row) update), at most 30 sweeps,
-// stopping when every off-diagonal |a_ij| <= 1e-14 sqrt(a_ii a_jj) among the directions above
-// 1e-12 of the largest (the relative test bounds the orthonormality of W M independently of the
-// block's conditioning); the directions with L > 1e-12 max(L) are kept in descending order and
-// M[:, q] = D U[:, keep_q] / sqrt(L[keep_q]) (columns past the rank are zero).  W M is then
-// orthonormal.  *rank_short is set to 1 when fewer than nb directions are kept.
-constexpr int kSvqbThreads = 128;
-__global__ void __launch_bounds__(kSvqbThreads) k_svqb_factor(const double* __restrict__ S, int nb,
+// Shared memory of k_rows with the fused Gram product.
+template <int NT>
+constexpr size_t rows_self_smem(int M) {
+  return rows_smem<NT>(M) + (size_t)(kThreads / 32) * 64 * NT * NT * sizeof(double);
+}
+
+// Orthonormalisation factor of a block W from its Gram matrix S = W^T W, given as nparts partial sums
+// (nb x nb each, nb <= 16), in one block, so that a Lanczos step needs no host round trip.  With
+// D = diag(S)^(-1/2) and D S D = R^T R (Cholesky), M = D R^(-1): W M is orthonormal to rounding times
+// the conditioning of the scaled block, as for a factor from the eigenvectors of D S D.  A column
+// whose pivot (the squared sine of its angle to the columns before it) is at most 1e-12, or whose
+// diagonal is at most 1e-28 of the largest, is a lost direction: its column of M is zero and
+// *rank_short is set.  One warp holds the matrix, lane = column; bound by the chain of nb square
+// roots and divisions: measured 12 us with the sum of 148 partial products, where a Jacobi
+// eigensolver took 88.
+constexpr int kSvqbThreads = 1024;
+__global__ void __launch_bounds__(kSvqbThreads) k_svqb_factor(const double* __restrict__ part,
+                                                              int nparts, int nb,
                                                               double* __restrict__ M,
                                                               int* __restrict__ rank_short) {
-  __shared__ double A[16][17], U[16][17], d[16], cs[8], sn[8], red[kSvqbThreads / 32];
-  __shared__ int pa[8], pb[8], keep[16];
-  __shared__ int stop, rr;
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  for (int x = tid; x < nb * nb; x += kSvqbThreads) A[x % nb][x / nb] = S[x];
-  __syncthreads();
-  if (tid == 0) {
-    double dmax = 0.0;
-    for (int i = 0; i < nb; ++i) dmax = fmax(dmax, A[i][i]);
-    for (int i = 0; i < nb; ++i) {
-      const double v = A[i][i];
-      d[i] = (v > 1e-28 * dmax && v > 1e-300) ? 1.0 / sqrt(v) : 0.0;
-    }
+  __shared__ double ps[4][256], A[16][17], R[16][17];
+  const int tid = threadIdx.x;
+  {  // four groups of threads add the partial sums q, q + 4, ...; then the groups in order
+    const int x = tid & 255, q0 = tid >> 8;
+    double t = 0.0;
+    if (x < nb * nb)
+#pragma unroll 8
+      for (int q = q0; q < nparts; q += 4) t += part[(int64_t)q * nb * nb + x];
+    ps[q0][x] = t;
   }
   __syncthreads();
-  for (int x = tid; x < 256; x += kSvqbThreads) {
-    const int i = x & 15, j = x >> 4;
-    if (i < nb && j < nb) {
-      A[i][j] *= d[i] * d[j];
-      U[i][j] = i == j ? 1.0 : 0.0;
+  if (tid >= 32) return;
+  for (int x = tid; x < nb * nb; x += 32)
+    A[x / nb][x % nb] = ((ps[0][x] + ps[1][x]) + ps[2][x]) + ps[3][x];
+  __syncwarp();
+  const int c = tid;
+  const bool in = c < nb;
+  const double dc = in ? A[c][c] : 0.0;
+  double dmax = dc;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) dmax = fmax(dmax, __shfl_xor_sync(~0u, dmax, o));
+  const bool live = in && dc > 1e-28 * dmax && dc > 1e-300;
+  const double d = live ? 1.0 / sqrt(dc) : 0.0;
+  // column c of the scaled matrix, from its upper triangle
+  double a[16], r[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const double di = __shfl_sync(~0u, d, i);
+    a[i] = (in && i <= c) ? A[i][c] * di * d : 0.0;
+    r[i] = 0.0;
+  }
+  int lost = in && !live;
+  // right-looking Cholesky: row i of R, then the trailing update of this lane's column
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    if (i < nb) {
+      const double piv = __shfl_sync(~0u, a[i], i);
+      const bool ok = piv > 1e-12;
+      const double inv = ok ? 1.0 / sqrt(piv) : 0.0;
+      if (!ok && c == i) lost = 1;
+      r[i] = (in && c >= i) ? a[i] * inv : 0.0;
+      if (in) R[i][c] = r[i];
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (j > i && j < nb && in && j <= c) a[j] = fma(-R[i][j], r[i], a[j]);
     }
   }
-  __syncthreads();
-  const int N = (nb + 1) & ~1;  // players of the round-robin (one idle index when nb is odd)
-  for (int sweep = 0; sweep < 30; ++sweep) {
-    // relative off-diagonal size over the directions that count
-    double dmx = 0.0;
-    for (int i = 0; i < nb; ++i) dmx = fmax(dmx, A[i][i]);
-    double mr = 0.0;
-    for (int x = tid; x < 256; x += kSvqbThreads) {
-      const int i = x & 15, j = x >> 4;
-      if (i < j && j < nb && A[i][i] > 1e-12 * dmx && A[j][j] > 1e-12 * dmx)
-        mr = fmax(mr, fabs(A[i][j]) / sqrt(A[i][i] * A[j][j]));
-    }
-    for (int o = 16; o > 0; o >>= 1) mr = fmax(mr, __shfl_xor_sync(~0u, mr, o));
-    if (lane == 0) red[wid] = mr;
-    __syncthreads();
-    if (tid == 0) {
-      double m = 0.0;
-      for (int w = 0; w < kSvqbThreads / 32; ++w) m = fmax(m, red[w]);
-      stop = m <= 1e-14 ? 1 : 0;
-    }
-    __syncthreads();
-    if (stop) break;
-    for (int round = 0; round < N - 1; ++round) {
-      if (tid < N / 2) {
-        int a = tid == 0 ? N - 1 : (tid + round) % (N - 1);
-        int b = tid == 0 ? round % (N - 1) : (N - 1 - tid + round) % (N - 1);
-        if (a > b) { const int t = a; a = b; b = t; }
-        double c = 1.0, sg = 0.0;
-        if (b < nb) {
-          const double apq = A[a][b];
-          if (fabs(apq) >= 1e-300) {
-            const double theta = (A[b][b] - A[a][a]) / (2.0 * apq);
-            const double t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-            c = 1.0 / sqrt(t * t + 1.0);
-            sg = t * c;
-          }
-        }
-        pa[tid] = a; pb[tid] = b; cs[tid] = c; sn[tid] = sg;
-      }
-      __syncthreads();
-      const int t = tid >> 4, k = tid & 15;  // rotation t, row / column k
-      const bool on = t < N / 2 && k < nb && pb[t] < nb;
-      if (on) {  // rows a, b
-        const int a = pa[t], b = pb[t];
-        const double ra = A[a][k], rb = A[b][k];
-        A[a][k] = cs[t] * ra - sn[t] * rb;
-        A[b][k] = sn[t] * ra + cs[t] * rb;
-      }
-      __syncthreads();
-      if (on) {  // columns a, b of A and U
-        const int a = pa[t], b = pb[t];
-        const double ca = A[k][a], cb = A[k][b];
-        A[k][a] = cs[t] * ca - sn[t] * cb;
-        A[k][b] = sn[t] * ca + cs[t] * cb;
-        const double ua = U[k][a], ub = U[k][b];
-        U[k][a] = cs[t] * ua - sn[t] * ub;
-        U[k][b] = sn[t] * ua + cs[t] * ub;
-      }
-      __syncthreads();
+  // column c of R^(-1) by back substitution (zero for a lost direction)
+  double x[16];
+#pragma unroll
+  for (int i = 15; i >= 0; --i) {
+    x[i] = 0.0;
+    if (i < nb && in && i <= c) {
+      double t = i == c ? 1.0 : 0.0;
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (j > i && j <= c) t = fma(-R[i][j], x[j], t);
+      const double p = R[i][i];
+      x[i] = p > 0.0 ? t / p : 0.0;
     }
   }
-  if (tid == 0) {
-    // descending eigenvalues above 1e-12 of the largest
-    int ord[16];
-    for (int i = 0; i < nb; ++i) ord[i] = i;
-    for (int i = 1; i < nb; ++i)
-      for (int j = i; j > 0 && A[ord[j]][ord[j]] > A[ord[j - 1]][ord[j - 1]]; --j) {
-        const int t = ord[j]; ord[j] = ord[j - 1]; ord[j - 1] = t;
-      }
-    const double lmax = A[ord[0]][ord[0]];
-    int r = 0;
-    for (int i = 0; i < nb; ++i) {
-      const double l = A[ord[i]][ord[i]];
-      if (l > 1e-12 * lmax && l > 0) keep[r++] = ord[i];
-    }
-    rr = r;
-    if (r < nb) *rank_short = 1;
+  const unsigned some = __ballot_sync(~0u, lost);
+  if (some && tid == 0) *rank_short = 1;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const double di = __shfl_sync(~0u, d, i);
+    if (i < nb && in) M[i + (int64_t)c * nb] = lost ? 0.0 : di * x[i];
   }
-  __syncthreads();
-  for (int x = tid; x < nb * nb; x += kSvqbThreads) {
-    const int i = x % nb, q = x / nb;
-    M[x] = q < rr ? d[i] * U[i][keep[q]] / sqrt(A[keep[q]][keep[q]]) : 0.0;
-  }
+}
+
+__global__ void k_add_cols(const double* __restrict__ src, int lds, int M, int P,
+                           double* __restrict__ dst, int ldd) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= M * P) return;
+  const int c = x / M, a = x - c * M;
+  dst[a + (int64_t)c * ldd] += src[a + (int64_t)c * lds];
 }
 
 // The dynamic shared-memory limits are set once per process to the largest size any launch uses,
@@ -489,24 +390,25 @@ __global__ void __launch_bounds__(kSvqbThreads) k_svqb_factor(const double* __re
 std::once_flag g_attr_once;
 void set_attributes() {
   std::call_once(g_attr_once, [] {
-    cudaFuncSetAttribute(k_rows<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(k_rows<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)rows_smem<1>(kRowsMaxM));
-    cudaFuncSetAttribute(k_rows<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(k_rows<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)rows_smem<2>(kRowsMaxM));
-    cudaFuncSetAttribute(k_rows<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(k_rows<4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)rows_smem<4>(kRowsMaxM4));
-    cudaFuncSetAttribute(k_rows_gram<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)fuse_smem<1>(kFuseMaxM));
-    cudaFuncSetAttribute(k_rows_gram<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)fuse_smem<2>(kFuseMaxM));
+    cudaFuncSetAttribute(k_rows<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)rows_self_smem<1>(kRowsSelfMaxM));
+    cudaFuncSetAttribute(k_rows<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)rows_self_smem<2>(kRowsSelfMaxM));
   });
 }
 
 }  // namespace
 
-void svqb_factor(const double* S, int nb, double* M, int* rank_short, cudaStream_t s) {
+void svqb_factor(const double* part, int nparts, int nb, double* M, int* rank_short,
+                 cudaStream_t s) {
   note_launch();
-  k_svqb_factor<<<1, kSvqbThreads, 0, s>>>(S, nb, M, rank_short);
+  k_svqb_factor<<<1, kSvqbThreads, 0, s>>>(part, nparts, nb, M, rank_short);
 }
 
 int64_t proj_gram_scratch(int M, int P) {
@@ -516,7 +418,8 @@ int64_t proj_gram_scratch(int M, int P) {
 }
 
 bool proj_gram(const double* A, int lda, const double* B, int ldb, int64_t n, int M, int P,
-               double alpha, double beta, double* C, int ldc, double* part, cudaStream_t s) {
+               double alpha, double beta, double* C, int ldc, double* part, cudaStream_t s,
+               double* Acc, int ldacc) {
   if (M <= 0 || P <= 0) return true;
   if (P > 16 || lda < M || ldb < P) return false;
   int nblk = kBlocks;
@@ -546,31 +449,15 @@ bool proj_gram(const double* A, int lda, const double* B, int ldb, int64_t n, in
     }
     note_launch();
     k_gram_reduce<<<(Mc * P + 31) / 32, kRedWarps * 32, 0, s>>>(part, nparts, Mc, P, alpha, beta,
-                                                                 C + a0, ldc);
+                                                                 C + a0, ldc, Acc ? Acc + a0 : nullptr,
+                                                                 ldacc);
   }
   return true;
 }
 
-bool proj_rows_gram(const double* A, int lda, const double* S1, int lds, double* W, int ldw,
-                    int64_t n, int M, int P, double* C, int ldc, double* part, cudaStream_t s) {
-  if (M <= 0 || P <= 0 || n <= 0) return true;
-  if (M > kFuseMaxM || P > 16 || lda < M || ldw < P) return false;
-  set_attributes();
-  int nblk = kBlocks;
-  if (n < (int64_t)nblk * kFuseChunk)
-    nblk = (int)std::max<int64_t>(1, (n + kFuseChunk - 1) / kFuseChunk);
-  note_launch();
-  if (P <= 8)
-    k_rows_gram<1><<<nblk, kThreads, fuse_smem<1>(M), s>>>(A, lda, S1, lds, W, ldw, n, M, P, part);
-  else
-    k_rows_gram<2><<<nblk, kThreads, fuse_smem<2>(M), s>>>(A, lda, S1, lds, W, ldw, n, M, P, part);
-  note_launch();
-  k_gram_reduce<<<(M * P + 31) / 32, kRedWarps * 32, 0, s>>>(part, nblk, M, P, 1.0, 0.0, C, ldc);
-  return true;
-}
-
 void proj_rows(const double* A, int lda, const double* S, int lds, int64_t n, int M, int P,
-               double alpha, double beta, double* Out, int ldo, cudaStream_t s) {
+               double alpha, double beta, double* Out, int ldo, cudaStream_t s, const double* In,
+               int ldi, double* Out2, int ldo2) {
   if (n <= 0 || P <= 0) return;
   set_attributes();
   const int64_t tiles = (n + 7) / 8;
@@ -585,18 +472,47 @@ void proj_rows(const double* A, int lda, const double* S, int lds, int64_t n, in
       const int Mc = std::min(kRowsMaxM, M - a0);
       const double* Sc = S + (int64_t)c0 * lds + a0;
       const double bt = a0 == 0 ? beta : 1.0;
+      const bool last = a0 + kRowsMaxM >= M;
+      const RowsTail t{a0 == 0 && In ? In + c0 : Oc, a0 == 0 && In ? ldi : ldo,
+                       last && Out2 ? Out2 + c0 : nullptr, ldo2, nullptr};
       note_launch();
       if (pc > 16)
-        k_rows<4><<<g, kThreads, rows_smem<4>(std::max(Mc, 1)), s>>>(A + a0, lda, Sc, lds, n,
-                                                                     Mc, pc, alpha, bt, Oc, ldo);
+        k_rows<4, false><<<g, kThreads, rows_smem<4>(std::max(Mc, 1)), s>>>(A + a0, lda, Sc, lds, n, Mc,
+                                                                            pc, alpha, bt, Oc, ldo, t);
       else if (pc <= 8)
-        k_rows<1><<<g, kThreads, rows_smem<1>(std::max(Mc, 1)), s>>>(A + a0, lda, Sc, lds, n,
-                                                                     Mc, pc, alpha, bt, Oc, ldo);
+        k_rows<1, false><<<g, kThreads, rows_smem<1>(std::max(Mc, 1)), s>>>(A + a0, lda, Sc, lds, n, Mc,
+                                                                            pc, alpha, bt, Oc, ldo, t);
       else
-        k_rows<2><<<g, kThreads, rows_smem<2>(std::max(Mc, 1)), s>>>(A + a0, lda, Sc, lds, n,
-                                                                     Mc, pc, alpha, bt, Oc, ldo);
+        k_rows<2, false><<<g, kThreads, rows_smem<2>(std::max(Mc, 1)), s>>>(A + a0, lda, Sc, lds, n, Mc,
+                                                                            pc, alpha, bt, Oc, ldo, t);
     }
   }
+}
+
+int proj_rows_self(const double* A, int lda, const double* S, int lds, int64_t n, int M, int P,
+                   double* W, int ldw, double* part, cudaStream_t s) {
+  if (n <= 0 || P <= 0 || P > 16 || M <= 0 || M > kRowsSelfMaxM) return 0;
+  set_attributes();
+  const int g = (int)std::min<int64_t>(kBlocks, ((n + 7) / 8 + 31) / 32);
+  const RowsTail t{W, ldw, nullptr, 0, part};
+  note_launch();
+  if (P <= 8)
+    k_rows<1, true><<<g, kThreads, rows_self_smem<1>(M), s>>>(A, lda, S, lds, n, M, P, -1.0, 1.0, W, ldw, t);
+  else
+    k_rows<2, true><<<g, kThreads, rows_self_smem<2>(M), s>>>(A, lda, S, lds, n, M, P, -1.0, 1.0, W, ldw, t);
+  return g;
+}
+
+void add_cols(const double* src, int lds, int M, int P, double* dst, int ldd, cudaStream_t s) {
+  if (M <= 0 || P <= 0) return;
+  note_launch();
+  k_add_cols<<<(M * P + 255) / 256, 256, 0, s>>>(src, lds, M, P, dst, ldd);
+}
+
+void gram_sum(const double* part, int nparts, int M, int P, double* C, int ldc, cudaStream_t s) {
+  note_launch();
+  k_gram_reduce<<<(M * P + 31) / 32, kRedWarps * 32, 0, s>>>(part, nparts, M, P, 1.0, 0.0, C, ldc,
+                                                              nullptr, 0);
 }
 
 }  // namespace vhci

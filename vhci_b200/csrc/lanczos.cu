@@ -3,9 +3,10 @@
 // Ham.cpp:347-370), organised for the GPU:
 //   * blocks of b = 16 vectors; the SpMM gathers from a compact n x b copy of the block and
 //     streams the matrix from HBM once per block;
-//   * full reorthogonalisation (classical Gram-Schmidt, two passes) with FP64 tensor-core
-//     projections (k_proj.cu), and the projected matrix T = Q^T H Q formed explicitly from the
-//     stored H Q blocks;
+//   * full reorthogonalisation with FP64 tensor-core projections (k_proj.cu): a first Gram-Schmidt
+//     pass over the columns that the product can couple to (the block itself and the one before; all
+//     of them in the first step after a restart), a second one over the whole basis, and the
+//     projected matrix T = Q^T H Q summed from the coefficients of both;
 //   * Rayleigh-Ritz (cuSOLVER syevd on T) only when the subspace is full; the kk = k + guard
 //     lowest Ritz vectors are kept (thick restart) together with the pending Lanczos block, so the
 //     kept Ritz vectors' residuals lie in the new subspace (Krylov-Schur property);
@@ -84,13 +85,14 @@ void jacobi_eig(int n, std::vector<double> A, std::vector<double>& w, std::vecto
 }
 
 struct LWork {
-  DBuf<double> Q, HQ, T, Yw, theta, Xb, HXb, W, S, M, part, rn2, Xc, gpart, Xg, gtmp;
+  DBuf<double> Q, HQ, T, Yw, theta, Xb, HXb, W, S, M, G, part, rn2, Xc, gpart, Xg, gtmp;
   DBuf<float> Xf, Xgf;  // FP32 copies of the vector block (mixed precision)
   DBuf<int> short_flag;   // set by the device SVQB when a block loses rank
   bool exact = false;   // mixed precision: products with FP64 gathers (the final sweep)
+  bool xc_ready = false;  // Xc already holds the block that the next product multiplies
   void release(cudaStream_t s) {
     Q.release(s); HQ.release(s); T.release(s); Yw.release(s); theta.release(s); Xb.release(s);
-    HXb.release(s); W.release(s); S.release(s); M.release(s); part.release(s); rn2.release(s);
+    HXb.release(s); W.release(s); S.release(s); M.release(s); G.release(s); part.release(s); rn2.release(s);
     Xc.release(s); gpart.release(s); Xg.release(s); gtmp.release(s); Xf.release(s);
     Xgf.release(s); short_flag.release(s);
   }
@@ -99,9 +101,10 @@ struct LWork {
 // Projections over the basis rows, on the FP64 tensor pipe (k_proj.cu).
 // C (M x P, column-major) = alpha A^T B + beta C, A n x M and B n x P row-major.  On a sharded
 // context the n rows are this rank's block and the partial product is summed over the ranks
-// (beta must be 0 there).
+// (beta must be 0 there).  Acc (ldacc), when given, also gets the product added.
 int gemm_gram(vhci_ctx* c, LWork& w, const double* A, int lda, const double* B, int ldb, int64_t n,
-              int M, int P, double alpha, double beta, double* C, int ldc) {
+              int M, int P, double alpha, double beta, double* C, int ldc, double* Acc = nullptr,
+              int ldacc = 0) {
   if (M <= 0 || P <= 0) return VHCI_OK;
   const bool sh = is_sharded(c);
   if (sh && beta != 0.0) return fail(c, VHCI_E_STATE, "accumulating projection on a sharded context");
@@ -113,7 +116,8 @@ int gemm_gram(vhci_ctx* c, LWork& w, const double* A, int lda, const double* B, 
     ldo = M;
   }
   VCK(w.gpart.reserve((size_t)proj_gram_scratch(M, P), c->st));
-  if (!proj_gram(A, lda, B, ldb, n, M, P, alpha, beta, out, ldo, w.gpart.p, c->st))
+  if (!proj_gram(A, lda, B, ldb, n, M, P, alpha, beta, out, ldo, w.gpart.p, c->st, sh ? nullptr : Acc,
+                 ldacc))
     return fail(c, VHCI_E_INPUT, "projection with more than 16 right-hand columns");
   if (sh) {
     VTRY(comm_sum(c, out, (int64_t)M * P));
@@ -132,29 +136,25 @@ int gemm_rows(vhci_ctx* c, const double* A, int lda, const double* S, int lds, i
   return VHCI_OK;
 }
 
-// The second and third Gram-Schmidt passes: W <- W - Q S1, then C = Q^T W (M x P, column-major),
-// fused into one pass over Q's rows when the shapes allow (k_proj.cu), else as two products.
-int gemm_rows_gram(vhci_ctx* c, LWork& w, const double* Q, int ldq, const double* S1, int lds,
-                   int64_t n, int M, int P, double* W, int ldw, double* C, int ldc) {
-  const bool sh = is_sharded(c);
-  double* out = C;
-  int ldo = ldc;
-  if (sh) {
-    VCK(w.gtmp.reserve((size_t)M * P, c->st));
-    out = w.gtmp.p;
-    ldo = M;
-  }
+// The last Gram-Schmidt pass, W <- W - Q S1, with the Gram matrix of the new W (P x P) as *nparts
+// partial sums in w.gpart (one, the sum over the ranks, on a sharded context).
+int gemm_rows_self(vhci_ctx* c, LWork& w, const double* Q, int ldq, const double* S1, int64_t n, int M,
+                   int P, double* W, int ldw, int* nparts) {
   VCK(w.gpart.reserve((size_t)proj_gram_scratch(M, P), c->st));
-  if (proj_rows_gram(Q, ldq, S1, lds, W, ldw, n, M, P, out, ldo, w.gpart.p, c->st)) {
-    if (sh) {
-      VTRY(comm_sum(c, out, (int64_t)M * P));
-      VCK(cudaMemcpy2DAsync(C, ldc * sizeof(double), out, M * sizeof(double),
-                            M * sizeof(double), P, cudaMemcpyDeviceToDevice, c->st));
-    }
-    return VHCI_OK;
+  *nparts = proj_rows_self(Q, ldq, S1, M, n, M, P, W, ldw, w.gpart.p, c->st);
+  const bool fused = *nparts > 0;
+  if (fused && !is_sharded(c)) return VHCI_OK;
+  VCK(w.G.reserve((size_t)P * P, c->st));
+  if (fused) {
+    gram_sum(w.gpart.p, *nparts, P, P, w.G.p, P, c->st);
+    VTRY(comm_sum(c, w.G.p, (int64_t)P * P));
+  } else {
+    VTRY(gemm_rows(c, Q, ldq, S1, M, n, M, P, -1.0, 1.0, W, ldw));
+    VTRY(gemm_gram(c, w, W, ldw, W, ldw, n, P, P, 1.0, 0.0, w.G.p, P));
   }
-  VTRY(gemm_rows(c, Q, ldq, S1, lds, n, M, P, -1.0, 1.0, W, ldw));
-  return gemm_gram(c, w, Q, ldq, W, ldw, n, M, P, 1.0, 0.0, C, ldc);
+  VCK(cudaMemcpyAsync(w.gpart.p, w.G.p, (size_t)P * P * sizeof(double), cudaMemcpyDeviceToDevice, c->st));
+  *nparts = 1;
+  return VHCI_OK;
 }
 
 int syevd_l(vhci_ctx* c, double* A, int m, int lda, double* w) {
@@ -170,6 +170,12 @@ int syevd_l(vhci_ctx* c, double* A, int m, int lda, double* w) {
   VCK(cudaStreamSynchronize(c->st));
   if (info != 0) return fail(c, VHCI_E_NOT_CONVERGED, "projected eigensolve failed");
   return VHCI_OK;
+}
+
+// Mixed precision: FP32 block gathers, FP64 accumulation and diagonal term (needs 16-byte gathers of
+// four columns; other widths and the final sweep gather FP64).
+bool gathers_f32(vhci_ctx* c, const LWork& w, int b) {
+  return c->o.precision == 1 && !w.exact && b % 4 == 0;
 }
 
 // Orthonormalise the nb columns of (B, ld) into (out, ldo) by SVQB with the small Gram matrix
@@ -212,16 +218,20 @@ int svqb_small(vhci_ctx* c, LWork& w, int64_t n, const double* B, int ld, int nb
   return VHCI_OK;
 }
 
-// svqb_small without the host round trip: the factor is formed on the device (svqb_factor) and
-// the block is assumed to keep its full rank nb, so nothing waits for the result; a lost
-// direction sets w.short_flag, which the caller reads at its next synchronisation.
-int svqb_dev(vhci_ctx* c, LWork& w, int64_t n, const double* B, int ld, int nb, double* out,
+// The same without the host round trip, from the block's Gram matrix (nparts partial sums in
+// w.gpart): the factor is formed on the device and the block is assumed to keep its full rank nb, so
+// nothing waits for the result; a lost direction sets w.short_flag, which the caller reads at its
+// next synchronisation.  The new block also goes to w.Xc for the product that follows (unless that
+// one gathers an FP32 copy).
+int svqb_dev(vhci_ctx* c, LWork& w, int64_t n, const double* B, int ld, int nb, int nparts, double* out,
              int ldo) {
-  VCK(w.S.reserve((size_t)nb * nb, c->st));
-  VTRY(gemm_gram(c, w, B, ld, B, ld, (int)n, nb, nb, 1.0, 0.0, w.S.p, nb));
   VCK(w.M.reserve((size_t)nb * nb, c->st));
-  svqb_factor(w.S.p, nb, w.M.p, w.short_flag.p, c->st);
-  return gemm_rows(c, B, ld, w.M.p, nb, (int)n, nb, nb, 1.0, 0.0, out, ldo);
+  svqb_factor(w.gpart.p, nparts, nb, w.M.p, w.short_flag.p, c->st);
+  w.xc_ready = !gathers_f32(c, w, nb);
+  if (w.xc_ready) VCK(w.Xc.reserve((size_t)std::max(n, c->rblk) * nb, c->st));
+  proj_rows(B, ld, w.M.p, nb, n, nb, nb, 1.0, 0.0, out, ldo, c->st, nullptr, 0,
+            w.xc_ready ? w.Xc.p : nullptr, nb);
+  return VHCI_OK;
 }
 
 // Y = H X for a block of the held rows: X is first copied to a compact rows x b buffer so the SpMM
@@ -233,9 +243,7 @@ int apply_h_l(vhci_ctx* c, LWork& w, const double* X, int ldx, int b, double* Y,
   cudaEvent_t e0 = ev_e0e1.a, e1 = ev_e0e1.b;
   const int64_t nl = c->nrow, rb = c->rblk;
   VCK(cudaEventRecord(e0, c->st));
-  // mixed precision: FP32 block gathers, FP64 accumulation and diagonal term (needs 16-byte
-  // gathers of four columns; other widths, the final sweep and column panels gather FP64)
-  const bool f32x = c->o.precision == 1 && !w.exact && b % 4 == 0;
+  const bool f32x = gathers_f32(c, w, b);
   if (f32x) {
     VCK(w.Xf.reserve((size_t)std::max(nl, rb) * b, c->st));
     copy_cols_f32(X, ldx, w.Xf.p, b, nl, b, c->st);
@@ -251,7 +259,7 @@ int apply_h_l(vhci_ctx* c, LWork& w, const double* X, int ldx, int b, double* Y,
       return fail(c, VHCI_E_STATE, "FP32 product with an unaligned block");
   } else {
     VCK(w.Xc.reserve((size_t)std::max(nl, rb) * b, c->st));
-    copy_cols(X, ldx, w.Xc.p, b, nl, b, c->st);
+    if (!w.xc_ready) copy_cols(X, ldx, w.Xc.p, b, nl, b, c->st);
     const double* Xfull = w.Xc.p;
     if (is_sharded(c)) {
       if (nl < rb) fill_zero(w.Xc.p + (size_t)nl * b, (rb - nl) * (int64_t)b, c->st);
@@ -261,6 +269,7 @@ int apply_h_l(vhci_ctx* c, LWork& w, const double* X, int ldx, int b, double* Y,
     }
     spmm_h(c, Xfull, b, b, Y, ldy);
   }
+  w.xc_ready = false;
   VCK(cudaEventRecord(e1, c->st));
   VCK(cudaEventSynchronize(e1));
   VCK(cudaGetLastError());
@@ -361,13 +370,14 @@ static int lanczos_guard(int k) {
 }
 
 // Working set of the block Lanczos over n states for subspace factor `span`, on a rank holding
-// `rows` of them: Q and H Q (rows x ld), the Ritz block and its product (rows x kk), the expansion
-// block and its compact copy (rows x b), and the gathered vector block (n x b), in doubles.
-static double lanczos_bytes(int64_t n, int64_t rows, int k, int span, int b) {
+// `rows` of them, in doubles: Q (rows x ld) and the Ritz block (rows x kk), in mixed precision the
+// products of both too, the pending block, the compact copy and the first pass's block (rows x b),
+// and the gathered vector block (n x b).
+static double lanczos_bytes(int64_t n, int64_t rows, int k, int span, int b, bool mixed) {
   const int kk = (int)std::min<int64_t>(n, k + lanczos_guard(k));
   const int mmax = (int)std::min<int64_t>(n, (int64_t)span * kk + 2 * b);
   const int ld = (mmax + b + 15) / 16 * 16;
-  return 8.0 * (double)rows * (2.0 * ld + 2.0 * kk + 2.0 * b) + (rows < n ? 8.0 * n * b : 0.0);
+  return 8.0 * (double)rows * ((mixed ? 2.0 : 1.0) * (ld + kk) + 3.0 * b) + (rows < n ? 8.0 * n * b : 0.0);
 }
 
 // Working set of the memory-lean variant: Q (n x ld, span 2), the expansion block, its product,
@@ -414,7 +424,7 @@ int block_lanczos_impl(vhci_ctx* c, int k, bool dev_svqb) {
   if (const char* e = std::getenv("VHCI_LANCZOS_LEAN"))
     if (std::atoi(e) == 1) return block_lanczos_lean(c, k);
   if (const char* e = std::getenv("VHCI_LANCZOS_SPAN")) span = std::max(2, std::min(8, std::atoi(e)));
-  if (lanczos_bytes(n, nl, k, span, b) + 1e9 > avail) return block_lanczos_lean(c, k);
+  if (lanczos_bytes(n, nl, k, span, b, c->o.precision == 1) + 1e9 > avail) return block_lanczos_lean(c, k);
   const int mmax = (int)std::min<int64_t>(n, (int64_t)span * kk + 2 * b);
   const bool dev = dev_svqb && n >= 8 * (int64_t)mmax;
   // row stride padded to whole 128-byte lines so every b-column gather touches whole L2 lines
@@ -428,7 +438,7 @@ int block_lanczos_impl(vhci_ctx* c, int k, bool dev_svqb) {
   const int plevel = prof ? std::atoi(prof) : 0;
   LWork w;
   VCK(w.Q.reserve((size_t)nl * ld, s));
-  VCK(w.HQ.reserve((size_t)nl * ld, s));
+  if (mixed) VCK(w.HQ.reserve((size_t)nl * ld, s));  // H Q, rotated for the explicit residuals
   VCK(w.T.reserve((size_t)ld * ld, s));
   VCK(w.Yw.reserve((size_t)ld * ld, s));
   VCK(w.theta.reserve(ld, s));
@@ -488,27 +498,38 @@ int block_lanczos_impl(vhci_ctx* c, int k, bool dev_svqb) {
   for (int cyc = 0; cyc < maxcyc; ++cyc) {
     // ---- expansion
     bool exhausted = (p == 0);
+    int loc = 0;  // first column of the first Gram-Schmidt pass: all after a (re)start
+    int pw = 0;   // columns of the pending block W when the loop ends with one
     while (p > 0) {
       auto t0 = now();
-      VTRY(apply_h_l(c, w, w.Q.p + m, ld, p, w.HQ.p + m, ld));
+      double* HX = mixed ? w.HQ.p + m : w.W.p;
+      const int ldh = mixed ? ld : b;
+      VTRY(apply_h_l(c, w, w.Q.p + m, ld, p, HX, ldh));
       t_spmm += msince(t0);
       t0 = now();
       ++steps;
-      // T[0:m+p, m:m+p] = Q^T (H Q_new)
-      VTRY(gemm_gram(c, w, w.Q.p, ld, w.HQ.p + m, ld, nl, m + p, p, 1.0, 0.0, w.T.p + (size_t)m * ld, ld));
-      m += p;
+      // First pass: W = H Q_new - Q_loc (Q_loc^T H Q_new).  The product of the newest block is
+      // orthogonal to every block but itself and the one before, to rounding (Q^T H Q is block
+      // tridiagonal there), so the other columns are left to the second pass, which reads the whole
+      // basis once for its coefficients S and once for the update.  T's new column is the sum of both
+      // passes' coefficients.
+      double* Tn = w.T.p + (size_t)m * ld;
+      const int mm = m + p;
+      VTRY(gemm_gram(c, w, w.Q.p + loc, ld, HX, ldh, nl, mm - loc, p, 1.0, 0.0, Tn + loc, ld));
+      proj_rows(w.Q.p + loc, ld, Tn + loc, ld, nl, mm - loc, p, -1.0, 1.0, w.W.p, b, s, HX, ldh);
+      VCK(w.S.reserve((size_t)std::max(mm, b) * p, s));
+      VTRY(gemm_gram(c, w, w.Q.p, ld, w.W.p, b, nl, mm, p, 1.0, 0.0, w.S.p, mm, Tn, ld));
+      m = mm;
+      loc = m - p;
       if (m + b > mmax || m >= n) {
+        pw = m < n ? p : 0;
         if (plevel) { cudaStreamSynchronize(s); t_orth += msince(t0); }
         break;
       }
-      // next block: W = H Q_new - Q T[:, new]; second Gram-Schmidt pass; SVQB
-      copy_cols(w.HQ.p + (m - p), ld, w.W.p, b, nl, p, s);
-      VCK(w.S.reserve((size_t)std::max(m, b) * p, s));
-      VTRY(gemm_rows_gram(c, w, w.Q.p, ld, w.T.p + (size_t)(m - p) * ld, ld, nl, m, p, w.W.p, b,
-                          w.S.p, m));
-      VTRY(gemm_rows(c, w.Q.p, ld, w.S.p, m, nl, m, p, -1.0, 1.0, w.W.p, b));
-      int p2 = p;
-      if (dev) VTRY(svqb_dev(c, w, nl, w.W.p, b, p, w.Q.p + m, ld));
+      // the rest of the second pass, and the next block from what is left
+      int nparts = 0, p2 = p;
+      VTRY(gemm_rows_self(c, w, w.Q.p, ld, w.S.p, nl, m, p, w.W.p, b, &nparts));
+      if (dev) VTRY(svqb_dev(c, w, nl, w.W.p, b, p, nparts, w.Q.p + m, ld));
       else VTRY(svqb_small(c, w, nl, w.W.p, b, p, w.Q.p + m, ld, &p2));
       t_orth += msince(t0);
       p = p2;
@@ -535,7 +556,7 @@ int block_lanczos_impl(vhci_ctx* c, int k, bool dev_svqb) {
     const int nk = std::min(kk, m);
     VTRY(gemm_rows(c, w.Q.p, ld, w.Yw.p, ld, nl, m, nk, 1.0, 0.0, w.Xb.p, kk));
     // Residuals from the Krylov relation H Q = Q T + W E_last^T, where W = (I - Q Q^T) H Q_last is
-    // the pending block (formed here; the restart continues from it): the residual of Ritz pair
+    // the pending block (completed here; the restart continues from it): the residual of Ritz pair
     // (theta_j, y_j) is W y_j[last block rows], so ||r_j||^2 = y_last^T (W^T W) y_last.  With the
     // full (two-pass) orthogonalisation the relation holds to rounding, far below the tolerance.
     // The whole space (m = n) or an invariant subspace (exhausted) leaves no residual.
@@ -543,9 +564,10 @@ int block_lanczos_impl(vhci_ctx* c, int k, bool dev_svqb) {
     // its FP32-gather products carry rounding noise of about 1e-8 relative, and the Krylov relation
     // (exact for the products as computed within one cycle) does not carry that noise across the
     // restarts' coupling terms, so it can stall at the 1e-7 tolerance.
-    const int pw = (!exhausted && m < n && !mixed) ? p : 0;
     std::fill(rn.begin(), rn.end(), 0.0);
     VCK(d2h(c, th.data(), w.theta.p, nk * sizeof(double)));
+    int nparts = 0;  // W's Gram matrix, for the residuals and for the block that continues from it
+    if (pw > 0) VTRY(gemm_rows_self(c, w, w.Q.p, ld, w.S.p, nl, m, pw, w.W.p, b, &nparts));
     if (mixed) {
       VTRY(gemm_rows(c, w.HQ.p, ld, w.Yw.p, ld, nl, m, nk, 1.0, 0.0, w.HXb.p, kk));
       residual_norms(w.Xb.p, w.HXb.p, nl, kk, nk, w.theta.p, w.part.p, nblk, w.rn2.p, s);
@@ -553,15 +575,10 @@ int block_lanczos_impl(vhci_ctx* c, int k, bool dev_svqb) {
       VCK(d2h(c, rn.data(), w.rn2.p, nk * sizeof(double)));
       VCK(cudaStreamSynchronize(s));
     } else if (pw > 0) {
-      copy_cols(w.HQ.p + (m - pw), ld, w.W.p, b, nl, pw, s);
-      VCK(w.S.reserve((size_t)std::max(m, b) * pw, s));
-      VTRY(gemm_rows_gram(c, w, w.Q.p, ld, w.T.p + (size_t)(m - pw) * ld, ld, nl, m, pw, w.W.p, b,
-                          w.S.p, m));
-      VTRY(gemm_rows(c, w.Q.p, ld, w.S.p, m, nl, m, pw, -1.0, 1.0, w.W.p, b));
-      VCK(w.M.reserve((size_t)pw * pw, s));
-      VTRY(gemm_gram(c, w, w.W.p, b, w.W.p, b, nl, pw, pw, 1.0, 0.0, w.M.p, pw));
+      VCK(w.G.reserve((size_t)pw * pw, s));
+      gram_sum(w.gpart.p, nparts, pw, pw, w.G.p, pw, s);
       std::vector<double> G((size_t)pw * pw), Yl((size_t)pw * nk);
-      VCK(d2h(c, G.data(), w.M.p, G.size() * sizeof(double)));
+      VCK(d2h(c, G.data(), w.G.p, G.size() * sizeof(double)));
       VCK(cudaMemcpy2DAsync(Yl.data(), pw * sizeof(double), w.Yw.p + (m - pw), ld * sizeof(double),
                             pw * sizeof(double), nk, cudaMemcpyDeviceToHost, s));
       VCK(cudaStreamSynchronize(s));
@@ -615,20 +632,13 @@ int block_lanczos_impl(vhci_ctx* c, int k, bool dev_svqb) {
       w.release(s);
       return VHCI_OK;
     }
-    // ---- thick restart: keep the Ritz block, continue from the pending block W (formed above
-    // with the residuals, or here in mixed precision, whose rotated products are kept with it)
+    // ---- thick restart: keep the Ritz block (in mixed precision its rotated products too), continue
+    // from the pending block W formed above
     t0 = now();
-    if (mixed) {
-      copy_cols(w.HQ.p + (m - p), ld, w.W.p, b, nl, p, s);
-      VCK(w.S.reserve((size_t)std::max(m, b) * p, s));
-      VTRY(gemm_rows_gram(c, w, w.Q.p, ld, w.T.p + (size_t)(m - p) * ld, ld, nl, m, p, w.W.p, b,
-                          w.S.p, m));
-      VTRY(gemm_rows(c, w.Q.p, ld, w.S.p, m, nl, m, p, -1.0, 1.0, w.W.p, b));
-      copy_cols(w.HXb.p, kk, w.HQ.p, ld, nl, nk, s);
-    }
+    if (mixed) copy_cols(w.HXb.p, kk, w.HQ.p, ld, nl, nk, s);
     copy_cols(w.Xb.p, kk, w.Q.p, ld, nl, nk, s);
     int p2 = p;
-    if (dev) VTRY(svqb_dev(c, w, nl, w.W.p, b, p, w.Q.p + nk, ld));
+    if (dev) VTRY(svqb_dev(c, w, nl, w.W.p, b, p, nparts, w.Q.p + nk, ld));
     else VTRY(svqb_small(c, w, nl, w.W.p, b, p, w.Q.p + nk, ld, &p2));
     std::vector<double> Th((size_t)ld * nk, 0.0);
     for (int j = 0; j < nk; ++j) Th[(size_t)j * ld + j] = th[j];
@@ -755,17 +765,19 @@ int block_lanczos_lean(vhci_ctx* c, int k) {
   for (int cyc = 0; cyc < maxcyc; ++cyc) {
     bool exhausted = false;
     int plast = 0;  // width of the block whose product formed the pending W
+    int loc = 0;    // first column of the first Gram-Schmidt pass
     while (true) {
       VTRY(apply_h_l(c, w, w.Q.p + m, ld, p, w.HQ.p, b));
       ++steps;
-      VTRY(gemm_gram(c, w, w.Q.p, ld, w.HQ.p, b, nl, m + p, p, 1.0, 0.0, w.T.p + (size_t)m * ld, ld));
+      // pending block W = H Q_new - Q T[:, new] in two Gram-Schmidt passes, as in block_lanczos
+      double* Tn = w.T.p + (size_t)m * ld;
+      VTRY(gemm_gram(c, w, w.Q.p + loc, ld, w.HQ.p, b, nl, m + p - loc, p, 1.0, 0.0, Tn + loc, ld));
+      proj_rows(w.Q.p + loc, ld, Tn + loc, ld, nl, m + p - loc, p, -1.0, 1.0, w.W.p, b, s, w.HQ.p, b);
       m += p;
       plast = p;
-      // pending block W = H Q_new - Q T[:, new], second Gram-Schmidt pass
-      VCK(cudaMemcpyAsync(w.W.p, w.HQ.p, (size_t)nl * b * sizeof(double), cudaMemcpyDeviceToDevice, s));
+      loc = m - p;
       VCK(w.S.reserve((size_t)m * p, s));
-      VTRY(gemm_rows_gram(c, w, w.Q.p, ld, w.T.p + (size_t)(m - p) * ld, ld, nl, m, p, w.W.p, b,
-                          w.S.p, m));
+      VTRY(gemm_gram(c, w, w.Q.p, ld, w.W.p, b, nl, m, p, 1.0, 0.0, w.S.p, m, Tn, ld));
       VTRY(gemm_rows(c, w.Q.p, ld, w.S.p, m, nl, m, p, -1.0, 1.0, w.W.p, b));
       if (m + b > mmax || m >= n) break;
       int p2 = 0;

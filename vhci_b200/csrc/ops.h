@@ -195,23 +195,31 @@ void fill_zero(double* p, int64_t n, cudaStream_t s);
 
 // ---- FP64 tensor-core projections (k_proj.cu) ----
 // C (M x P, column-major, ldc) = alpha A^T B + beta C with A n x M and B n x P row-major (lda,
-// ldb); any M (slabs of 1024), P <= 16; part holds proj_gram_scratch(M, P) doubles.  Returns
-// false (nothing launched) for P > 16 or strides shorter than the rows.
+// ldb); any M (slabs of 768), P <= 16; part holds proj_gram_scratch(M, P) doubles.  Acc (ldacc), when
+// given, also gets C added.  Returns false (nothing launched) for P > 16 or strides shorter than the
+// rows.
 int64_t proj_gram_scratch(int M, int P);
 bool proj_gram(const double* A, int lda, const double* B, int ldb, int64_t n, int M, int P,
-               double alpha, double beta, double* C, int ldc, double* part, cudaStream_t s);
-// Out (n x P row-major, ldo) = alpha A S + beta Out with A n x M row-major and S M x P
-// column-major (lds); any P (column chunks of 64).
+               double alpha, double beta, double* C, int ldc, double* part, cudaStream_t s,
+               double* Acc = nullptr, int ldacc = 0);
+// Out (n x P row-major, ldo) = alpha A S + beta In (In = Out unless given) with A n x M row-major and
+// S M x P column-major (lds); any P (column slabs of 16 or 32).  Out2 (ldo2), when given, gets a
+// copy.
 void proj_rows(const double* A, int lda, const double* S, int lds, int64_t n, int M, int P,
-               double alpha, double beta, double* Out, int ldo, cudaStream_t s);
-// W <- W - A S1, then C (M x P, column-major) = A^T W, in one pass over A; M <= 768, P <= 16
-// (false, nothing launched, otherwise); part holds proj_gram_scratch(M, P) doubles.
-bool proj_rows_gram(const double* A, int lda, const double* S1, int lds, double* W, int ldw,
-                    int64_t n, int M, int P, double* C, int ldc, double* part, cudaStream_t s);
-// SVQB factor M (nb x nb, column-major) of the Gram matrix S = W^T W (nb <= 16) on the device:
-// W M is orthonormal over the directions above 1e-12 of the largest, further columns of M are
-// zero and *rank_short is set to 1 when there are any.
-void svqb_factor(const double* S, int nb, double* M, int* rank_short, cudaStream_t s);
+               double alpha, double beta, double* Out, int ldo, cudaStream_t s,
+               const double* In = nullptr, int ldi = 0, double* Out2 = nullptr, int ldo2 = 0);
+// W <- W - A S with the partial sums of W^T W (P x P each) of the new W in part; returns how many
+// partial sums there are, 0 (nothing launched) for P > 16 or M > 960.
+int proj_rows_self(const double* A, int lda, const double* S, int lds, int64_t n, int M, int P,
+                   double* W, int ldw, double* part, cudaStream_t s);
+// C (M x P, column-major) = the sum of nparts partial sums (M x P a-major each).
+void gram_sum(const double* part, int nparts, int M, int P, double* C, int ldc, cudaStream_t s);
+// dst (M x P, column-major, ldd) += src (lds)
+void add_cols(const double* src, int lds, int M, int P, double* dst, int ldd, cudaStream_t s);
+// Factor M (nb x nb, column-major) of the Gram matrix W^T W (the sum of nparts partial sums, nb x nb,
+// nb <= 16) on the device: W M is orthonormal; the column of a lost direction is zero, and
+// *rank_short is set to 1 when there are any.
+void svqb_factor(const double* part, int nparts, int nb, double* M, int* rank_short, cudaStream_t s);
 
 // ---- PT2 (k_pt2.cu) ----
 void pt2_count(const uint64_t* keys, int64_t n, KeyLayout L, HashView pert, ConnDev cd,
