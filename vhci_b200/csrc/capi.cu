@@ -387,6 +387,21 @@ double device_available(vhci_ctx* c) {
   return avail;
 }
 
+// Whether `need` bytes can be allocated.  The driver's free-memory query usually takes 65 us and at
+// times several ms, so it is asked last: not when the pool's idle reserve covers the need, and not
+// for less than 1/64 of the device, where the callers leave a shortage to the allocation itself.
+bool device_fits(vhci_ctx* c, double need) {
+  if (need <= c->dev_bytes / 64) return true;
+  cudaMemPool_t pool;
+  uint64_t reserved = 0, used = 0;
+  if (cudaDeviceGetDefaultMemPool(&pool, c->o.device) == cudaSuccess &&
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess &&
+      reserved > used && need <= (double)(reserved - used))
+    return true;
+  return need <= device_available(c);
+}
+
 void spmm_h(vhci_ctx* c, const double* X, int ldx, int b, double* Y, int ldy) {
   const bool f = c->o.precision == 1;
   if (c->npanel > 0)
@@ -628,29 +643,39 @@ static int build_h_incremental(vhci_ctx* c) {
                       (double)n * 40.0 + 8.0 * radix_hist_elems(nnz_new);
   const double eig = lanczos_min_bytes(c, c->M.nstate);
   const double old_bytes = (double)c->nnz * (4.0 + vb) + 16.0 * (double)n_old;
-  // the kept connections give way when the matrix needs their room
-  double avail = device_available(c);
-  auto fits = [&] { return need <= 0.9 * avail && nnz_all_max * (4.0 + vb) + eig <= avail + old_bytes; };
-  if (nbatch > 0 && !fits()) {
-    avail += 264.0 * (double)stage.view.cap;
+  const double room = std::max(need / 0.9, nnz_all_max * (4.0 + vb) + eig - old_bytes);
+  bool fits = device_fits(c, room);
+  if (!fits && nbatch > 0) {  // the kept connections give way when the matrix needs their room
     stage.release(s);
     nbatch = 0;
+    fits = device_fits(c, room);
   }
-  if (nnz_new >= 0xFFFFFFFFll || !fits()) {
+  if (nnz_new >= 0xFFFFFFFFll || !fits) {
     release_all();
     return 1;
   }
-  VCK(tcol.reserve(std::max<int64_t>(nnz_new, 1), s));
-  if (f) VCK(tvalf.reserve(std::max<int64_t>(nnz_new, 1), s));
-  else VCK(tval.reserve(std::max<int64_t>(nnz_new, 1), s));
-  VCK(tdiag.reserve(nn, s));
+  // a buffer that cannot be had after all: also left to the build from scratch
+#define VHCI_INC(call)                              \
+  do {                                              \
+    const cudaError_t e_ = (call);                  \
+    if (e_ == cudaErrorMemoryAllocation) {          \
+      cudaGetLastError();                           \
+      release_all();                                \
+      return 1;                                     \
+    }                                               \
+    if (e_ != cudaSuccess) return cuda_fail(c, e_, #call); \
+  } while (0)
+  VHCI_INC(tcol.reserve(std::max<int64_t>(nnz_new, 1), s));
+  if (f) VHCI_INC(tvalf.reserve(std::max<int64_t>(nnz_new, 1), s));
+  else VHCI_INC(tval.reserve(std::max<int64_t>(nnz_new, 1), s));
+  VHCI_INC(tdiag.reserve(nn, s));
   fill_rows(c, stage, nbatch, n_old, nn, rp_new.p, tcol.p, f ? nullptr : tval.p,
             f ? tvalf.p : nullptr, tdiag.p);
   // transposed entries: per old column counts and (column, entry) keys, sorted
-  VCK(add.reserve(n_old, s));
+  VHCI_INC(add.reserve(n_old, s));
   VCK(cudaMemsetAsync(add.p, 0, n_old * sizeof(int32_t), s));
-  VCK(keys.reserve(std::max<int64_t>(nnz_new, 1), s));
-  VCK(kc.reserve(1, s));
+  VHCI_INC(keys.reserve(std::max<int64_t>(nnz_new, 1), s));
+  VHCI_INC(kc.reserve(1, s));
   VCK(cudaMemsetAsync(kc.p, 0, sizeof(unsigned long long), s));
   hmerge_cross_keys(tcol.p, nnz_new, n_old, add.p, keys.p, kc.p, s);
   unsigned long long ncross_u = 0;
@@ -660,24 +685,24 @@ static int build_h_incremental(vhci_ctx* c) {
   if (ncross > 0) {
     int cbits = 1;
     while (cbits < 32 && ((int64_t)1 << cbits) < n_old) ++cbits;
-    VCK(alt.reserve(ncross, s));
-    VCK(hist.reserve(std::max<int64_t>(radix_hist_elems(ncross), 1), s));
+    VHCI_INC(alt.reserve(ncross, s));
+    VHCI_INC(hist.reserve(std::max<int64_t>(radix_hist_elems(ncross), 1), s));
     radix_sort_keys(keys.p, alt.p, ncross, 1, 32 + cbits, hist.p, s);
   }
-  VCK(xoff.reserve(n_old + 1, s));
+  VHCI_INC(xoff.reserve(n_old + 1, s));
   exclusive_scan_i32(add.p, xoff.p, n_old, c->scan_tmp.p, s);
-  VCK(erow.reserve(std::max<int64_t>(nnz_new, 1), s));
+  VHCI_INC(erow.reserve(std::max<int64_t>(nnz_new, 1), s));
   hmerge_entry_rows(rp_new.p, nn, erow.p, s);
   // merged row pointers and arrays
-  VCK(len.reserve(n, s));
+  VHCI_INC(len.reserve(n, s));
   hmerge_lengths(c->rowptr.p, add.p, rp_new.p, n_old, nn, len.p, s);
-  VCK(rp_all.reserve(n + 1, s));
+  VHCI_INC(rp_all.reserve(n + 1, s));
   exclusive_scan_i32(len.p, rp_all.p, n, c->scan_tmp.p, s);
   const int64_t nnz_all = c->nnz + nnz_new + ncross;
-  VCK(col_all.reserve(std::max<int64_t>(nnz_all, 1), s));
-  if (f) VCK(valf_all.reserve(std::max<int64_t>(nnz_all, 1), s));
-  else VCK(val_all.reserve(std::max<int64_t>(nnz_all, 1), s));
-  VCK(diag_all.reserve(n, s));
+  VHCI_INC(col_all.reserve(std::max<int64_t>(nnz_all, 1), s));
+  if (f) VHCI_INC(valf_all.reserve(std::max<int64_t>(nnz_all, 1), s));
+  else VHCI_INC(val_all.reserve(std::max<int64_t>(nnz_all, 1), s));
+  VHCI_INC(diag_all.reserve(n, s));
   hmerge_copy_rows(c->rowptr.p, c->col.p, f ? nullptr : c->val.p, f ? c->valf.p : nullptr, n_old,
                    rp_all.p, col_all.p, val_all.p, valf_all.p, s);
   hmerge_copy_rows(rp_new.p, tcol.p, f ? nullptr : tval.p, f ? tvalf.p : nullptr, nn,
@@ -687,6 +712,7 @@ static int build_h_incremental(vhci_ctx* c) {
                        valf_all.p, s);
   VCK(cudaMemcpyAsync(diag_all.p, c->diag.p, n_old * sizeof(double), cudaMemcpyDeviceToDevice, s));
   VCK(cudaMemcpyAsync(diag_all.p + n_old, tdiag.p, nn * sizeof(double), cudaMemcpyDeviceToDevice, s));
+  #undef VHCI_INC
   // the merged matrix replaces the stored one (the old arrays leave with the temporaries)
   std::swap(c->rowptr.p, rp_all.p); std::swap(c->rowptr.cap, rp_all.cap);
   std::swap(c->col.p, col_all.p); std::swap(c->col.cap, col_all.cap);
@@ -748,15 +774,16 @@ int build_h(vhci_ctx* c, bool all_rows) {
   if ((int64_t)c->valf.cap < nnz) c->valf.release(c->st);
   {  // admission: the matrix and the eigensolver's smallest working set must fit together
     const double hbytes = (double)nnz * (4.0 + (c->o.precision == 1 ? 4.0 : 8.0)) + 8.0 * nr;
-    double avail = device_available(c) + 8.0 * (double)c->x_rows * c->ldx;
-    const double eig = lanczos_min_bytes(c, c->M.nstate);
-    if (nbatch > 0 && hbytes + eig > avail) {  // the kept connections give way
-      avail += 264.0 * (double)stage.view.cap;
+    const double xb = 8.0 * (double)c->x_rows * c->ldx, eig = lanczos_min_bytes(c, c->M.nstate);
+    bool fits = device_fits(c, hbytes + eig - xb);
+    if (!fits && nbatch > 0) {  // the kept connections give way
       stage.release(c->st);
       nbatch = 0;
+      fits = device_fits(c, hbytes + eig - xb);
     }
-    if (hbytes + eig > avail) {
+    if (!fits) {
       stage.release(c->st);
+      const double avail = device_available(c) + xb;
       char msg[320];
       std::snprintf(msg, sizeof msg,
                     "Hamiltonian rows of %lld states and %lld off-diagonal entries need %.1f GB "

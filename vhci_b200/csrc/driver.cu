@@ -75,50 +75,59 @@ int pt2(vhci_ctx* c, double eps2, double* dE_out, int64_t* n_pert) {
       nbatch = 0;
     }
     c->stats.pt2_entries += total;
-    // chunk the perturber range so one chunk's entries fit the budget
-    // entries (12 bytes) plus, in the worst case, the same again as scratch for long-row ordering
-    auto chunk_budget = [&] {
-      const int64_t e = c->o.pt2_chunk > 0 ? c->o.pt2_chunk : (int64_t)(device_available(c) * 0.4 / 12.0);
-      return std::max<int64_t>(e, 1 << 20);
-    };
-    int64_t budget = chunk_budget();
-    if (nbatch > 0 && total > budget && c->o.pt2_chunk <= 0) {  // the kept connections give way
-      stage.release(s);
-      nbatch = 0;
-      budget = chunk_budget();
-    }
+    // chunk the perturber range so one chunk's entries fit the budget: 12 bytes each plus, in the worst
+    // case, the same again as scratch for long-row ordering, in 40 % of the memory to be had
+    DBuf<int32_t> ecol;
+    DBuf<double> eval, part, dEd, Ed, ediag;
+    std::vector<int64_t> bounds, arow_h;
     // chunk bounds in perturber indices (arow_h is indexed from A0); one chunk needs only the total,
     // several the host copy of the row offsets
-    std::vector<int64_t> bounds{A0};
-    std::vector<int64_t> arow_h;
-    if (total <= budget) {
-      bounds.push_back(A1);
-    } else {
-      arow_h.resize(NA + 1);
-      VCK(d2h(c, arow_h.data(), arow.p, (NA + 1) * sizeof(int64_t)));
-      VCK(cudaStreamSynchronize(s));
-    }
     auto chunk_entries = [&](int64_t a0, int64_t a1) {
       return arow_h.empty() ? total : arow_h[a1 - A0] - arow_h[a0 - A0];
     };
-    while (bounds.back() < A1) {
-      const int64_t a0 = bounds.back();
-      const int64_t lim = arow_h[a0 - A0] + budget;
-      int64_t a1 = A0 + (std::upper_bound(arow_h.begin() + (a0 - A0) + 1, arow_h.end(), lim) -
-                         arow_h.begin()) - 1;
-      if (a1 <= a0) a1 = a0 + 1;
-      bounds.push_back(std::min(a1, A1));
-    }
-    DBuf<int32_t> ecol;
-    DBuf<double> eval, part, dEd, Ed, ediag;
-    const int64_t maxchunk = [&] {
-      int64_t mx = 0;
+    bool whole = c->o.pt2_chunk <= 0 && device_fits(c, (double)total * 30.0);
+    for (;;) {
+      bounds.assign(1, A0);
+      if (!whole) {
+        auto chunk_budget = [&] {
+          const int64_t e = c->o.pt2_chunk > 0 ? c->o.pt2_chunk : (int64_t)(device_available(c) * 0.4 / 12.0);
+          return std::max<int64_t>(e, 1 << 20);
+        };
+        int64_t budget = chunk_budget();
+        if (nbatch > 0 && total > budget && c->o.pt2_chunk <= 0) {  // the kept connections give way
+          stage.release(s);
+          nbatch = 0;
+          budget = chunk_budget();
+        }
+        if (total > budget) {
+          arow_h.resize(NA + 1);
+          VCK(d2h(c, arow_h.data(), arow.p, (NA + 1) * sizeof(int64_t)));
+          VCK(cudaStreamSynchronize(s));
+          while (bounds.back() < A1) {
+            const int64_t a0 = bounds.back();
+            const int64_t lim = arow_h[a0 - A0] + budget;
+            int64_t a1 = A0 + (std::upper_bound(arow_h.begin() + (a0 - A0) + 1, arow_h.end(), lim) -
+                               arow_h.begin()) - 1;
+            if (a1 <= a0) a1 = a0 + 1;
+            bounds.push_back(std::min(a1, A1));
+          }
+        }
+      }
+      if (arow_h.empty()) bounds.push_back(A1);
+      int64_t maxchunk = 1;
       for (size_t q = 1; q < bounds.size(); ++q)
-        mx = std::max(mx, chunk_entries(bounds[q - 1], bounds[q]));
-      return mx;
-    }();
-    VCK(ecol.reserve(std::max<int64_t>(maxchunk, 1), s));
-    VCK(eval.reserve(std::max<int64_t>(maxchunk, 1), s));
+        maxchunk = std::max(maxchunk, chunk_entries(bounds[q - 1], bounds[q]));
+      cudaError_t e = ecol.reserve(maxchunk, s);
+      if (e == cudaSuccess) e = eval.reserve(maxchunk, s);
+      if (e == cudaErrorMemoryAllocation && whole) {  // not to be had in one: by the budget
+        cudaGetLastError();
+        ecol.release(s);
+        whole = false;
+        continue;
+      }
+      VCK(e);
+      break;
+    }
     const int nblk = pt2_en_blocks();
     VCK(part.reserve((size_t)nblk * nopt, s));
     VCK(cudaMemsetAsync(part.p, 0, (size_t)nblk * nopt * sizeof(double), s));

@@ -94,6 +94,7 @@ int structural_count(vhci_ctx* c, int64_t* out);
 void spmm_h(vhci_ctx* c, const double* X, int ldx, int b, double* Y, int ldy);
 // Device memory a new allocation can use: free memory plus the pool's idle reserve.
 double device_available(vhci_ctx* c);
+bool device_fits(vhci_ctx* c, double need);
 // Device bytes the block Lanczos needs for k eigenpairs on the current basis with its smallest
 // subspace (span 2).
 double lanczos_min_bytes(vhci_ctx* c, int k);

@@ -84,7 +84,36 @@ void jacobi_eig(int n, std::vector<double> A, std::vector<double>& w, std::vecto
   V.swap(V2);
 }
 
+// Device times of the products, read when the stream has been synchronised anyway.
+struct ProductTimes {
+  std::vector<cudaEvent_t> ev;
+  size_t used = 0;
+  cudaError_t record(cudaStream_t s) {
+    if (used == ev.size()) {
+      cudaEvent_t e = nullptr;
+      const cudaError_t r = cudaEventCreate(&e);
+      if (r != cudaSuccess) return r;
+      ev.push_back(e);
+    }
+    return cudaEventRecord(ev[used++], s);
+  }
+  // adds the recorded pairs' times (after a synchronisation) and forgets them
+  double collect() {
+    double sum = 0.0;
+    for (size_t i = 0; i + 1 < used; i += 2) {
+      float ms = 0.f;
+      if (cudaEventElapsedTime(&ms, ev[i], ev[i + 1]) == cudaSuccess) sum += ms;
+    }
+    used = 0;
+    return sum;
+  }
+  ~ProductTimes() {
+    for (cudaEvent_t e : ev) cudaEventDestroy(e);
+  }
+};
+
 struct LWork {
+  ProductTimes times;
   DBuf<double> Q, HQ, T, Yw, theta, Xb, HXb, W, S, M, G, part, rn2, Xc, gpart, Xg, gtmp;
   DBuf<float> Xf, Xgf;  // FP32 copies of the vector block (mixed precision)
   DBuf<int> short_flag;   // set by the device SVQB when a block loses rank
@@ -157,7 +186,7 @@ int gemm_rows_self(vhci_ctx* c, LWork& w, const double* Q, int ldq, const double
   return VHCI_OK;
 }
 
-int syevd_l(vhci_ctx* c, double* A, int m, int lda, double* w) {
+int syevd_l(vhci_ctx* c, LWork& wk, double* A, int m, int lda, double* w) {
   int lwork = 0;
   VBL(cusolverDnDsyevd_bufferSize(c->sol, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_UPPER, m, A,
                                   lda, w, &lwork));
@@ -168,6 +197,7 @@ int syevd_l(vhci_ctx* c, double* A, int m, int lda, double* w) {
   int info = 0;
   VCK(d2h(c, &info, c->solver_info.p, sizeof(int)));
   VCK(cudaStreamSynchronize(c->st));
+  c->stats.ms_spmm += wk.times.collect();
   if (info != 0) return fail(c, VHCI_E_NOT_CONVERGED, "projected eigensolve failed");
   return VHCI_OK;
 }
@@ -238,11 +268,8 @@ int svqb_dev(vhci_ctx* c, LWork& w, int64_t n, const double* B, int ld, int nb, 
 // gathers from a small, L2-resident array instead of rows of the wide basis; on a sharded context
 // the ranks' compact blocks (rblk rows each) are all-gathered into the whole vector block first.
 int apply_h_l(vhci_ctx* c, LWork& w, const double* X, int ldx, int b, double* Y, int ldy) {
-  EventPair ev_e0e1;
-  VCK(ev_e0e1.create());
-  cudaEvent_t e0 = ev_e0e1.a, e1 = ev_e0e1.b;
   const int64_t nl = c->nrow, rb = c->rblk;
-  VCK(cudaEventRecord(e0, c->st));
+  VCK(w.times.record(c->st));
   const bool f32x = gathers_f32(c, w, b);
   if (f32x) {
     VCK(w.Xf.reserve((size_t)std::max(nl, rb) * b, c->st));
@@ -270,12 +297,8 @@ int apply_h_l(vhci_ctx* c, LWork& w, const double* X, int ldx, int b, double* Y,
     spmm_h(c, Xfull, b, b, Y, ldy);
   }
   w.xc_ready = false;
-  VCK(cudaEventRecord(e1, c->st));
-  VCK(cudaEventSynchronize(e1));
+  VCK(w.times.record(c->st));
   VCK(cudaGetLastError());
-  float ms = 0.f;
-  cudaEventElapsedTime(&ms, e0, e1);
-  c->stats.ms_spmm += ms;
   c->stats.spmm_calls += 1;
   c->stats.spmm_cols += b;
   const int64_t sval = c->o.precision == 1 ? 4 : 8;
@@ -307,7 +330,7 @@ int fp64_sweep(vhci_ctx* c, LWork& w, int kk, int nk, int keff, int ld, std::vec
   }
   VCK(cudaMemcpy2DAsync(w.Yw.p, ld * sizeof(double), w.T.p, ld * sizeof(double),
                         nk * sizeof(double), nk, cudaMemcpyDeviceToDevice, s));
-  VTRY(syevd_l(c, w.Yw.p, nk, ld, w.theta.p));
+  VTRY(syevd_l(c, w, w.Yw.p, nk, ld, w.theta.p));
   VTRY(comm_bcast0(c, w.Yw.p, (int64_t)ld * nk));
   VTRY(comm_bcast0(c, w.theta.p, nk));
   VTRY(gemm_rows(c, w.Xb.p, kk, w.Yw.p, ld, nl, nk, nk, 1.0, 0.0, w.Q.p, ld));
@@ -420,11 +443,11 @@ int block_lanczos_impl(vhci_ctx* c, int k, bool dev_svqb) {
   // subspace size: 2 kk + 2 b (VHCI_LANCZOS_SPAN overrides the factor 2); a basis too large for
   // that working set in the free device memory runs the memory-lean variant
   int span = 2;
-  const double avail = device_available(c);
   if (const char* e = std::getenv("VHCI_LANCZOS_LEAN"))
     if (std::atoi(e) == 1) return block_lanczos_lean(c, k);
   if (const char* e = std::getenv("VHCI_LANCZOS_SPAN")) span = std::max(2, std::min(8, std::atoi(e)));
-  if (lanczos_bytes(n, nl, k, span, b, c->o.precision == 1) + 1e9 > avail) return block_lanczos_lean(c, k);
+  if (!device_fits(c, lanczos_bytes(n, nl, k, span, b, c->o.precision == 1) + 1e9))
+    return block_lanczos_lean(c, k);
   const int mmax = (int)std::min<int64_t>(n, (int64_t)span * kk + 2 * b);
   const bool dev = dev_svqb && n >= 8 * (int64_t)mmax;
   // row stride padded to whole 128-byte lines so every b-column gather touches whole L2 lines
@@ -437,17 +460,26 @@ int block_lanczos_impl(vhci_ctx* c, int k, bool dev_svqb) {
   const char* prof = std::getenv("VHCI_PROFILE");
   const int plevel = prof ? std::atoi(prof) : 0;
   LWork w;
-  VCK(w.Q.reserve((size_t)nl * ld, s));
-  if (mixed) VCK(w.HQ.reserve((size_t)nl * ld, s));  // H Q, rotated for the explicit residuals
-  VCK(w.T.reserve((size_t)ld * ld, s));
-  VCK(w.Yw.reserve((size_t)ld * ld, s));
-  VCK(w.theta.reserve(ld, s));
-  VCK(w.Xb.reserve((size_t)rb * kk, s));  // rblk rows: the block each rank gathers at the end
-  if (mixed) VCK(w.HXb.reserve((size_t)nl * kk, s));  // the final FP64 sweep's products
-  VCK(w.W.reserve((size_t)nl * b, s));
   const int nblk = residual_blocks(nl);
-  VCK(w.part.reserve((size_t)nblk * kk, s));
-  VCK(w.rn2.reserve(kk, s));
+  auto reserve_all = [&]() -> cudaError_t {
+    cudaError_t e = w.Q.reserve((size_t)nl * ld, s);
+    if (!e && mixed) e = w.HQ.reserve((size_t)nl * ld, s);  // H Q, rotated for the explicit residuals
+    if (!e) e = w.T.reserve((size_t)ld * ld, s);
+    if (!e) e = w.Yw.reserve((size_t)ld * ld, s);
+    if (!e) e = w.theta.reserve(ld, s);
+    if (!e) e = w.Xb.reserve((size_t)rb * kk, s);  // rblk rows: the block each rank gathers at the end
+    if (!e && mixed) e = w.HXb.reserve((size_t)nl * kk, s);  // the final FP64 sweep's products
+    if (!e) e = w.W.reserve((size_t)nl * b, s);
+    if (!e) e = w.part.reserve((size_t)nblk * kk, s);
+    if (!e) e = w.rn2.reserve(kk, s);
+    return e;
+  };
+  if (const cudaError_t e = reserve_all()) {
+    w.release(s);
+    if (e != cudaErrorMemoryAllocation) return cuda_fail(c, e, "eigensolver buffers");
+    cudaGetLastError();  // too little memory after all
+    return block_lanczos_lean(c, k);
+  }
   VCK(w.short_flag.reserve(1, s));
   VCK(cudaMemsetAsync(w.short_flag.p, 0, sizeof(int), s));
   fill_zero(w.Q.p, nl * (int64_t)ld, s);
@@ -540,7 +572,7 @@ int block_lanczos_impl(vhci_ctx* c, int k, bool dev_svqb) {
     c->stats.eig_iterations += 1;
     VCK(cudaMemcpy2DAsync(w.Yw.p, ld * sizeof(double), w.T.p, ld * sizeof(double),
                           m * sizeof(double), m, cudaMemcpyDeviceToDevice, s));
-    VTRY(syevd_l(c, w.Yw.p, m, ld, w.theta.p));
+    VTRY(syevd_l(c, w, w.Yw.p, m, ld, w.theta.p));
     if (dev) {  // a block that lost rank on the device: redo with the host factorisation
       int short_rank = 0;
       VCK(d2h(c, &short_rank, w.short_flag.p, sizeof(int)));
@@ -754,6 +786,7 @@ int block_lanczos_lean(vhci_ctx* c, int k) {
     VCK(out.reserve((size_t)rb * kk, s));
     copy_cols(w.Q.p, ld, out.p, kk, nl, nk, s);
     VTRY(publish_ritz(c, out, kk, nk, th));
+    c->stats.ms_spmm += w.times.collect();
     out.release(s);
     w.release(s);
     return VHCI_OK;
@@ -789,7 +822,7 @@ int block_lanczos_lean(vhci_ctx* c, int k) {
     c->stats.eig_iterations += 1;
     VCK(cudaMemcpy2DAsync(w.Yw.p, ld * sizeof(double), w.T.p, ld * sizeof(double),
                           m * sizeof(double), m, cudaMemcpyDeviceToDevice, s));
-    VTRY(syevd_l(c, w.Yw.p, m, ld, w.theta.p));
+    VTRY(syevd_l(c, w, w.Yw.p, m, ld, w.theta.p));
     VTRY(comm_bcast0(c, w.Yw.p, (int64_t)ld * m));
     VTRY(comm_bcast0(c, w.theta.p, m));
     const int nk = std::min(kk, m);
