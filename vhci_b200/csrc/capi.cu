@@ -921,6 +921,7 @@ vhci_status vhci_destroy(vhci_ctx* c) {
     c->d64a.release(c->st); c->u64a.release(c->st); c->u64b.release(c->st);
     c->u8a.release(c->st); c->ull.release(c->st); c->solver_work.release(c->st);
     c->solver_info.release(c->st);
+    c->eig_work.release(c->st); c->eig_dev.release(c->st);
     c->prow.release(c->st); c->pcol.release(c->st); c->pval.release(c->st);
     c->pvalf.release(c->st); c->gate_dev.release(c->st);
     cudaStreamSynchronize(c->st);

@@ -145,6 +145,8 @@ struct vhci_ctx {
   vhci::DBuf<unsigned long long> ull;
   vhci::DBuf<double> solver_work;
   vhci::DBuf<int> solver_info;
+  vhci::DBuf<double> eig_work;
+  vhci::DBuf<unsigned long long> eig_dev;
 
   std::string err;
   vhci_stats stats{};

@@ -1,6 +1,7 @@
 // Lowest eigenpairs of the sparse Hamiltonian (reference: SparseDiagonalize / DenseDiagonalize,
 // Ham.cpp:347-379).  Small bases (and the first heat-bath step over the initial basis) use a dense
-// symmetric eigensolve on the device (cuSOLVER syevd over the matrix expanded from its CSR form);
+// symmetric eigensolve on the device over the matrix expanded from its CSR form (k_eig.cu up to 640
+// states, cuSOLVER's syevd beyond);
 // larger ones use the block thick-restart Lanczos of lanczos.cu, whose projections run on the
 // FP64 tensor pipe (k_proj.cu).  Convergence follows the reference eigensolver's rule
 // ||r_j|| <= tol * max(eps^(2/3), |theta_j|) for the wanted pairs (tol = 1e-10, Ham.cpp:363).
@@ -43,6 +44,21 @@ int syevd(vhci_ctx* c, double* A, int m, int lda, double* w) {
 
 }  // namespace
 
+int small_eigs(vhci_ctx* c, const double* T, int m, int ld, int nk, double* theta, double* Y, bool* done) {
+  *done = false;
+  if (m > kSmallEigMax) return VHCI_OK;
+  VCK(c->eig_work.reserve(small_eig_elems(m, nk), c->st));
+  VCK(c->eig_dev.reserve(2, c->st));
+  if (!small_eig(T, ld, m, nk, theta, Y, ld, c->eig_work.p, c->eig_dev.p, c->st)) return VHCI_OK;
+  double dev[2];
+  static_assert(sizeof(double) == sizeof(unsigned long long), "deviations are doubles' bits");
+  VCK(d2h(c, dev, c->eig_dev.p, sizeof(dev)));
+  VCK(cudaStreamSynchronize(c->st));
+  VCK(cudaGetLastError());
+  *done = small_eig_good(dev[0], dev[1]);
+  return VHCI_OK;
+}
+
 int apply_h(vhci_ctx* c, const double* X, int ldx, int b, double* Y, int ldy) {
   EventPair ev_e0e1;
   VCK(ev_e0e1.create());
@@ -73,19 +89,26 @@ int dense_eigs(vhci_ctx* c, int keep) {
   VCK(w.reserve(n, c->st));
   dense_from_csr(n, c->rowptr.p, c->col.p, c->o.precision == 1 ? nullptr : c->val.p,
                  c->o.precision == 1 ? c->valf.p : nullptr, c->diag.p, A.p, c->st);
-  VTRY(syevd(c, A.p, (int)n, (int)n, w.p));
+  DBuf<double> Y;  // the vectors, column-major
+  bool done = false;
+  if (n <= kSmallEigMax) {
+    VCK(Y.reserve((size_t)n * keep, c->st));
+    VTRY(small_eigs(c, A.p, (int)n, (int)n, keep, w.p, Y.p, &done));
+  }
+  if (!done) VTRY(syevd(c, A.p, (int)n, (int)n, w.p));
   VCK(c->X.reserve((size_t)n * keep, c->st));
   {
     const int64_t tot = n * keep;
     const int g = (int)std::min<int64_t>(148 * 16, std::max<int64_t>(1, (tot + 255) / 256));
     note_launch();
-    k_cols_to_rows<<<g, 256, 0, c->st>>>(A.p, n, keep, c->X.p);
+    k_cols_to_rows<<<g, 256, 0, c->st>>>(done ? Y.p : A.p, n, keep, c->X.p);
   }
   std::vector<double> wh(keep);
   VCK(d2h(c, wh.data(), w.p, keep * sizeof(double)));
   VCK(cudaStreamSynchronize(c->st));
   A.release(c->st);
   w.release(c->st);
+  Y.release(c->st);
   c->ldx = keep;
   c->nvec = keep;
   c->x_rows = n;

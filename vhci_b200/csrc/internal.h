@@ -101,6 +101,10 @@ double lanczos_min_bytes(vhci_ctx* c, int k);
 // Lowest k eigenpairs; dense_all keeps every eigenpair of a dense solve (first HCI step).
 int eigs(vhci_ctx* c, int k);
 int dense_eigs(vhci_ctx* c, int keep);
+// The nk lowest eigenpairs of the m x m matrix in T (upper triangle, column-major, ld) by small_eig:
+// values in theta, vectors in Y (ld).  *done = false when the caller has to use another solver.
+// Synchronises.
+int small_eigs(vhci_ctx* c, const double* T, int m, int ld, int nk, double* theta, double* Y, bool* done);
 // Block thick-restart Lanczos (lanczos.cu).
 int block_lanczos(vhci_ctx* c, int k);
 int lanczos_block(int64_t n);

@@ -1,0 +1,563 @@
+// Lowest eigenpairs of a small dense symmetric matrix (the projected matrix of the Lanczos solver,
+// 100 to 640 rows, once per cycle; the first dense heat-bath steps), the role of the dense
+// eigensolvers behind Spectra and Eigen in the reference (Ham.cpp:347-379).
+//
+//   1. k_tridiag: Householder tridiagonalisation in one cluster of thread blocks that hold the whole
+//      matrix in their shared memory (rows dealt cyclically), one cluster barrier a column;
+//   2. k_tri_vectors: one warp per wanted eigenvalue: Sturm counts at 32 points a round, then the
+//      vector from the twisted factorisation of T - lambda I;
+//   3. two Newton-Schulz steps Z <- Z (3 I - Z^T Z) / 2 take out the mixing of close eigenvalues
+//      (k_eig_gram, k_eig_mul, FP64 tensor cores), with the deviation from orthonormality before each;
+//   4. k_back: the reflectors applied to the vectors, one warp per vector.
+//
+// All steps at 192, 352 and 640 rows (half of the vectors wanted): 0.66, 1.4 and 3.7 ms, against 1.9,
+// 3.5 and 7 ms for syevd with its host steps.
+//
+// Vectors of eigenvalues closer than about 1e-12 of the norm come out too far from orthogonal for
+// step 3; the deviations tell, and the caller takes the library's solver instead.
+#include <cooperative_groups.h>
+
+#include <algorithm>
+#include <cstdint>
+#include <mutex>
+
+#include "ops.h"
+
+namespace cg = cooperative_groups;
+
+namespace vhci {
+
+namespace {
+
+constexpr int kTriThreads = 256, kTriWarps = kTriThreads / 32;
+constexpr int kTriRows = 8;   // rows a warp holds at most
+constexpr int kVecWarps = 4;
+
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// Dynamic shared memory: the block's rows (m values each), p and the next row as they arrive (two
+// buffers each), v at the block's own rows (two buffers).
+__host__ __device__ constexpr size_t tri_smem(int m, int blocks) {
+  const size_t rows = (size_t)((m + blocks - 1) / blocks);
+  return (rows * m + 4 * (size_t)m + 2 * rows) * sizeof(double);
+}
+
+// A = H_0 .. H_{m-3} (tridiagonal d, e) H_{m-3} .. H_0 with H_k = I - tau_k v_k v_k^T, v_k (zero up to
+// k, one at k + 1) in row k of V.  T holds the upper triangle of A, column-major.  m <= 32 NR.
+//
+// Row l C + r of the matrix is kept by block r of the cluster, in its warp l % kTriWarps.  Column k
+// takes one cluster barrier: every warp of every block holds v_{k-1} in registers (columns lane + 32 q)
+// and finds p_{k-1} = tau A v_{k-1} and row k, as it was before the update with them, in its block's
+// shared memory; it forms the updated row k, the reflector v_k and tau_k from it by itself, then in
+// one pass over its own rows applies the update A - v p^T - (p + K v) v^T, K = - tau v^T p, and
+// multiplies by v_k, and hands p_k and (the keeper of that row) row k + 1 to all blocks.  Bound by
+// latency: the barrier, three warp sums, a square root and a division a column.  Measured at 192, 352
+// and 640 rows: 0.42, 0.99 and 2.9 ms; with two barriers, one of which waits for one block to form v
+// and hand it round, 0.72, 1.8 and 4.9 ms; the tridiagonalisation of cuSOLVER's syevd takes 1.0 ms
+// at 192 and 2.5 at 352.  The barriers wait only for blocks of the same cluster, which run together.
+template <int NR>
+__global__ void __launch_bounds__(kTriThreads) k_tridiag(const double* __restrict__ T, int ldt, int m,
+                                                         double* __restrict__ d, double* __restrict__ e,
+                                                         double* __restrict__ tau,
+                                                         double* __restrict__ V, double* rowx) {
+  constexpr bool kRowGlobal = NR > 8;
+  extern __shared__ double sm[];
+  cg::cluster_group cl = cg::this_cluster();
+  const int C = (int)cl.num_blocks(), r = (int)cl.block_rank();
+  const int sh = 31 - __clz(C), lm = C - 1;  // C is a power of two
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int R = (m + C - 1) / C;
+  double* A = sm;                     // local row l is row l C + r
+  double* sp = A + (size_t)R * m;     // [2][m] p
+  double* srow = sp + 2 * m;          // [2][m] the next row
+  double* svr = srow + 2 * m;         // [2][R] v at the local rows
+  const int rows = r < m ? (m - r + C - 1) / C : 0;
+  for (int l = wid; l < rows; l += kTriWarps) {
+    const int i = l * C + r;
+    for (int j = lane; j < m; j += 32)
+      A[(size_t)l * m + j] = i <= j ? T[i + (int64_t)j * ldt] : T[j + (int64_t)i * ldt];
+  }
+  for (int j = tid; j < m; j += kTriThreads) {
+    sp[j] = 0.0;
+    const double y = T[(int64_t)j * ldt];  // row 0
+    srow[j] = y;
+    if (kRowGlobal && r == 0) rowx[j] = y;
+  }
+  for (int l = tid; l < 2 * R; l += kTriThreads) svr[l] = 0.0;
+  double v[NR];  // v_{k-1}
+#pragma unroll
+  for (int q = 0; q < NR; ++q) v[q] = 0.0;
+  double t = 0.0;  // tau_{k-1}
+  cl.sync();
+  for (int k = 0; k + 1 < m; ++k) {
+    const int par = k & 1, q0 = (k + 1) >> 5;  // chunks before q0 are done
+    const double* p_in = sp + par * m;
+    double p[NR], x[NR], s = 0.0, s1 = 0.0;
+#pragma unroll
+    for (int q = 0; q < NR; ++q) {
+      const int j = lane + 32 * q;
+      const bool in = j >= k && j < m;
+      p[q] = in ? p_in[j] : 0.0;
+      x[q] = !in ? 0.0 : kRowGlobal ? __ldcg(rowx + par * m + j) : srow[par * m + j];
+    }
+#pragma unroll
+    for (int q = 0; q < NR; ++q)
+      if (q & 1) s1 = fma(v[q], p[q], s1); else s = fma(v[q], p[q], s);
+    const double K = -t * warp_sum(s + s1);
+    {  // row k, updated
+      const double vk = k > 0 ? 1.0 : 0.0, ck = fma(K, vk, p_in[k]);
+      s = s1 = 0.0;
+#pragma unroll
+      for (int q = 0; q < NR; ++q) {
+        const int j = lane + 32 * q;
+        x[q] -= fma(vk, p[q], ck * v[q]);
+        const double y = j > k + 1 ? x[q] : 0.0;
+        if (q & 1) s1 = fma(y, y, s1); else s = fma(y, y, s);
+      }
+    }
+    const double ss = warp_sum(s + s1);
+    double alpha = 0.0;
+#pragma unroll
+    for (int q = 0; q < NR; ++q)
+      if (q == q0) alpha = x[q];
+    alpha = __shfl_sync(0xffffffffu, alpha, (k + 1) & 31);
+    double beta = alpha, inv = 0.0, tn = 0.0;
+    if (ss > 0.0 && k + 2 < m) {
+      beta = -copysign(sqrt(fma(alpha, alpha, ss)), alpha);
+      const double g = 1.0 / (beta * (alpha - beta));  // both quotients from one division
+      inv = beta * g;
+      tn = (beta - alpha) * ((alpha - beta) * g);
+    }
+    const bool keeper = r == (k & lm) && wid == 0;
+    double vn[NR];
+#pragma unroll
+    for (int q = 0; q < NR; ++q) {
+      const int j = lane + 32 * q;
+      vn[q] = j > k + 1 ? x[q] * inv : (j == k + 1 ? 1.0 : 0.0);
+      if (keeper) {
+        if (j == k) d[k] = x[q];
+        if (j > k && j < m) V[(int64_t)k * m + j] = vn[q];
+      }
+      if (wid == 0 && j < m && (j & lm) == r) svr[par * R + (j >> sh)] = vn[q];
+    }
+    if (keeper && lane == 0) {
+      e[k] = beta;
+      tau[k] = tn;
+    }
+    // own rows below k: update with v, p; multiply by the new reflector
+    const double* vr = svr + (par ^ 1) * R;
+    const int lr = (k + 1) >> sh;
+    const bool has_next = r == ((k + 1) & lm);  // this block keeps row k + 1
+    double sum[kTriRows];
+    auto pass = [&](int l, bool out) -> double {
+      const int i = (l << sh) + r;
+      const double vi = vr[l], ci = fma(K, vi, p_in[i]);
+      double* a = A + (size_t)l * m;
+      double y[NR], u = 0.0, u1 = 0.0;
+#pragma unroll
+      for (int q = 0; q < NR; ++q) {
+        const int j = lane + 32 * q;
+        y[q] = q >= q0 && j < m ? a[j] : 0.0;
+      }
+#pragma unroll
+      for (int q = 0; q < NR; ++q) y[q] -= fma(vi, p[q], ci * v[q]);
+#pragma unroll
+      for (int q = 0; q < NR; ++q) {
+        const int j = lane + 32 * q;
+        if (q >= q0 && j < m) a[j] = y[q];
+        if (kRowGlobal && out && q >= q0 && j < m) __stcg(rowx + (par ^ 1) * m + j, y[q]);
+        if (q & 1) u1 = fma(y[q], vn[q], u1); else u = fma(y[q], vn[q], u);
+      }
+      return u + u1;
+    };
+    // the keeper of row k + 1 updates it first; it goes to all blocks through their shared memory by
+    // the whole block, or for long rows (320 stores a lane otherwise) through L2
+    double first = 0.0;
+    if (has_next) {
+      if (wid == lr % kTriWarps) first = pass(lr, true);
+      if (!kRowGlobal) {
+        __syncthreads();
+        for (int j = k + 1 + tid; j < m; j += kTriThreads) {
+          const double y = A[(size_t)lr * m + j];
+          for (int c = 0; c < C; ++c) cl.map_shared_rank(srow, c)[(par ^ 1) * m + j] = y;
+        }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < kTriRows; ++q) {
+      const int l = wid + q * kTriWarps;
+      sum[q] = 0.0;
+      if (l < rows && (l << sh) + r > k) sum[q] = has_next && l == lr ? first : pass(l, false);
+    }
+#pragma unroll
+    for (int q = 0; q < kTriRows; ++q) {
+      const int l = wid + q * kTriWarps, i = (l << sh) + r;
+      if (!(l < rows && i > k)) continue;
+      const double pi = tn * warp_sum(sum[q]);
+      if (lane < C) cl.map_shared_rank(sp, lane)[(par ^ 1) * m + i] = pi;
+    }
+#pragma unroll
+    for (int q = 0; q < NR; ++q) v[q] = vn[q];
+    t = tn;
+    cl.sync();  // p and the next row have arrived
+  }
+  // the last diagonal element (its row has had every update)
+  if (r == (m - 1) % C && tid == 0) d[m - 1] = A[(size_t)((m - 1) / C) * m + m - 1];
+}
+
+// Eigenvalue j (j < nk; the last warp takes the largest, for its value alone) of the tridiagonal
+// matrix, scaled to norm 1, and its vector in column j of Z (leading dimension m).  The Sturm count
+// uses the three-term recurrence of the characteristic polynomials (one multiply-add of latency a
+// step where the quotient form has a division), rescaled every eight steps; squared off-diagonals
+// below 1e-34 are raised to that, a change below the rounding of the matrix.
+__global__ void __launch_bounds__(32 * kVecWarps) k_tri_vectors(const double* __restrict__ d,
+                                                                const double* __restrict__ e, int m,
+                                                                int nk, double* __restrict__ theta,
+                                                                double* __restrict__ Z) {
+  extern __shared__ double sm[];
+  __shared__ double s_red[kVecWarps];
+  double* sd = sm;              // [m]
+  double* se = sd + m;          // [m] off-diagonals, zero at the end
+  double* se2 = se + m;         // [m] their squares
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  double* P = se2 + m + (size_t)wid * 2 * m;  // forward pivots, then the vector
+  double* M = P + m;                          // backward pivots
+  // norm: the largest row sum
+  double nrm = 0.0;
+  for (int i = tid; i < m; i += blockDim.x) {
+    const double a = i > 0 ? fabs(e[i - 1]) : 0.0, b = i + 1 < m ? fabs(e[i]) : 0.0;
+    nrm = fmax(nrm, a + fabs(d[i]) + b);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) nrm = fmax(nrm, __shfl_xor_sync(0xffffffffu, nrm, o));
+  if (lane == 0) s_red[wid] = nrm;
+  __syncthreads();
+  nrm = s_red[0];
+#pragma unroll
+  for (int q = 1; q < kVecWarps; ++q) nrm = fmax(nrm, s_red[q]);
+  const double scale = nrm > 0.0 ? 1.0 / nrm : 1.0;
+  for (int i = tid; i < m; i += blockDim.x) {
+    const double x = i + 1 < m ? e[i] * scale : 0.0;
+    sd[i] = d[i] * scale;
+    se[i] = x;
+    se2[i] = fmax(x * x, 1e-34);
+  }
+  __syncthreads();
+  const int w = blockIdx.x * kVecWarps + wid;
+  if (w > nk || (w == nk && nk >= m)) return;
+  const int j = w < nk ? w : m - 1;
+
+  // eigenvalue j lies in [lo, hi): counts of the eigenvalues below 32 points inside
+  double lo = -1.0000001, hi = 1.0000001;
+  for (int round = 0; round < 12; ++round) {
+    const double x = lo + (hi - lo) * ((lane + 1) * (1.0 / 33.0));
+    double p0 = 1.0, p1 = sd[0] - x;
+    int below = (unsigned)__double2hiint(p1) >> 31;  // sign changes, by the sign bits
+    for (int i = 1; i < m; i += 8) {
+      const int n = min(8, m - i);
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (q < n) {
+          const double p2 = fma(sd[i + q] - x, p1, -se2[i + q - 1] * p0);
+          below += (unsigned)(__double2hiint(p2) ^ __double2hiint(p1)) >> 31;
+          p0 = p1;
+          p1 = p2;
+        }
+      const double big = fmax(fabs(p0), fabs(p1));
+      if (big > 1e100) { p0 *= 1e-100; p1 *= 1e-100; }
+      else if (big < 1e-100) { p0 *= 1e100; p1 *= 1e100; }
+    }
+    const int n = __popc(__ballot_sync(0xffffffffu, below <= j));
+    const double a = __shfl_sync(0xffffffffu, x, max(0, n - 1)), b = __shfl_sync(0xffffffffu, x, min(31, n));
+    if (n > 0) lo = a;
+    if (n < 32) hi = b;
+    if (hi - lo <= 1e-17) break;
+  }
+  const double lam = 0.5 * (lo + hi);
+  if (lane == 0) theta[j] = lam * nrm;
+  if (w >= nk) return;
+
+  // twisted factorisation of T - lam: forward pivots by lane 0, backward ones by lane 1
+  constexpr double tiny = 1e-17;
+  if (lane == 0) {
+    double q = sd[0] - lam;
+    for (int i = 0;; ) {
+      if (fabs(q) < tiny) q = copysign(tiny, q);
+      P[i] = q;
+      if (++i >= m) break;
+      q = (sd[i] - lam) - se2[i - 1] / q;
+    }
+  } else if (lane == 1) {
+    double q = sd[m - 1] - lam;
+    for (int i = m - 1;; ) {
+      if (fabs(q) < tiny) q = copysign(tiny, q);
+      M[i] = q;
+      if (--i < 0) break;
+      q = (sd[i] - lam) - se2[i] / q;
+    }
+  }
+  __syncwarp();
+  double best = 1e300;
+  int twist = 0;
+  for (int i = lane; i < m; i += 32) {
+    const double g = fabs(P[i] + M[i] - (sd[i] - lam));
+    if (g < best) { best = g; twist = i; }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+    const int ot = __shfl_xor_sync(0xffffffffu, twist, o);
+    if (ob < best || (ob == best && ot < twist)) { best = ob; twist = ot; }
+  }
+  // ratios of neighbouring components, then their running products away from the twist
+  __syncwarp();
+  for (int i = lane; i < m; i += 32) {
+    const double up = i < twist ? -se[i] / P[i] : 0.0;        // z_i = up z_{i+1}
+    const double dn = i > twist ? -se[i - 1] / M[i] : 0.0;    // z_i = dn z_{i-1}
+    P[i] = i < twist ? up : (i > twist ? dn : 1.0);
+  }
+  __syncwarp();
+  if (lane == 0) {
+    double z = 1.0;
+    for (int i = twist - 1; i >= 0; --i) P[i] = z = P[i] * z;
+  } else if (lane == 1) {
+    double z = 1.0;
+    for (int i = twist + 1; i < m; ++i) P[i] = z = P[i] * z;
+  }
+  __syncwarp();
+  double s = 0.0;
+  for (int i = lane; i < m; i += 32) s = fma(P[i], P[i], s);
+  s = 1.0 / sqrt(warp_sum(s));
+  for (int i = lane; i < m; i += 32) Z[(int64_t)j * m + i] = P[i] * s;
+}
+
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
+}
+
+// One warp per 8 x 32 tile of S = (3 I - Z^T Z) / 2 (nk x nk); *dev: the largest |Z^T Z - I| seen, as
+// the bits of a non-negative double.
+__global__ void __launch_bounds__(128) k_eig_gram(const double* __restrict__ Z, int m, int nk,
+                                                  double* __restrict__ S,
+                                                  unsigned long long* __restrict__ dev) {
+  const int lane = threadIdx.x & 31, w = blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int tr = (nk + 7) / 8, tc = (nk + 31) / 32;
+  if (w >= tr * tc) return;
+  const int a0 = (w / tc) * 8, b0 = (w % tc) * 32;
+  const int q = lane >> 2, kl = lane & 3;
+  double acc[4][2];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) acc[u][0] = acc[u][1] = 0.0;
+  const double* za = Z + (int64_t)min(a0 + q, nk - 1) * m;
+  for (int k0 = 0; k0 < m; k0 += 16) {
+    double a[4], b[4][4];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const int k = k0 + 4 * s + kl;
+      a[s] = k < m ? __ldg(za + k) : 0.0;
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        b[s][u] = k < m ? __ldg(Z + (int64_t)min(b0 + 8 * u + q, nk - 1) * m + k) : 0.0;
+    }
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) dmma(acc[u], a[s], b[s][u]);
+  }
+  double worst = 0.0;
+  bool bad = false;
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int i = a0 + q, j = b0 + 8 * u + 2 * kl + h;
+      if (i >= nk || j >= nk) continue;
+      const double g = acc[u][h] - (i == j ? 1.0 : 0.0);
+      bad |= !(fabs(g) < 1e300);
+      worst = fmax(worst, fabs(g));
+      S[i + (int64_t)j * nk] = (i == j ? 1.0 : 0.0) - 0.5 * g;
+    }
+  if (bad) worst = 1e300;  // a NaN counts as the largest deviation
+  atomicMax(dev, (unsigned long long)__double_as_longlong(worst));
+}
+
+// Out (m x nk) = Z S, one warp per 8 x 32 tile.
+__global__ void __launch_bounds__(128) k_eig_mul(const double* __restrict__ Z, const double* __restrict__ S,
+                                                 int m, int nk, double* __restrict__ Out) {
+  const int lane = threadIdx.x & 31, w = blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int tr = (m + 7) / 8, tc = (nk + 31) / 32;
+  if (w >= tr * tc) return;
+  const int i0 = (w / tc) * 8, j0 = (w % tc) * 32;
+  const int q = lane >> 2, kl = lane & 3;
+  double acc[4][2];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) acc[u][0] = acc[u][1] = 0.0;
+  for (int k0 = 0; k0 < nk; k0 += 16) {
+    double a[4], b[4][4];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const int k = k0 + 4 * s + kl;
+      a[s] = k < nk ? __ldg(Z + (int64_t)k * m + min(i0 + q, m - 1)) : 0.0;
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        b[s][u] = k < nk ? __ldg(S + (int64_t)min(j0 + 8 * u + q, nk - 1) * nk + k) : 0.0;
+    }
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) dmma(acc[u], a[s], b[s][u]);
+  }
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int i = i0 + q, j = j0 + 8 * u + 2 * kl + h;
+      if (i < m && j < nk) Out[i + (int64_t)j * m] = acc[u][h];
+    }
+}
+
+// Y[:, j] = H_0 .. H_{m-3} Z[:, j], one warp per column with the column in registers (32 NR >= m) and
+// the next PF reflectors' loads in flight.
+template <int NR, int PF>
+__global__ void __launch_bounds__(64) k_back(const double* __restrict__ Z, const double* __restrict__ V,
+                                             const double* __restrict__ tau, int m, int nk,
+                                             double* __restrict__ Y, int ldy) {
+  const int lane = threadIdx.x & 31, j = blockIdx.x * 2 + (threadIdx.x >> 5);
+  if (j >= nk) return;
+  double z[NR], v[PF][NR], t[PF];
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    const int i = lane + 32 * r;
+    z[r] = i < m ? Z[(int64_t)j * m + i] : 0.0;
+  }
+  auto fetch = [&](int k, double (&u)[NR], double& tk) {
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+      const int i = lane + 32 * r;
+      u[r] = (k >= 0 && i > k && i < m) ? __ldg(V + (int64_t)k * m + i) : 0.0;
+    }
+    tk = k >= 0 ? __ldg(tau + k) : 0.0;
+  };
+#pragma unroll
+  for (int f = 0; f < PF; ++f) fetch(m - 3 - f, v[f], t[f]);
+  for (int k = m - 3; k >= 0; k -= PF) {
+#pragma unroll
+    for (int f = 0; f < PF; ++f) {  // a reflector before the first has tau = 0
+      double s = 0.0, s1 = 0.0;
+#pragma unroll
+      for (int r = 0; r < NR; ++r)
+        if (r & 1) s1 = fma(v[f][r], z[r], s1); else s = fma(v[f][r], z[r], s);
+      s = -t[f] * warp_sum(s + s1);
+#pragma unroll
+      for (int r = 0; r < NR; ++r) z[r] = fma(s, v[f][r], z[r]);
+      fetch(k - f - PF, v[f], t[f]);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    const int i = lane + 32 * r;
+    if (i < m) Y[(int64_t)j * ldy + i] = z[r];
+  }
+}
+
+constexpr size_t vec_smem(int m) { return (size_t)m * (3 + 2 * kVecWarps) * sizeof(double); }
+
+// Blocks of the cluster for m rows (its rows must fit the shared memory and kTriRows rounds): 16 (the
+// barrier reaches over more of the chip, the pass over the rows is shorter) pay from 256 rows on:
+// 0.64 : 0.66 ms there, 0.99 : 1.17 at 352; four are 10 to 20 % slower than eight from 128 on.
+int tri_blocks(int m) {
+  return m <= 32 ? 4 : (m < 256 ? 8 : 16);
+}
+
+using TriKernel = void (*)(const double*, int, int, double*, double*, double*, double*, double*);
+TriKernel tri_kernel(int m) {
+  return m <= 64 ? k_tridiag<2> : m <= 128 ? k_tridiag<4> : m <= 192 ? k_tridiag<6> : m <= 256 ? k_tridiag<8>
+         : m <= 384 ? k_tridiag<12> : k_tridiag<20>;
+}
+
+// Shared-memory and cluster limits of the kernels, set once per device.
+constexpr int kMaxDevices = 64;
+std::once_flag g_eig_once[kMaxDevices];
+bool g_eig_ok[kMaxDevices];
+
+bool eig_attributes() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return false;
+  std::call_once(g_eig_once[dev], [dev] {
+    bool ok = cudaFuncSetAttribute(k_tri_vectors, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)vec_smem(kSmallEigMax)) == cudaSuccess;
+    for (int m : {64, 128, 192, 256, 384, kSmallEigMax}) {
+      const TriKernel k = tri_kernel(m);
+      ok = ok && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) == cudaSuccess &&
+           cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    }
+    g_eig_ok[dev] = ok;
+    if (!g_eig_ok[dev]) cudaGetLastError();
+  });
+  return g_eig_ok[dev];
+}
+
+}  // namespace
+
+size_t small_eig_elems(int m, int nk) {
+  // d, e, tau; the row exchange; V; two vector blocks; S
+  return 5 * (size_t)m + (size_t)m * m + 2 * (size_t)m * nk + (size_t)nk * nk;
+}
+
+bool small_eig(const double* T, int ldt, int m, int nk, double* theta, double* Y, int ldy, double* work,
+               unsigned long long* dev, cudaStream_t s) {
+  if (m < 1 || m > kSmallEigMax || nk < 1 || nk > m) return false;
+  if (!eig_attributes()) return false;
+  double* d = work;
+  double* e = d + m;
+  double* tau = e + m;
+  double* rowx = tau + m;
+  double* V = rowx + 2 * m;
+  double* Za = V + (size_t)m * m;
+  double* Zb = Za + (size_t)m * nk;
+  double* S = Zb + (size_t)m * nk;
+  const int C = tri_blocks(m);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(C);
+  cfg.blockDim = dim3(kTriThreads);
+  cfg.dynamicSmemBytes = tri_smem(m, C);
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = C;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  note_launch();
+  if (cudaLaunchKernelEx(&cfg, tri_kernel(m), T, ldt, m, d, e, tau, V, rowx) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  note_launch();
+  k_tri_vectors<<<(nk + 1 + kVecWarps - 1) / kVecWarps, 32 * kVecWarps, vec_smem(m), s>>>(d, e, m, nk,
+                                                                                          theta, Za);
+  cudaMemsetAsync(dev, 0, 2 * sizeof(unsigned long long), s);
+  const int tr = (nk + 7) / 8, tc = (nk + 31) / 32, tm = (m + 7) / 8;
+  for (int it = 0; it < 2; ++it) {
+    note_launch();
+    k_eig_gram<<<(tr * tc + 3) / 4, 128, 0, s>>>(it ? Zb : Za, m, nk, S, dev + it);
+    note_launch();
+    k_eig_mul<<<(tm * tc + 3) / 4, 128, 0, s>>>(it ? Zb : Za, S, m, nk, it ? Za : Zb);
+  }
+  note_launch();
+  const int g = (nk + 1) / 2;
+  if (m <= 64) k_back<2, 4><<<g, 64, 0, s>>>(Za, V, tau, m, nk, Y, ldy);
+  else if (m <= 128) k_back<4, 4><<<g, 64, 0, s>>>(Za, V, tau, m, nk, Y, ldy);
+  else if (m <= 256) k_back<8, 4><<<g, 64, 0, s>>>(Za, V, tau, m, nk, Y, ldy);
+  else if (m <= 384) k_back<12, 3><<<g, 64, 0, s>>>(Za, V, tau, m, nk, Y, ldy);
+  else k_back<20, 2><<<g, 64, 0, s>>>(Za, V, tau, m, nk, Y, ldy);
+  return true;
+}
+
+}  // namespace vhci

@@ -7,7 +7,7 @@
 //     pass over the columns that the product can couple to (the block itself and the one before; all
 //     of them in the first step after a restart), a second one over the whole basis, and the
 //     projected matrix T = Q^T H Q summed from the coefficients of both;
-//   * Rayleigh-Ritz (cuSOLVER syevd on T) only when the subspace is full; the kk = k + guard
+//   * Rayleigh-Ritz (k_eig.cu on T) only when the subspace is full; the kk = k + guard
 //     lowest Ritz vectors are kept (thick restart) together with the pending Lanczos block, so the
 //     kept Ritz vectors' residuals lie in the new subspace (Krylov-Schur property);
 //   * convergence: ||H x - theta x|| <= tol * max(eps^(2/3), |theta|) for the k wanted pairs,
@@ -208,6 +208,28 @@ bool gathers_f32(vhci_ctx* c, const LWork& w, int b) {
   return c->o.precision == 1 && !w.exact && b % 4 == 0;
 }
 
+// The nk lowest eigenpairs of T[0:m, 0:m] into w.theta and the columns of w.Yw (k_eig.cu, or cuSOLVER's
+// syevd beyond its sizes and for eigenvalues too close for it); also the largest, in theta[m - 1].
+int project_eigs(vhci_ctx* c, LWork& w, int m, int ld, int nk) {
+  bool done = false;
+  VTRY(small_eigs(c, w.T.p, m, ld, nk, w.theta.p, w.Yw.p, &done));
+  if (done) {
+    c->stats.ms_spmm += w.times.collect();
+    return VHCI_OK;
+  }
+  VCK(cudaMemcpy2DAsync(w.Yw.p, ld * sizeof(double), w.T.p, ld * sizeof(double), m * sizeof(double), m,
+                        cudaMemcpyDeviceToDevice, c->st));
+  return syevd_l(c, w, w.Yw.p, m, ld, w.theta.p);
+}
+
+// Subspace size span kk + 2 b; one up to a tenth above what k_eig.cu takes is cut to that (fewer steps
+// a cycle, but a Rayleigh-Ritz step of 3.7 ms instead of 7).
+int subspace_size(int64_t n, int span, int kk, int b) {
+  int64_t m = (int64_t)span * kk + 2 * b;
+  if (m > kSmallEigMax && 10 * m <= 11 * kSmallEigMax) m = kSmallEigMax;
+  return (int)std::min<int64_t>(n, m);
+}
+
 // Orthonormalise the nb columns of (B, ld) into (out, ldo) by SVQB with the small Gram matrix
 // decomposed on the host; directions below 1e-12 of the largest are dropped.  *r = rank.
 int svqb_small(vhci_ctx* c, LWork& w, int64_t n, const double* B, int ld, int nb, double* out,
@@ -328,9 +350,7 @@ int fp64_sweep(vhci_ctx* c, LWork& w, int kk, int nk, int keff, int ld, std::vec
     VTRY(gemm_gram(c, w, w.Xb.p, kk, w.HQ.p + j0, ld, nl, nk, bw, 1.0, 0.0,
                    w.T.p + (size_t)j0 * ld, ld));
   }
-  VCK(cudaMemcpy2DAsync(w.Yw.p, ld * sizeof(double), w.T.p, ld * sizeof(double),
-                        nk * sizeof(double), nk, cudaMemcpyDeviceToDevice, s));
-  VTRY(syevd_l(c, w, w.Yw.p, nk, ld, w.theta.p));
+  VTRY(project_eigs(c, w, nk, ld, nk));
   VTRY(comm_bcast0(c, w.Yw.p, (int64_t)ld * nk));
   VTRY(comm_bcast0(c, w.theta.p, nk));
   VTRY(gemm_rows(c, w.Xb.p, kk, w.Yw.p, ld, nl, nk, nk, 1.0, 0.0, w.Q.p, ld));
@@ -398,7 +418,7 @@ static int lanczos_guard(int k) {
 // and the gathered vector block (n x b).
 static double lanczos_bytes(int64_t n, int64_t rows, int k, int span, int b, bool mixed) {
   const int kk = (int)std::min<int64_t>(n, k + lanczos_guard(k));
-  const int mmax = (int)std::min<int64_t>(n, (int64_t)span * kk + 2 * b);
+  const int mmax = subspace_size(n, span, kk, b);
   const int ld = (mmax + b + 15) / 16 * 16;
   return 8.0 * (double)rows * ((mixed ? 2.0 : 1.0) * (ld + kk) + 3.0 * b) + (rows < n ? 8.0 * n * b : 0.0);
 }
@@ -407,7 +427,7 @@ static double lanczos_bytes(int64_t n, int64_t rows, int k, int span, int b, boo
 // the compact copy (n x b each), the rotation chunk, and the output Ritz block (n x kk).
 static double lanczos_lean_bytes(int64_t n, int64_t rows, int k, int b, int span = 2) {
   const int kk = (int)std::min<int64_t>(n, k + lanczos_guard(k));
-  const int mmax = (int)std::min<int64_t>(n, (int64_t)span * kk + 2 * b);
+  const int mmax = subspace_size(n, span, kk, b);
   const int ld = (mmax + b + 15) / 16 * 16;
   return 8.0 * (double)rows * (ld + 3.0 * b + kk) + (rows < n ? 8.0 * n * (b + kk) : 0.0) + 2.6e8;
 }
@@ -448,7 +468,7 @@ int block_lanczos_impl(vhci_ctx* c, int k, bool dev_svqb) {
   if (const char* e = std::getenv("VHCI_LANCZOS_SPAN")) span = std::max(2, std::min(8, std::atoi(e)));
   if (!device_fits(c, lanczos_bytes(n, nl, k, span, b, c->o.precision == 1) + 1e9))
     return block_lanczos_lean(c, k);
-  const int mmax = (int)std::min<int64_t>(n, (int64_t)span * kk + 2 * b);
+  const int mmax = subspace_size(n, span, kk, b);
   const bool dev = dev_svqb && n >= 8 * (int64_t)mmax;
   // row stride padded to whole 128-byte lines so every b-column gather touches whole L2 lines
   const int ld = (mmax + b + 15) / 16 * 16;
@@ -570,9 +590,7 @@ int block_lanczos_impl(vhci_ctx* c, int k, bool dev_svqb) {
     // ---- Rayleigh-Ritz on T[0:m, 0:m]
     auto t0 = now();
     c->stats.eig_iterations += 1;
-    VCK(cudaMemcpy2DAsync(w.Yw.p, ld * sizeof(double), w.T.p, ld * sizeof(double),
-                          m * sizeof(double), m, cudaMemcpyDeviceToDevice, s));
-    VTRY(syevd_l(c, w, w.Yw.p, m, ld, w.theta.p));
+    VTRY(project_eigs(c, w, m, ld, std::min(kk, m)));
     if (dev) {  // a block that lost rank on the device: redo with the host factorisation
       int short_rank = 0;
       VCK(d2h(c, &short_rank, w.short_flag.p, sizeof(int)));
@@ -711,7 +729,7 @@ int block_lanczos_lean(vhci_ctx* c, int k) {
   const int kk = (int)std::min<int64_t>(n, k + guard);
   const int b = lanczos_block(n);
   const int span = 2;
-  const int mmax = (int)std::min<int64_t>(n, (int64_t)span * kk + 2 * b);
+  const int mmax = subspace_size(n, span, kk, b);
   const int ld = (mmax + b + 15) / 16 * 16;
   const double tol = c->o.eig_tol > 0 ? c->o.eig_tol : 1e-10;
   const double eps23 = std::pow(DBL_EPSILON, 2.0 / 3.0);
@@ -820,9 +838,7 @@ int block_lanczos_lean(vhci_ctx* c, int k) {
     }
     // Rayleigh-Ritz
     c->stats.eig_iterations += 1;
-    VCK(cudaMemcpy2DAsync(w.Yw.p, ld * sizeof(double), w.T.p, ld * sizeof(double),
-                          m * sizeof(double), m, cudaMemcpyDeviceToDevice, s));
-    VTRY(syevd_l(c, w, w.Yw.p, m, ld, w.theta.p));
+    VTRY(project_eigs(c, w, m, ld, std::min(kk, m)));
     VTRY(comm_bcast0(c, w.Yw.p, (int64_t)ld * m));
     VTRY(comm_bcast0(c, w.theta.p, m));
     const int nk = std::min(kk, m);
