@@ -141,6 +141,10 @@ __device__ __forceinline__ void load_slots(const uint64_t* p, ulonglong2& a, ulo
       : "l"(p));
 }
 
+// Presence bits of a table's keys by the upper hash bits, small enough for a block's shared memory.
+constexpr int kBitsLog = 20, kBitsWords = 1 << (kBitsLog - 5);
+__device__ __forceinline__ uint32_t bits_index(uint64_t h) { return (uint32_t)(h >> (64 - kBitsLog)); }
+
 // Returns the key's index or -1.
 template <int W>
 __device__ __forceinline__ int64_t hash_find(const HashView& t, const uint64_t (&k)[W],

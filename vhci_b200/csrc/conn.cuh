@@ -6,25 +6,63 @@
 
 namespace vhci {
 
+// One term record, read as one 32-byte load (as its own fields it takes four, and the L1 tag stage is
+// what the element sums are bound by).
+struct TermRegs {
+  double fc;
+  uint64_t a, b, c;  // bytes 8 .. 31 of TermDev: nk, mode[6], pw[6], dl[6]
+  __device__ __forceinline__ int nk() const { return (int)(a & 255u); }
+  template <int J> __device__ __forceinline__ int mode() const { return (int)((a >> (8 * (1 + J))) & 255u); }
+  template <int J> __device__ __forceinline__ int pw() const {
+    return (int)((J == 0 ? a >> 56 : b >> (8 * (J - 1))) & 255u);
+  }
+  template <int J> __device__ __forceinline__ int dl() const {
+    return (int)(int8_t)(J < 3 ? b >> (8 * (5 + J)) : c >> (8 * (J - 3)));
+  }
+};
+__device__ __forceinline__ TermRegs load_term(const TermDev* t) {
+  TermRegs r;
+  uint64_t fc;
+  asm("ld.global.nc.v4.u64 {%0,%1,%2,%3}, [%4];" : "=l"(fc), "=l"(r.a), "=l"(r.b), "=l"(r.c) : "l"(t));
+  r.fc = __longlong_as_double((long long)fc);
+  return r;
+}
+
 // Sum of a group's terms for ket key k: each term is fc * prod_j T[pw_j][q(mode_j)][dl_j], multiplied
 // left to right and summed in table order (the reference's AnharmPot product and Vij sum order).
 // Products and sums use explicit round-to-nearest operations so no multiply-add is contracted:
-// the results are the same bits as the reference's separate multiplies and adds.
+// the results are the same bits as the reference's separate multiplies and adds.  T: the ladder
+// table, in global or shared memory.
 template <int W>
-__device__ __forceinline__ double group_value(const ConnDev& cd, int tb, int te,
+__device__ __forceinline__ double group_value(const ConnDev& cd, const double* T, int tb, int te,
                                               const uint64_t (&k)[W], const KeyLayout& L) {
   const int qs = L.qmax + 1;
   double v = 0.0;
   for (int t = tb; t < te; ++t) {
-    const TermDev tm = cd.terms[t];
+    const TermRegs tm = load_term(cd.terms + t);
+    const int nk = tm.nk();
     double tv = tm.fc;
-    for (int j = 0; j < tm.nk; ++j) {
-      const int q = key_q<W>(k, tm.mode[j], L.mpw, L.bits);
-      tv = __dmul_rn(tv, __ldg(cd.T + ((int64_t)tm.pw[j] * qs + q) * 13 + tm.dl[j] + 6));
-    }
+    auto factor = [&](int mode, int pw, int dl) {
+      const int q = key_q<W>(k, mode, L.mpw, L.bits);
+      tv = __dmul_rn(tv, T[(pw * qs + q) * 13 + dl + 6]);
+    };
+    factor(tm.mode<0>(), tm.pw<0>(), tm.dl<0>());
+    if (nk > 1) factor(tm.mode<1>(), tm.pw<1>(), tm.dl<1>());
+    if (nk > 2) factor(tm.mode<2>(), tm.pw<2>(), tm.dl<2>());
+    if (nk > 3) factor(tm.mode<3>(), tm.pw<3>(), tm.dl<3>());
+    if (nk > 4) factor(tm.mode<4>(), tm.pw<4>(), tm.dl<4>());
+    if (nk > 5) factor(tm.mode<5>(), tm.pw<5>(), tm.dl<5>());
     v = __dadd_rn(v, tv);
   }
   return v;
+}
+
+// The ladder table of 4-bit keys (7 powers, 16 quanta, 13 changes) fits a block's shared memory.
+constexpr int kLadder4 = 7 * 16 * 13;
+__device__ __forceinline__ const double* stage_ladder(const ConnDev& cd, const KeyLayout& L, double* s) {
+  if (L.qmax != 15) return cd.T;
+  for (int x = threadIdx.x; x < kLadder4; x += blockDim.x) s[x] = cd.T[x];
+  return s;  // the caller synchronises the block
 }
 
 // Diagonal element: harmonic energy (Ham.cpp:211-220 operation order) plus the Delta = 0 terms
@@ -107,14 +145,18 @@ __device__ __forceinline__ void seg_find(const ConnDev& cd, uint64_t key, int& f
 
 // ---- the connection walk ---------------------------------------------------------------------
 
-// Probes in flight per lane, and the ring of possible hits they feed (31 waiting + 32 kWalkIlp new).
-constexpr int kWalkIlp = 2;
-constexpr unsigned kWalkRing = 128;
 constexpr int kWalkThreads = 128, kWalkWarps = kWalkThreads / 32;
 
-struct WalkScratch {        // one per warp, in shared memory
-  uint2 ring[kWalkRing];    // (index found, group)
+// Visits in flight per lane and the rings of one warp, in shared memory.  Plain: two probes a lane, a
+// ring of possible hits (31 waiting + 64 new).  Filtered: four visits a lane, a ring of the groups
+// whose target may be in the table (31 + 128), and of the possible hits (31 + 32).
+template <bool FILTER>
+struct WalkScratch {
+  static constexpr int kIlp = FILTER ? 4 : 2;
+  static constexpr unsigned kRing = FILTER ? 64 : 128, kMaybe = FILTER ? 256 : 1;
+  uint2 ring[kRing];        // (index found, group)
   int2 seg[32];             // segments of a batch: end in the flattened list, group - position
+  uint32_t maybe[kMaybe];   // groups that passed the filter
   uint8_t exc[128];         // excited modes of the state
 };
 
@@ -136,14 +178,21 @@ struct WalkScratch {        // one per warp, in shared memory
 // 3.2 ms, against visits that checked the bounds first and probed one slot at a time; two probes in
 // flight per lane beat four (13.3 : 15.7 ms, fewer registers), one 32-byte load beats a 16-byte one
 // over two slots (14.8 ms) or two of them over four (19.2 ms, four in flight).
-template <int W, class Hit>
+//
+// FILTER: the table's presence bits are in shared memory (sbits).  A visit is then one bit test (a few
+// bank conflicts instead of 32 L1 tag cycles), and only what passes is probed, 32 groups at a time
+// with every lane busy.
+template <int W, bool FILTER = false, class Hit>
 __device__ __forceinline__ void walk_connections(const ConnDev& cd, const HashView& tab,
                                                  const uint64_t (&k)[W], const KeyLayout& L,
-                                                 WalkScratch& ws, const uint32_t* binom, Hit&& hit) {
+                                                 WalkScratch<FILTER>& ws, const uint32_t* binom,
+                                                 const uint32_t* sbits, Hit&& hit) {
+  using WS = WalkScratch<FILTER>;
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const uint64_t hk = hash_lin<W>(k);
   unsigned head = 0, tail = 0;  // ring positions, the same in every lane
+  unsigned mhead = 0, mtail = 0;
 
   // hands on ring entries, 32 at a time (`all`: the rest too)
   auto drain = [&](bool all) {
@@ -153,7 +202,7 @@ __device__ __forceinline__ void walk_connections(const ConnDev& cd, const HashVi
       int64_t j = -1;
       uint32_t u = 0;
       if (lane < have) {
-        const uint2 r = ws.ring[(head + lane) % kWalkRing];
+        const uint2 r = ws.ring[(head + lane) % WS::kRing];
         u = r.y;
         uint64_t t[W];
 #pragma unroll
@@ -167,16 +216,52 @@ __device__ __forceinline__ void walk_connections(const ConnDev& cd, const HashVi
     }
     __syncwarp();
   };
+  // slots a, b hold the home of a target with linear hash h of group u: what matches goes to the ring
+  auto probe = [&](uint64_t h, uint32_t u, const ulonglong2& a, const ulonglong2& b) {
+    const uint32_t fp = hash_fp(h);
+    uint64_t s = hash_home(h, tab.mask);
+    SlotHit r = match_slots(a, b, fp);
+    for (uint64_t it = 0; r.more && it <= tab.mask; it += 4) {
+      s = (s + 4) & tab.mask;
+      ulonglong2 c, d;
+      load_slots(tab.slots + s, c, d);
+      r = match_slots(c, d, fp);
+    }
+    const bool on = r.idx != kNoIndex;
+    const unsigned m = __ballot_sync(full, on);
+    if (on) ws.ring[(tail + __popc(m & lanemask_lt())) % WS::kRing] = make_uint2(r.idx, u);
+    tail += __popc(m);
+  };
+  const ulonglong2 none = make_ulonglong2(kEmptySlot, kEmptySlot);
+  // probes the groups that passed the filter, 32 at a time (`all`: the rest too)
+  auto probe_maybe = [&](bool all) {
+    __syncwarp();
+    while (mtail - mhead >= 32 || (all && mtail != mhead)) {
+      const unsigned have = min(32u, mtail - mhead);
+      uint32_t u = 0;
+      uint64_t h = 0;
+      ulonglong2 a = none, b = none;
+      if (lane < have) {
+        u = ws.maybe[(mhead + lane) % WS::kMaybe];
+        h = hash_final(hk + __ldg(cd.hdelta + u));
+        load_slots(tab.slots + hash_home(h, tab.mask), a, b);
+      }
+      probe(h, u, a, b);
+      mhead += have;
+      if (tail - head >= 32) drain(false);
+    }
+    __syncwarp();
+  };
   // visits the flattened list of the segments in ws.seg
   auto visit = [&](int total) {
+    constexpr int ILP = WS::kIlp;
     int at = 0;
     int2 sg = ws.seg[0];
-    for (int f0 = 0; f0 < total; f0 += 32 * kWalkIlp) {
-      uint32_t u[kWalkIlp];
-      uint64_t h[kWalkIlp], s[kWalkIlp];
-      ulonglong2 a[kWalkIlp], b[kWalkIlp];
+    for (int f0 = 0; f0 < total; f0 += 32 * ILP) {
+      uint32_t u[ILP];
+      uint64_t h[ILP];
 #pragma unroll
-      for (int t = 0; t < kWalkIlp; ++t) {
+      for (int t = 0; t < ILP; ++t) {
         const int f = f0 + 32 * t + lane;
         h[t] = 0;
         u[t] = kNoIndex;
@@ -186,29 +271,28 @@ __device__ __forceinline__ void walk_connections(const ConnDev& cd, const HashVi
           h[t] = __ldg(cd.hdelta + u[t]);
         }
       }
+      if constexpr (FILTER) {
 #pragma unroll
-      for (int t = 0; t < kWalkIlp; ++t) {
-        h[t] = hash_final(hk + h[t]);
-        s[t] = hash_home(h[t], tab.mask);
-        if (u[t] != kNoIndex) load_slots(tab.slots + s[t], a[t], b[t]);
-        else a[t] = b[t] = make_ulonglong2(kEmptySlot, kEmptySlot);
-      }
-#pragma unroll
-      for (int t = 0; t < kWalkIlp; ++t) {
-        const uint32_t fp = hash_fp(h[t]);
-        SlotHit r = match_slots(a[t], b[t], fp);
-        for (uint64_t it = 0; r.more && it <= tab.mask; it += 4) {
-          s[t] = (s[t] + 4) & tab.mask;
-          ulonglong2 c, d;
-          load_slots(tab.slots + s[t], c, d);
-          r = match_slots(c, d, fp);
+        for (int t = 0; t < ILP; ++t) {
+          const uint32_t x = bits_index(hash_final(hk + h[t]));
+          const bool on = u[t] != kNoIndex && ((sbits[x >> 5] >> (x & 31)) & 1u);
+          const unsigned m = __ballot_sync(full, on);
+          if (on) ws.maybe[(mtail + __popc(m & lanemask_lt())) % WS::kMaybe] = u[t];
+          mtail += __popc(m);
         }
-        const bool on = r.idx != kNoIndex;
-        const unsigned m = __ballot_sync(full, on);
-        if (on) ws.ring[(tail + __popc(m & lanemask_lt())) % kWalkRing] = make_uint2(r.idx, u[t]);
-        tail += __popc(m);
+        if (mtail - mhead >= 32) probe_maybe(false);
+      } else {
+        ulonglong2 a[ILP], b[ILP];
+#pragma unroll
+        for (int t = 0; t < ILP; ++t) {
+          h[t] = hash_final(hk + h[t]);
+          if (u[t] != kNoIndex) load_slots(tab.slots + hash_home(h[t], tab.mask), a[t], b[t]);
+          else a[t] = b[t] = none;
+        }
+#pragma unroll
+        for (int t = 0; t < ILP; ++t) probe(h[t], u[t], a[t], b[t]);
+        if (tail - head >= 32) drain(false);
       }
-      if (tail - head >= 32) drain(false);
     }
   };
 
@@ -266,6 +350,7 @@ __device__ __forceinline__ void walk_connections(const ConnDev& cd, const HashVi
     visit(total);
     __syncwarp();
   }
+  if constexpr (FILTER) probe_maybe(true);
   drain(true);
 }
 

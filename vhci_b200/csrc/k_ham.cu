@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_hbuild(
     const int64_t* __restrict__ rowptr, int32_t* __restrict__ col, double* __restrict__ val,
     float* __restrict__ valf) {
   __shared__ uint32_t s_binom[kBinomElems];
-  __shared__ WalkScratch s_walk[kWalkWarps];
+  __shared__ WalkScratch<false> s_walk[kWalkWarps];
   fill_binom(s_binom);
   __syncthreads();
   const int64_t i = blockIdx.x * (int64_t)kWalkWarps + (threadIdx.x >> 5);
@@ -44,14 +44,14 @@ __global__ void __launch_bounds__(kWalkThreads) k_hbuild(
   load_key<W>(keys, row0 + stride * i, k);
   const int64_t pos = FILL ? rowptr[i] : 0;
   int cnt = 0;
-  walk_connections<W>(cd, basis, k, L, s_walk[threadIdx.x >> 5], s_binom, [&](int64_t j, uint32_t u) {
+  walk_connections<W>(cd, basis, k, L, s_walk[threadIdx.x >> 5], s_binom, nullptr, [&](int64_t j, uint32_t u) {
     const unsigned b = __ballot_sync(0xffffffffu, j >= 0);
     if (FILL) {
       if (j >= 0) {
         const int64_t p = pos + cnt + __popc(b & lanemask_lt());
         const GroupDev g = cd.groups[u];
         col[p] = (int32_t)j;
-        const double v = group_value<W>(cd, g.tb, g.te, k, L);
+        const double v = group_value<W>(cd, cd.T, g.tb, g.te, k, L);
         if (valf) valf[p] = (float)v; else val[p] = v;
       }
     } else if (stage.cap > 0) {
@@ -62,28 +62,95 @@ __global__ void __launch_bounds__(kWalkThreads) k_hbuild(
   if (!FILL && (threadIdx.x & 31) == 0) rowcnt[i] = cnt;
 }
 
+// The presence bits of the table's keys (zeroed by the caller).
+template <int W>
+__global__ void __launch_bounds__(256) k_hash_bits(const uint64_t* __restrict__ keys, int64_t n,
+                                                   uint32_t* __restrict__ bits) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    uint64_t k[W];
+    load_key<W>(keys, i, k);
+    const uint32_t x = bits_index(key_hash<W>(k));
+    atomicOr(bits + (x >> 5), 1u << (x & 31));
+  }
+}
+
+// The count pass with the table's presence bits in shared memory: one block of 32 warps per SM, each
+// warp taking the next row when it has done one.  Bound by instruction issue (65 a round of 32 visits,
+// 73 % of the issue slots).  Measured against the plain count pass: 200,000 states of 48 modes 13.3 ->
+// 7.7 ms, 40,000 of 30 modes 3.7 -> 1.7 ms, 150,001 of 15 modes 3.2 -> 2.5 ms.
+constexpr int kFiltThreads = 1024, kFiltWarps = kFiltThreads / 32;
+constexpr size_t kFiltSmem = kBitsWords * sizeof(uint32_t) + kFiltWarps * sizeof(WalkScratch<true>) +
+                             kBinomElems * sizeof(uint32_t);
+
+template <int W>
+__global__ void __launch_bounds__(kFiltThreads, 1) k_hcount_filtered(
+    const uint64_t* __restrict__ keys, int64_t row0, int64_t n, KeyLayout L, HashView basis, ConnDev cd,
+    const uint4* __restrict__ bits, int32_t* __restrict__ rowcnt, StageView stage,
+    unsigned long long* __restrict__ next) {
+  extern __shared__ __align__(16) unsigned char s_raw[];
+  uint32_t* s_bits = reinterpret_cast<uint32_t*>(s_raw);
+  WalkScratch<true>* s_walk = reinterpret_cast<WalkScratch<true>*>(s_bits + kBitsWords);
+  uint32_t* s_binom = reinterpret_cast<uint32_t*>(s_walk + kFiltWarps);
+  for (int x = threadIdx.x; x < kBitsWords / 4; x += kFiltThreads) reinterpret_cast<uint4*>(s_bits)[x] = bits[x];
+  fill_binom(s_binom);
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  for (;;) {
+    unsigned long long i = 0;
+    if (lane == 0) i = atomicAdd(next, 1ull);
+    i = __shfl_sync(0xffffffffu, i, 0);
+    if ((int64_t)i >= n) return;
+    uint64_t k[W];
+    load_key<W>(keys, row0 + (int64_t)i, k);
+    int cnt = 0;
+    walk_connections<W, true>(cd, basis, k, L, s_walk[threadIdx.x >> 5], s_binom, s_bits,
+                              [&](int64_t j, uint32_t u) {
+      const unsigned b = __ballot_sync(0xffffffffu, j >= 0);
+      if (stage.cap > 0) stage_hits(stage, (uint32_t)i, (uint32_t)cnt, j, u);
+      cnt += __popc(b);
+    });
+    if (lane == 0) rowcnt[i] = cnt;
+  }
+}
+
+template <int W>
+void hcount_filtered_launch(const uint64_t* keys, int64_t row0, int64_t n, KeyLayout L, HashView basis,
+                            int64_t nkeys, ConnDev cd, uint32_t* bits, int32_t* rowcnt, StageView stage,
+                            unsigned long long* next, cudaStream_t s) {
+  cudaFuncSetAttribute(k_hcount_filtered<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFiltSmem);
+  note_launch(); k_hash_bits<W><<<grid_for(nkeys, 256), 256, 0, s>>>(basis.keys, nkeys, bits);
+  note_launch(); k_hcount_filtered<W><<<148, kFiltThreads, kFiltSmem, s>>>(
+      keys, row0, n, L, basis, cd, reinterpret_cast<const uint4*>(bits), rowcnt, stage, next);
+}
+
 // The entries from kept batches, one warp per batch: every lane has an element to form and the
 // writes are consecutive, where a second walk costs as much as the first (fill of 200,000 states of
-// 48 modes 15.0 -> 0.7 ms, of 150,001 of 15 modes 5.8 -> 2.1 ms).  Bound by the term sums: a group
-// that changes one or two quanta has up to 16 terms, and the batch waits for its longest.
+// 48 modes 15.0 -> 0.42 ms, of 150,001 of 15 modes 5.8 -> 0.88 ms).  Bound by the L1 tag stage
+// (scattered group and term records): one 32-byte load a term and the ladder table in shared memory
+// took 2.1 ms to 0.88; sharing the groups' terms evenly among the lanes gave a tenth.
 template <int W>
 __global__ void __launch_bounds__(256) k_hfill_staged(
     const uint64_t* __restrict__ keys, int64_t row0, KeyLayout L, ConnDev cd, StageView stage,
     int64_t nbatch, const int64_t* __restrict__ rowptr, int32_t* __restrict__ col,
     double* __restrict__ val, float* __restrict__ valf) {
-  const int64_t b = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (b >= nbatch) return;
+  __shared__ double s_T[kLadder4];
+  const double* T = stage_ladder(cd, L, s_T);
+  __syncthreads();
   const int lane = threadIdx.x & 31;
-  const uint2 h = stage.batch[b];
-  const uint2 e = stage.pair[b * 32 + lane];
-  if (e.x == kNoIndex) return;
-  uint64_t k[W];
-  load_key<W>(keys, row0 + h.x, k);
-  const GroupDev g = cd.groups[e.y];
-  const double v = group_value<W>(cd, g.tb, g.te, k, L);
-  const int64_t p = rowptr[h.x] + h.y + lane;
-  col[p] = (int32_t)e.x;
-  if (valf) valf[p] = (float)v; else val[p] = v;
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t b = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); b < nbatch; b += warps) {
+    const uint2 e = stage.pair[b * 32 + lane];
+    if (e.x == kNoIndex) continue;
+    const uint2 h = stage.batch[b];
+    uint64_t k[W];
+    load_key<W>(keys, row0 + h.x, k);
+    const int2 terms = __ldg(reinterpret_cast<const int2*>(cd.groups + e.y));
+    const double v = group_value<W>(cd, T, terms.x, terms.y, k, L);
+    const int64_t p = rowptr[h.x] + h.y + lane;
+    col[p] = (int32_t)e.x;
+    if (valf) valf[p] = (float)v; else val[p] = v;
+  }
 }
 
 // One thread per state (the terms are the same for all, their loads broadcast).
@@ -115,7 +182,7 @@ template <int W>
 void hbuild_fill_staged_launch(const uint64_t* keys, int64_t row0, KeyLayout L, ConnDev cd,
                                StageView stage, int64_t nbatch, const int64_t* rowptr, int32_t* col,
                                double* val, float* valf, cudaStream_t s) {
-  note_launch(); k_hfill_staged<W><<<(unsigned)((nbatch + 7) / 8), 256, 0, s>>>(
+  note_launch(); k_hfill_staged<W><<<grid_for(nbatch * 32, 256, 148 * 24), 256, 0, s>>>(
       keys, row0, L, cd, stage, nbatch, rowptr, col, val, valf);
 }
 template <int W>
@@ -321,6 +388,17 @@ void hbuild_count(const uint64_t* keys, int64_t row0, int64_t stride, int64_t n,
                   HashView basis, ConnDev cd, int32_t* rowcnt, StageView stage, cudaStream_t s) {
   if (n <= 0) return;
   VHCI_DISPATCH_W(L.W, hbuild_count_launch, keys, row0, stride, n, L, basis, cd, rowcnt, stage, s);
+}
+
+bool hcount_filter_pays(int64_t n, int64_t nkeys) { return n >= 16384 && nkeys <= (1 << (kBitsLog - 1)); }
+
+void hcount_filtered(const uint64_t* keys, int64_t row0, int64_t n, KeyLayout L, HashView basis,
+                     int64_t nkeys, ConnDev cd, uint32_t* bits, int32_t* rowcnt, StageView stage,
+                     unsigned long long* next, cudaStream_t s) {
+  cudaMemsetAsync(bits, 0, kBitsWords * sizeof(uint32_t), s);
+  cudaMemsetAsync(next, 0, sizeof(unsigned long long), s);
+  VHCI_DISPATCH_W(L.W, hcount_filtered_launch, keys, row0, n, L, basis, nkeys, cd, bits, rowcnt, stage,
+                  next, s);
 }
 
 void hbuild_fill(const uint64_t* keys, int64_t row0, int64_t n, KeyLayout L, HashView basis,

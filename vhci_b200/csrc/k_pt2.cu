@@ -33,14 +33,14 @@ __global__ void __launch_bounds__(kWalkThreads) k_pt2_gen(
     int64_t a_lo, int64_t a_hi, int32_t* __restrict__ acount, StageView stage,
     const int64_t* __restrict__ arowptr, int32_t* __restrict__ ecol, double* __restrict__ eval) {
   __shared__ uint32_t s_binom[kBinomElems];
-  __shared__ WalkScratch s_walk[kWalkWarps];
+  __shared__ WalkScratch<false> s_walk[kWalkWarps];
   fill_binom(s_binom);
   __syncthreads();
   const int64_t i = blockIdx.x * (int64_t)kWalkWarps + (threadIdx.x >> 5);
   if (i >= n) return;
   uint64_t k[W];
   load_key<W>(keys, i, k);
-  walk_connections<W>(cd, pert, k, L, s_walk[threadIdx.x >> 5], s_binom, [&](int64_t a, uint32_t u) {
+  walk_connections<W>(cd, pert, k, L, s_walk[threadIdx.x >> 5], s_binom, nullptr, [&](int64_t a, uint32_t u) {
     if (a < a_lo || a >= a_hi) a = -1;
     if (!FILL) {
       if (a >= 0) atomicAdd(acount + (a - a_lo), 1);
@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_pt2_gen(
       const int64_t p = arowptr[a - a_lo] + atomicAdd(acount + (a - a_lo), 1);
       const GroupDev g = cd.groups[u];
       ecol[p] = (int32_t)i;
-      eval[p] = group_value<W>(cd, g.tb, g.te, k, L);
+      eval[p] = group_value<W>(cd, cd.T, g.tb, g.te, k, L);
     }
   });
 }
@@ -64,16 +64,16 @@ __global__ void __launch_bounds__(256) k_pt2_fill_staged(
     int32_t* __restrict__ ecol, double* __restrict__ eval) {
   const int64_t b = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
   if (b >= nbatch) return;
-  const uint32_t i = stage.batch[b].x;
   const uint2 e = stage.pair[b * 32 + (threadIdx.x & 31)];
   const int64_t a = e.x;
   if (e.x == kNoIndex || a < a_lo || a >= a_hi) return;
   const int64_t p = arowptr[a - a_lo] + atomicAdd(afill + (a - a_lo), 1);
+  const uint32_t i = stage.batch[b].x;
   uint64_t k[W];
   load_key<W>(keys, i, k);
-  const GroupDev g = cd.groups[e.y];
+  const int2 terms = __ldg(reinterpret_cast<const int2*>(cd.groups + e.y));
   ecol[p] = (int32_t)i;
-  eval[p] = group_value<W>(cd, g.tb, g.te, k, L);
+  eval[p] = group_value<W>(cd, cd.T, terms.x, terms.y, k, L);
 }
 
 template <int W>

@@ -13,7 +13,7 @@ void note_launch();
 long long launch_count();
 
 // ---- device table records ----
-struct GroupDev {   // one connection group (a fixed quanta change)
+struct __align__(8) GroupDev {   // one connection group (a fixed quanta change)
   int32_t tb, te;   // term range
   uint8_t nchg;
   uint8_t mode[6];
@@ -141,6 +141,13 @@ void hmerge_cross_scatter(const uint64_t* keys, int64_t ncross, const int64_t* x
 // the nbatch kept batches when none was lost.
 void hbuild_count(const uint64_t* keys, int64_t row0, int64_t stride, int64_t n, KeyLayout L,
                   HashView basis, ConnDev cd, int32_t* rowcnt, StageView stage, cudaStream_t s);
+// hbuild_count (stride 1) with presence bits of the table's nkeys keys in shared memory; bits:
+// kBitsWords words, next: one counter.  For many rows over a table that leaves the bits sparse: from
+// 16,384 rows (the bits cost each SM a 128 KB read) up to 2^19 keys (40 % of absent targets pass).
+bool hcount_filter_pays(int64_t n, int64_t nkeys);
+void hcount_filtered(const uint64_t* keys, int64_t row0, int64_t n, KeyLayout L, HashView basis,
+                     int64_t nkeys, ConnDev cd, uint32_t* bits, int32_t* rowcnt, StageView stage,
+                     unsigned long long* next, cudaStream_t s);
 void hbuild_fill(const uint64_t* keys, int64_t row0, int64_t n, KeyLayout L, HashView basis,
                  ConnDev cd, const int64_t* rowptr, int32_t* col, double* val, float* valf,
                  cudaStream_t s);
