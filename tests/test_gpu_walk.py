@@ -148,3 +148,26 @@ def test_pt2_sums(nm, n, k, chunk):
         num[j] += h * C[i]
     ref = (num ** 2 / (E - Ea[:, None])).sum(0)
     assert np.abs(dE - ref).max() <= 1e-12 * np.abs(ref).max()
+
+
+def test_pt2_chunks():
+    """More entries than one chunk holds: the rows of every chunk are filled and ordered by themselves."""
+    from vhci_b200 import VHCI
+    nm, n, k = 10, 4000, 7
+    freq, fcs = problem(nm, 4, 0.8)
+    q = states(nm, n, 5, 0.25)
+    rng = np.random.default_rng(6)
+    C = np.asfortranarray(rng.standard_normal((n, k)) / math.sqrt(n))
+    E = 0.5 * sum(freq) - np.linspace(4000.0, 2000.0, k)
+    out = []
+    for chunk in (0, 1 << 20):
+        with VHCI(problem=dict(freq=freq, cap=[8] * nm, ntot=1, fcs=fcs, eps1=0.0, nstate=k, pt2=1),
+                  pt2_chunk=chunk) as v:
+            v.set_basis(q)
+            v.set_vectors(C, E)
+            out.append(v.pt2(0.02))
+            entries = v.stats()["pt2_entries"]
+    assert entries > 2 << 20  # three chunks at least
+    assert out[0][1] == out[1][1]
+    # the same rows, summed over the perturbers in another grouping
+    assert np.abs(out[0][0] - out[1][0]).max() <= 1e-12 * np.abs(out[0][0]).max()

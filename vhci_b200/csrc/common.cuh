@@ -151,14 +151,15 @@ __device__ __forceinline__ int64_t hash_find(const HashView& t, const uint64_t (
                                              uint64_t h) {
   uint64_t s = hash_home(h, t.mask);
   const uint32_t fp = hash_fp(h);
-  for (uint64_t it = 0; it <= t.mask; ++it) {
-    const uint64_t v = __ldg(t.slots + s);
-    if (v == kEmptySlot) return -1;
-    if ((uint32_t)(v >> 32) == fp) {
-      const uint32_t idx = (uint32_t)v;
-      if (key_eq<W>(t.keys, idx, k)) return idx;
-    }
-    s = (s + 1) & t.mask;
+  for (uint64_t it = 0; it <= t.mask; it += 4) {
+    ulonglong2 a, b;
+    load_slots(t.slots + s, a, b);
+    if ((uint32_t)(a.x >> 32) == fp && key_eq<W>(t.keys, (uint32_t)a.x, k)) return (uint32_t)a.x;
+    if ((uint32_t)(a.y >> 32) == fp && key_eq<W>(t.keys, (uint32_t)a.y, k)) return (uint32_t)a.y;
+    if ((uint32_t)(b.x >> 32) == fp && key_eq<W>(t.keys, (uint32_t)b.x, k)) return (uint32_t)b.x;
+    if ((uint32_t)(b.y >> 32) == fp && key_eq<W>(t.keys, (uint32_t)b.y, k)) return (uint32_t)b.y;
+    if (b.y == kEmptySlot) return -1;
+    s = (s + 4) & t.mask;
   }
   return -1;
 }

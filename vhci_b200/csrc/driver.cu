@@ -75,22 +75,22 @@ int pt2(vhci_ctx* c, double eps2, double* dE_out, int64_t* n_pert) {
       nbatch = 0;
     }
     c->stats.pt2_entries += total;
-    // chunk the perturber range so one chunk's entries fit the budget: 12 bytes each plus, in the worst
-    // case, the same again as scratch for long-row ordering, in 40 % of the memory to be had
-    DBuf<int32_t> ecol;
-    DBuf<double> eval, part, dEd, Ed, ediag;
+    // chunk the perturber range so one chunk's entries fit the budget: 16 bytes each plus, in the worst
+    // case, the same again as scratch for long-row ordering, in 80 % of the memory to be had
+    DBuf<PtEntry> ent, ltmp;
+    DBuf<double> part, dEd, Ed, ediag;
     std::vector<int64_t> bounds, arow_h;
     // chunk bounds in perturber indices (arow_h is indexed from A0); one chunk needs only the total,
     // several the host copy of the row offsets
     auto chunk_entries = [&](int64_t a0, int64_t a1) {
       return arow_h.empty() ? total : arow_h[a1 - A0] - arow_h[a0 - A0];
     };
-    bool whole = c->o.pt2_chunk <= 0 && device_fits(c, (double)total * 30.0);
+    bool whole = c->o.pt2_chunk <= 0 && device_fits(c, (double)total * 40.0);
     for (;;) {
       bounds.assign(1, A0);
       if (!whole) {
         auto chunk_budget = [&] {
-          const int64_t e = c->o.pt2_chunk > 0 ? c->o.pt2_chunk : (int64_t)(device_available(c) * 0.4 / 12.0);
+          const int64_t e = c->o.pt2_chunk > 0 ? c->o.pt2_chunk : (int64_t)(device_available(c) * 0.4 / 16.0);
           return std::max<int64_t>(e, 1 << 20);
         };
         int64_t budget = chunk_budget();
@@ -117,11 +117,9 @@ int pt2(vhci_ctx* c, double eps2, double* dE_out, int64_t* n_pert) {
       int64_t maxchunk = 1;
       for (size_t q = 1; q < bounds.size(); ++q)
         maxchunk = std::max(maxchunk, chunk_entries(bounds[q - 1], bounds[q]));
-      cudaError_t e = ecol.reserve(maxchunk, s);
-      if (e == cudaSuccess) e = eval.reserve(maxchunk, s);
+      const cudaError_t e = ent.reserve(maxchunk, s);
       if (e == cudaErrorMemoryAllocation && whole) {  // not to be had in one: by the budget
         cudaGetLastError();
-        ecol.release(s);
         whole = false;
         continue;
       }
@@ -136,15 +134,14 @@ int pt2(vhci_ctx* c, double eps2, double* dE_out, int64_t* n_pert) {
     VCK(cudaMemsetAsync(dEd.p, 0, nopt * sizeof(double), s));
     VCK(h2d(c, Ed.p, c->E.data(), nopt * sizeof(double)));
     DBuf<int64_t> crow, lrow_d, loff_d;
-    DBuf<int32_t> lcol;
-    DBuf<double> lval;
-    DBuf<unsigned long long> lcnt;
+    DBuf<unsigned long long> lcnt, apos;
     VCK(lcnt.reserve(2, s));
     for (size_t q = 1; q < bounds.size(); ++q) {
       const int64_t a0 = bounds[q - 1], a1 = bounds[q], na = a1 - a0;
       // this chunk's row offsets, rebased on the device
       VCK(crow.reserve(na + 1, s));
-      pt2_rebase_rows(arow.p + (a0 - A0), na, crow.p, s);
+      VCK(apos.reserve(na + 1, s));
+      pt2_rebase_rows(arow.p + (a0 - A0), na, crow.p, apos.p, s);
       // rows too long for one warp's ordering, listed on the device; only their count and
       // entries come back, to size the scratch and the launch
       const int64_t maxlong = std::min<int64_t>(na, chunk_entries(a0, a1) / pt2_sort_long_min() + 1);
@@ -155,23 +152,19 @@ int pt2(vhci_ctx* c, double eps2, double* dE_out, int64_t* n_pert) {
       unsigned long long lc[2] = {0, 0};
       VCK(d2h(c, lc, lcnt.p, sizeof(lc)));
       VCK(cudaStreamSynchronize(s));
-      VCK(cudaMemsetAsync(acount.p, 0, na * sizeof(int32_t), s));
       if (nbatch > 0)
-        pt2_fill_staged(c->keys.p, L, conn_view(c), stage.view, (int64_t)nbatch, a0, a1, crow.p, acount.p,
-                        ecol.p, eval.p, s);
+        pt2_fill_staged(c->keys.p, L, conn_view(c), stage.view, (int64_t)nbatch, a0, a1, apos.p, ent.p, s);
       else
-        pt2_fill(c->keys.p, n, L, pv, conn_view(c), a0, a1, crow.p, acount.p, ecol.p, eval.p, s);
+        pt2_fill(c->keys.p, n, L, pv, conn_view(c), a0, a1, apos.p, ent.p, s);
       if (a1 == A1) stage.release(s);
       // fixed entry order per row (the fill's atomics leave it arbitrary): short rows by one warp
       // each, long rows by one block each
-      pt2_sort_rows(crow.p, na, ecol.p, eval.p, s);
+      pt2_sort_rows(crow.p, na, ent.p, s);
       if (lc[0] > 0) {
-        VCK(lcol.reserve((int64_t)lc[1], s));
-        VCK(lval.reserve((int64_t)lc[1], s));
+        VCK(ltmp.reserve((int64_t)lc[1], s));
         for (int64_t q0 = 0; q0 < (int64_t)lc[0]; q0 += 65535)
           pt2_sort_long(crow.p, lrow_d.p + q0, loff_d.p + q0,
-                        (int)std::min<int64_t>(65535, (int64_t)lc[0] - q0), ecol.p, eval.p, lcol.p,
-                        lval.p, s);
+                        (int)std::min<int64_t>(65535, (int64_t)lc[0] - q0), ent.p, ltmp.p, s);
       }
       VCK(ediag.reserve(std::max<int64_t>(na, 1), s));
       diag_energies(pkeys.p, a0, na, L, conn_view(c), ediag.p, s);
@@ -179,7 +172,7 @@ int pt2(vhci_ctx* c, double eps2, double* dE_out, int64_t* n_pert) {
       VCK(ev_r0r1.create());
       cudaEvent_t r0 = ev_r0r1.a, r1 = ev_r0r1.b;
       VCK(cudaEventRecord(r0, s));
-      if (!pt2_en(ediag.p, na, crow.p, ecol.p, eval.p, c->X.p, c->ldx, nopt, Ed.p, part.p, s))
+      if (!pt2_en(ediag.p, na, crow.p, ent.p, c->X.p, c->ldx, nopt, Ed.p, part.p, s))
         return fail(c, VHCI_E_INPUT, "PT2: unsupported state count");
       VCK(cudaEventRecord(r1, s));
       reduce_parts(part.p, nblk, nopt, dEd.p, s);
@@ -187,8 +180,8 @@ int pt2(vhci_ctx* c, double eps2, double* dE_out, int64_t* n_pert) {
       float ms = 0.f;
       cudaEventElapsedTime(&ms, r0, r1);
       c->stats.ms_pt2_reduce += ms;
-      const int64_t ent = chunk_entries(a0, a1);
-      c->stats.pt2_reduce_bytes += ent * (4 + 8) + ent * (int64_t)nopt * 8 + (a1 - a0) * (8 + 8 * L.W);
+      const int64_t nent = chunk_entries(a0, a1);
+      c->stats.pt2_reduce_bytes += nent * 16 + nent * (int64_t)nopt * 8 + (a1 - a0) * (8 + 8 * L.W);
     }
     VTRY(comm_sum(c, dEd.p, nopt));  // the ranks' shares of the perturber sum
     VCK(d2h(c, dE.data(), dEd.p, nopt * sizeof(double)));
@@ -198,9 +191,9 @@ int pt2(vhci_ctx* c, double eps2, double* dE_out, int64_t* n_pert) {
     VTRY(read_flags(c, &fl));
     if (fl & kFlagTableFull) return fail(c, VHCI_E_TABLE_FULL, "perturber hash full");
     pkeys.release(s); pslots.release(s); acount.release(s); arow.release(s); tmp.release(s);
-    ecol.release(s); eval.release(s); part.release(s); dEd.release(s); Ed.release(s); crow.release(s);
+    ent.release(s); apos.release(s); part.release(s); dEd.release(s); Ed.release(s); crow.release(s);
     ediag.release(s);
-    lrow_d.release(s); loff_d.release(s); lcol.release(s); lval.release(s); lcnt.release(s);
+    lrow_d.release(s); loff_d.release(s); ltmp.release(s); lcnt.release(s);
   }
   for (int j = 0; j < nopt; ++j) {
     c->E[j] += dE[j];

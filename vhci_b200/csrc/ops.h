@@ -244,37 +244,43 @@ bool small_eig(const double* T, int ldt, int m, int nk, double* theta, double* Y
 inline bool small_eig_good(double dev0, double dev1) { return dev0 <= 1e-3 && dev1 <= 1e-9; }
 
 // ---- PT2 (k_pt2.cu) ----
+// One entry H_ai = v of a perturber row.
+struct __align__(16) PtEntry {
+  double v;
+  int32_t i, pad;
+};
+static_assert(sizeof(PtEntry) == 16, "PtEntry layout");
 void pt2_count(const uint64_t* keys, int64_t n, KeyLayout L, HashView pert, ConnDev cd,
                int64_t a_lo, int64_t a_hi, int32_t* acount, StageView stage, cudaStream_t s);
+// The entries of perturbers [a_lo, a_hi), from the kept batches or by a walk; apos[a - a_lo]: the next
+// free place of each row.
 void pt2_fill_staged(const uint64_t* keys, KeyLayout L, ConnDev cd, StageView stage, int64_t nbatch,
-                     int64_t a_lo, int64_t a_hi, const int64_t* arowptr, int32_t* afill,
-                     int32_t* ecol, double* eval, cudaStream_t s);
-void pt2_fill(const uint64_t* keys, int64_t n, KeyLayout L, HashView pert, ConnDev cd,
-              int64_t a_lo, int64_t a_hi, const int64_t* arowptr, int32_t* afill, int32_t* ecol,
-              double* eval, cudaStream_t s);
-// Fused EN reduction over na perturber rows: num_a = sum_e eval_e X[ecol_e, :nopt];
+                     int64_t a_lo, int64_t a_hi, unsigned long long* apos, PtEntry* ent,
+                     cudaStream_t s);
+void pt2_fill(const uint64_t* keys, int64_t n, KeyLayout L, HashView pert, ConnDev cd, int64_t a_lo,
+              int64_t a_hi, unsigned long long* apos, PtEntry* ent, cudaStream_t s);
+// Fused EN reduction over na perturber rows: num_a = sum_e v_e X[i_e, :nopt];
 // part[blk][n] += num_a^2 / (E_n - ediag_a) (ediag: the perturbers' diagonal elements).
 // Every block writes all nopt columns of its part row; any nopt >= 1 (column tiles of 256);
 // returns false for nopt < 1 (nothing launched).
 int pt2_en_blocks();
-bool pt2_en(const double* ediag, int64_t na, const int64_t* arowptr, const int32_t* ecol,
-            const double* eval, const double* X, int ldx, int nopt, const double* E, double* part,
-            cudaStream_t s);
+bool pt2_en(const double* ediag, int64_t na, const int64_t* arowptr, const PtEntry* ent, const double* X,
+            int ldx, int nopt, const double* E, double* part, cudaStream_t s);
 // Orders the entries of each perturber row [arowptr[r], arowptr[r+1]) by ascending state index,
 // so the EN sums run in one fixed order.  pt2_sort_rows handles rows shorter than
 // pt2_sort_long_min() entries; pt2_sort_long the listed longer rows (rows[q], with scratch
-// tcol/tval of their total length, row q's part at soff[q]).
-void pt2_sort_rows(const int64_t* arowptr, int64_t nrows, int32_t* ecol, double* eval,
-                   cudaStream_t s);
+// tmp of their total length, row q's part at soff[q]).
+void pt2_sort_rows(const int64_t* arowptr, int64_t nrows, PtEntry* ent, cudaStream_t s);
 int pt2_sort_long_min();
-// crow[i] = arow[i] - arow[0] for i in [0, nrows]
-void pt2_rebase_rows(const int64_t* arow, int64_t nrows, int64_t* crow, cudaStream_t s);
+// crow[i] = apos[i] = arow[i] - arow[0] for i in [0, nrows]
+void pt2_rebase_rows(const int64_t* arow, int64_t nrows, int64_t* crow, unsigned long long* apos,
+                     cudaStream_t s);
 // rows of at least pt2_sort_long_min() entries into rows[] with disjoint scratch offsets soff[]
 // (cnt[0] += rows listed, cnt[1] += their entries; both zeroed by the caller)
 void pt2_list_long(const int64_t* arowptr, int64_t nrows, int64_t* rows, int64_t* soff,
                    unsigned long long* cnt, cudaStream_t s);
 void pt2_sort_long(const int64_t* arowptr, const int64_t* rows, const int64_t* soff, int nlong,
-                   int32_t* ecol, double* eval, int32_t* tcol, double* tval, cudaStream_t s);
+                   PtEntry* ent, PtEntry* tmp, cudaStream_t s);
 void reduce_parts(const double* part, int nblk, int nopt, double* out_accum, cudaStream_t s);
 
 }  // namespace vhci
