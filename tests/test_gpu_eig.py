@@ -1,6 +1,6 @@
-"""The small dense eigensolver through the dense path (bases up to 640 states), against LAPACK: one
-state, sizes on both sides of every cluster and register form, all eigenvectors wanted, and spectra it
-has to hand on to the library's solver (exactly degenerate states).
+"""The small dense eigensolver through the dense path (bases up to 2,000 states), against LAPACK: one
+state, sizes on both sides of every cluster, grid and register form and beyond the largest, all
+eigenvectors wanted, and spectra it has to hand on to the library's solver (exactly degenerate states).
 
 Tolerance: both solvers are backward stable, so an eigenvalue is within a few n 2^-53 ||H|| of the
 exact one; the vectors' residuals are held to the same size and their orthonormality to n 2^-53."""
@@ -40,7 +40,7 @@ def make(n, nstate, seed, nm=7, couple=1.0):
 
 @pytest.mark.parametrize("n,k", [(1, 1), (2, 2), (3, 1), (5, 5), (28, 10), (64, 64), (65, 7), (127, 40), (129, 129),
                                  (255, 100), (257, 30), (383, 20), (385, 385), (513, 64), (639, 10), (640, 640),
-                                 (641, 10)])
+                                 (641, 10), (700, 70), (1184, 20), (1185, 5), (1500, 150), (1799, 12), (1801, 3)])
 def test_dense_eigenpairs(n, k):
     with make(n, k, n) as v:
         check(v, k)

@@ -1,12 +1,13 @@
 // Lowest eigenpairs of the sparse Hamiltonian (reference: SparseDiagonalize / DenseDiagonalize,
 // Ham.cpp:347-379).  Small bases (and the first heat-bath step over the initial basis) use a dense
-// symmetric eigensolve on the device over the matrix expanded from its CSR form (k_eig.cu up to 640
+// symmetric eigensolve on the device over the matrix expanded from its CSR form (k_eig.cu up to 1,800
 // states, cuSOLVER's syevd beyond);
 // larger ones use the block thick-restart Lanczos of lanczos.cu, whose projections run on the
 // FP64 tensor pipe (k_proj.cu).  Convergence follows the reference eigensolver's rule
 // ||r_j|| <= tol * max(eps^(2/3), |theta_j|) for the wanted pairs (tol = 1e-10, Ham.cpp:363).
 #include <algorithm>
 #include <cstdlib>
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -48,14 +49,15 @@ int small_eigs(vhci_ctx* c, const double* T, int m, int ld, int nk, double* thet
   *done = false;
   if (m > kSmallEigMax) return VHCI_OK;
   VCK(c->eig_work.reserve(small_eig_elems(m, nk), c->st));
-  VCK(c->eig_dev.reserve(2, c->st));
+  VCK(c->eig_dev.reserve(kSmallEigDev, c->st));
   if (!small_eig(T, ld, m, nk, theta, Y, ld, c->eig_work.p, c->eig_dev.p, c->st)) return VHCI_OK;
-  double dev[2];
-  static_assert(sizeof(double) == sizeof(unsigned long long), "deviations are doubles' bits");
-  VCK(d2h(c, dev, c->eig_dev.p, sizeof(dev)));
+  unsigned long long w[kSmallEigDev];
+  VCK(d2h(c, w, c->eig_dev.p, sizeof(w)));
   VCK(cudaStreamSynchronize(c->st));
   VCK(cudaGetLastError());
-  *done = small_eig_good(dev[0], dev[1]);
+  double dev[2];
+  std::memcpy(dev, w, sizeof(dev));
+  *done = small_eig_good(dev[0], dev[1], w[3]);
   return VHCI_OK;
 }
 

@@ -3,7 +3,8 @@
 // eigensolvers behind Spectra and Eigen in the reference (Ham.cpp:347-379).
 //
 //   1. k_tridiag: Householder tridiagonalisation in one cluster of thread blocks that hold the whole
-//      matrix in their shared memory (rows dealt cyclically), one cluster barrier a column;
+//      matrix in their shared memory (rows dealt cyclically), one cluster barrier a column; beyond
+//      640 rows k_tridiag_grid, the same over all SMs;
 //   2. k_tri_vectors: one warp per wanted eigenvalue: Sturm counts at 32 points a round, then the
 //      vector from the twisted factorisation of T - lambda I;
 //   3. two Newton-Schulz steps Z <- Z (3 I - Z^T Z) / 2 take out the mixing of close eigenvalues
@@ -207,6 +208,179 @@ __global__ void __launch_bounds__(kTriThreads) k_tridiag(const double* __restric
   }
   // the last diagonal element (its row has had every update)
   if (r == (m - 1) % C && tid == 0) d[m - 1] = A[(size_t)((m - 1) / C) * m + m - 1];
+}
+
+// The same for matrices beyond one cluster's shared memory (m <= kSmallEigMax), over the whole GPU: row
+// l G + r of the matrix is kept by block r of G in its shared memory, and a thread works on columns
+// tid + kGridThreads c of all the block's rows, so that v, p and the row being reduced stay in its
+// registers.  p and the next row go through L2, and the blocks meet once a column: block 0 .. G - 1
+// each count up *ctr, and wait for all with a limit, after which *err is set and the kernel gives up
+// (launched cooperatively, so that all blocks run together).  Bound by latency: the meeting and the
+// exchange (2 us), two block sums, a square root and a division a column.  Measured at 672, 1,225 and
+// 1,500 rows 3.0, 6.1 and 7.6 ms (one cluster at 640: 2.9); the whole solve 4.0, 7.8 and 9.7 ms, where
+// cuSOLVER's syevd takes 7.8, 15.6 and 19.6.
+constexpr int kGridThreads = 512, kGridWarps = kGridThreads / 32;
+constexpr int kGridCols = 4;    // columns a thread: m <= 2048
+constexpr int kGridRows = 16;   // rows a block
+__device__ __forceinline__ double grid_block_sum(double v, double (&red)[2][kGridWarps], int& buf) {
+  const int lane = threadIdx.x & 31;
+  v = warp_sum(v);
+  if (lane == 0) red[buf][threadIdx.x >> 5] = v;
+  __syncthreads();
+  double t = red[buf][lane % kGridWarps];
+#pragma unroll
+  for (int o = kGridWarps / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  buf ^= 1;
+  return t;
+}
+
+__global__ void __launch_bounds__(kGridThreads, 1) k_tridiag_grid(
+    const double* __restrict__ T, int ldt, int m, double* __restrict__ d, double* __restrict__ e,
+    double* __restrict__ tau, double* __restrict__ V, double* xch, unsigned long long* ctr,
+    unsigned long long* err) {
+  extern __shared__ double sm[];
+  __shared__ double red[2][kGridWarps], s_v[kGridRows], s_p[kGridRows], s_x[2];
+  __shared__ double s_part[kGridWarps][kGridRows];
+  __shared__ int s_stop;
+  const int G = gridDim.x, r = blockIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  double* A = sm;  // local row l is row l G + r
+  const int rows = r < m ? (m - r + G - 1) / G : 0;
+  for (int l = wid; l < rows; l += kGridWarps) {
+    const int i = l * G + r;
+    for (int j = lane; j < m; j += 32)
+      A[(size_t)l * m + j] = i <= j ? T[i + (int64_t)j * ldt] : T[j + (int64_t)i * ldt];
+  }
+  int own[kGridCols];  // local row with this column's index, or -1
+  double v[kGridCols], p[kGridCols], x[kGridCols];
+#pragma unroll
+  for (int c = 0; c < kGridCols; ++c) {
+    const int j = tid + kGridThreads * c;
+    own[c] = j < m && j % G == r ? j / G : -1;
+    v[c] = p[c] = 0.0;
+    x[c] = j < m ? T[(int64_t)j * ldt] : 0.0;  // row 0
+  }
+  if (tid < kGridRows) s_v[tid] = s_p[tid] = 0.0;
+  if (tid == 0) s_stop = 0;
+  __syncthreads();
+  double t = 0.0;
+  int buf = 0;
+  for (int k = 0; k + 1 < m; ++k) {
+    const int par = k & 1;
+    if (k > 0) {
+      if (tid == 0) {  // all blocks have handed on p and row k
+        const unsigned long long want = (unsigned long long)k * G;
+        unsigned long long seen = 0;
+        int polls = 0;
+        do {
+          asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(seen) : "l"(ctr) : "memory");
+        } while (seen < want && ++polls < (1 << 21));
+        if (seen < want) {
+          s_stop = 1;
+          *err = 1;
+        }
+        __threadfence();
+      }
+      __syncthreads();
+      if (s_stop) return;
+#pragma unroll
+      for (int c = 0; c < kGridCols; ++c) {
+        const int j = tid + kGridThreads * c;
+        const bool in = j >= k && j < m;
+        p[c] = in ? __ldcg(xch + (size_t)par * 2 * m + j) : 0.0;
+        x[c] = in ? __ldcg(xch + (size_t)par * 2 * m + m + j) : 0.0;
+        if (own[c] >= 0) s_p[own[c]] = p[c];
+        if (j == k) s_x[0] = p[c];
+      }
+    }
+    double s = 0.0;
+#pragma unroll
+    for (int c = 0; c < kGridCols; ++c) s = fma(v[c], p[c], s);
+    const double K = -t * grid_block_sum(s, red, buf);
+    const double vk = k > 0 ? 1.0 : 0.0, ck = k > 0 ? s_x[0] + K : 0.0;
+    s = 0.0;
+#pragma unroll
+    for (int c = 0; c < kGridCols; ++c) {
+      const int j = tid + kGridThreads * c;
+      x[c] -= fma(vk, p[c], ck * v[c]);
+      if (j > k + 1) s = fma(x[c], x[c], s);
+      if (j == k + 1) s_x[1] = x[c];
+      if (j == k && r == 0) d[k] = x[c];
+    }
+    const double ss = grid_block_sum(s, red, buf), alpha = s_x[1];
+    double beta = alpha, inv = 0.0, tn = 0.0;
+    if (ss > 0.0 && k + 2 < m) {
+      beta = -copysign(sqrt(fma(alpha, alpha, ss)), alpha);
+      const double g = 1.0 / (beta * (alpha - beta));
+      inv = beta * g;
+      tn = (beta - alpha) * ((alpha - beta) * g);
+    }
+    if (r == 0 && tid == 0) {
+      e[k] = beta;
+      tau[k] = tn;
+    }
+    double vi[kGridRows], sum[kGridRows];
+#pragma unroll
+    for (int l = 0; l < kGridRows; ++l) {
+      vi[l] = s_v[l];
+      sum[l] = 0.0;
+    }
+    const int lr = (k + 1) / G;
+    const bool has_next = r == (k + 1) % G;
+#pragma unroll
+    for (int c = 0; c < kGridCols; ++c) {
+      const int j = tid + kGridThreads * c;
+      const double y = j > k + 1 ? x[c] * inv : (j == k + 1 ? 1.0 : 0.0);
+      if (j > k && j < m) {
+        if (r == k % G) V[(int64_t)k * m + j] = y;
+#pragma unroll
+        for (int l = 0; l < kGridRows; ++l) {
+          if (l < rows && l * G + r > k) {
+            const double a = A[(size_t)l * m + j] - fma(vi[l], p[c], fma(K, vi[l], s_p[l]) * v[c]);
+            A[(size_t)l * m + j] = a;
+            sum[l] = fma(a, y, sum[l]);
+            if (has_next && l == lr) __stcg(xch + (size_t)(par ^ 1) * 2 * m + m + j, a);
+          }
+        }
+      }
+      x[c] = y;
+    }
+    // sums of the rows over the warp, halving the rows a lane carries at each step: lane l ends with
+    // row l / 2
+#pragma unroll
+    for (int o = 16, h = kGridRows / 2; h > 0; o >>= 1, h >>= 1) {
+      const bool up = lane & o;
+#pragma unroll
+      for (int l = 0; l < kGridRows / 2; ++l)
+        if (l < h) {
+          const double give = up ? sum[l] : sum[l + h], keep = up ? sum[l + h] : sum[l];
+          sum[l] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    const double wsum = sum[0] + __shfl_xor_sync(0xffffffffu, sum[0], 1);
+    if ((lane & 1) == 0) s_part[wid][lane >> 1] = wsum;
+    __syncthreads();  // also: every thread has read s_v and s_p
+    {
+      double q = s_part[lane % kGridWarps][wid];  // row wid over the warps
+#pragma unroll
+      for (int o = kGridWarps / 2; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+      const int i = wid * G + r;
+      if (lane == 0 && wid < rows && i > k) __stcg(xch + (size_t)(par ^ 1) * 2 * m + i, tn * q);
+    }
+#pragma unroll
+    for (int c = 0; c < kGridCols; ++c) {
+      v[c] = x[c];
+      if (own[c] >= 0) s_v[own[c]] = x[c];
+    }
+    t = tn;
+    __syncthreads();
+    if (tid == 0) {
+      __threadfence();
+      atomicAdd(ctr, 1ull);
+    }
+  }
+  const int l = (m - 1) / G;
+  if (r == (m - 1) % G && tid == 0) d[m - 1] = A[(size_t)l * m + m - 1];
 }
 
 // Eigenvalue j (j < nk; the last warp takes the largest, for its value alone) of the tridiagonal
@@ -466,6 +640,51 @@ __global__ void __launch_bounds__(64) k_back(const double* __restrict__ Z, const
   }
 }
 
+// The same with one block of four warps per column (m <= 128 NR).
+template <int NR>
+__global__ void __launch_bounds__(128) k_back_block(const double* __restrict__ Z, const double* __restrict__ V,
+                                                    const double* __restrict__ tau, int m, int nk,
+                                                    double* __restrict__ Y, int ldy) {
+  __shared__ double red[2][4];
+  const int tid = threadIdx.x, lane = tid & 31, j = blockIdx.x;
+  double z[NR], v[NR], u[NR];
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    const int i = tid + 128 * r;
+    z[r] = i < m ? Z[(int64_t)j * m + i] : 0.0;
+  }
+  auto fetch = [&](int k, double (&w)[NR]) {
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+      const int i = tid + 128 * r;
+      w[r] = (k >= 0 && i > k && i < m) ? __ldg(V + (int64_t)k * m + i) : 0.0;
+    }
+  };
+  fetch(m - 3, v);
+  for (int k = m - 3; k >= 0; --k) {
+    fetch(k - 1, u);
+    const double tk = __ldg(tau + k);
+    double s = 0.0, s1 = 0.0;
+#pragma unroll
+    for (int r = 0; r < NR; ++r)
+      if (r & 1) s1 = fma(v[r], z[r], s1); else s = fma(v[r], z[r], s);
+    s = warp_sum(s + s1);
+    if (lane == 0) red[k & 1][tid >> 5] = s;
+    __syncthreads();
+    s = -tk * ((red[k & 1][0] + red[k & 1][1]) + (red[k & 1][2] + red[k & 1][3]));
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+      z[r] = fma(s, v[r], z[r]);
+      v[r] = u[r];
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    const int i = tid + 128 * r;
+    if (i < m) Y[(int64_t)j * ldy + i] = z[r];
+  }
+}
+
 constexpr size_t vec_smem(int m) { return (size_t)m * (3 + 2 * kVecWarps) * sizeof(double); }
 
 // Blocks of the cluster for m rows (its rows must fit the shared memory and kTriRows rounds): 16 (the
@@ -474,6 +693,10 @@ constexpr size_t vec_smem(int m) { return (size_t)m * (3 + 2 * kVecWarps) * size
 int tri_blocks(int m) {
   return m <= 32 ? 4 : (m < 256 ? 8 : 16);
 }
+
+// Blocks of the grid for m rows: eight rows a block, fewer when the GPU has no more SMs.
+int grid_blocks(int m) { return std::min(148, (m + 7) / 8); }
+size_t grid_smem(int m) { return (size_t)((m + grid_blocks(m) - 1) / grid_blocks(m)) * m * sizeof(double); }
 
 using TriKernel = void (*)(const double*, int, int, double*, double*, double*, double*, double*);
 TriKernel tri_kernel(int m) {
@@ -492,12 +715,13 @@ bool eig_attributes() {
   std::call_once(g_eig_once[dev], [dev] {
     bool ok = cudaFuncSetAttribute(k_tri_vectors, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)vec_smem(kSmallEigMax)) == cudaSuccess;
-    for (int m : {64, 128, 192, 256, 384, kSmallEigMax}) {
+    for (int m : {64, 128, 192, 256, 384, kClusterEigMax}) {
       const TriKernel k = tri_kernel(m);
       ok = ok && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) == cudaSuccess &&
            cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
     }
-    g_eig_ok[dev] = ok;
+    g_eig_ok[dev] = ok && cudaFuncSetAttribute(k_tridiag_grid, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)grid_smem(kSmallEigMax)) == cudaSuccess;
     if (!g_eig_ok[dev]) cudaGetLastError();
   });
   return g_eig_ok[dev];
@@ -506,8 +730,8 @@ bool eig_attributes() {
 }  // namespace
 
 size_t small_eig_elems(int m, int nk) {
-  // d, e, tau; the row exchange; V; two vector blocks; S
-  return 5 * (size_t)m + (size_t)m * m + 2 * (size_t)m * nk + (size_t)nk * nk;
+  // d, e, tau; the exchange; V; two vector blocks; S
+  return 7 * (size_t)m + (size_t)m * m + 2 * (size_t)m * nk + (size_t)nk * nk;
 }
 
 bool small_eig(const double* T, int ldt, int m, int nk, double* theta, double* Y, int ldy, double* work,
@@ -518,31 +742,43 @@ bool small_eig(const double* T, int ldt, int m, int nk, double* theta, double* Y
   double* e = d + m;
   double* tau = e + m;
   double* rowx = tau + m;
-  double* V = rowx + 2 * m;
+  double* V = rowx + 4 * m;
   double* Za = V + (size_t)m * m;
   double* Zb = Za + (size_t)m * nk;
   double* S = Zb + (size_t)m * nk;
-  const int C = tri_blocks(m);
+  cudaMemsetAsync(dev, 0, kSmallEigDev * sizeof(unsigned long long), s);
+  const bool cluster = m <= kClusterEigMax;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(C);
-  cfg.blockDim = dim3(kTriThreads);
-  cfg.dynamicSmemBytes = tri_smem(m, C);
   cfg.stream = s;
   cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = C;
-  at.val.clusterDim.y = at.val.clusterDim.z = 1;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
+  cudaError_t err;
   note_launch();
-  if (cudaLaunchKernelEx(&cfg, tri_kernel(m), T, ldt, m, d, e, tau, V, rowx) != cudaSuccess) {
+  if (cluster) {
+    const int C = tri_blocks(m);
+    cfg.gridDim = dim3(C);
+    cfg.blockDim = dim3(kTriThreads);
+    cfg.dynamicSmemBytes = tri_smem(m, C);
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = C;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    err = cudaLaunchKernelEx(&cfg, tri_kernel(m), T, ldt, m, d, e, tau, V, rowx);
+  } else {
+    cfg.gridDim = dim3(grid_blocks(m));
+    cfg.blockDim = dim3(kGridThreads);
+    cfg.dynamicSmemBytes = grid_smem(m);
+    at.id = cudaLaunchAttributeCooperative;
+    at.val.cooperative = 1;
+    err = cudaLaunchKernelEx(&cfg, k_tridiag_grid, T, ldt, m, d, e, tau, V, rowx, dev + 2, dev + 3);
+  }
+  if (err != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
   note_launch();
   k_tri_vectors<<<(nk + 1 + kVecWarps - 1) / kVecWarps, 32 * kVecWarps, vec_smem(m), s>>>(d, e, m, nk,
                                                                                           theta, Za);
-  cudaMemsetAsync(dev, 0, 2 * sizeof(unsigned long long), s);
   const int tr = (nk + 7) / 8, tc = (nk + 31) / 32, tm = (m + 7) / 8;
   for (int it = 0; it < 2; ++it) {
     note_launch();
@@ -556,7 +792,8 @@ bool small_eig(const double* T, int ldt, int m, int nk, double* theta, double* Y
   else if (m <= 128) k_back<4, 4><<<g, 64, 0, s>>>(Za, V, tau, m, nk, Y, ldy);
   else if (m <= 256) k_back<8, 4><<<g, 64, 0, s>>>(Za, V, tau, m, nk, Y, ldy);
   else if (m <= 384) k_back<12, 3><<<g, 64, 0, s>>>(Za, V, tau, m, nk, Y, ldy);
-  else k_back<20, 2><<<g, 64, 0, s>>>(Za, V, tau, m, nk, Y, ldy);
+  else if (cluster) k_back<20, 2><<<g, 64, 0, s>>>(Za, V, tau, m, nk, Y, ldy);
+  else k_back_block<15><<<nk, 128, 0, s>>>(Za, V, tau, m, nk, Y, ldy);
   return true;
 }
 

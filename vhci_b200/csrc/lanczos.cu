@@ -222,14 +222,6 @@ int project_eigs(vhci_ctx* c, LWork& w, int m, int ld, int nk) {
   return syevd_l(c, w, w.Yw.p, m, ld, w.theta.p);
 }
 
-// Subspace size span kk + 2 b; one up to a tenth above what k_eig.cu takes is cut to that (fewer steps
-// a cycle, but a Rayleigh-Ritz step of 3.7 ms instead of 7).
-int subspace_size(int64_t n, int span, int kk, int b) {
-  int64_t m = (int64_t)span * kk + 2 * b;
-  if (m > kSmallEigMax && 10 * m <= 11 * kSmallEigMax) m = kSmallEigMax;
-  return (int)std::min<int64_t>(n, m);
-}
-
 // Orthonormalise the nb columns of (B, ld) into (out, ldo) by SVQB with the small Gram matrix
 // decomposed on the host; directions below 1e-12 of the largest are dropped.  *r = rank.
 int svqb_small(vhci_ctx* c, LWork& w, int64_t n, const double* B, int ld, int nb, double* out,
@@ -418,7 +410,7 @@ static int lanczos_guard(int k) {
 // and the gathered vector block (n x b).
 static double lanczos_bytes(int64_t n, int64_t rows, int k, int span, int b, bool mixed) {
   const int kk = (int)std::min<int64_t>(n, k + lanczos_guard(k));
-  const int mmax = subspace_size(n, span, kk, b);
+  const int mmax = (int)std::min<int64_t>(n, (int64_t)span * kk + 2 * b);
   const int ld = (mmax + b + 15) / 16 * 16;
   return 8.0 * (double)rows * ((mixed ? 2.0 : 1.0) * (ld + kk) + 3.0 * b) + (rows < n ? 8.0 * n * b : 0.0);
 }
@@ -427,7 +419,7 @@ static double lanczos_bytes(int64_t n, int64_t rows, int k, int span, int b, boo
 // the compact copy (n x b each), the rotation chunk, and the output Ritz block (n x kk).
 static double lanczos_lean_bytes(int64_t n, int64_t rows, int k, int b, int span = 2) {
   const int kk = (int)std::min<int64_t>(n, k + lanczos_guard(k));
-  const int mmax = subspace_size(n, span, kk, b);
+  const int mmax = (int)std::min<int64_t>(n, (int64_t)span * kk + 2 * b);
   const int ld = (mmax + b + 15) / 16 * 16;
   return 8.0 * (double)rows * (ld + 3.0 * b + kk) + (rows < n ? 8.0 * n * (b + kk) : 0.0) + 2.6e8;
 }
@@ -468,7 +460,7 @@ int block_lanczos_impl(vhci_ctx* c, int k, bool dev_svqb) {
   if (const char* e = std::getenv("VHCI_LANCZOS_SPAN")) span = std::max(2, std::min(8, std::atoi(e)));
   if (!device_fits(c, lanczos_bytes(n, nl, k, span, b, c->o.precision == 1) + 1e9))
     return block_lanczos_lean(c, k);
-  const int mmax = subspace_size(n, span, kk, b);
+  const int mmax = (int)std::min<int64_t>(n, (int64_t)span * kk + 2 * b);
   const bool dev = dev_svqb && n >= 8 * (int64_t)mmax;
   // row stride padded to whole 128-byte lines so every b-column gather touches whole L2 lines
   const int ld = (mmax + b + 15) / 16 * 16;
@@ -729,7 +721,7 @@ int block_lanczos_lean(vhci_ctx* c, int k) {
   const int kk = (int)std::min<int64_t>(n, k + guard);
   const int b = lanczos_block(n);
   const int span = 2;
-  const int mmax = subspace_size(n, span, kk, b);
+  const int mmax = (int)std::min<int64_t>(n, (int64_t)span * kk + 2 * b);
   const int ld = (mmax + b + 15) / 16 * 16;
   const double tol = c->o.eig_tol > 0 ? c->o.eig_tol : 1e-10;
   const double eps23 = std::pow(DBL_EPSILON, 2.0 / 3.0);

@@ -231,17 +231,21 @@ void svqb_factor(const double* part, int nparts, int nb, double* M, int* rank_sh
 // ---- small dense eigensolver (k_eig.cu) ----
 // The nk lowest eigenpairs of the symmetric m x m matrix whose upper triangle is in T (column-major,
 // ldt), m <= kSmallEigMax: theta[0..nk) ascending, and the largest eigenvalue in theta[m - 1]; the
-// vectors in the columns of Y (ldy).  work: small_eig_elems(m, nk) doubles.  dev[0], dev[1]: the
-// vectors' largest deviations from orthonormality before the first and before the second correction
-// (as doubles' bits); the result is good when small_eig_good says so.  Returns false (nothing usable
-// launched) when the size or the device does not allow it.
-constexpr int kSmallEigMax = 640;
+// vectors in the columns of Y (ldy).  work: small_eig_elems(m, nk) doubles.  dev (kSmallEigDev words):
+// the vectors' largest deviations from orthonormality before the first and before the second
+// correction (as doubles' bits), a counter, and a word that is not zero when a wait ran out; the
+// result is good when small_eig_good says so.  Returns false (nothing usable launched) when the size
+// or the device does not allow it.  Up to kClusterEigMax rows one thread block cluster does the
+// tridiagonalisation, beyond that the whole GPU.
+constexpr int kClusterEigMax = 640, kSmallEigMax = 1800, kSmallEigDev = 4;
 size_t small_eig_elems(int m, int nk);
 bool small_eig(const double* T, int ldt, int m, int nk, double* theta, double* Y, int ldy, double* work,
                unsigned long long* dev, cudaStream_t s);
 // Each correction squares the deviation (times 3/4 of the number of vectors at worst): from these
 // bounds the second leaves less than 1e-15 of it.
-inline bool small_eig_good(double dev0, double dev1) { return dev0 <= 1e-3 && dev1 <= 1e-9; }
+inline bool small_eig_good(double dev0, double dev1, unsigned long long err) {
+  return dev0 <= 1e-3 && dev1 <= 1e-9 && err == 0;
+}
 
 // ---- PT2 (k_pt2.cu) ----
 // One entry H_ai = v of a perturber row.
