@@ -99,6 +99,7 @@ struct HandleSet {
   cublasHandle_t blas;
   cusolverDnHandle_t sol;
   double dev_bytes;  // the device's memory
+  double* pinned;    // page-locked host memory for small results
 };
 std::mutex g_handle_mu;
 std::vector<HandleSet> g_handle_pool;
@@ -123,6 +124,7 @@ static int acquire_handles(vhci_ctx* c) {
         c->blas = g_handle_pool[i].blas;
         c->sol = g_handle_pool[i].sol;
         c->dev_bytes = g_handle_pool[i].dev_bytes;
+        c->pinned = g_handle_pool[i].pinned;
         g_handle_pool.erase(g_handle_pool.begin() + i);
         return VHCI_OK;
       }
@@ -135,11 +137,13 @@ static int acquire_handles(vhci_ctx* c) {
   size_t freeb = 0, totb = 0;
   VCK(cudaMemGetInfo(&freeb, &totb));
   c->dev_bytes = (double)totb;
+  VCK(cudaMallocHost((void**)&c->pinned, kPinnedDoubles * sizeof(double)));
   return VHCI_OK;
 }
 
 static void release_handles(vhci_ctx* c) {
-  if (!c->st || !c->blas || !c->sol) {  // a partly built set is not pooled
+  if (!c->st || !c->blas || !c->sol || !c->pinned) {  // a partly built set is not pooled
+    if (c->pinned) cudaFreeHost(c->pinned);
     if (c->blas) cublasDestroy(c->blas);
     if (c->sol) cusolverDnDestroy(c->sol);
     if (c->st) cudaStreamDestroy(c->st);
@@ -147,7 +151,7 @@ static void release_handles(vhci_ctx* c) {
   }
   cudaStreamSynchronize(c->st);
   std::lock_guard<std::mutex> lk(g_handle_mu);
-  g_handle_pool.push_back(HandleSet{c->o.device, c->o.stream_priority, c->st, c->blas, c->sol, c->dev_bytes});
+  g_handle_pool.push_back(HandleSet{c->o.device, c->o.stream_priority, c->st, c->blas, c->sol, c->dev_bytes, c->pinned});
 }
 
 // Layout-dependent tables (packed key deltas, ladder factors) and the layout-free ones.

@@ -58,6 +58,8 @@ struct DevGroups {
   }
 };
 
+constexpr int kPinnedDoubles = 8192;
+
 struct Status {
   int code = VHCI_OK;
   std::string msg;
@@ -78,6 +80,7 @@ struct vhci_ctx {
   cusolverDnHandle_t sol = nullptr;
   cudaEvent_t ev_a = nullptr, ev_b = nullptr;
   double dev_bytes = 0;  // the device's memory
+  double* pinned = nullptr;  // kPinnedDoubles of page-locked host memory
 
   vhci::KeyLayout L{};
 
@@ -146,7 +149,7 @@ struct vhci_ctx {
   vhci::DBuf<double> solver_work;
   vhci::DBuf<int> solver_info;
   vhci::DBuf<double> eig_work;
-  vhci::DBuf<unsigned long long> eig_dev;
+  vhci::DBuf<double> eig_dev;
 
   std::string err;
   vhci_stats stats{};

@@ -45,19 +45,31 @@ int syevd(vhci_ctx* c, double* A, int m, int lda, double* w) {
 
 }  // namespace
 
-int small_eigs(vhci_ctx* c, const double* T, int m, int ld, int nk, double* theta, double* Y, bool* done) {
-  *done = false;
+int small_eigs_start(vhci_ctx* c, const double* T, int m, int ld, int nk, double* theta, double* Y,
+                     double* words, bool* started) {
+  *started = false;
   if (m > kSmallEigMax) return VHCI_OK;
   VCK(c->eig_work.reserve(small_eig_elems(m, nk), c->st));
+  *started = small_eig(T, ld, m, nk, theta, Y, ld, c->eig_work.p,
+                       reinterpret_cast<unsigned long long*>(words), c->st);
+  return VHCI_OK;
+}
+
+bool small_eigs_verdict(const double* words) {
+  unsigned long long err;
+  std::memcpy(&err, words + 3, sizeof(err));
+  return small_eig_good(words[0], words[1], err);
+}
+
+int small_eigs(vhci_ctx* c, const double* T, int m, int ld, int nk, double* theta, double* Y, bool* done) {
   VCK(c->eig_dev.reserve(kSmallEigDev, c->st));
-  if (!small_eig(T, ld, m, nk, theta, Y, ld, c->eig_work.p, c->eig_dev.p, c->st)) return VHCI_OK;
-  unsigned long long w[kSmallEigDev];
+  VTRY(small_eigs_start(c, T, m, ld, nk, theta, Y, c->eig_dev.p, done));
+  if (!*done) return VHCI_OK;
+  double w[kSmallEigDev];
   VCK(d2h(c, w, c->eig_dev.p, sizeof(w)));
   VCK(cudaStreamSynchronize(c->st));
   VCK(cudaGetLastError());
-  double dev[2];
-  std::memcpy(dev, w, sizeof(dev));
-  *done = small_eig_good(dev[0], dev[1], w[3]);
+  *done = small_eigs_verdict(w);
   return VHCI_OK;
 }
 

@@ -105,6 +105,11 @@ int dense_eigs(vhci_ctx* c, int keep);
 // values in theta, vectors in Y (ld).  *done = false when the caller has to use another solver.
 // Synchronises.
 int small_eigs(vhci_ctx* c, const double* T, int m, int ld, int nk, double* theta, double* Y, bool* done);
+// The same without the wait: started, with the kSmallEigDev words that tell whether it worked in device
+// memory (`words`); *started = false when it cannot be tried.
+int small_eigs_start(vhci_ctx* c, const double* T, int m, int ld, int nk, double* theta, double* Y,
+                     double* words, bool* started);
+bool small_eigs_verdict(const double* words);
 // Block thick-restart Lanczos (lanczos.cu).
 int block_lanczos(vhci_ctx* c, int k);
 int lanczos_block(int64_t n);

@@ -1,6 +1,7 @@
 // Basis-state kernels: prefix scans, key packing, the basis hash, Cmax, heat-bath candidate
 // generation with warp-free load balancing, candidate compaction and an LSD radix sort of packed
 // keys.  All are memory-bound integer/byte kernels sized in grid-stride loops.
+#include <algorithm>
 #include <atomic>
 
 #include "ops.h"
@@ -465,9 +466,56 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_scatter(
   }
 }
 
+// Few keys: one block sorts them in shared memory (bitonic network on whole keys, padded with the
+// largest), one launch where the passes take three for every eight bits.  2,048 keys of one to three
+// words fit: 40 us of launches less for 24 bits, 80 us for 48.
+constexpr int kSmallSort = 2048;
+template <int W>
+constexpr int small_sort_keys() { return W <= 3 ? kSmallSort : 512; }
+
+template <int W>
+__global__ void __launch_bounds__(1024) k_sort_small(uint64_t* __restrict__ keys, int n, int P) {
+  __shared__ uint64_t sk[small_sort_keys<W>() * W];  // [W][P]
+  for (int x = threadIdx.x; x < P; x += blockDim.x)
+#pragma unroll
+    for (int w = 0; w < W; ++w) sk[w * P + x] = x < n ? keys[(int64_t)x * W + w] : ~0ull;
+  __syncthreads();
+  for (int k = 2; k <= P; k <<= 1)
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      for (int t = threadIdx.x; t < P / 2; t += blockDim.x) {
+        const int x = 2 * t - (t & (j - 1)), y = x + j;
+        bool gt = false, lt = false;  // the last word is the most significant
+#pragma unroll
+        for (int w = W - 1; w >= 0; --w) {
+          const uint64_t a = sk[w * P + x], b = sk[w * P + y];
+          gt = gt || (!lt && a > b);
+          lt = lt || (!gt && a < b);
+        }
+        if (((x & k) == 0) ? gt : lt) {
+#pragma unroll
+          for (int w = 0; w < W; ++w) {
+            const uint64_t a = sk[w * P + x];
+            sk[w * P + x] = sk[w * P + y];
+            sk[w * P + y] = a;
+          }
+        }
+      }
+      __syncthreads();
+    }
+  for (int x = threadIdx.x; x < n; x += blockDim.x)
+#pragma unroll
+    for (int w = 0; w < W; ++w) keys[(int64_t)x * W + w] = sk[w * P + x];
+}
+
 template <int W>
 void radix_launch(uint64_t* keys, uint64_t* alt, int64_t n, int nbits, int64_t* hist,
                   cudaStream_t s) {
+  if (n <= small_sort_keys<W>()) {
+    int P = 2;
+    while (P < n) P <<= 1;
+    note_launch(); k_sort_small<W><<<1, std::min(1024, std::max(32, P / 2)), 0, s>>>(keys, (int)n, P);
+    return;
+  }
   const int nblk = (int)((n + kRadixTile - 1) / kRadixTile);
   const int64_t hn = (int64_t)256 * nblk;
   int64_t* offs = hist;

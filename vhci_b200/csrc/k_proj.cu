@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(kSvqbThreads) k_svqb_factor(const double* __re
                                                               int nparts, int nb,
                                                               double* __restrict__ M,
                                                               int* __restrict__ rank_short) {
-  __shared__ double ps[4][256], A[16][17], R[16][17];
+  __shared__ double ps[4][256], A[16][17], R[16][17], rinv[16];
   const int tid = threadIdx.x;
   {  // four groups of threads add the partial sums q, q + 4, ...; then the groups in order
     const int x = tid & 255, q0 = tid >> 8;
@@ -344,8 +344,9 @@ __global__ void __launch_bounds__(kSvqbThreads) k_svqb_factor(const double* __re
     if (i < nb) {
       const double piv = __shfl_sync(~0u, a[i], i);
       const bool ok = piv > 1e-12;
-      const double inv = ok ? 1.0 / sqrt(piv) : 0.0;
+      const double inv = ok ? rsqrt(piv) : 0.0;
       if (!ok && c == i) lost = 1;
+      if (c == i) rinv[i] = inv;
       r[i] = (in && c >= i) ? a[i] * inv : 0.0;
       if (in) R[i][c] = r[i];
       __syncwarp();
@@ -364,8 +365,7 @@ __global__ void __launch_bounds__(kSvqbThreads) k_svqb_factor(const double* __re
 #pragma unroll
       for (int j = 0; j < 16; ++j)
         if (j > i && j <= c) t = fma(-R[i][j], x[j], t);
-      const double p = R[i][i];
-      x[i] = p > 0.0 ? t / p : 0.0;
+      x[i] = t * rinv[i];
     }
   }
   const unsigned some = __ballot_sync(~0u, lost);
@@ -374,6 +374,43 @@ __global__ void __launch_bounds__(kSvqbThreads) k_svqb_factor(const double* __re
   for (int i = 0; i < 16; ++i) {
     const double di = __shfl_sync(~0u, d, i);
     if (i < nb && in) M[i + (int64_t)c * nb] = lost ? 0.0 : di * x[i];
+  }
+}
+
+// One block per 32 vectors; the partial sums of G are added as in k_svqb_factor.
+__global__ void __launch_bounds__(1024) k_krylov_residuals(const double* __restrict__ Y, int ldy, int nk,
+                                                           const double* __restrict__ part, int nparts,
+                                                           int P, double* __restrict__ rn2) {
+  __shared__ double ps[4][256], G[256];
+  const int tid = threadIdx.x;
+  {
+    const int x = tid & 255, q0 = tid >> 8;
+    double t = 0.0;
+    if (x < P * P)
+#pragma unroll 8
+      for (int q = q0; q < nparts; q += 4) t += part[(int64_t)q * P * P + x];
+    ps[q0][x] = t;
+  }
+  __syncthreads();
+  if (tid < P * P) G[tid] = ((ps[0][tid] + ps[1][tid]) + ps[2][tid]) + ps[3][tid];
+  __syncthreads();
+  const int j = blockIdx.x * 32 + (tid >> 5), a = tid & 31;
+  if (j >= nk) return;
+  double q = 0.0;
+  if (a < P) {
+    const double* y = Y + (int64_t)j * ldy;
+    for (int e = 0; e < P; ++e) q = fma(G[a * P + e], y[e], q);
+    q *= y[a];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(~0u, q, o);
+  if (a == 0) rn2[j] = q;
+}
+
+__global__ void k_restart_matrix(double* __restrict__ T, int ld, const double* __restrict__ theta, int nk) {
+  for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < ld * ld; x += gridDim.x * blockDim.x) {
+    const int c = x / ld, r = x - c * ld;
+    T[x] = r == c && r < nk ? theta[r] : 0.0;
   }
 }
 
@@ -501,6 +538,18 @@ int proj_rows_self(const double* A, int lda, const double* S, int lds, int64_t n
   else
     k_rows<2, true><<<g, kThreads, rows_self_smem<2>(M), s>>>(A, lda, S, lds, n, M, P, -1.0, 1.0, W, ldw, t);
   return g;
+}
+
+void krylov_residuals(const double* Y, int ldy, int nk, const double* part, int nparts, int P,
+                      double* rn2, cudaStream_t s) {
+  if (nk <= 0) return;
+  note_launch();
+  k_krylov_residuals<<<(nk + 31) / 32, 1024, 0, s>>>(Y, ldy, nk, part, nparts, P, rn2);
+}
+
+void restart_matrix(double* T, int ld, const double* theta, int nk, cudaStream_t s) {
+  note_launch();
+  k_restart_matrix<<<std::min(592, (ld * ld + 255) / 256), 256, 0, s>>>(T, ld, theta, nk);
 }
 
 void add_cols(const double* src, int lds, int M, int P, double* dst, int ldd, cudaStream_t s) {

@@ -25,6 +25,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -116,14 +117,18 @@ struct LWork {
   ProductTimes times;
   DBuf<double> Q, HQ, T, Yw, theta, Xb, HXb, W, S, M, G, part, rn2, Xc, gpart, Xg, gtmp;
   DBuf<float> Xf, Xgf;  // FP32 copies of the vector block (mixed precision)
-  DBuf<int> short_flag;   // set by the device SVQB when a block loses rank
+  // what the host reads at a Rayleigh-Ritz step: eigenvalues (ld), squared residuals (kk), the words of
+  // small_eig and, in the last place, the flag that the device factorisation sets when a block loses
+  // rank
+  DBuf<double> out;
+  int* short_flag = nullptr;
   bool exact = false;   // mixed precision: products with FP64 gathers (the final sweep)
   bool xc_ready = false;  // Xc already holds the block that the next product multiplies
   void release(cudaStream_t s) {
     Q.release(s); HQ.release(s); T.release(s); Yw.release(s); theta.release(s); Xb.release(s);
     HXb.release(s); W.release(s); S.release(s); M.release(s); G.release(s); part.release(s); rn2.release(s);
     Xc.release(s); gpart.release(s); Xg.release(s); gtmp.release(s); Xf.release(s);
-    Xgf.release(s); short_flag.release(s);
+    Xgf.release(s); out.release(s);
   }
 };
 
@@ -208,18 +213,20 @@ bool gathers_f32(vhci_ctx* c, const LWork& w, int b) {
   return c->o.precision == 1 && !w.exact && b % 4 == 0;
 }
 
+// All eigenpairs of T[0:m, 0:m] into w.theta and w.Yw by cuSOLVER's syevd.
+int library_eigs(vhci_ctx* c, LWork& w, int m, int ld) {
+  VCK(cudaMemcpy2DAsync(w.Yw.p, ld * sizeof(double), w.T.p, ld * sizeof(double), m * sizeof(double), m,
+                        cudaMemcpyDeviceToDevice, c->st));
+  return syevd_l(c, w, w.Yw.p, m, ld, w.theta.p);
+}
+
 // The nk lowest eigenpairs of T[0:m, 0:m] into w.theta and the columns of w.Yw (k_eig.cu, or cuSOLVER's
 // syevd beyond its sizes and for eigenvalues too close for it); also the largest, in theta[m - 1].
 int project_eigs(vhci_ctx* c, LWork& w, int m, int ld, int nk) {
   bool done = false;
   VTRY(small_eigs(c, w.T.p, m, ld, nk, w.theta.p, w.Yw.p, &done));
-  if (done) {
-    c->stats.ms_spmm += w.times.collect();
-    return VHCI_OK;
-  }
-  VCK(cudaMemcpy2DAsync(w.Yw.p, ld * sizeof(double), w.T.p, ld * sizeof(double), m * sizeof(double), m,
-                        cudaMemcpyDeviceToDevice, c->st));
-  return syevd_l(c, w, w.Yw.p, m, ld, w.theta.p);
+  c->stats.ms_spmm += w.times.collect();
+  return done ? VHCI_OK : library_eigs(c, w, m, ld);
 }
 
 // Orthonormalise the nb columns of (B, ld) into (out, ldo) by SVQB with the small Gram matrix
@@ -270,7 +277,7 @@ int svqb_small(vhci_ctx* c, LWork& w, int64_t n, const double* B, int ld, int nb
 int svqb_dev(vhci_ctx* c, LWork& w, int64_t n, const double* B, int ld, int nb, int nparts, double* out,
              int ldo) {
   VCK(w.M.reserve((size_t)nb * nb, c->st));
-  svqb_factor(w.gpart.p, nparts, nb, w.M.p, w.short_flag.p, c->st);
+  svqb_factor(w.gpart.p, nparts, nb, w.M.p, w.short_flag, c->st);
   w.xc_ready = !gathers_f32(c, w, nb);
   if (w.xc_ready) VCK(w.Xc.reserve((size_t)std::max(n, c->rblk) * nb, c->st));
   proj_rows(B, ld, w.M.p, nb, n, nb, nb, 1.0, 0.0, out, ldo, c->st, nullptr, 0,
@@ -331,6 +338,7 @@ int fp64_sweep(vhci_ctx* c, LWork& w, int kk, int nk, int keff, int ld, std::vec
   const int64_t nl = c->nrow;
   cudaStream_t s = c->st;
   w.exact = true;
+  w.xc_ready = false;  // a restart started ahead may have left its block there
   for (int j0 = 0; j0 < nk; j0 += 16) {
     const int bw = std::min(16, nk - j0);
     VTRY(apply_h_l(c, w, w.Xb.p + j0, kk, bw, w.HQ.p + j0, ld));
@@ -479,6 +487,7 @@ int block_lanczos_impl(vhci_ctx* c, int k, bool dev_svqb) {
     if (!e) e = w.T.reserve((size_t)ld * ld, s);
     if (!e) e = w.Yw.reserve((size_t)ld * ld, s);
     if (!e) e = w.theta.reserve(ld, s);
+    if (!e) e = w.out.reserve((size_t)ld + kk + kSmallEigDev + 1, s);
     if (!e) e = w.Xb.reserve((size_t)rb * kk, s);  // rblk rows: the block each rank gathers at the end
     if (!e && mixed) e = w.HXb.reserve((size_t)nl * kk, s);  // the final FP64 sweep's products
     if (!e) e = w.W.reserve((size_t)nl * b, s);
@@ -492,8 +501,13 @@ int block_lanczos_impl(vhci_ctx* c, int k, bool dev_svqb) {
     cudaGetLastError();  // too little memory after all
     return block_lanczos_lean(c, k);
   }
-  VCK(w.short_flag.reserve(1, s));
-  VCK(cudaMemsetAsync(w.short_flag.p, 0, sizeof(int), s));
+  const int nout = ld + kk + kSmallEigDev + 1;
+  w.short_flag = reinterpret_cast<int*>(w.out.p + nout - 1);
+  VCK(cudaMemsetAsync(w.out.p, 0, nout * sizeof(double), s));
+  std::vector<double> out_pageable(nout <= kPinnedDoubles ? 0 : nout);
+  double* out_h = nout <= kPinnedDoubles ? c->pinned : out_pageable.data();
+  EventPair rr_done;  // a: the projected solve's verdict, b: values and residuals have arrived
+  VCK(rr_done.create());
   fill_zero(w.Q.p, nl * (int64_t)ld, s);
   VCK(cudaMemsetAsync(w.T.p, 0, (size_t)ld * ld * sizeof(double), s));
 
@@ -530,7 +544,7 @@ int block_lanczos_impl(vhci_ctx* c, int k, bool dev_svqb) {
     if (p == 0) return fail(c, VHCI_E_NOT_CONVERGED, "empty start block");
   }
 
-  std::vector<double> th(ld), rn(kk);
+  std::vector<double> th(ld), rn(kk, 0.0);
   const int maxcyc = c->o.eig_maxit > 0 ? c->o.eig_maxit : 1000;
   auto t_start = std::chrono::steady_clock::now();
   double t_spmm = 0, t_orth = 0, t_rr = 0;
@@ -582,23 +596,13 @@ int block_lanczos_impl(vhci_ctx* c, int k, bool dev_svqb) {
     // ---- Rayleigh-Ritz on T[0:m, 0:m]
     auto t0 = now();
     c->stats.eig_iterations += 1;
-    VTRY(project_eigs(c, w, m, ld, std::min(kk, m)));
-    if (dev) {  // a block that lost rank on the device: redo with the host factorisation
-      int short_rank = 0;
-      VCK(d2h(c, &short_rank, w.short_flag.p, sizeof(int)));
-      VCK(cudaStreamSynchronize(s));
-      if (short_rank) {
-        w.release(s);
-        return block_lanczos_impl(c, k, false);
-      }
-    }
-    // one projected solution for every rank: rank 0's
-    VTRY(comm_bcast0(c, w.Yw.p, (int64_t)ld * m));
-    VTRY(comm_bcast0(c, w.theta.p, m));
     const int nk = std::min(kk, m);
-    VTRY(gemm_rows(c, w.Q.p, ld, w.Yw.p, ld, nl, m, nk, 1.0, 0.0, w.Xb.p, kk));
+    int nparts = 0;  // W's Gram matrix, for the residuals and for the block that continues from it
+    if (pw > 0) VTRY(gemm_rows_self(c, w, w.Q.p, ld, w.S.p, nl, m, pw, w.W.p, b, &nparts));
+    // Rotation, residuals and the copy of what the host needs, once w.theta and w.Yw are set.
+    //
     // Residuals from the Krylov relation H Q = Q T + W E_last^T, where W = (I - Q Q^T) H Q_last is
-    // the pending block (completed here; the restart continues from it): the residual of Ritz pair
+    // the pending block (completed above; the restart continues from it): the residual of Ritz pair
     // (theta_j, y_j) is W y_j[last block rows], so ||r_j||^2 = y_last^T (W^T W) y_last.  With the
     // full (two-pass) orthogonalisation the relation holds to rounding, far below the tolerance.
     // The whole space (m = n) or an invariant subspace (exhausted) leaves no residual.
@@ -606,36 +610,79 @@ int block_lanczos_impl(vhci_ctx* c, int k, bool dev_svqb) {
     // its FP32-gather products carry rounding noise of about 1e-8 relative, and the Krylov relation
     // (exact for the products as computed within one cycle) does not carry that noise across the
     // restarts' coupling terms, so it can stall at the 1e-7 tolerance.
-    std::fill(rn.begin(), rn.end(), 0.0);
-    VCK(d2h(c, th.data(), w.theta.p, nk * sizeof(double)));
-    int nparts = 0;  // W's Gram matrix, for the residuals and for the block that continues from it
-    if (pw > 0) VTRY(gemm_rows_self(c, w, w.Q.p, ld, w.S.p, nl, m, pw, w.W.p, b, &nparts));
-    if (mixed) {
-      VTRY(gemm_rows(c, w.HQ.p, ld, w.Yw.p, ld, nl, m, nk, 1.0, 0.0, w.HXb.p, kk));
-      residual_norms(w.Xb.p, w.HXb.p, nl, kk, nk, w.theta.p, w.part.p, nblk, w.rn2.p, s);
-      VTRY(comm_sum(c, w.rn2.p, nk));
-      VCK(d2h(c, rn.data(), w.rn2.p, nk * sizeof(double)));
-      VCK(cudaStreamSynchronize(s));
-    } else if (pw > 0) {
-      VCK(w.G.reserve((size_t)pw * pw, s));
-      gram_sum(w.gpart.p, nparts, pw, pw, w.G.p, pw, s);
-      std::vector<double> G((size_t)pw * pw), Yl((size_t)pw * nk);
-      VCK(d2h(c, G.data(), w.G.p, G.size() * sizeof(double)));
-      VCK(cudaMemcpy2DAsync(Yl.data(), pw * sizeof(double), w.Yw.p + (m - pw), ld * sizeof(double),
-                            pw * sizeof(double), nk, cudaMemcpyDeviceToHost, s));
-      VCK(cudaStreamSynchronize(s));
-      for (int j = 0; j < nk; ++j) {
-        const double* y = Yl.data() + (size_t)j * pw;
-        double q = 0.0;
-        for (int a = 0; a < pw; ++a) {
-          double ga = 0.0;
-          for (int e = 0; e < pw; ++e) ga += G[(size_t)e * pw + a] * y[e];
-          q += y[a] * ga;
-        }
-        rn[j] = q;
+    double* rn2 = w.out.p + ld;
+    auto rotate = [&]() -> int {
+      // one projected solution for every rank: rank 0's
+      VTRY(comm_bcast0(c, w.Yw.p, (int64_t)ld * m));
+      VTRY(comm_bcast0(c, w.theta.p, m));
+      VTRY(gemm_rows(c, w.Q.p, ld, w.Yw.p, ld, nl, m, nk, 1.0, 0.0, w.Xb.p, kk));
+      if (mixed) {
+        VTRY(gemm_rows(c, w.HQ.p, ld, w.Yw.p, ld, nl, m, nk, 1.0, 0.0, w.HXb.p, kk));
+        residual_norms(w.Xb.p, w.HXb.p, nl, kk, nk, w.theta.p, w.part.p, nblk, rn2, s);
+        VTRY(comm_sum(c, rn2, nk));
+      } else if (pw > 0) {
+        krylov_residuals(w.Yw.p + (m - pw), ld, nk, w.gpart.p, nparts, pw, rn2, s);
+      } else {
+        VCK(cudaMemsetAsync(rn2, 0, kk * sizeof(double), s));
+      }
+      VCK(cudaMemcpyAsync(w.out.p, w.theta.p, m * sizeof(double), cudaMemcpyDeviceToDevice, s));
+      VCK(d2h(c, out_h, w.out.p, nout * sizeof(double)));
+      VCK(cudaEventRecord(rr_done.b, s));
+      return VHCI_OK;
+    };
+    // the restart from the rotated block: kept Ritz vectors (in mixed precision their products too), T
+    // of their values, and the pending block behind them
+    int p2 = p;
+    auto restart = [&]() -> int {
+      if (mixed) copy_cols(w.HXb.p, kk, w.HQ.p, ld, nl, nk, s);
+      copy_cols(w.Xb.p, kk, w.Q.p, ld, nl, nk, s);
+      if (dev) VTRY(svqb_dev(c, w, nl, w.W.p, b, p, nparts, w.Q.p + nk, ld));
+      else VTRY(svqb_small(c, w, nl, w.W.p, b, p, w.Q.p + nk, ld, &p2));
+      restart_matrix(w.T.p, ld, w.theta.p, nk, s);
+      return VHCI_OK;
+    };
+    // The host decides twice, and the GPU has work queued both times: whether the projected solve is
+    // good (the rotation runs meanwhile), and whether the pairs have converged (the restart does; it
+    // leaves the rotated block alone).  A rank of a sharded solve waits for each answer.
+    const bool ahead = dev && !is_sharded(c);
+    bool started = false;
+    if (ahead) {
+      bool fast = false;
+      VTRY(small_eigs_start(c, w.T.p, m, ld, nk, w.theta.p, w.Yw.p, w.out.p + ld + kk, &fast));
+      if (fast) {
+        double* verdict = out_h + nout;  // its own place behind the copy below
+        if (nout + kSmallEigDev > kPinnedDoubles) verdict = nullptr;
+        if (verdict) VCK(d2h(c, verdict, w.out.p + ld + kk, kSmallEigDev * sizeof(double)));
+        VCK(cudaEventRecord(rr_done.a, s));
+        VTRY(rotate());
+        VCK(cudaEventSynchronize(verdict ? rr_done.a : rr_done.b));
+        fast = small_eigs_verdict(verdict ? verdict : out_h + ld + kk);
+      }
+      if (fast && pw > 0 && !exhausted) {
+        VTRY(restart());
+        started = true;
+      }
+      if (!fast) {
+        VTRY(library_eigs(c, w, m, ld));
+        VTRY(rotate());
       }
     } else {
-      VCK(cudaStreamSynchronize(s));
+      VTRY(project_eigs(c, w, m, ld, nk));
+      VTRY(rotate());
+    }
+    VCK(cudaEventSynchronize(rr_done.b));
+    VCK(cudaGetLastError());
+    c->stats.ms_spmm += w.times.collect();
+    std::copy(out_h, out_h + m, th.begin());
+    std::copy(out_h + ld, out_h + ld + nk, rn.begin());
+    if (dev) {  // a block that lost rank on the device: redo with the host factorisation
+      int lost = 0;
+      std::memcpy(&lost, out_h + nout - 1, sizeof(int));
+      if (lost) {
+        VCK(cudaStreamSynchronize(s));
+        w.release(s);
+        return block_lanczos_impl(c, k, false);
+      }
     }
     const int keff = std::min(k, nk);
     // Mixed precision measures the residual against the spectrum's scale (the largest |Ritz
@@ -643,9 +690,7 @@ int block_lanczos_impl(vhci_ctx* c, int k, bool dev_svqb) {
     // to ||H||, which a pair with small |theta| cannot get under; the FP64 sweep refines the pairs.
     double scale = 0.0;
     if (mixed) {
-      double tl = 0.0;
-      VCK(d2h(c, &tl, w.theta.p + (m - 1), sizeof(double)));
-      scale = std::max(std::fabs(th[0]), std::fabs(tl));
+      scale = std::max(std::fabs(th[0]), std::fabs(th[m - 1]));
     }
     auto thresh = [&](int j) { return tol * std::max({eps23, std::fabs(th[j]), scale}); };
     int nconv = 0;
@@ -674,18 +719,9 @@ int block_lanczos_impl(vhci_ctx* c, int k, bool dev_svqb) {
       w.release(s);
       return VHCI_OK;
     }
-    // ---- thick restart: keep the Ritz block (in mixed precision its rotated products too), continue
-    // from the pending block W formed above
+    // ---- thick restart
     t0 = now();
-    if (mixed) copy_cols(w.HXb.p, kk, w.HQ.p, ld, nl, nk, s);
-    copy_cols(w.Xb.p, kk, w.Q.p, ld, nl, nk, s);
-    int p2 = p;
-    if (dev) VTRY(svqb_dev(c, w, nl, w.W.p, b, p, nparts, w.Q.p + nk, ld));
-    else VTRY(svqb_small(c, w, nl, w.W.p, b, p, w.Q.p + nk, ld, &p2));
-    std::vector<double> Th((size_t)ld * nk, 0.0);
-    for (int j = 0; j < nk; ++j) Th[(size_t)j * ld + j] = th[j];
-    VCK(cudaMemsetAsync(w.T.p, 0, (size_t)ld * ld * sizeof(double), s));
-    VCK(h2d(c, w.T.p, Th.data(), Th.size() * sizeof(double)));
+    if (!started) VTRY(restart());
     m = nk;
     p = p2;
     t_rr += msince(t0);

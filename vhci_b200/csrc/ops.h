@@ -223,6 +223,12 @@ int proj_rows_self(const double* A, int lda, const double* S, int lds, int64_t n
 void gram_sum(const double* part, int nparts, int M, int P, double* C, int ldc, cudaStream_t s);
 // dst (M x P, column-major, ldd) += src (lds)
 void add_cols(const double* src, int lds, int M, int P, double* dst, int ldd, cudaStream_t s);
+// rn2[j] = y_j^T G y_j, j < nk, with y_j the P values at Y + j ldy and G (P x P) the sum of nparts
+// partial sums: the squared residuals of the Krylov relation.
+void krylov_residuals(const double* Y, int ldy, int nk, const double* part, int nparts, int P,
+                      double* rn2, cudaStream_t s);
+// T (ld x ld) = diag(theta[0..nk)) with zeros elsewhere.
+void restart_matrix(double* T, int ld, const double* theta, int nk, cudaStream_t s);
 // Factor M (nb x nb, column-major) of the Gram matrix W^T W (the sum of nparts partial sums, nb x nb,
 // nb <= 16) on the device: W M is orthonormal; the column of a lost direction is zero, and
 // *rank_short is set to 1 when there are any.
