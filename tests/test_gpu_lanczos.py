@@ -46,3 +46,22 @@ def test_lowest_states(n, k, precision):
         C, E = v.vectors(k)
         # orthonormal to the rounding of two Gram-Schmidt passes and the rotations
         assert np.abs(C.T @ C - np.eye(k)).max() <= 1e-11
+
+
+@pytest.mark.parametrize("n,k", [(9001, 301), (9002, 61), (1203, 5)])
+def test_subspace_widths(n, k):
+    """Subspaces of several slabs of the projections' columns, with blocks that begin past a 32-byte
+    boundary after a restart (wanted counts that are no multiple of four), and the narrowest ones: the
+    same matrix through the eigensolver and a dense eigensolve; tolerance as above."""
+    with context(n, k, 0) as v:
+        H = v.h_csr()
+        w = np.linalg.eigvalsh(H.toarray())[:k] if n < 4000 else None
+        E = v.eigs(k)
+        C, _ = v.vectors(k)
+        scale = np.abs(H).sum(1).max()
+        # ||H c - E c|| <= 1e-10 |E| for a converged pair, plus the rounding of the product here
+        R = H @ C - C * E
+        assert (np.linalg.norm(R, axis=0) <= 1e-10 * np.abs(E) + 64 * 2.0 ** -53 * scale).all()
+        assert np.abs(C.T @ C - np.eye(k)).max() <= 1e-11
+        if w is not None:
+            assert (np.abs(E - w) <= 1e-10 * np.abs(w) + n * 2.0 ** -53 * scale).all()

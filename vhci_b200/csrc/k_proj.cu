@@ -3,13 +3,14 @@
 // implicitly restarted Lanczos, Ham.cpp:347-370) does these with Eigen's dense products; here they
 // are skinny products over the whole basis, written for B200's FP64 tensor pipe (DMMA,
 // mma.sync.m8n8k4.f64).  Both read the tall operand once, straight from global memory into the
-// DMMA fragment registers (each lane's fragment element is 8 bytes of a 32-byte row segment, so
-// the sectors are fully used), with several k-steps of loads in flight per lane and 32 warps per
-// SM; the main loops have no block-wide barriers:
+// DMMA fragment registers, 32 bytes a lane: what a lane holds of four (or two) adjacent columns is
+// its element of four fragments, so that a fragment's columns lie four apart in the operand.  An
+// 8-byte load a lane visits one cache line for every 32 bytes, and the line lookups of the first
+// cache level were the limit (84 % of its peak at 42 % of the memory's bandwidth, 100,000 rows).
 //
 //   proj_gram:  C = alpha * A^T B + beta * C   A: n x M, B: n x P (row-major), C: M x P col-major,
 //               P <= 16.  A persistent grid splits the n rows over the blocks; each warp keeps
-//               the partial products of its 8-row tiles of C in registers; the blocks' partials
+//               the partial products of its 16 or 32 rows of C in registers; the blocks' partials
 //               go to scratch and a second kernel sums them in block order, so the result does not
 //               depend on scheduling.
 //   proj_rows:  Out = alpha * A S + beta * In    A: n x M row-major, S: M x P col-major,
@@ -18,7 +19,8 @@
 //
 // A Lanczos step reads the basis twice (coefficients, update).  Three passes with the first two fused
 // over 128-row chunks took 240 + 110 us of projections at 120,011 rows and 512 columns on average,
-// 44 us at 24,000 rows and 150 columns; now 140 + 114 and 15 + 13 us.
+// 44 us at 24,000 rows and 150 columns; with 8-byte loads 150 + 110 and 16 + 13 us, now 99 + 100 and 13 +
+// 11 us (the bytes of one pass take 75 us at 120,011 rows, and its products 52 us at 37 TFLOP/s).
 //
 // Fragment layouts of m8n8k4 (row.col): A[m][k] sits in lane 4 m + k, B[k][n] in lane 4 n + k,
 // D[m][n] in lane 4 m + n / 2 (element n % 2).
@@ -38,100 +40,174 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
                : "d"(a), "d"(b));
 }
 
-constexpr int kThreads = 1024;      // proj_rows: 32 warps, one block per SM
+constexpr int kThreads = 512;       // proj_rows: 16 warps with up to 128 registers each, one block per SM
+constexpr int kAhead = 4;           // proj_rows: loads of 16 columns in flight per warp
 constexpr int kBlocks = 148;
-constexpr int kUnroll = 8;          // proj_rows: k-steps of loads issued ahead
-constexpr int kGramThreads = 512;   // proj_gram: 16 warps with up to 128 registers each
-constexpr int kGramWarps = kGramThreads / 32;
-constexpr int kGramTiles = 6;       // 8-row tiles of C per warp: a slab of 16 x 6 x 8 = 768 rows
-constexpr int kGramSlab = kGramWarps * kGramTiles * 8;
-constexpr int kGramUnroll = 2;
+constexpr int kGramSlab = 764;      // columns of A in one launch of k_gram: 24 tiles of 32 with any skew
 
-// Partial A^T B over this block's rows for the columns a0 .. a0 + Mc - 1 of A.  The 8-row tiles
-// of C are dealt to a group of WG = ceil(tiles / TILES) warps (warp g of a group owns tiles g,
-// g + WG, ...); the block's 16 warps form 16 / WG such groups, which take turns over the block's
-// rows in steps of 4 UNROLL rows, so a narrow C (few tiles) still keeps every warp streaming.
-// When a group would need more than half the warps, all 16 form one group.
-// Group r of block x writes its partial to part[x * groups + r] (Mc x P, a-major).
-template <int NT, int TILES, int UNROLL, int NWARP>
+// Four adjacent doubles at p, of which those with first <= k < last (k: the index of p[0]) are wanted.
+// wide: p is 32-byte aligned, and the four are one load; a sector that holds a wanted element lies
+// within its allocation, and mask4 clears the others before they are used.
+__device__ __forceinline__ void load4(double (&v)[4], const double* p, int k, int first, int last,
+                                      bool wide) {
+  v[0] = v[1] = v[2] = v[3] = 0.0;
+  if (wide) {
+    if (k + 3 >= first && k < last)
+      asm volatile("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];"
+                   : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
+                   : "l"(p));
+  } else {
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+      if (k + s >= first && k + s < last) v[s] = __ldg(p + s);
+  }
+}
+
+__device__ __forceinline__ void mask4(double (&v)[4], int k, int first, int last) {
+  if (k < first || k + 3 >= last) {
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+      if (k + s < first || k + s >= last) v[s] = 0.0;
+  }
+}
+
+// How far a pointer lies past a 32-byte boundary, in doubles, where its rows all start alike; 0 and
+// wide = false where they do not.
+inline int row_skew(const double* A, int lda, bool* wide) {
+  *wide = lda % 4 == 0;
+  return *wide ? (int)(reinterpret_cast<uintptr_t>(A) / sizeof(double) % 4) : 0;
+}
+
+// Partial A^T B over this block's rows for Mc columns of A (A points skew columns before the first).
+// The columns are dealt in tiles of 8 CT to a group of WG warps, one tile a warp; the block's warps
+// form NWARP / WG groups, which take turns over the block's rows in steps of 4 UNROLL rows, so a
+// narrow C (few tiles) still keeps every warp streaming.  A lane loads CT adjacent columns of its row:
+// its elements of CT fragments, fragment t holding the columns t, t + CT, ... of the tile; B's columns
+// are taken NT apart likewise.  Each step's registers are loaded anew, for the next round, as soon as
+// its products are issued, so that loads and products of one warp overlap.
+// Block x writes its partial to part[x] (Mc x P, a-major).
+template <int NT, int CT, int UNROLL, int NWARP>
 __global__ void __launch_bounds__(NWARP * 32, 1) k_gram(const double* __restrict__ A, int lda,
                                                     const double* __restrict__ B, int ldb,
-                                                    int64_t n, int Mc, int P,
-                                                    double* __restrict__ part) {
+                                                    int64_t n, int Mc, int P, int skew, bool wide,
+                                                    bool bwide, double* __restrict__ part) {
+  static_assert(CT == 2 || CT == 4, "");
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int mt_total = (Mc + 7) / 8;
-  int WG = (mt_total + TILES - 1) / TILES;
-  if (2 * WG > NWARP) WG = NWARP;  // one group: spread the tiles over all warps
+  const int last = skew + Mc;
+  const int WG = (last + 8 * CT - 1) / (8 * CT);
   const int RG = NWARP / WG;
-  const int rg = wid / WG, wg = wid - rg * WG;
-  if (rg >= RG) return;
+  const int rg = wid / WG, wg = wid - rg * WG;  // warps with rg >= RG have no rows
   const int64_t per = ((n + gridDim.x - 1) / gridDim.x + 3) & ~int64_t(3);
   const int64_t r0 = (int64_t)blockIdx.x * per, r1 = min(n, r0 + per);
-  double acc[TILES][NT][2];
+  double acc[CT][NT][2];
 #pragma unroll
-  for (int t = 0; t < TILES; ++t)
+  for (int t = 0; t < CT; ++t)
 #pragma unroll
     for (int u = 0; u < NT; ++u) acc[t][u][0] = acc[t][u][1] = 0.0;
-  int acol[TILES];
-  bool aon[TILES];
-#pragma unroll
-  for (int t = 0; t < TILES; ++t) {
-    acol[t] = 8 * (wg + WG * t) + (lane >> 2);
-    aon[t] = (wg + WG * t) < mt_total && acol[t] < Mc;
-  }
+  const int acol = 8 * CT * wg + CT * (lane >> 2);  // from A, so the lane's columns start at acol - skew
+  const bool ain = acol + CT - 1 >= skew && acol < last, aall = acol >= skew && acol + CT <= last;
+  const int bcol = NT * (lane >> 2);
   const int kl = lane & 3;
-  for (int64_t k0 = r0 + 4 * UNROLL * rg; k0 < r1; k0 += 4 * UNROLL * RG) {
-    double a[UNROLL][TILES], b[UNROLL][NT];
+  double a[UNROLL][CT], b[UNROLL][NT];
+  auto load = [&](int s, int64_t i) {
+    const bool rin = i < r1;
+    const double* p = A + i * lda + acol;
+#pragma unroll
+    for (int t = 0; t < CT; ++t) a[s][t] = 0.0;
+    if (wide) {
+      if (rin && ain) {
+        if constexpr (CT == 4) {
+          asm volatile("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];"
+                       : "=d"(a[s][0]), "=d"(a[s][1]), "=d"(a[s][2]), "=d"(a[s][3])
+                       : "l"(p));
+        } else {
+          asm volatile("ld.global.nc.v2.f64 {%0,%1}, [%2];" : "=d"(a[s][0]), "=d"(a[s][1]) : "l"(p));
+        }
+      }
+    } else {
+#pragma unroll
+      for (int t = 0; t < CT; ++t)
+        if (rin && acol + t < last) a[s][t] = __ldg(p + t);
+    }
+    const double* q = B + i * ldb + bcol;
+#pragma unroll
+    for (int u = 0; u < NT; ++u) b[s][u] = 0.0;
+    if (NT == 2 && bwide) {
+      if (rin) asm volatile("ld.global.nc.v2.f64 {%0,%1}, [%2];" : "=d"(b[s][0]), "=d"(b[s][NT - 1]) : "l"(q));
+    } else {
+#pragma unroll
+      for (int u = 0; u < NT; ++u)
+        if (rin && bcol + u < P) b[s][u] = __ldg(q + u);
+    }
+  };
+  const int64_t first = rg < RG ? r0 + 4 * UNROLL * rg + kl : r1 + kl;
+#pragma unroll
+  for (int s = 0; s < UNROLL; ++s) load(s, first + 4 * s);
+  for (int64_t k0 = first; k0 - kl < r1; k0 += 4 * UNROLL * RG) {
 #pragma unroll
     for (int s = 0; s < UNROLL; ++s) {
-      const int64_t i = k0 + 4 * s + kl;
-      const bool rin = i < r1;
+      if (wide && !aall)
 #pragma unroll
-      for (int t = 0; t < TILES; ++t)
-        a[s][t] = (rin && aon[t]) ? __ldg(A + i * lda + acol[t]) : 0.0;
+        for (int t = 0; t < CT; ++t)
+          if (acol + t < skew || acol + t >= last) a[s][t] = 0.0;
 #pragma unroll
-      for (int u = 0; u < NT; ++u) {
-        const int c = 8 * u + (lane >> 2);
-        b[s][u] = (rin && c < P) ? __ldg(B + i * ldb + c) : 0.0;
-      }
+      for (int t = 0; t < CT; ++t)
+#pragma unroll
+        for (int u = 0; u < NT; ++u) dmma(acc[t][u], a[s][t], b[s][u]);
+      load(s, k0 + 4 * UNROLL * RG + 4 * s);
     }
-#pragma unroll
-    for (int s = 0; s < UNROLL; ++s)
-#pragma unroll
-      for (int t = 0; t < TILES; ++t)
-        if ((wg + WG * t) < mt_total)
-#pragma unroll
-          for (int u = 0; u < NT; ++u) dmma(acc[t][u], a[s][t], b[s][u]);
   }
-  double* out = part + ((int64_t)blockIdx.x * RG + rg) * Mc * P;
+  if (RG > 1) {  // the groups' sums, added in order by the first
+    constexpr int kTile = CT * NT * 2;
+    extern __shared__ double sg[];  // [RG - 1][WG][kTile][32]
+    double* own = sg + ((rg - 1) * WG + wg) * kTile * 32 + lane;
+    if (rg > 0 && rg < RG)
 #pragma unroll
-  for (int t = 0; t < TILES; ++t) {
-    const int mt = wg + WG * t;
-    if (mt >= mt_total) continue;
-    const int r = 8 * mt + (lane >> 2);
-    if (r >= Mc) continue;
+      for (int x = 0; x < kTile; ++x) own[x * 32] = acc[x / (2 * NT)][x / 2 % NT][x % 2];
+    __syncthreads();
+    if (rg == 0)
+      for (int q = 0; q < RG - 1; ++q)
+#pragma unroll
+        for (int x = 0; x < kTile; ++x)
+          acc[x / (2 * NT)][x / 2 % NT][x % 2] += sg[((q * WG + wg) * kTile + x) * 32 + lane];
+  }
+  if (rg > 0) return;
+  double* out = part + (int64_t)blockIdx.x * Mc * P;
+#pragma unroll
+  for (int t = 0; t < CT; ++t) {
+    const int r = acol + t - skew;
+    if (r < 0 || r >= Mc) continue;
 #pragma unroll
     for (int u = 0; u < NT; ++u)
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
-        const int c = 8 * u + 2 * (lane & 3) + j;
+        const int c = NT * (2 * (lane & 3) + j) + u;
         if (c < P) out[(int64_t)r * P + c] = acc[t][u][j];
       }
   }
 }
 
-// Row groups of one k_gram launch (as the kernel computes them).
-inline int gram_groups(int Mc, int tiles_per_warp, int nwarp) {
-  const int mt = (Mc + 7) / 8;
-  const int wg = (mt + tiles_per_warp - 1) / tiles_per_warp;
-  return 2 * wg > nwarp ? 1 : nwarp / wg;
+template <int CT, int UNROLL, int NWARP>
+void launch_gram(const double* A, int lda, const double* B, int ldb, int64_t n, int nblk, int Mc, int P,
+                 int skew, bool wide, double* part, cudaStream_t s) {
+  // all of a row's 16 columns of B as pairs
+  const bool bwide = P == 16 && ldb % 2 == 0 && reinterpret_cast<uintptr_t>(B) % 16 == 0;
+  const int wg = (skew + Mc + 8 * CT - 1) / (8 * CT);
+  const size_t tiles = (size_t)(NWARP / wg - 1) * wg;  // of the groups beside the first: 12 of 32 columns, 15 of 16
+  const size_t smem = tiles * 8 * CT * (P <= 8 ? 8 : 16) * sizeof(double);
+  note_launch();
+  if (P <= 8)
+    k_gram<1, CT, UNROLL, NWARP><<<nblk, NWARP * 32, smem, s>>>(A - skew, lda, B, ldb, n, Mc, P, skew, wide,
+                                                                bwide, part);
+  else
+    k_gram<2, CT, UNROLL, NWARP><<<nblk, NWARP * 32, smem, s>>>(A - skew, lda, B, ldb, n, Mc, P, skew, wide,
+                                                                bwide, part);
 }
 
 // Sums the blocks' partials: a block of kRedWarps warps owns 32 consecutive entries of C; warp w
 // adds the partials of blocks w, w + kRedWarps, ... (lane = entry, so each partial row is read as
 // one 256-byte segment) and the warps' sums are combined in warp order, so the result is the same
-// on every run.  32 warps: a narrow product leaves thousands of partials (148 blocks x 16 row
-// groups) for few entries of C.
+// on every run.
 constexpr int kRedWarps = 32;
 __global__ void __launch_bounds__(kRedWarps * 32) k_gram_reduce(const double* __restrict__ part,
                                                                 int nblk, int M, int P, double alpha,
@@ -159,15 +235,23 @@ __global__ void __launch_bounds__(kRedWarps * 32) k_gram_reduce(const double* __
   }
 }
 
-// Shared row stride of the S slab: 8 NT + 4 doubles puts the four k-rows of one fragment load into
-// distinct 32-byte bank groups.
 constexpr int kRowsMaxM = 1280;     // rows of S held in shared memory per pass over A
 constexpr int kRowsMaxM4 = 768;     // the same for 32-column slabs
 constexpr int kRowsSelfMaxM = 960;  // the same beside the fused Gram product's reduction
 
+// Place of element (k, c) of the S slab in shared memory.  A fragment load takes row 16 j + 4 q + s of
+// column pairs c, c + 1 (NT = 2; single columns for 1, two pairs for 4), q and c / NT differing over the
+// lanes: the rows are rotated in 32-byte groups, or padded, such that these lie in distinct banks.
+template <int NT>
+__host__ __device__ constexpr int s_place(int k, int c) {
+  return NT == 1   ? k * 9 + c
+         : NT == 2 ? k * 16 + (c ^ ((k & 12) | ((k & 1) << 1)))
+                   : k * 32 + (c ^ (((k & 4) << 1) | ((k & 8) >> 2)));
+}
+
 template <int NT>
 constexpr size_t rows_smem(int M) {
-  return (size_t)M * (8 * NT + 4) * sizeof(double);
+  return (size_t)((M + 3 + 15) / 16 * 16) * (NT == 1 ? 9 : 8 * NT) * sizeof(double);
 }
 
 // What k_rows does beside its product.
@@ -179,28 +263,45 @@ struct RowsTail {
   double* part;      // partial Gram products Out^T Out, P x P per block, or null
 };
 
-// Out[i][c] = alpha sum_a A[i][a] S[a + c lds] + beta In[i][c] for Mc rows of S; warps stream 8-row
-// tiles of A over the whole grid.  SELF: the tile's new rows also go, as they are in the accumulators
-// (moved into operand layout by shuffles), into the warp's share of Out^T Out, so that the block
-// orthonormalisation that follows a Gram-Schmidt pass needs no pass of its own (114 us at 120,011 rows
-// and 512 columns on average, where the pass without it took 110 and the Gram product another 16).
+// Out[i][c] = alpha sum_a A[i][a] S[a + c lds] + beta In[i][c] for Mc rows of S (A points skew columns
+// before the first; vec: rows of Out, In and Out2 are 16-byte aligned and P = 8 NT); warps stream 8-row
+// tiles of A over the whole grid, 16 columns in one 32-byte load a lane, each load issued as soon as its
+// registers' products are (the next tile's first ones too).  Fragment u of
+// the result holds the columns u, u + NT, ..., so that a lane's elements of a row are adjacent.
+// SELF: the tile's new rows also go, as they are in the accumulators (moved into operand layout by
+// shuffles), into the warp's share of Out^T Out, so that the block orthonormalisation that follows a
+// Gram-Schmidt pass needs no pass of its own.  Updates of 120,011 rows by 320 to 672
+// columns take 100 us (110 with 8-byte loads of 32 warps and the tiles of the last round on a third of the
+// SMs); a 32-column rotation of 672 columns takes 197 us, of which the tensor pipe needs 140 (231 before).
 template <int NT, bool SELF>
 __global__ void __launch_bounds__(kThreads, 1) k_rows(const double* __restrict__ A, int lda,
                                                       const double* __restrict__ S, int lds,
-                                                      int64_t n, int Mc, int P, double alpha,
-                                                      double beta, double* Out, int ldo,
-                                                      RowsTail tail) {
-  extern __shared__ double ss[];  // [Mc][8 NT + 4]; SELF: then [warps][64 NT NT] for the reduction
-  constexpr int SW = 8 * NT + 4;
-  for (int x = threadIdx.x; x < Mc * 8 * NT; x += blockDim.x) {
-    const int c = x / Mc, a = x - c * Mc;  // consecutive threads read one column of S
-    ss[a * SW + c] = c < P ? S[a + (int64_t)c * lds] : 0.0;
-  }
-  __syncthreads();
+                                                      int64_t n, int Mc, int P, int skew, bool wide,
+                                                      bool vec, double alpha, double beta, double* Out,
+                                                      int ldo, RowsTail tail) {
+  extern __shared__ __align__(16) double ss[];  // the S slab; SELF: then [warps][64 NT NT] for the reduction
+  const int last = skew + Mc, Mr = (last + 15) / 16 * 16;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int kl = lane & 3;
   const int64_t tiles = (n + 7) / 8;
   const int64_t wstride = (int64_t)gridDim.x * (blockDim.x >> 5);
+  // a round's tiles go over the blocks first, so that the last round is spread over all of them
+  const int64_t tile0 = (int64_t)wid * gridDim.x + blockIdx.x;
+  double a[kAhead][4];
+  {
+    const int64_t i = tile0 * 8 + (lane >> 2);
+#pragma unroll
+    for (int h = 0; h < kAhead; ++h)
+      load4(a[h], A + (i < n ? i : 0) * lda + 16 * h + 4 * kl, 16 * h + 4 * kl, skew, i < n ? last : 0, wide);
+  }
+  for (int c = wid; c < 8 * NT; c += blockDim.x >> 5) {
+    const double* Sc = S - skew + (int64_t)c * lds;
+#pragma unroll 4
+    for (int k = lane; k < Mr; k += 32)
+      ss[s_place<NT>(k, c)] = c < P && k >= skew && k < last ? __ldg(Sc + k) : 0.0;
+  }
+  __syncthreads();
+  const int c0 = 2 * NT * kl;  // the lane's columns of the result: c0 + NT j + u
   double g[SELF ? NT : 1][SELF ? NT : 1][2];
   if constexpr (SELF) {
 #pragma unroll
@@ -208,46 +309,77 @@ __global__ void __launch_bounds__(kThreads, 1) k_rows(const double* __restrict__
 #pragma unroll
       for (int v = 0; v < NT; ++v) g[u][v][0] = g[u][v][1] = 0.0;
   }
-  for (int64_t tile = (int64_t)blockIdx.x * (blockDim.x >> 5) + wid; tile < tiles; tile += wstride) {
+  for (int64_t tile = tile0; tile < tiles; tile += wstride) {
     const int64_t i = tile * 8 + (lane >> 2);
     const bool rin = i < n;
-    const double* arow = A + (rin ? i : 0) * lda;
+    const int64_t inext = i + 8 * wstride;
+    const double* arow = A + (rin ? i : 0) * lda + 4 * kl;
+    const double* anext = A + (inext < n ? inext : 0) * lda + 4 * kl;
+    const int rlast = rin ? last : 0, nlast = inext < n ? last : 0;
     double acc[NT][2];
 #pragma unroll
     for (int u = 0; u < NT; ++u) acc[u][0] = acc[u][1] = 0.0;
-    for (int k0 = 0; k0 < Mc; k0 += 4 * kUnroll) {
-      double a[kUnroll];
+    for (int k0 = 0; k0 < Mr; k0 += 16 * kAhead) {
+      const bool more = k0 + 16 * kAhead < Mr;
 #pragma unroll
-      for (int s = 0; s < kUnroll; ++s) {
-        const int k = k0 + 4 * s + kl;
-        a[s] = (rin && k < Mc) ? __ldg(arow + k) : 0.0;
-      }
+      for (int h = 0; h < kAhead; ++h) {
+        mask4(a[h], k0 + 16 * h + 4 * kl, skew, rlast);
+        const int k = k0 + 16 * h + 4 * kl;
+        if (k0 + 16 * h < Mr)
 #pragma unroll
-      for (int s = 0; s < kUnroll; ++s) {
-        const int k = k0 + 4 * s + kl;
-        if (k0 + 4 * s < Mc) {
+          for (int s = 0; s < 4; ++s) {
+            if constexpr (NT == 1) {
+              dmma(acc[0], a[h][s], ss[s_place<1>(k + s, lane >> 2)]);
+            } else {
 #pragma unroll
-          for (int u = 0; u < NT; ++u)
-            dmma(acc[u], a[s], k < Mc ? ss[k * SW + 8 * u + (lane >> 2)] : 0.0);
-        }
+              for (int u = 0; u < NT; u += 2) {
+                const double2 v =
+                    *reinterpret_cast<const double2*>(ss + s_place<NT>(k + s, NT * (lane >> 2) + u));
+                dmma(acc[u], a[h][s], v.x);
+                dmma(acc[u + 1], a[h][s], v.y);
+              }
+            }
+          }
+        const int kn = (more ? k0 + 16 * kAhead : 0) + 16 * h;
+        load4(a[h], (more ? arow : anext) + kn, kn + 4 * kl, skew, more ? rlast : nlast, wide);
       }
     }
+    if (vec) {
 #pragma unroll
-    for (int u = 0; u < NT; ++u)
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const int c = 8 * u + 2 * (lane & 3) + j;
-        double o = 0.0;
-        if (rin && c < P) {
-          o = beta == 0.0 ? alpha * acc[u][j] : alpha * acc[u][j] + beta * tail.In[i * tail.ldi + c];
-          Out[i * ldo + c] = o;
-          if (tail.Out2) tail.Out2[i * tail.ldo2 + c] = o;
+      for (int x = 0; x < 2 * NT; x += 2) {  // place x of the lane's row segment: j = x / NT, u = x % NT
+        double2 o = make_double2(0.0, 0.0);
+        if (rin) {
+          o.x = alpha * acc[x % NT][x / NT];
+          o.y = alpha * acc[(x + 1) % NT][(x + 1) / NT];
+          if (beta != 0.0) {
+            const double2 v = *reinterpret_cast<const double2*>(tail.In + i * tail.ldi + c0 + x);
+            o.x += beta * v.x;
+            o.y += beta * v.y;
+          }
+          *reinterpret_cast<double2*>(Out + i * ldo + c0 + x) = o;
+          if (tail.Out2) *reinterpret_cast<double2*>(tail.Out2 + i * tail.ldo2 + c0 + x) = o;
         }
-        acc[u][j] = o;
+        acc[x % NT][x / NT] = o.x;
+        acc[(x + 1) % NT][(x + 1) / NT] = o.y;
       }
+    } else {
+#pragma unroll
+      for (int u = 0; u < NT; ++u)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int c = c0 + NT * j + u;
+          double o = 0.0;
+          if (rin && c < P) {
+            o = beta == 0.0 ? alpha * acc[u][j] : alpha * acc[u][j] + beta * tail.In[i * tail.ldi + c];
+            Out[i * ldo + c] = o;
+            if (tail.Out2) tail.Out2[i * tail.ldo2 + c] = o;
+          }
+          acc[u][j] = o;
+        }
+    }
     if constexpr (SELF) {
-      // operand element (row 4 h + (lane & 3), column 8 u + lane / 4) sits in lane
-      // 4 row + (column % 8) / 2, place column % 2
+      // operand element (row 4 h + (lane & 3), place lane / 4 of fragment u) sits in lane
+      // 4 row + place / 2, element place % 2
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         double w[NT];
@@ -267,14 +399,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_rows(const double* __restrict__
   }
   if constexpr (SELF) {
     // the warps' shares, added in warp order
-    double* sg = ss + Mc * SW;
+    double* sg = ss + Mr * (NT == 1 ? 9 : 8 * NT);
 #pragma unroll
     for (int u = 0; u < NT; ++u)
 #pragma unroll
       for (int v = 0; v < NT; ++v)
 #pragma unroll
         for (int j = 0; j < 2; ++j)
-          sg[wid * 64 * NT * NT + (8 * u + (lane >> 2)) * 8 * NT + 8 * v + 2 * (lane & 3) + j] = g[u][v][j];
+          sg[wid * 64 * NT * NT + (NT * (lane >> 2) + u) * 8 * NT + NT * (2 * (lane & 3) + j) + v] =
+              g[u][v][j];
     __syncthreads();
     for (int x = threadIdx.x; x < 64 * NT * NT; x += blockDim.x) {
       const int r = x / (8 * NT), c = x - r * (8 * NT);
@@ -290,6 +423,23 @@ __global__ void __launch_bounds__(kThreads, 1) k_rows(const double* __restrict__
 template <int NT>
 constexpr size_t rows_self_smem(int M) {
   return rows_smem<NT>(M) + (size_t)(kThreads / 32) * 64 * NT * NT * sizeof(double);
+}
+
+inline bool pair_rows(const double* p, int ld) {
+  return ld % 2 == 0 && reinterpret_cast<uintptr_t>(p) % 16 == 0;
+}
+
+template <int NT, bool SELF>
+void launch_rows(const double* A, int lda, const double* S, int lds, int64_t n, int Mc, int P, double alpha,
+                 double beta, double* Out, int ldo, const RowsTail& t, int blocks, cudaStream_t s) {
+  bool wide;
+  const int skew = row_skew(A, lda, &wide);
+  const bool vec = P == 8 * NT && pair_rows(Out, ldo) && (beta == 0.0 || pair_rows(t.In, t.ldi)) &&
+                   (!t.Out2 || pair_rows(t.Out2, t.ldo2));
+  const size_t smem = SELF ? rows_self_smem<NT>(Mc) : rows_smem<NT>(Mc);
+  note_launch();
+  k_rows<NT, SELF><<<blocks, kThreads, smem, s>>>(A - skew, lda, S, lds, n, Mc, P, skew, wide, vec, alpha,
+                                                  beta, Out, ldo, t);
 }
 
 // Orthonormalisation factor of a block W from its Gram matrix S = W^T W, given as nparts partial sums
@@ -449,7 +599,7 @@ void svqb_factor(const double* part, int nparts, int nb, double* M, int* rank_sh
 }
 
 int64_t proj_gram_scratch(int M, int P) {
-  // blocks x row groups x Mc <= kBlocks x kGramSlab for every slab width (groups x tiles <= 96)
+  // a partial of at most kGramSlab x P a block
   (void)M;
   return (int64_t)kBlocks * kGramSlab * P;
 }
@@ -463,29 +613,20 @@ bool proj_gram(const double* A, int lda, const double* B, int ldb, int64_t n, in
   if (n < (int64_t)nblk * 64) nblk = (int)std::max<int64_t>(1, (n + 63) / 64);
   for (int a0 = 0; a0 < M; a0 += kGramSlab) {
     const int Mc = std::min(kGramSlab, M - a0);
-    // up to 16 tiles of C: 16 warps, one tile each, eight k-steps in flight; up to 64 tiles: 32
-    // warps, two tiles each, four k-steps; wider: 16 warps, six tiles each, two k-steps (measured
-    // on 380k rows, P = 16: 0.39 ms against 0.47 ms at M = 512 for the middle form, and 0.50
-    // against 0.55 ms at M = 672 for the wide one)
-    const int form = Mc <= 8 * kGramWarps ? 0 : (Mc <= 8 * 2 * 32 ? 1 : 2);
-    const int nparts = nblk * (form == 0   ? gram_groups(Mc, 1, kGramWarps)
-                               : form == 1 ? gram_groups(Mc, 2, 32)
-                                           : gram_groups(Mc, kGramTiles, kGramWarps));
+    bool wide;
+    const int skew = row_skew(A + a0, lda, &wide);
+    // Up to 128 columns: tiles of 16, so that the warps of a narrow C share the rows among at least two
+    // groups.  Wider: tiles of 32, one a warp; 24 warps where 16 would leave 4 or more of them idle
+    // (9 to 12 tiles), or are too few.  At 120,011 rows and P = 16: 88 us for 13 to 16 tiles on average,
+    // 107 for 17 to 21 (130 and 134 with each round's loads waited for before its products).
+    const int t32 = (skew + Mc + 31) / 32;
+    if (skew + Mc <= 128) launch_gram<2, 8, 16>(A + a0, lda, B, ldb, n, nblk, Mc, P, skew, wide, part, s);
+    else if (t32 <= 8 || (t32 > 12 && t32 <= 16))
+      launch_gram<4, 4, 16>(A + a0, lda, B, ldb, n, nblk, Mc, P, skew, wide, part, s);
+    else
+      launch_gram<4, 2, 24>(A + a0, lda, B, ldb, n, nblk, Mc, P, skew, wide, part, s);
     note_launch();
-    if (form == 0) {
-      if (P <= 8) k_gram<1, 1, 8, kGramWarps><<<nblk, kGramThreads, 0, s>>>(A + a0, lda, B, ldb, n, Mc, P, part);
-      else k_gram<2, 1, 8, kGramWarps><<<nblk, kGramThreads, 0, s>>>(A + a0, lda, B, ldb, n, Mc, P, part);
-    } else if (form == 1) {
-      if (P <= 8) k_gram<1, 2, 4, 32><<<nblk, 1024, 0, s>>>(A + a0, lda, B, ldb, n, Mc, P, part);
-      else k_gram<2, 2, 4, 32><<<nblk, 1024, 0, s>>>(A + a0, lda, B, ldb, n, Mc, P, part);
-    } else {
-      if (P <= 8)
-        k_gram<1, kGramTiles, kGramUnroll, kGramWarps><<<nblk, kGramThreads, 0, s>>>(A + a0, lda, B, ldb, n, Mc, P, part);
-      else
-        k_gram<2, kGramTiles, kGramUnroll, kGramWarps><<<nblk, kGramThreads, 0, s>>>(A + a0, lda, B, ldb, n, Mc, P, part);
-    }
-    note_launch();
-    k_gram_reduce<<<(Mc * P + 31) / 32, kRedWarps * 32, 0, s>>>(part, nparts, Mc, P, alpha, beta,
+    k_gram_reduce<<<(Mc * P + 31) / 32, kRedWarps * 32, 0, s>>>(part, nblk, Mc, P, alpha, beta,
                                                                  C + a0, ldc, Acc ? Acc + a0 : nullptr,
                                                                  ldacc);
   }
@@ -498,7 +639,7 @@ void proj_rows(const double* A, int lda, const double* S, int lds, int64_t n, in
   if (n <= 0 || P <= 0) return;
   set_attributes();
   const int64_t tiles = (n + 7) / 8;
-  const int g = (int)std::min<int64_t>(kBlocks, (tiles + 31) / 32);
+  const int g = (int)std::min<int64_t>(kBlocks, (tiles + 15) / 16);
   // 32-column slabs when S's rows fit beside them in shared memory: half the passes over A
   const int cw = (P > 16 && M <= kRowsMaxM4) ? 32 : 16;
   for (int c0 = 0; c0 < P; c0 += cw) {
@@ -512,16 +653,9 @@ void proj_rows(const double* A, int lda, const double* S, int lds, int64_t n, in
       const bool last = a0 + kRowsMaxM >= M;
       const RowsTail t{a0 == 0 && In ? In + c0 : Oc, a0 == 0 && In ? ldi : ldo,
                        last && Out2 ? Out2 + c0 : nullptr, ldo2, nullptr};
-      note_launch();
-      if (pc > 16)
-        k_rows<4, false><<<g, kThreads, rows_smem<4>(std::max(Mc, 1)), s>>>(A + a0, lda, Sc, lds, n, Mc,
-                                                                            pc, alpha, bt, Oc, ldo, t);
-      else if (pc <= 8)
-        k_rows<1, false><<<g, kThreads, rows_smem<1>(std::max(Mc, 1)), s>>>(A + a0, lda, Sc, lds, n, Mc,
-                                                                            pc, alpha, bt, Oc, ldo, t);
-      else
-        k_rows<2, false><<<g, kThreads, rows_smem<2>(std::max(Mc, 1)), s>>>(A + a0, lda, Sc, lds, n, Mc,
-                                                                            pc, alpha, bt, Oc, ldo, t);
+      if (pc > 16) launch_rows<4, false>(A + a0, lda, Sc, lds, n, Mc, pc, alpha, bt, Oc, ldo, t, g, s);
+      else if (pc <= 8) launch_rows<1, false>(A + a0, lda, Sc, lds, n, Mc, pc, alpha, bt, Oc, ldo, t, g, s);
+      else launch_rows<2, false>(A + a0, lda, Sc, lds, n, Mc, pc, alpha, bt, Oc, ldo, t, g, s);
     }
   }
 }
@@ -530,13 +664,10 @@ int proj_rows_self(const double* A, int lda, const double* S, int lds, int64_t n
                    double* W, int ldw, double* part, cudaStream_t s) {
   if (n <= 0 || P <= 0 || P > 16 || M <= 0 || M > kRowsSelfMaxM) return 0;
   set_attributes();
-  const int g = (int)std::min<int64_t>(kBlocks, ((n + 7) / 8 + 31) / 32);
+  const int g = (int)std::min<int64_t>(kBlocks, ((n + 7) / 8 + 15) / 16);
   const RowsTail t{W, ldw, nullptr, 0, part};
-  note_launch();
-  if (P <= 8)
-    k_rows<1, true><<<g, kThreads, rows_self_smem<1>(M), s>>>(A, lda, S, lds, n, M, P, -1.0, 1.0, W, ldw, t);
-  else
-    k_rows<2, true><<<g, kThreads, rows_self_smem<2>(M), s>>>(A, lda, S, lds, n, M, P, -1.0, 1.0, W, ldw, t);
+  if (P <= 8) launch_rows<1, true>(A, lda, S, lds, n, M, P, -1.0, 1.0, W, ldw, t, g, s);
+  else launch_rows<2, true>(A, lda, S, lds, n, M, P, -1.0, 1.0, W, ldw, t, g, s);
   return g;
 }
 

@@ -202,7 +202,7 @@ void fill_zero(double* p, int64_t n, cudaStream_t s);
 
 // ---- FP64 tensor-core projections (k_proj.cu) ----
 // C (M x P, column-major, ldc) = alpha A^T B + beta C with A n x M and B n x P row-major (lda,
-// ldb); any M (slabs of 768), P <= 16; part holds proj_gram_scratch(M, P) doubles.  Acc (ldacc), when
+// ldb); any M (slabs of 764), P <= 16; part holds proj_gram_scratch(M, P) doubles.  Acc (ldacc), when
 // given, also gets C added.  Returns false (nothing launched) for P > 16 or strides shorter than the
 // rows.
 int64_t proj_gram_scratch(int M, int P);
