@@ -22,6 +22,7 @@
 #include <cstdint>
 #include <mutex>
 
+#include "chain.cuh"
 #include "ops.h"
 
 namespace cg = cooperative_groups;
@@ -392,6 +393,7 @@ __global__ void __launch_bounds__(32 * kVecWarps) k_tri_vectors(const double* __
                                                                 const double* __restrict__ e, int m,
                                                                 int nk, double* __restrict__ theta,
                                                                 double* __restrict__ Z) {
+  chain_wait();
   extern __shared__ double sm[];
   __shared__ double s_red[kVecWarps];
   double* sd = sm;              // [m]
@@ -520,6 +522,7 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
 __global__ void __launch_bounds__(128) k_eig_gram(const double* __restrict__ Z, int m, int nk,
                                                   double* __restrict__ S,
                                                   unsigned long long* __restrict__ dev) {
+  chain_wait();
   const int lane = threadIdx.x & 31, w = blockIdx.x * 4 + (threadIdx.x >> 5);
   const int tr = (nk + 7) / 8, tc = (nk + 31) / 32;
   if (w >= tr * tc) return;
@@ -564,6 +567,7 @@ __global__ void __launch_bounds__(128) k_eig_gram(const double* __restrict__ Z, 
 // Out (m x nk) = Z S, one warp per 8 x 32 tile.
 __global__ void __launch_bounds__(128) k_eig_mul(const double* __restrict__ Z, const double* __restrict__ S,
                                                  int m, int nk, double* __restrict__ Out) {
+  chain_wait();
   const int lane = threadIdx.x & 31, w = blockIdx.x * 4 + (threadIdx.x >> 5);
   const int tr = (m + 7) / 8, tc = (nk + 31) / 32;
   if (w >= tr * tc) return;
@@ -602,6 +606,7 @@ template <int NR, int PF>
 __global__ void __launch_bounds__(64) k_back(const double* __restrict__ Z, const double* __restrict__ V,
                                              const double* __restrict__ tau, int m, int nk,
                                              double* __restrict__ Y, int ldy) {
+  chain_wait();
   const int lane = threadIdx.x & 31, j = blockIdx.x * 2 + (threadIdx.x >> 5);
   if (j >= nk) return;
   double z[NR], v[PF][NR], t[PF];
@@ -645,6 +650,7 @@ template <int NR>
 __global__ void __launch_bounds__(128) k_back_block(const double* __restrict__ Z, const double* __restrict__ V,
                                                     const double* __restrict__ tau, int m, int nk,
                                                     double* __restrict__ Y, int ldy) {
+  chain_wait();
   __shared__ double red[2][4];
   const int tid = threadIdx.x, lane = tid & 31, j = blockIdx.x;
   double z[NR], v[NR], u[NR];
@@ -777,23 +783,23 @@ bool small_eig(const double* T, int ldt, int m, int nk, double* theta, double* Y
     return false;
   }
   note_launch();
-  k_tri_vectors<<<(nk + 1 + kVecWarps - 1) / kVecWarps, 32 * kVecWarps, vec_smem(m), s>>>(d, e, m, nk,
+  launch_chained(k_tri_vectors, (nk + 1 + kVecWarps - 1) / kVecWarps, 32 * kVecWarps, vec_smem(m), s, d, e, m, nk,
                                                                                           theta, Za);
   const int tr = (nk + 7) / 8, tc = (nk + 31) / 32, tm = (m + 7) / 8;
   for (int it = 0; it < 2; ++it) {
     note_launch();
-    k_eig_gram<<<(tr * tc + 3) / 4, 128, 0, s>>>(it ? Zb : Za, m, nk, S, dev + it);
+    launch_chained(k_eig_gram, (tr * tc + 3) / 4, 128, 0, s, it ? Zb : Za, m, nk, S, dev + it);
     note_launch();
-    k_eig_mul<<<(tm * tc + 3) / 4, 128, 0, s>>>(it ? Zb : Za, S, m, nk, it ? Za : Zb);
+    launch_chained(k_eig_mul, (tm * tc + 3) / 4, 128, 0, s, it ? Zb : Za, S, m, nk, it ? Za : Zb);
   }
   note_launch();
   const int g = (nk + 1) / 2;
-  if (m <= 64) k_back<2, 4><<<g, 64, 0, s>>>(Za, V, tau, m, nk, Y, ldy);
-  else if (m <= 128) k_back<4, 4><<<g, 64, 0, s>>>(Za, V, tau, m, nk, Y, ldy);
-  else if (m <= 256) k_back<8, 4><<<g, 64, 0, s>>>(Za, V, tau, m, nk, Y, ldy);
-  else if (m <= 384) k_back<12, 3><<<g, 64, 0, s>>>(Za, V, tau, m, nk, Y, ldy);
-  else if (cluster) k_back<20, 2><<<g, 64, 0, s>>>(Za, V, tau, m, nk, Y, ldy);
-  else k_back_block<15><<<nk, 128, 0, s>>>(Za, V, tau, m, nk, Y, ldy);
+  if (m <= 64) launch_chained(k_back<2, 4>, g, 64, 0, s, Za, V, tau, m, nk, Y, ldy);
+  else if (m <= 128) launch_chained(k_back<4, 4>, g, 64, 0, s, Za, V, tau, m, nk, Y, ldy);
+  else if (m <= 256) launch_chained(k_back<8, 4>, g, 64, 0, s, Za, V, tau, m, nk, Y, ldy);
+  else if (m <= 384) launch_chained(k_back<12, 3>, g, 64, 0, s, Za, V, tau, m, nk, Y, ldy);
+  else if (cluster) launch_chained(k_back<20, 2>, g, 64, 0, s, Za, V, tau, m, nk, Y, ldy);
+  else launch_chained(k_back_block<15>, nk, 128, 0, s, Za, V, tau, m, nk, Y, ldy);
   return true;
 }
 

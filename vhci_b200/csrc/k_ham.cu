@@ -5,6 +5,7 @@
 #include <cstdlib>
 #include <string>
 
+#include "chain.cuh"
 #include "conn.cuh"
 #include "ops.h"
 #include "rowprod.cuh"
@@ -207,6 +208,7 @@ __global__ void __launch_bounds__(256, 5) k_spmm(int64_t n, const int64_t* __res
                                                  const double* __restrict__ X, int ldx, int bq,
                                                  double* __restrict__ Y, int ldy, int accum,
                                                  int64_t xrow0) {
+  chain_wait();
   const int lane = threadIdx.x & 31, cc = lane % BQ;
   const bool on = cc < bq;
   const int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -239,6 +241,7 @@ __global__ void __launch_bounds__(256, 4) k_spmm_f32x(int64_t n, const int64_t* 
                                                    const float* __restrict__ X, int ldx, int bq,
                                                    const double* __restrict__ Xd, int ldd,
                                                    double* __restrict__ Y, int ldy) {
+  chain_wait();
   const int lane = threadIdx.x & 31, cc = lane % BQ;
   const bool on = cc < bq;
   const int64_t stride = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -271,7 +274,7 @@ void spmm_rows_launch(int64_t n, const int64_t* rowptr, const int32_t* col, cons
     const int w = std::min(32, b - c0), q = pairs ? w / 2 : w;
     note_launch();
 #define VHCI_SPMM(BQ, VEC)                                                                        \
-  k_spmm<BQ, VEC, VT><<<(unsigned)gr, 256, 0, s>>>(n, rowptr, col, val, diag, X + c0, ldx, q,       \
+  launch_chained(k_spmm<BQ, VEC, VT>, (unsigned)gr, 256, 0, s, n, rowptr, col, val, diag, X + c0, ldx, q,       \
                                                    Y + c0, ldy, accum, xrow0)
     if (pairs) {
       if (q == 1) VHCI_SPMM(1, 2);
@@ -327,6 +330,7 @@ __global__ void __launch_bounds__(256) k_sum_parts(const double* __restrict__ pa
 
 __global__ void k_copy_cols(const double* __restrict__ src, int lds, double* __restrict__ dst,
                             int ldd, int64_t n, int ncol) {
+  chain_wait();
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < n * ncol;
        idx += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = idx / ncol;
@@ -534,9 +538,9 @@ bool spmm_f32x(int64_t n, const int64_t* rowptr, const int32_t* col, const float
     const int bq = std::min(BQ, (b - c0) / 4);
     note_launch();
     if (BQ == 8)
-      k_spmm_f32x<8><<<gr, 256, 0, s>>>(n, rowptr, col, val, diag, X + c0, ldx, bq, Xd + c0, ldd, Y + c0, ldy);
+      launch_chained(k_spmm_f32x<8>, gr, 256, 0, s, n, rowptr, col, val, diag, X + c0, ldx, bq, Xd + c0, ldd, Y + c0, ldy);
     else
-      k_spmm_f32x<4><<<gr, 256, 0, s>>>(n, rowptr, col, val, diag, X + c0, ldx, bq, Xd + c0, ldd, Y + c0, ldy);
+      launch_chained(k_spmm_f32x<4>, gr, 256, 0, s, n, rowptr, col, val, diag, X + c0, ldx, bq, Xd + c0, ldd, Y + c0, ldy);
   }
   return true;
 }
@@ -544,6 +548,7 @@ bool spmm_f32x(int64_t n, const int64_t* rowptr, const int32_t* col, const float
 // Compact FP32 copy of ncol columns of a row-major FP64 block (rounded to nearest).
 __global__ void k_copy_cols_f32(const double* __restrict__ src, int lds, float* __restrict__ dst,
                                 int ldd, int64_t n, int ncol) {
+  chain_wait();
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < n * ncol;
        idx += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = idx / ncol;
@@ -556,7 +561,7 @@ void copy_cols_f32(const double* src, int lds, float* dst, int ldd, int64_t n, i
                    cudaStream_t s) {
   if (n <= 0 || ncol <= 0) return;
   note_launch();
-  k_copy_cols_f32<<<grid_for(n * ncol, 256), 256, 0, s>>>(src, lds, dst, ldd, n, ncol);
+  launch_chained(k_copy_cols_f32, grid_for(n * ncol, 256), 256, 0, s, src, lds, dst, ldd, n, ncol);
 }
 
 void spmm(int64_t n, const int64_t* rowptr, const int32_t* col, const double* val,
@@ -583,7 +588,7 @@ void residual_norms(const double* X, const double* HX, int64_t n, int ld, int kk
 void copy_cols(const double* src, int lds, double* dst, int ldd, int64_t n, int ncol,
                cudaStream_t s) {
   if (n <= 0 || ncol <= 0) return;
-  note_launch(); k_copy_cols<<<grid_for(n * ncol, 256), 256, 0, s>>>(src, lds, dst, ldd, n, ncol);
+  note_launch(); launch_chained(k_copy_cols, grid_for(n * ncol, 256), 256, 0, s, src, lds, dst, ldd, n, ncol);
 }
 
 void cols_to_rows(const double* src, int64_t n, int w, double* dst, int ldd, cudaStream_t s) {

@@ -28,6 +28,7 @@
 #include <cstdint>
 #include <mutex>
 
+#include "chain.cuh"
 #include "ops.h"
 
 namespace vhci {
@@ -91,6 +92,7 @@ __global__ void __launch_bounds__(NWARP * 32, 1) k_gram(const double* __restrict
                                                     const double* __restrict__ B, int ldb,
                                                     int64_t n, int Mc, int P, int skew, bool wide,
                                                     bool bwide, double* __restrict__ part) {
+  chain_wait();
   static_assert(CT == 2 || CT == 4, "");
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int last = skew + Mc;
@@ -197,10 +199,10 @@ void launch_gram(const double* A, int lda, const double* B, int ldb, int64_t n, 
   const size_t smem = tiles * 8 * CT * (P <= 8 ? 8 : 16) * sizeof(double);
   note_launch();
   if (P <= 8)
-    k_gram<1, CT, UNROLL, NWARP><<<nblk, NWARP * 32, smem, s>>>(A - skew, lda, B, ldb, n, Mc, P, skew, wide,
+    launch_chained(k_gram<1, CT, UNROLL, NWARP>, nblk, NWARP * 32, smem, s, A - skew, lda, B, ldb, n, Mc, P, skew, wide,
                                                                 bwide, part);
   else
-    k_gram<2, CT, UNROLL, NWARP><<<nblk, NWARP * 32, smem, s>>>(A - skew, lda, B, ldb, n, Mc, P, skew, wide,
+    launch_chained(k_gram<2, CT, UNROLL, NWARP>, nblk, NWARP * 32, smem, s, A - skew, lda, B, ldb, n, Mc, P, skew, wide,
                                                                 bwide, part);
 }
 
@@ -214,6 +216,7 @@ __global__ void __launch_bounds__(kRedWarps * 32) k_gram_reduce(const double* __
                                                                 double beta, double* __restrict__ C,
                                                                 int ldc, double* __restrict__ Acc,
                                                                 int ldacc) {
+  chain_wait();
   __shared__ double ws[kRedWarps][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int x = blockIdx.x * 32 + lane;
@@ -279,6 +282,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_rows(const double* __restrict__
                                                       int64_t n, int Mc, int P, int skew, bool wide,
                                                       bool vec, double alpha, double beta, double* Out,
                                                       int ldo, RowsTail tail) {
+  chain_wait();
   extern __shared__ __align__(16) double ss[];  // the S slab; SELF: then [warps][64 NT NT] for the reduction
   const int last = skew + Mc, Mr = (last + 15) / 16 * 16;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -438,7 +442,7 @@ void launch_rows(const double* A, int lda, const double* S, int lds, int64_t n, 
                    (!t.Out2 || pair_rows(t.Out2, t.ldo2));
   const size_t smem = SELF ? rows_self_smem<NT>(Mc) : rows_smem<NT>(Mc);
   note_launch();
-  k_rows<NT, SELF><<<blocks, kThreads, smem, s>>>(A - skew, lda, S, lds, n, Mc, P, skew, wide, vec, alpha,
+  launch_chained(k_rows<NT, SELF>, blocks, kThreads, smem, s, A - skew, lda, S, lds, n, Mc, P, skew, wide, vec, alpha,
                                                   beta, Out, ldo, t);
 }
 
@@ -456,6 +460,7 @@ __global__ void __launch_bounds__(kSvqbThreads) k_svqb_factor(const double* __re
                                                               int nparts, int nb,
                                                               double* __restrict__ M,
                                                               int* __restrict__ rank_short) {
+  chain_wait();
   __shared__ double ps[4][256], A[16][17], R[16][17], rinv[16];
   const int tid = threadIdx.x;
   {  // four groups of threads add the partial sums q, q + 4, ...; then the groups in order
@@ -531,6 +536,7 @@ __global__ void __launch_bounds__(kSvqbThreads) k_svqb_factor(const double* __re
 __global__ void __launch_bounds__(1024) k_krylov_residuals(const double* __restrict__ Y, int ldy, int nk,
                                                            const double* __restrict__ part, int nparts,
                                                            int P, double* __restrict__ rn2) {
+  chain_wait();
   __shared__ double ps[4][256], G[256];
   const int tid = threadIdx.x;
   {
@@ -558,6 +564,7 @@ __global__ void __launch_bounds__(1024) k_krylov_residuals(const double* __restr
 }
 
 __global__ void k_restart_matrix(double* __restrict__ T, int ld, const double* __restrict__ theta, int nk) {
+  chain_wait();
   for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < ld * ld; x += gridDim.x * blockDim.x) {
     const int c = x / ld, r = x - c * ld;
     T[x] = r == c && r < nk ? theta[r] : 0.0;
@@ -566,6 +573,7 @@ __global__ void k_restart_matrix(double* __restrict__ T, int ld, const double* _
 
 __global__ void k_add_cols(const double* __restrict__ src, int lds, int M, int P,
                            double* __restrict__ dst, int ldd) {
+  chain_wait();
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= M * P) return;
   const int c = x / M, a = x - c * M;
@@ -595,7 +603,7 @@ void set_attributes() {
 void svqb_factor(const double* part, int nparts, int nb, double* M, int* rank_short,
                  cudaStream_t s) {
   note_launch();
-  k_svqb_factor<<<1, kSvqbThreads, 0, s>>>(part, nparts, nb, M, rank_short);
+  launch_chained(k_svqb_factor, 1, kSvqbThreads, 0, s, part, nparts, nb, M, rank_short);
 }
 
 int64_t proj_gram_scratch(int M, int P) {
@@ -626,7 +634,7 @@ bool proj_gram(const double* A, int lda, const double* B, int ldb, int64_t n, in
     else
       launch_gram<4, 2, 24>(A + a0, lda, B, ldb, n, nblk, Mc, P, skew, wide, part, s);
     note_launch();
-    k_gram_reduce<<<(Mc * P + 31) / 32, kRedWarps * 32, 0, s>>>(part, nblk, Mc, P, alpha, beta,
+    launch_chained(k_gram_reduce, (Mc * P + 31) / 32, kRedWarps * 32, 0, s, part, nblk, Mc, P, alpha, beta,
                                                                  C + a0, ldc, Acc ? Acc + a0 : nullptr,
                                                                  ldacc);
   }
@@ -675,23 +683,23 @@ void krylov_residuals(const double* Y, int ldy, int nk, const double* part, int 
                       double* rn2, cudaStream_t s) {
   if (nk <= 0) return;
   note_launch();
-  k_krylov_residuals<<<(nk + 31) / 32, 1024, 0, s>>>(Y, ldy, nk, part, nparts, P, rn2);
+  launch_chained(k_krylov_residuals, (nk + 31) / 32, 1024, 0, s, Y, ldy, nk, part, nparts, P, rn2);
 }
 
 void restart_matrix(double* T, int ld, const double* theta, int nk, cudaStream_t s) {
   note_launch();
-  k_restart_matrix<<<std::min(592, (ld * ld + 255) / 256), 256, 0, s>>>(T, ld, theta, nk);
+  launch_chained(k_restart_matrix, std::min(592, (ld * ld + 255) / 256), 256, 0, s, T, ld, theta, nk);
 }
 
 void add_cols(const double* src, int lds, int M, int P, double* dst, int ldd, cudaStream_t s) {
   if (M <= 0 || P <= 0) return;
   note_launch();
-  k_add_cols<<<(M * P + 255) / 256, 256, 0, s>>>(src, lds, M, P, dst, ldd);
+  launch_chained(k_add_cols, (M * P + 255) / 256, 256, 0, s, src, lds, M, P, dst, ldd);
 }
 
 void gram_sum(const double* part, int nparts, int M, int P, double* C, int ldc, cudaStream_t s) {
   note_launch();
-  k_gram_reduce<<<(M * P + 31) / 32, kRedWarps * 32, 0, s>>>(part, nparts, M, P, 1.0, 0.0, C, ldc,
+  launch_chained(k_gram_reduce, (M * P + 31) / 32, kRedWarps * 32, 0, s, part, nparts, M, P, 1.0, 0.0, C, ldc,
                                                               nullptr, 0);
 }
 
