@@ -4,15 +4,17 @@
 //
 //   1. k_tridiag: Householder tridiagonalisation in one cluster of thread blocks that hold the whole
 //      matrix in their shared memory (rows dealt cyclically), one cluster barrier a column; beyond
-//      640 rows k_tridiag_grid, the same over all SMs;
+//      640 rows k_tridiag_grid, the same over all SMs; the last 128 columns, and matrices that have no
+//      more, by k_tridiag_block, one block with the matrix in its registers;
 //   2. k_tri_vectors: one warp per wanted eigenvalue: Sturm counts at 32 points a round, then the
 //      vector from the twisted factorisation of T - lambda I;
 //   3. two Newton-Schulz steps Z <- Z (3 I - Z^T Z) / 2 take out the mixing of close eigenvalues
 //      (k_eig_gram, k_eig_mul, FP64 tensor cores), with the deviation from orthonormality before each;
 //   4. k_back: the reflectors applied to the vectors, one warp per vector.
 //
-// All steps at 192, 352 and 640 rows (half of the vectors wanted): 0.66, 1.4 and 3.7 ms, against 1.9,
-// 3.5 and 7 ms for syevd with its host steps.
+// All steps at 192, 352 and 640 rows (half of the vectors wanted) took 0.66, 1.4 and 3.7 ms, against
+// 1.9, 3.5 and 7 ms for syevd with its host steps, when step 1 was k_tridiag alone (0.42, 0.99 and
+// 2.9 ms); with the last 128 columns in one block step 1 takes 0.30 ms at 192 rows and 0.82 at 352.
 //
 // Vectors of eigenvalues closer than about 1e-12 of the norm come out too far from orthogonal for
 // step 3; the deviations tell, and the caller takes the library's solver instead.
@@ -34,11 +36,53 @@ namespace {
 constexpr int kTriThreads = 256, kTriWarps = kTriThreads / 32;
 constexpr int kTriRows = 8;   // rows a warp holds at most
 constexpr int kVecWarps = 4;
+constexpr int kTriTail = 128;       // rows of k_tridiag_block
+constexpr int kBlockThreads = 256;
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
+}
+
+// The same by the tensor pipe (the order of the lanes is another): 126 cycles against 187 alone on an SM,
+// 155 against 189 with eight warps.
+__device__ __forceinline__ double warp_sum_mma(double v) {
+  double s0 = 0.0, s1 = 0.0, z = 0.0;
+  // lane 4 m + k gives element (m, k); times ones: row m's sum, in lanes 4 m .. 4 m + 3
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(s0), "+d"(z) : "d"(v), "d"(1.0));
+  const int k = threadIdx.x & 3;
+  const double lo = __shfl_sync(0xffffffffu, s0, 4 * k), hi = __shfl_sync(0xffffffffu, s0, 4 * k + 16);
+  s0 = s1 = 0.0;
+  double z0 = 0.0, z1 = 0.0;
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(s0), "+d"(z0) : "d"(1.0), "d"(lo));
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(s1), "+d"(z1) : "d"(1.0), "d"(hi));
+  return s0 + s1;
+}
+
+// Sums of N values (a power of two) over the warp, halving the values a lane carries at each step: lane l
+// returns the sum of value l N / 32.
+template <int N>
+__device__ __forceinline__ double warp_sums(double (&v)[N]) {
+  const int lane = threadIdx.x & 31;
+  int o = 16;
+#pragma unroll
+  for (int h = N / 2; h > 0; o >>= 1, h >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int q = 0; q < N / 2; ++q)
+      if (q < h) {
+        const double give = up ? v[q] : v[q + h], keep = up ? v[q + h] : v[q];
+        v[q] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+      }
+  }
+  double s = v[0];
+#pragma unroll
+  for (int x = 16 / N; x > 0; x >>= 1) s += __shfl_xor_sync(0xffffffffu, s, x);
+  return s;
 }
 
 // Dynamic shared memory: the block's rows (m values each), p and the next row as they arrive (two
@@ -58,14 +102,16 @@ __host__ __device__ constexpr size_t tri_smem(int m, int blocks) {
 // one pass over its own rows applies the update A - v p^T - (p + K v) v^T, K = - tau v^T p, and
 // multiplies by v_k, and hands p_k and (the keeper of that row) row k + 1 to all blocks.  Bound by
 // latency: the barrier, three warp sums, a square root and a division a column.  Measured at 192, 352
-// and 640 rows: 0.42, 0.99 and 2.9 ms; with two barriers, one of which waits for one block to form v
-// and hand it round, 0.72, 1.8 and 4.9 ms; the tridiagonalisation of cuSOLVER's syevd takes 1.0 ms
-// at 192 and 2.5 at 352.  The barriers wait only for blocks of the same cluster, which run together.
+// and 640 rows, to the last column: 0.42, 0.99 and 2.9 ms (now it stops 128 columns before: 0.15 and
+// 0.67 ms at 192 and 352); with two barriers, one of which waits for one block to form v and hand it
+// round, 0.72, 1.8 and 4.9 ms; the tridiagonalisation of cuSOLVER's syevd takes 1.0 ms at 192 and 2.5
+// at 352.  The barriers wait only for blocks of the same cluster, which run together.
 template <int NR>
 __global__ void __launch_bounds__(kTriThreads) k_tridiag(const double* __restrict__ T, int ldt, int m,
                                                          double* __restrict__ d, double* __restrict__ e,
                                                          double* __restrict__ tau,
-                                                         double* __restrict__ V, double* rowx) {
+                                                         double* __restrict__ V, double* rowx,
+                                                         double* __restrict__ tail) {
   constexpr bool kRowGlobal = NR > 8;
   extern __shared__ double sm[];
   cg::cluster_group cl = cg::this_cluster();
@@ -95,7 +141,8 @@ __global__ void __launch_bounds__(kTriThreads) k_tridiag(const double* __restric
   for (int q = 0; q < NR; ++q) v[q] = 0.0;
   double t = 0.0;  // tau_{k-1}
   cl.sync();
-  for (int k = 0; k + 1 < m; ++k) {
+  const int k0 = m - kTriTail;
+  for (int k = 0; k < k0; ++k) {
     const int par = k & 1, q0 = (k + 1) >> 5;  // chunks before q0 are done
     const double* p_in = sp + par * m;
     double p[NR], x[NR], s = 0.0, s1 = 0.0;
@@ -109,7 +156,7 @@ __global__ void __launch_bounds__(kTriThreads) k_tridiag(const double* __restric
 #pragma unroll
     for (int q = 0; q < NR; ++q)
       if (q & 1) s1 = fma(v[q], p[q], s1); else s = fma(v[q], p[q], s);
-    const double K = -t * warp_sum(s + s1);
+    const double K = -t * warp_sum_mma(s + s1);
     {  // row k, updated
       const double vk = k > 0 ? 1.0 : 0.0, ck = fma(K, vk, p_in[k]);
       s = s1 = 0.0;
@@ -121,7 +168,7 @@ __global__ void __launch_bounds__(kTriThreads) k_tridiag(const double* __restric
         if (q & 1) s1 = fma(y, y, s1); else s = fma(y, y, s);
       }
     }
-    const double ss = warp_sum(s + s1);
+    const double ss = warp_sum_mma(s + s1);
     double alpha = 0.0;
 #pragma unroll
     for (int q = 0; q < NR; ++q)
@@ -195,20 +242,39 @@ __global__ void __launch_bounds__(kTriThreads) k_tridiag(const double* __restric
       sum[q] = 0.0;
       if (l < rows && (l << sh) + r > k) sum[q] = has_next && l == lr ? first : pass(l, false);
     }
-#pragma unroll
-    for (int q = 0; q < kTriRows; ++q) {
-      const int l = wid + q * kTriWarps, i = (l << sh) + r;
-      if (!(l < rows && i > k)) continue;
-      const double pi = tn * warp_sum(sum[q]);
-      if (lane < C) cl.map_shared_rank(sp, lane)[(par ^ 1) * m + i] = pi;
+    {
+      const double pi = tn * warp_sums<kTriRows>(sum);
+      const int l = wid + (lane / 4) * kTriWarps, i = (l << sh) + r;
+      if (l < rows && i > k)
+        for (int c = lane & 3; c < C; c += 4) cl.map_shared_rank(sp, c)[(par ^ 1) * m + i] = pi;
     }
 #pragma unroll
     for (int q = 0; q < NR; ++q) v[q] = vn[q];
     t = tn;
     cl.sync();  // p and the next row have arrived
   }
-  // the last diagonal element (its row has had every update)
-  if (r == (m - 1) % C && tid == 0) d[m - 1] = A[(size_t)((m - 1) / C) * m + m - 1];
+  // the rest of the matrix, with its last update, for k_tridiag_block
+  const double* p_in = sp + (k0 & 1) * m;
+  const double* vr = svr + ((k0 & 1) ^ 1) * R;
+  double p[NR], s = 0.0;
+#pragma unroll
+  for (int q = 0; q < NR; ++q) {
+    const int j = lane + 32 * q;
+    p[q] = j >= k0 && j < m ? p_in[j] : 0.0;
+    s = fma(v[q], p[q], s);
+  }
+  const double K = -t * warp_sum(s);
+  for (int l = wid; l < rows; l += kTriWarps) {
+    const int i = (l << sh) + r;
+    if (i < k0) continue;
+    const double vi = vr[l], ci = fma(K, vi, p_in[i]);
+#pragma unroll
+    for (int q = 0; q < NR; ++q) {
+      const int j = lane + 32 * q;
+      if (j >= k0 && j < m)
+        tail[(i - k0) * kTriTail + j - k0] = A[(size_t)l * m + j] - fma(vi, p[q], ci * v[q]);
+    }
+  }
 }
 
 // The same for matrices beyond one cluster's shared memory (m <= kSmallEigMax), over the whole GPU: row
@@ -218,7 +284,8 @@ __global__ void __launch_bounds__(kTriThreads) k_tridiag(const double* __restric
 // each count up *ctr, and wait for all with a limit, after which *err is set and the kernel gives up
 // (launched cooperatively, so that all blocks run together).  Bound by latency: the meeting and the
 // exchange (2 us), two block sums, a square root and a division a column.  Measured at 672, 1,225 and
-// 1,500 rows 3.0, 6.1 and 7.6 ms (one cluster at 640: 2.9); the whole solve 4.0, 7.8 and 9.7 ms, where
+// 1,500 rows, to the last column, 3.0, 6.1 and 7.6 ms (one cluster at 640: 2.9; at 672 now 2.52, 128
+// columns short of the last); the whole solve 4.0, 7.8 and 9.7 ms, where
 // cuSOLVER's syevd takes 7.8, 15.6 and 19.6.
 constexpr int kGridThreads = 512, kGridWarps = kGridThreads / 32;
 constexpr int kGridCols = 4;    // columns a thread: m <= 2048
@@ -238,7 +305,7 @@ __device__ __forceinline__ double grid_block_sum(double v, double (&red)[2][kGri
 __global__ void __launch_bounds__(kGridThreads, 1) k_tridiag_grid(
     const double* __restrict__ T, int ldt, int m, double* __restrict__ d, double* __restrict__ e,
     double* __restrict__ tau, double* __restrict__ V, double* xch, unsigned long long* ctr,
-    unsigned long long* err) {
+    unsigned long long* err, double* __restrict__ tail) {
   extern __shared__ double sm[];
   __shared__ double red[2][kGridWarps], s_v[kGridRows], s_p[kGridRows], s_x[2];
   __shared__ double s_part[kGridWarps][kGridRows];
@@ -266,7 +333,8 @@ __global__ void __launch_bounds__(kGridThreads, 1) k_tridiag_grid(
   __syncthreads();
   double t = 0.0;
   int buf = 0;
-  for (int k = 0; k + 1 < m; ++k) {
+  const int k0 = m - kTriTail;
+  for (int k = 0; k <= k0; ++k) {
     const int par = k & 1;
     if (k > 0) {
       if (tid == 0) {  // all blocks have handed on p and row k
@@ -298,6 +366,10 @@ __global__ void __launch_bounds__(kGridThreads, 1) k_tridiag_grid(
 #pragma unroll
     for (int c = 0; c < kGridCols; ++c) s = fma(v[c], p[c], s);
     const double K = -t * grid_block_sum(s, red, buf);
+    if (k == k0) {
+      t = K;
+      break;
+    }
     const double vk = k > 0 ? 1.0 : 0.0, ck = k > 0 ? s_x[0] + K : 0.0;
     s = 0.0;
 #pragma unroll
@@ -346,19 +418,7 @@ __global__ void __launch_bounds__(kGridThreads, 1) k_tridiag_grid(
       }
       x[c] = y;
     }
-    // sums of the rows over the warp, halving the rows a lane carries at each step: lane l ends with
-    // row l / 2
-#pragma unroll
-    for (int o = 16, h = kGridRows / 2; h > 0; o >>= 1, h >>= 1) {
-      const bool up = lane & o;
-#pragma unroll
-      for (int l = 0; l < kGridRows / 2; ++l)
-        if (l < h) {
-          const double give = up ? sum[l] : sum[l + h], keep = up ? sum[l + h] : sum[l];
-          sum[l] = keep + __shfl_xor_sync(0xffffffffu, give, o);
-        }
-    }
-    const double wsum = sum[0] + __shfl_xor_sync(0xffffffffu, sum[0], 1);
+    const double wsum = warp_sums<kGridRows>(sum);
     if ((lane & 1) == 0) s_part[wid][lane >> 1] = wsum;
     __syncthreads();  // also: every thread has read s_v and s_p
     {
@@ -380,8 +440,150 @@ __global__ void __launch_bounds__(kGridThreads, 1) k_tridiag_grid(
       atomicAdd(ctr, 1ull);
     }
   }
-  const int l = (m - 1) / G;
-  if (r == (m - 1) % G && tid == 0) d[m - 1] = A[(size_t)l * m + m - 1];
+  // the rest of the matrix, with its last update (t: K), for k_tridiag_block
+#pragma unroll
+  for (int c = 0; c < kGridCols; ++c) {
+    const int j = tid + kGridThreads * c;
+    if (j < k0 || j >= m) continue;
+    for (int l = 0; l < rows; ++l)
+      if (l * G + r >= k0)
+        tail[(l * G + r - k0) * kTriTail + j - k0] =
+            A[(size_t)l * m + j] - fma(s_v[l], p[c], fma(t, s_v[l], s_p[l]) * v[c]);
+  }
+}
+
+// A warp's share of a column in k_tridiag_block: its rows from 32 C0 on, in the columns from 32 C0 on,
+// updated (A - v w^T - w v^T, w = p + K / 2 v, K2 = K / 2) and multiplied by the new reflector vn; row k + 1 is put out.
+template <int C0>
+__device__ __forceinline__ void block_pass(double (&a)[16][4], double (&sum)[16], const double (&w)[4],
+                                           const double (&v)[4], const double (&vn)[4], double K2,
+                                           const double* sv, const double* sp, double* srow, int k, int wid,
+                                           int lane) {
+#pragma unroll
+  for (int q = 0; q < 16; ++q) sum[q] = 0.0;
+#pragma unroll
+  for (int q = 4 * C0; q < 16; ++q) {
+    const int i = 8 * q + wid;
+    const double vi = i > k ? -sv[i] : 0.0, wi = i > k ? fma(K2, vi, -sp[i]) : 0.0;  // -v, -w
+#pragma unroll
+    for (int c = C0; c < 4; ++c) a[q][c] = fma(wi, v[c], fma(vi, w[c], a[q][c]));
+#pragma unroll
+    for (int c = C0; c < 4; ++c) sum[q] = fma(a[q][c], vn[c], sum[q]);
+  }
+  if (wid == ((k + 1) & 7))
+#pragma unroll
+    for (int q = 4 * C0; q < 16; ++q)
+      if (8 * q + wid == k + 1)
+#pragma unroll
+        for (int c = C0; c < 4; ++c) srow[lane + 32 * c] = a[q][c];
+}
+
+// The same for n <= 128 rows, in one block that holds the matrix in registers: warp w keeps the rows
+// 8 q + w, a lane their columns lane + 32 c; p, v and the next row go through shared memory, and the
+// block meets once a column.  T holds the upper triangle, column-major; V's rows lie ldv apart.  Bound by
+// latency (two warp sums, a square root and a division, the sums of the rows), and at its first columns by
+// the FP64 rate of one SM: 128 rows take 155 us, 1.2 us a column (16 warps with the finished rows left out
+// by a branch each: 250).  128 rows because half as many again would not fit the registers; it also ends
+// the larger matrices, where a column costs a meeting of the cluster (2.3 us at 192 rows) or the grid.
+__global__ void __launch_bounds__(kBlockThreads, 1) k_tridiag_block(const double* __restrict__ T, int ldt, int n,
+                                                                    double* __restrict__ d,
+                                                                    double* __restrict__ e,
+                                                                    double* __restrict__ tau,
+                                                                    double* __restrict__ V, int ldv) {
+  constexpr int W = kBlockThreads / 32, RQ = kTriTail / W, NC = kTriTail / 32;
+  static_assert(W == 8 && RQ == 16 && NC == 4, "block_pass is written for these");
+  chain_wait();
+  __shared__ double sp[2][kTriTail], srow[2][kTriTail], sv[2][kTriTail];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  double a[RQ][NC];
+#pragma unroll
+  for (int q = 0; q < RQ; ++q)
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const int i = W * q + wid, j = lane + 32 * c;
+      a[q][c] = i < n && j < n ? (i <= j ? T[i + (int64_t)j * ldt] : T[j + (int64_t)i * ldt]) : 0.0;
+    }
+  if (threadIdx.x < kTriTail) {
+    const int j = threadIdx.x;
+    sp[0][j] = sp[1][j] = sv[0][j] = sv[1][j] = srow[1][j] = 0.0;
+    srow[0][j] = j < n ? T[(int64_t)j * ldt] : 0.0;  // row 0
+  }
+  double v[NC], t = 0.0;
+#pragma unroll
+  for (int c = 0; c < NC; ++c) v[c] = 0.0;
+  __syncthreads();
+  for (int k = 0; k + 1 < n; ++k) {
+    const int par = k & 1, c0 = (k + 1) >> 5;  // columns before chunk c0 are done
+    double p[NC], x[NC], w[NC], s = 0.0, s1 = 0.0;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const int j = lane + 32 * c;
+      p[c] = j >= k ? sp[par][j] : 0.0;
+      x[c] = j >= k ? srow[par][j] : 0.0;
+      if (c & 1) s1 = fma(v[c], p[c], s1); else s = fma(v[c], p[c], s);
+    }
+    const double K = -t * warp_sum_mma(s + s1);
+    const double vk = k > 0 ? 1.0 : 0.0, ck = fma(K, vk, sp[par][k]);
+    const double K2 = 0.5 * K;
+    s = s1 = 0.0;
+    double alpha = 0.0;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {  // row k, updated
+      const int j = lane + 32 * c;
+      x[c] -= fma(vk, p[c], ck * v[c]);
+      const double y = j > k + 1 ? x[c] : 0.0;
+      if (c & 1) s1 = fma(y, y, s1); else s = fma(y, y, s);
+      w[c] = fma(K2, v[c], p[c]);
+      if (c == c0) alpha = x[c];
+    }
+    alpha = __shfl_sync(0xffffffffu, alpha, (k + 1) & 31);
+    const double ss = warp_sum_mma(s + s1);
+    double beta = alpha, inv = 0.0, tn = 0.0;
+    if (ss > 0.0 && k + 2 < n) {
+      beta = -copysign(sqrt(fma(alpha, alpha, ss)), alpha);
+      const double g = 1.0 / (beta * (alpha - beta));
+      inv = beta * g;
+      tn = (beta - alpha) * ((alpha - beta) * g);
+    }
+    double vn[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const int j = lane + 32 * c;
+      vn[c] = j > k + 1 ? x[c] * inv : (j == k + 1 ? 1.0 : 0.0);
+    }
+    if (wid == (k & (W - 1))) {
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const int j = lane + 32 * c;
+        sv[par][j] = vn[c];
+        if (j == k) d[k] = x[c];
+        if (j > k && j < n) V[(int64_t)k * ldv + j] = vn[c];
+      }
+      if (lane == 0) {
+        e[k] = beta;
+        tau[k] = tn;
+      }
+    }
+    double sum[RQ];
+    switch (c0) {  // finished rows and columns are left out 32 at a time, without a branch a row
+      case 0: block_pass<0>(a, sum, w, v, vn, K2, sv[par ^ 1], sp[par], srow[par ^ 1], k, wid, lane); break;
+      case 1: block_pass<1>(a, sum, w, v, vn, K2, sv[par ^ 1], sp[par], srow[par ^ 1], k, wid, lane); break;
+      case 2: block_pass<2>(a, sum, w, v, vn, K2, sv[par ^ 1], sp[par], srow[par ^ 1], k, wid, lane); break;
+      default: block_pass<3>(a, sum, w, v, vn, K2, sv[par ^ 1], sp[par], srow[par ^ 1], k, wid, lane); break;
+    }
+    const double pi = tn * warp_sums<RQ>(sum);
+    const int i = W * (lane >> 1) + wid;
+    if ((lane & 1) == 0 && i > k) sp[par ^ 1][i] = pi;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) v[c] = vn[c];
+    t = tn;
+    __syncthreads();
+  }
+#pragma unroll
+  for (int q = 0; q < RQ; ++q)
+#pragma unroll
+    for (int c = 0; c < NC; ++c)
+      if (W * q + wid == n - 1 && lane + 32 * c == n - 1) d[n - 1] = a[q][c];
 }
 
 // Eigenvalue j (j < nk; the last warp takes the largest, for its value alone) of the tridiagonal
@@ -696,18 +898,15 @@ constexpr size_t vec_smem(int m) { return (size_t)m * (3 + 2 * kVecWarps) * size
 // Blocks of the cluster for m rows (its rows must fit the shared memory and kTriRows rounds): 16 (the
 // barrier reaches over more of the chip, the pass over the rows is shorter) pay from 256 rows on:
 // 0.64 : 0.66 ms there, 0.99 : 1.17 at 352; four are 10 to 20 % slower than eight from 128 on.
-int tri_blocks(int m) {
-  return m <= 32 ? 4 : (m < 256 ? 8 : 16);
-}
+int tri_blocks(int m) { return m < 256 ? 8 : 16; }
 
 // Blocks of the grid for m rows: eight rows a block, fewer when the GPU has no more SMs.
 int grid_blocks(int m) { return std::min(148, (m + 7) / 8); }
 size_t grid_smem(int m) { return (size_t)((m + grid_blocks(m) - 1) / grid_blocks(m)) * m * sizeof(double); }
 
-using TriKernel = void (*)(const double*, int, int, double*, double*, double*, double*, double*);
+using TriKernel = void (*)(const double*, int, int, double*, double*, double*, double*, double*, double*);
 TriKernel tri_kernel(int m) {
-  return m <= 64 ? k_tridiag<2> : m <= 128 ? k_tridiag<4> : m <= 192 ? k_tridiag<6> : m <= 256 ? k_tridiag<8>
-         : m <= 384 ? k_tridiag<12> : k_tridiag<20>;
+  return m <= 192 ? k_tridiag<6> : m <= 256 ? k_tridiag<8> : m <= 384 ? k_tridiag<12> : k_tridiag<20>;
 }
 
 // Shared-memory and cluster limits of the kernels, set once per device.
@@ -721,7 +920,7 @@ bool eig_attributes() {
   std::call_once(g_eig_once[dev], [dev] {
     bool ok = cudaFuncSetAttribute(k_tri_vectors, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)vec_smem(kSmallEigMax)) == cudaSuccess;
-    for (int m : {64, 128, 192, 256, 384, kClusterEigMax}) {
+    for (int m : {192, 256, 384, kClusterEigMax}) {
       const TriKernel k = tri_kernel(m);
       ok = ok && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) == cudaSuccess &&
            cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
@@ -736,8 +935,8 @@ bool eig_attributes() {
 }  // namespace
 
 size_t small_eig_elems(int m, int nk) {
-  // d, e, tau; the exchange; V; two vector blocks; S
-  return 7 * (size_t)m + (size_t)m * m + 2 * (size_t)m * nk + (size_t)nk * nk;
+  // d, e, tau; the exchange; V; two vector blocks; S; the last rows
+  return 7 * (size_t)m + (size_t)m * m + 2 * (size_t)m * nk + (size_t)nk * nk + kTriTail * kTriTail;
 }
 
 bool small_eig(const double* T, int ldt, int m, int nk, double* theta, double* Y, int ldy, double* work,
@@ -752,36 +951,43 @@ bool small_eig(const double* T, int ldt, int m, int nk, double* theta, double* Y
   double* Za = V + (size_t)m * m;
   double* Zb = Za + (size_t)m * nk;
   double* S = Zb + (size_t)m * nk;
+  double* tail = S + (size_t)nk * nk;
   cudaMemsetAsync(dev, 0, kSmallEigDev * sizeof(unsigned long long), s);
   const bool cluster = m <= kClusterEigMax;
-  cudaLaunchConfig_t cfg{};
-  cfg.stream = s;
-  cudaLaunchAttribute at{};
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  cudaError_t err;
+  const int k0 = std::max(0, m - kTriTail);  // columns before the last ones
+  if (k0 > 0) {
+    cudaLaunchConfig_t cfg{};
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaError_t err;
+    note_launch();
+    if (cluster) {
+      const int C = tri_blocks(m);
+      cfg.gridDim = dim3(C);
+      cfg.blockDim = dim3(kTriThreads);
+      cfg.dynamicSmemBytes = tri_smem(m, C);
+      at.id = cudaLaunchAttributeClusterDimension;
+      at.val.clusterDim.x = C;
+      at.val.clusterDim.y = at.val.clusterDim.z = 1;
+      err = cudaLaunchKernelEx(&cfg, tri_kernel(m), T, ldt, m, d, e, tau, V, rowx, tail);
+    } else {
+      cfg.gridDim = dim3(grid_blocks(m));
+      cfg.blockDim = dim3(kGridThreads);
+      cfg.dynamicSmemBytes = grid_smem(m);
+      at.id = cudaLaunchAttributeCooperative;
+      at.val.cooperative = 1;
+      err = cudaLaunchKernelEx(&cfg, k_tridiag_grid, T, ldt, m, d, e, tau, V, rowx, dev + 2, dev + 3, tail);
+    }
+    if (err != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+  }
   note_launch();
-  if (cluster) {
-    const int C = tri_blocks(m);
-    cfg.gridDim = dim3(C);
-    cfg.blockDim = dim3(kTriThreads);
-    cfg.dynamicSmemBytes = tri_smem(m, C);
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = C;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    err = cudaLaunchKernelEx(&cfg, tri_kernel(m), T, ldt, m, d, e, tau, V, rowx);
-  } else {
-    cfg.gridDim = dim3(grid_blocks(m));
-    cfg.blockDim = dim3(kGridThreads);
-    cfg.dynamicSmemBytes = grid_smem(m);
-    at.id = cudaLaunchAttributeCooperative;
-    at.val.cooperative = 1;
-    err = cudaLaunchKernelEx(&cfg, k_tridiag_grid, T, ldt, m, d, e, tau, V, rowx, dev + 2, dev + 3);
-  }
-  if (err != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
+  launch_chained(k_tridiag_block, 1, kBlockThreads, 0, s, k0 > 0 ? tail : T, k0 > 0 ? kTriTail : ldt, m - k0,
+                 d + k0, e + k0, tau + k0, V + (size_t)k0 * m + k0, m);
   note_launch();
   launch_chained(k_tri_vectors, (nk + 1 + kVecWarps - 1) / kVecWarps, 32 * kVecWarps, vec_smem(m), s, d, e, m, nk,
                                                                                           theta, Za);
