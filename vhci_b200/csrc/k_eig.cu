@@ -587,7 +587,9 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_tridiag_block(const double
 }
 
 // Eigenvalue j (j < nk; the last warp takes the largest, for its value alone) of the tridiagonal
-// matrix, scaled to norm 1, and its vector in column j of Z (leading dimension m).  The Sturm count
+// matrix, scaled to norm 1, and its vector in column j of Z (leading dimension m).  Bound by the latency of
+// the recurrences: 192 rows take 51 us, 672 rows 170 (with one point a lane and the pivots by division
+// 130 and 455).  The Sturm count
 // uses the three-term recurrence of the characteristic polynomials (one multiply-add of latency a
 // step where the quotient form has a division), rescaled every eight steps; squared off-diagonals
 // below 1e-34 are raised to that, a change below the rounding of the matrix.
@@ -604,6 +606,8 @@ __global__ void __launch_bounds__(32 * kVecWarps) k_tri_vectors(const double* __
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   double* P = se2 + m + (size_t)wid * 2 * m;  // forward pivots, then the vector
   double* M = P + m;                          // backward pivots
+  const int fs = m / 8 + 1;
+  double* F = se2 + m + (size_t)kVecWarps * 2 * m + (size_t)wid * 2 * fs;  // their rescalings, every 8 rows
   // norm: the largest row sum
   double nrm = 0.0;
   for (int i = tid; i < m; i += blockDim.x) {
@@ -629,56 +633,114 @@ __global__ void __launch_bounds__(32 * kVecWarps) k_tri_vectors(const double* __
   if (w > nk || (w == nk && nk >= m)) return;
   const int j = w < nk ? w : m - 1;
 
-  // eigenvalue j lies in [lo, hi): counts of the eigenvalues below 32 points inside
+  // eigenvalue j lies in [lo, hi): counts of the eigenvalues below 64 points inside, two a lane, whose
+  // recurrences overlap
   double lo = -1.0000001, hi = 1.0000001;
-  for (int round = 0; round < 12; ++round) {
-    const double x = lo + (hi - lo) * ((lane + 1) * (1.0 / 33.0));
-    double p0 = 1.0, p1 = sd[0] - x;
-    int below = (unsigned)__double2hiint(p1) >> 31;  // sign changes, by the sign bits
-    for (int i = 1; i < m; i += 8) {
-      const int n = min(8, m - i);
+  for (int round = 0; round < 10; ++round) {
+    const double wd = (hi - lo) * (1.0 / 65.0);
+    double x[2], p0[2], p1[2];
+    int below[2];
 #pragma unroll
-      for (int q = 0; q < 8; ++q)
-        if (q < n) {
-          const double p2 = fma(sd[i + q] - x, p1, -se2[i + q - 1] * p0);
-          below += (unsigned)(__double2hiint(p2) ^ __double2hiint(p1)) >> 31;
-          p0 = p1;
-          p1 = p2;
-        }
-      const double big = fmax(fabs(p0), fabs(p1));
-      if (big > 1e100) { p0 *= 1e-100; p1 *= 1e-100; }
-      else if (big < 1e-100) { p0 *= 1e100; p1 *= 1e100; }
+    for (int h = 0; h < 2; ++h) {
+      x[h] = lo + wd * (2 * lane + h + 1);
+      p0[h] = 1.0;
+      p1[h] = sd[0] - x[h];
+      below[h] = (unsigned)__double2hiint(p1[h]) >> 31;  // sign changes, by the sign bits
     }
-    const int n = __popc(__ballot_sync(0xffffffffu, below <= j));
-    const double a = __shfl_sync(0xffffffffu, x, max(0, n - 1)), b = __shfl_sync(0xffffffffu, x, min(31, n));
-    if (n > 0) lo = a;
-    if (n < 32) hi = b;
+    auto step = [&](double di, double e2) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const double p2 = fma(di - x[h], p1[h], -e2 * p0[h]);
+        below[h] += (unsigned)(__double2hiint(p2) ^ __double2hiint(p1[h])) >> 31;
+        p0[h] = p1[h];
+        p1[h] = p2;
+      }
+    };
+    auto rescale = [&] {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const double big = fmax(fabs(p0[h]), fabs(p1[h]));
+        const double f = big > 1e100 ? 1e-100 : (big < 1e-100 ? 1e100 : 1.0);
+        p0[h] *= f;
+        p1[h] *= f;
+      }
+    };
+    int i = 1;
+    for (; i + 8 <= m; i += 8) {
+      double di[8], e2[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        di[q] = sd[i + q];
+        e2[q] = se2[i + q - 1];
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q) step(di[q], e2[q]);
+      rescale();
+    }
+    for (; i < m; ++i) step(sd[i], se2[i - 1]);
+    const int n = __popc(__ballot_sync(0xffffffffu, below[0] <= j)) +
+                  __popc(__ballot_sync(0xffffffffu, below[1] <= j));  // points up to the eigenvalue
+    const double l0 = lo;
+    if (n > 0) lo = l0 + wd * n;
+    if (n < 64) hi = l0 + wd * (n + 1);
     if (hi - lo <= 1e-17) break;
   }
   const double lam = 0.5 * (lo + hi);
   if (lane == 0) theta[j] = lam * nrm;
   if (w >= nk) return;
 
-  // twisted factorisation of T - lam: forward pivots by lane 0, backward ones by lane 1
+  // twisted factorisation of T - lam: forward pivots by lane 0, backward ones by lane 1, at once.  The
+  // lanes run the recurrence of the characteristic polynomials too; a pivot is the ratio of two that follow
+  // one another, and all lanes take the ratios afterwards (with a division in the recurrence, one lane
+  // after the other, 192 rows took 26 us more).
   constexpr double tiny = 1e-17;
-  if (lane == 0) {
-    double q = sd[0] - lam;
-    for (int i = 0;; ) {
-      if (fabs(q) < tiny) q = copysign(tiny, q);
-      P[i] = q;
-      if (++i >= m) break;
-      q = (sd[i] - lam) - se2[i - 1] / q;
-    }
-  } else if (lane == 1) {
-    double q = sd[m - 1] - lam;
-    for (int i = m - 1;; ) {
-      if (fabs(q) < tiny) q = copysign(tiny, q);
-      M[i] = q;
-      if (--i < 0) break;
-      q = (sd[i] - lam) - se2[i] / q;
+  if (lane < 2) {
+    double* out = lane ? M : P;
+    double* fo = F + lane * fs;
+    const int s = lane ? -1 : 1, o = lane ? m - 1 : 0, o2 = lane ? m - 1 : -1;  // row of step i: o + s i
+    double p0 = 1.0, p1 = sd[o] - lam;
+    if (fabs(p1) < tiny) p1 = copysign(tiny, p1);
+    out[o] = p1;
+    for (int i = 1; i < m; i += 8) {
+      double di[8], e2[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const bool in = i + q < m;
+        di[q] = in ? sd[o + s * (i + q)] - lam : 0.0;
+        e2[q] = in ? se2[o2 + s * (i + q)] : 0.0;
+      }
+      const double big = fmax(fabs(p0), fabs(p1));
+      const double f = big > 1e100 ? 1e-100 : (big < 1e-100 ? 1e100 : 1.0);
+      p0 *= f;
+      p1 *= f;
+      fo[i >> 3] = f;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        double p2 = fma(di[q], p1, -e2[q] * p0);
+        const double least = tiny * fabs(p1);
+        if (fabs(p2) < least) p2 = copysign(least, p2);
+        if (i + q < m) out[o + s * (i + q)] = p2;
+        p0 = p1;
+        p1 = p2;
+      }
     }
   }
   __syncwarp();
+  for (int c = (m - 1) / 32 * 32; c >= 0; c -= 32) {  // forward ones from the end, backward ones from row 0
+    const int i = c + lane, jr = m - 1 - i;
+    double q = 0.0, r = 0.0;
+    if (i < m) {
+      const bool f = (i & 7) == 1;
+      q = i > 0 ? P[i] / (P[i - 1] * (f ? F[i >> 3] : 1.0)) : P[0];
+      r = i > 0 ? M[jr] / (M[jr + 1] * (f ? F[fs + (i >> 3)] : 1.0)) : M[jr];
+    }
+    __syncwarp();
+    if (i < m) {
+      P[i] = q;
+      M[jr] = r;
+    }
+    __syncwarp();
+  }
   double best = 1e300;
   int twist = 0;
   for (int i = lane; i < m; i += 32) {
@@ -699,12 +761,14 @@ __global__ void __launch_bounds__(32 * kVecWarps) k_tri_vectors(const double* __
     P[i] = i < twist ? up : (i > twist ? dn : 1.0);
   }
   __syncwarp();
-  if (lane == 0) {
-    double z = 1.0;
-    for (int i = twist - 1; i >= 0; --i) P[i] = z = P[i] * z;
-  } else if (lane == 1) {
-    double z = 1.0;
-    for (int i = twist + 1; i < m; ++i) P[i] = z = P[i] * z;
+  if (lane < 2) {
+    const int s = lane ? 1 : -1, n = lane ? m - 1 - twist : twist;
+    double z = 1.0, next = n > 0 ? P[twist + s] : 0.0;
+    for (int x = 1; x <= n; ++x) {
+      const double y = next;
+      next = x < n ? P[twist + s * (x + 1)] : 0.0;
+      P[twist + s * x] = z = y * z;
+    }
   }
   __syncwarp();
   double s = 0.0;
@@ -893,7 +957,9 @@ __global__ void __launch_bounds__(128) k_back_block(const double* __restrict__ Z
   }
 }
 
-constexpr size_t vec_smem(int m) { return (size_t)m * (3 + 2 * kVecWarps) * sizeof(double); }
+constexpr size_t vec_smem(int m) {
+  return ((size_t)m * (3 + 2 * kVecWarps) + (size_t)(m / 8 + 1) * 2 * kVecWarps) * sizeof(double);
+}
 
 // Blocks of the cluster for m rows (its rows must fit the shared memory and kTriRows rounds): 16 (the
 // barrier reaches over more of the chip, the pass over the rows is shorter) pay from 256 rows on:
