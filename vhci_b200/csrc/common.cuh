@@ -141,9 +141,17 @@ __device__ __forceinline__ void load_slots(const uint64_t* p, ulonglong2& a, ulo
       : "l"(p));
 }
 
-// Presence bits of a table's keys by the upper hash bits, small enough for a block's shared memory.
+// Presence bits of a table's keys by the upper hash bits, small enough for a block's shared memory: a key
+// sets two bits of one word.  A key that is not there finds both set in 11 % of the cases with 200,000
+// keys in the table, where one bit a key is found set in 17 %; at 2^19 keys the two are equal (40 %).
 constexpr int kBitsLog = 20, kBitsWords = 1 << (kBitsLog - 5);
-__device__ __forceinline__ uint32_t bits_index(uint64_t h) { return (uint32_t)(h >> (64 - kBitsLog)); }
+struct KeyBits {
+  uint32_t word, first, second;  // shifts: modulo 32
+};
+__device__ __forceinline__ KeyBits key_bits(uint64_t h) {
+  const uint32_t x = (uint32_t)(h >> 32);
+  return {x >> (37 - kBitsLog), x >> (32 - kBitsLog), x >> (27 - kBitsLog)};
+}
 
 // Returns the key's index or -1.
 template <int W>

@@ -274,8 +274,9 @@ __device__ __forceinline__ void walk_connections(const ConnDev& cd, const HashVi
       if constexpr (FILTER) {
 #pragma unroll
         for (int t = 0; t < ILP; ++t) {
-          const uint32_t x = bits_index(hash_final(hk + h[t]));
-          const bool on = u[t] != kNoIndex && ((sbits[x >> 5] >> (x & 31)) & 1u);
+          const KeyBits x = key_bits(hash_final(hk + h[t]));
+          const uint32_t s = sbits[x.word];
+          const bool on = u[t] != kNoIndex && ((s >> (x.first & 31)) & (s >> (x.second & 31)) & 1u);
           const unsigned m = __ballot_sync(full, on);
           if (on) ws.maybe[(mtail + __popc(m & lanemask_lt())) % WS::kMaybe] = u[t];
           mtail += __popc(m);

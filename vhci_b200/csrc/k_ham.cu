@@ -71,15 +71,15 @@ __global__ void __launch_bounds__(256) k_hash_bits(const uint64_t* __restrict__ 
        i += (int64_t)gridDim.x * blockDim.x) {
     uint64_t k[W];
     load_key<W>(keys, i, k);
-    const uint32_t x = bits_index(key_hash<W>(k));
-    atomicOr(bits + (x >> 5), 1u << (x & 31));
+    const KeyBits x = key_bits(key_hash<W>(k));
+    atomicOr(bits + x.word, 1u << (x.first & 31) | 1u << (x.second & 31));
   }
 }
 
 // The count pass with the table's presence bits in shared memory: one block of 32 warps per SM, each
-// warp taking the next row when it has done one.  Bound by instruction issue (65 a round of 32 visits,
-// 73 % of the issue slots).  Measured against the plain count pass: 200,000 states of 48 modes 13.3 ->
-// 7.7 ms, 40,000 of 30 modes 3.7 -> 1.7 ms, 150,001 of 15 modes 3.2 -> 2.5 ms.
+// warp taking the next row when it has done one.  Bound by instruction issue (about 60 a round of 32
+// visits).  Measured against the plain count pass: 200,000 states of 48 modes 13.3 -> 6.9 ms (7.7 with
+// one presence bit a key), 40,000 of 30 modes 3.7 -> 1.7 ms, 150,001 of 15 modes 3.2 -> 2.35 ms.
 constexpr int kFiltThreads = 1024, kFiltWarps = kFiltThreads / 32;
 constexpr size_t kFiltSmem = kBitsWords * sizeof(uint32_t) + kFiltWarps * sizeof(WalkScratch<true>) +
                              kBinomElems * sizeof(uint32_t);
