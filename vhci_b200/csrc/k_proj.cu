@@ -453,7 +453,7 @@ void launch_rows(const double* A, int lda, const double* S, int lds, int64_t n, 
 // whose pivot (the squared sine of its angle to the columns before it) is at most 1e-12, or whose
 // diagonal is at most 1e-28 of the largest, is a lost direction: its column of M is zero and
 // *rank_short is set.  One warp holds the matrix, lane = column; bound by the chain of nb square
-// roots and divisions: measured 12 us with the sum of 148 partial products, where a Jacobi
+// roots and divisions: measured 11 us with the sum of 148 partial products, where a Jacobi
 // eigensolver took 88.
 constexpr int kSvqbThreads = 1024;
 __global__ void __launch_bounds__(kSvqbThreads) k_svqb_factor(const double* __restrict__ part,
