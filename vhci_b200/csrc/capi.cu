@@ -416,11 +416,12 @@ void spmm_h(vhci_ctx* c, const double* X, int ldx, int b, double* Y, int ldy) {
          c->diag.p, X, ldx, b, Y, ldy, c->row0, c->st);
 }
 
-// Column panels for the product: one 16-column FP64 block row is 128 bytes, and each panel's rows
-// take about 96 MB of the 126 MB L2, so panels start at two when the block's rows exceed 96 MB
-// (N > 750k).  VHCI_PANEL_MB sets the panel size; VHCI_PANELS=0 turns panels off.  On the 6.1M-state, 1.17e9-entry matrix
-// 96 MB panels measured 3 % faster than one pass and 48 MB ones no faster: the product there is
-// bound by the dependent index-then-gather loads more than by where the block rows live.  Skipped when the regrouped copy does not fit
+// Column panels for the product, on request: VHCI_PANEL_MB sets the size of a panel's block rows (128
+// bytes a state and 16 columns; VHCI_PANELS=0 turns them off again).  With one warp per row they lose
+// at every size measured, since each panel's part of a row is short: one pass against panels of 96 MB,
+// 1.0M and 2.0M states of 15 modes (537 and 624 entries a row) 5.8 : 6.2 and 13.9 : 15.3 ms, 1.5M and
+// 3.0M of 48 modes (133 and 152 entries) 3.05 : 3.7 and 7.05 : 10.5 ms, 6.0M of 48 modes 16.2 ms.  (Four
+// rows per warp with panels: 6.5, 15.8, 3.2, 8.1 and 20.0.)  Skipped when the regrouped copy does not fit
 // in free device memory.
 static int build_panels(vhci_ctx* c) {
   c->npanel = 0;
@@ -428,8 +429,9 @@ static int build_panels(vhci_ctx* c) {
   const int64_t nr = c->nrow;  // rows held
   if (const char* e = std::getenv("VHCI_PANELS"))
     if (std::atoi(e) == 0) return VHCI_OK;
-  double pbytes = 96e6;
-  if (const char* e = std::getenv("VHCI_PANEL_MB")) pbytes = std::max(0.01, std::atof(e)) * 1e6;
+  const char* asked = std::getenv("VHCI_PANEL_MB");
+  if (!asked) return VHCI_OK;
+  const double pbytes = std::max(0.01, std::atof(asked)) * 1e6;
   int P = (int)std::ceil((double)n * 128.0 / pbytes);
   if (P < 2 || c->nnz == 0) return VHCI_OK;
   P = std::min(P, kMaxPanels);

@@ -121,7 +121,7 @@ struct vhci_ctx {
   vhci::DBuf<double> val;
   vhci::DBuf<float> valf;
   vhci::DBuf<double> diag;
-  // column panels of the off-diagonal entries (built with H when the gathered block outgrows L2)
+  // column panels of the off-diagonal entries (built with H on request)
   int npanel = 0;
   int64_t panel_cw = 0;
   vhci::DBuf<int64_t> prow;

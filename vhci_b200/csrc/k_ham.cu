@@ -437,8 +437,8 @@ void diag_energies(const uint64_t* keys, int64_t row0, int64_t n, KeyLayout L, C
 }
 
 // ---- column panels: the off-diagonal entries regrouped by column range -----------------------
-// When the gathered block no longer fits in L2, the product runs once per column panel, so the
-// rows gathered in one pass (one panel of the block) stay L2-resident while H streams once.
+// On request (capi.cu) the product runs once per column panel, so that the rows gathered in one
+// pass (one panel of the block) stay L2-resident while H streams once.
 // Layout: entries of panel p for row i at [prow[p n + i], prow[p n + i + 1]); within a (panel,
 // row) cell entries keep their CSR order, so the product is deterministic.
 
