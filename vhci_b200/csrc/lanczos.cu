@@ -157,6 +157,7 @@ int gemm_gram(vhci_ctx* c, LWork& w, const double* A, int lda, const double* B, 
     VTRY(comm_sum(c, out, (int64_t)M * P));
     VCK(cudaMemcpy2DAsync(C, ldc * sizeof(double), out, M * sizeof(double), M * sizeof(double), P,
                           cudaMemcpyDeviceToDevice, c->st));
+    if (Acc) add_cols(out, M, M, P, Acc, ldacc, c->st);  // the sum over the ranks, as the kernel does alone
   }
   return VHCI_OK;
 }
