@@ -9,6 +9,11 @@
 // returns when that kernel has ended and its writes are visible.  (It ended after its own chain_wait, so
 // all that came before it has ended too.)  A kernel that does not call chain_wait is launched plainly,
 // before or after a chained one, as ever.
+//
+// k's life overlaps that of the kernel before it, so what that kernel writes is not read-only during k:
+// k reads it by ordinary loads, never by __ldg or ld.global.nc (which a compiler may also move to before
+// the wait) nor through const __restrict__ pointers (whose loads it may turn into such).  The matrix and
+// other tables are complete before the kernel before k begins, and stay with the read-only loads.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -485,7 +485,7 @@ __device__ __forceinline__ void block_pass(double (&a)[16][4], double (&sum)[16]
 // the FP64 rate of one SM: 128 rows take 155 us, 1.2 us a column (16 warps with the finished rows left out
 // by a branch each: 250).  128 rows because half as many again would not fit the registers; it also ends
 // the larger matrices, where a column costs a meeting of the cluster (2.3 us at 192 rows) or the grid.
-__global__ void __launch_bounds__(kBlockThreads, 1) k_tridiag_block(const double* __restrict__ T, int ldt, int n,
+__global__ void __launch_bounds__(kBlockThreads, 1) k_tridiag_block(const double* T, int ldt, int n,
                                                                     double* __restrict__ d,
                                                                     double* __restrict__ e,
                                                                     double* __restrict__ tau,
@@ -593,8 +593,8 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_tridiag_block(const double
 // uses the three-term recurrence of the characteristic polynomials (one multiply-add of latency a
 // step where the quotient form has a division), rescaled every eight steps; squared off-diagonals
 // below 1e-34 are raised to that, a change below the rounding of the matrix.
-__global__ void __launch_bounds__(32 * kVecWarps) k_tri_vectors(const double* __restrict__ d,
-                                                                const double* __restrict__ e, int m,
+__global__ void __launch_bounds__(32 * kVecWarps) k_tri_vectors(const double* d,
+                                                                const double* e, int m,
                                                                 int nk, double* __restrict__ theta,
                                                                 double* __restrict__ Z) {
   chain_wait();
@@ -785,7 +785,7 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
 
 // One warp per 8 x 32 tile of S = (3 I - Z^T Z) / 2 (nk x nk); *dev: the largest |Z^T Z - I| seen, as
 // the bits of a non-negative double.
-__global__ void __launch_bounds__(128) k_eig_gram(const double* __restrict__ Z, int m, int nk,
+__global__ void __launch_bounds__(128) k_eig_gram(const double* Z, int m, int nk,
                                                   double* __restrict__ S,
                                                   unsigned long long* __restrict__ dev) {
   chain_wait();
@@ -803,10 +803,10 @@ __global__ void __launch_bounds__(128) k_eig_gram(const double* __restrict__ Z, 
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
       const int k = k0 + 4 * s + kl;
-      a[s] = k < m ? __ldg(za + k) : 0.0;
+      a[s] = k < m ? za[k] : 0.0;
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-        b[s][u] = k < m ? __ldg(Z + (int64_t)min(b0 + 8 * u + q, nk - 1) * m + k) : 0.0;
+        b[s][u] = k < m ? Z[(int64_t)min(b0 + 8 * u + q, nk - 1) * m + k] : 0.0;
     }
 #pragma unroll
     for (int s = 0; s < 4; ++s)
@@ -831,7 +831,7 @@ __global__ void __launch_bounds__(128) k_eig_gram(const double* __restrict__ Z, 
 }
 
 // Out (m x nk) = Z S, one warp per 8 x 32 tile.
-__global__ void __launch_bounds__(128) k_eig_mul(const double* __restrict__ Z, const double* __restrict__ S,
+__global__ void __launch_bounds__(128) k_eig_mul(const double* Z, const double* S,
                                                  int m, int nk, double* __restrict__ Out) {
   chain_wait();
   const int lane = threadIdx.x & 31, w = blockIdx.x * 4 + (threadIdx.x >> 5);
@@ -847,10 +847,10 @@ __global__ void __launch_bounds__(128) k_eig_mul(const double* __restrict__ Z, c
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
       const int k = k0 + 4 * s + kl;
-      a[s] = k < nk ? __ldg(Z + (int64_t)k * m + min(i0 + q, m - 1)) : 0.0;
+      a[s] = k < nk ? Z[(int64_t)k * m + min(i0 + q, m - 1)] : 0.0;
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-        b[s][u] = k < nk ? __ldg(S + (int64_t)min(j0 + 8 * u + q, nk - 1) * nk + k) : 0.0;
+        b[s][u] = k < nk ? S[(int64_t)min(j0 + 8 * u + q, nk - 1) * nk + k] : 0.0;
     }
 #pragma unroll
     for (int s = 0; s < 4; ++s)
@@ -869,8 +869,8 @@ __global__ void __launch_bounds__(128) k_eig_mul(const double* __restrict__ Z, c
 // Y[:, j] = H_0 .. H_{m-3} Z[:, j], one warp per column with the column in registers (32 NR >= m) and
 // the next PF reflectors' loads in flight.
 template <int NR, int PF>
-__global__ void __launch_bounds__(64) k_back(const double* __restrict__ Z, const double* __restrict__ V,
-                                             const double* __restrict__ tau, int m, int nk,
+__global__ void __launch_bounds__(64) k_back(const double* Z, const double* V,
+                                             const double* tau, int m, int nk,
                                              double* __restrict__ Y, int ldy) {
   chain_wait();
   const int lane = threadIdx.x & 31, j = blockIdx.x * 2 + (threadIdx.x >> 5);
@@ -885,9 +885,9 @@ __global__ void __launch_bounds__(64) k_back(const double* __restrict__ Z, const
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
       const int i = lane + 32 * r;
-      u[r] = (k >= 0 && i > k && i < m) ? __ldg(V + (int64_t)k * m + i) : 0.0;
+      u[r] = (k >= 0 && i > k && i < m) ? V[(int64_t)k * m + i] : 0.0;
     }
-    tk = k >= 0 ? __ldg(tau + k) : 0.0;
+    tk = k >= 0 ? tau[k] : 0.0;
   };
 #pragma unroll
   for (int f = 0; f < PF; ++f) fetch(m - 3 - f, v[f], t[f]);
@@ -913,8 +913,8 @@ __global__ void __launch_bounds__(64) k_back(const double* __restrict__ Z, const
 
 // The same with one block of four warps per column (m <= 128 NR).
 template <int NR>
-__global__ void __launch_bounds__(128) k_back_block(const double* __restrict__ Z, const double* __restrict__ V,
-                                                    const double* __restrict__ tau, int m, int nk,
+__global__ void __launch_bounds__(128) k_back_block(const double* Z, const double* V,
+                                                    const double* tau, int m, int nk,
                                                     double* __restrict__ Y, int ldy) {
   chain_wait();
   __shared__ double red[2][4];
@@ -929,13 +929,13 @@ __global__ void __launch_bounds__(128) k_back_block(const double* __restrict__ Z
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
       const int i = tid + 128 * r;
-      w[r] = (k >= 0 && i > k && i < m) ? __ldg(V + (int64_t)k * m + i) : 0.0;
+      w[r] = (k >= 0 && i > k && i < m) ? V[(int64_t)k * m + i] : 0.0;
     }
   };
   fetch(m - 3, v);
   for (int k = m - 3; k >= 0; --k) {
     fetch(k - 1, u);
-    const double tk = __ldg(tau + k);
+    const double tk = tau[k];
     double s = 0.0, s1 = 0.0;
 #pragma unroll
     for (int r = 0; r < NR; ++r)

@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(256, 5) k_spmm(int64_t n, const int64_t* __res
                                                  const int32_t* __restrict__ col,
                                                  const VT* __restrict__ val,
                                                  const double* __restrict__ diag,
-                                                 const double* __restrict__ X, int ldx, int bq,
+                                                 const double* X, int ldx, int bq,
                                                  double* __restrict__ Y, int ldy, int accum,
                                                  int64_t xrow0) {
   chain_wait();
@@ -238,8 +238,8 @@ __global__ void __launch_bounds__(256, 4) k_spmm_f32x(int64_t n, const int64_t* 
                                                    const int32_t* __restrict__ col,
                                                    const float* __restrict__ val,
                                                    const double* __restrict__ diag,
-                                                   const float* __restrict__ X, int ldx, int bq,
-                                                   const double* __restrict__ Xd, int ldd,
+                                                   const float* X, int ldx, int bq,
+                                                   const double* Xd, int ldd,
                                                    double* __restrict__ Y, int ldy) {
   chain_wait();
   const int lane = threadIdx.x & 31, cc = lane % BQ;
@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(256) k_sum_parts(const double* __restrict__ pa
   if (lane == 0) out[c] = accumulate ? out[c] + s : s;
 }
 
-__global__ void k_copy_cols(const double* __restrict__ src, int lds, double* __restrict__ dst,
+__global__ void k_copy_cols(const double* src, int lds, double* __restrict__ dst,
                             int ldd, int64_t n, int ncol) {
   chain_wait();
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < n * ncol;
@@ -546,7 +546,7 @@ bool spmm_f32x(int64_t n, const int64_t* rowptr, const int32_t* col, const float
 }
 
 // Compact FP32 copy of ncol columns of a row-major FP64 block (rounded to nearest).
-__global__ void k_copy_cols_f32(const double* __restrict__ src, int lds, float* __restrict__ dst,
+__global__ void k_copy_cols_f32(const double* src, int lds, float* __restrict__ dst,
                                 int ldd, int64_t n, int ncol) {
   chain_wait();
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < n * ncol;

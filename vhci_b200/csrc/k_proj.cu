@@ -54,13 +54,13 @@ __device__ __forceinline__ void load4(double (&v)[4], const double* p, int k, in
   v[0] = v[1] = v[2] = v[3] = 0.0;
   if (wide) {
     if (k + 3 >= first && k < last)
-      asm volatile("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];"
+      asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];"
                    : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
                    : "l"(p));
   } else {
 #pragma unroll
     for (int s = 0; s < 4; ++s)
-      if (k + s >= first && k + s < last) v[s] = __ldg(p + s);
+      if (k + s >= first && k + s < last) v[s] = p[s];
   }
 }
 
@@ -88,8 +88,8 @@ inline int row_skew(const double* A, int lda, bool* wide) {
 // its products are issued, so that loads and products of one warp overlap.
 // Block x writes its partial to part[x] (Mc x P, a-major).
 template <int NT, int CT, int UNROLL, int NWARP>
-__global__ void __launch_bounds__(NWARP * 32, 1) k_gram(const double* __restrict__ A, int lda,
-                                                    const double* __restrict__ B, int ldb,
+__global__ void __launch_bounds__(NWARP * 32, 1) k_gram(const double* A, int lda,
+                                                    const double* B, int ldb,
                                                     int64_t n, int Mc, int P, int skew, bool wide,
                                                     bool bwide, double* __restrict__ part) {
   chain_wait();
@@ -119,27 +119,27 @@ __global__ void __launch_bounds__(NWARP * 32, 1) k_gram(const double* __restrict
     if (wide) {
       if (rin && ain) {
         if constexpr (CT == 4) {
-          asm volatile("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];"
+          asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];"
                        : "=d"(a[s][0]), "=d"(a[s][1]), "=d"(a[s][2]), "=d"(a[s][3])
                        : "l"(p));
         } else {
-          asm volatile("ld.global.nc.v2.f64 {%0,%1}, [%2];" : "=d"(a[s][0]), "=d"(a[s][1]) : "l"(p));
+          asm volatile("ld.global.v2.f64 {%0,%1}, [%2];" : "=d"(a[s][0]), "=d"(a[s][1]) : "l"(p));
         }
       }
     } else {
 #pragma unroll
       for (int t = 0; t < CT; ++t)
-        if (rin && acol + t < last) a[s][t] = __ldg(p + t);
+        if (rin && acol + t < last) a[s][t] = p[t];
     }
     const double* q = B + i * ldb + bcol;
 #pragma unroll
     for (int u = 0; u < NT; ++u) b[s][u] = 0.0;
     if (NT == 2 && bwide) {
-      if (rin) asm volatile("ld.global.nc.v2.f64 {%0,%1}, [%2];" : "=d"(b[s][0]), "=d"(b[s][NT - 1]) : "l"(q));
+      if (rin) asm volatile("ld.global.v2.f64 {%0,%1}, [%2];" : "=d"(b[s][0]), "=d"(b[s][NT - 1]) : "l"(q));
     } else {
 #pragma unroll
       for (int u = 0; u < NT; ++u)
-        if (rin && bcol + u < P) b[s][u] = __ldg(q + u);
+        if (rin && bcol + u < P) b[s][u] = q[u];
     }
   };
   const int64_t first = rg < RG ? r0 + 4 * UNROLL * rg + kl : r1 + kl;
@@ -211,7 +211,7 @@ void launch_gram(const double* A, int lda, const double* B, int ldb, int64_t n, 
 // one 256-byte segment) and the warps' sums are combined in warp order, so the result is the same
 // on every run.
 constexpr int kRedWarps = 32;
-__global__ void __launch_bounds__(kRedWarps * 32) k_gram_reduce(const double* __restrict__ part,
+__global__ void __launch_bounds__(kRedWarps * 32) k_gram_reduce(const double* part,
                                                                 int nblk, int M, int P, double alpha,
                                                                 double beta, double* __restrict__ C,
                                                                 int ldc, double* __restrict__ Acc,
@@ -277,8 +277,8 @@ struct RowsTail {
 // columns take 100 us (110 with 8-byte loads of 32 warps and the tiles of the last round on a third of the
 // SMs); a 32-column rotation of 672 columns takes 197 us, of which the tensor pipe needs 140 (231 before).
 template <int NT, bool SELF>
-__global__ void __launch_bounds__(kThreads, 1) k_rows(const double* __restrict__ A, int lda,
-                                                      const double* __restrict__ S, int lds,
+__global__ void __launch_bounds__(kThreads, 1) k_rows(const double* A, int lda,
+                                                      const double* S, int lds,
                                                       int64_t n, int Mc, int P, int skew, bool wide,
                                                       bool vec, double alpha, double beta, double* Out,
                                                       int ldo, RowsTail tail) {
@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_rows(const double* __restrict__
     const double* Sc = S - skew + (int64_t)c * lds;
 #pragma unroll 4
     for (int k = lane; k < Mr; k += 32)
-      ss[s_place<NT>(k, c)] = c < P && k >= skew && k < last ? __ldg(Sc + k) : 0.0;
+      ss[s_place<NT>(k, c)] = c < P && k >= skew && k < last ? Sc[k] : 0.0;
   }
   __syncthreads();
   const int c0 = 2 * NT * kl;  // the lane's columns of the result: c0 + NT j + u
@@ -456,7 +456,7 @@ void launch_rows(const double* A, int lda, const double* S, int lds, int64_t n, 
 // roots and divisions: measured 11 us with the sum of 148 partial products, where a Jacobi
 // eigensolver took 88.
 constexpr int kSvqbThreads = 1024;
-__global__ void __launch_bounds__(kSvqbThreads) k_svqb_factor(const double* __restrict__ part,
+__global__ void __launch_bounds__(kSvqbThreads) k_svqb_factor(const double* part,
                                                               int nparts, int nb,
                                                               double* __restrict__ M,
                                                               int* __restrict__ rank_short) {
@@ -533,8 +533,8 @@ __global__ void __launch_bounds__(kSvqbThreads) k_svqb_factor(const double* __re
 }
 
 // One block per 32 vectors; the partial sums of G are added as in k_svqb_factor.
-__global__ void __launch_bounds__(1024) k_krylov_residuals(const double* __restrict__ Y, int ldy, int nk,
-                                                           const double* __restrict__ part, int nparts,
+__global__ void __launch_bounds__(1024) k_krylov_residuals(const double* Y, int ldy, int nk,
+                                                           const double* part, int nparts,
                                                            int P, double* __restrict__ rn2) {
   chain_wait();
   __shared__ double ps[4][256], G[256];
@@ -563,7 +563,7 @@ __global__ void __launch_bounds__(1024) k_krylov_residuals(const double* __restr
   if (a == 0) rn2[j] = q;
 }
 
-__global__ void k_restart_matrix(double* __restrict__ T, int ld, const double* __restrict__ theta, int nk) {
+__global__ void k_restart_matrix(double* __restrict__ T, int ld, const double* theta, int nk) {
   chain_wait();
   for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < ld * ld; x += gridDim.x * blockDim.x) {
     const int c = x / ld, r = x - c * ld;
@@ -571,7 +571,7 @@ __global__ void k_restart_matrix(double* __restrict__ T, int ld, const double* _
   }
 }
 
-__global__ void k_add_cols(const double* __restrict__ src, int lds, int M, int P,
+__global__ void k_add_cols(const double* src, int lds, int M, int P,
                            double* __restrict__ dst, int ldd) {
   chain_wait();
   const int x = blockIdx.x * blockDim.x + threadIdx.x;

@@ -46,19 +46,20 @@ __device__ __forceinline__ void load_vals4(const float* p, float* v) {
 
 // Sum over the entries [beg, end) of one row of val * X[col, this lane's columns] into a; ldv: row
 // stride of X in lane vectors, cv: this lane's vector of a row.  The whole warp calls this together;
-// with on = false a lane gathers nothing.  Every lane returns the sum over the whole row.
+// with on = false a lane gathers nothing.  Every lane returns the sum over the whole row.  X is read by
+// ordinary loads: the kernel before a chained product may write it (chain.cuh).
 template <int U, int BQ, int VEC, typename VT, typename XT>
 __device__ __forceinline__ void row_product(int64_t beg, int64_t end, const int32_t* __restrict__ col,
-                                            const VT* __restrict__ val, const XT* __restrict__ X,
+                                            const VT* __restrict__ val, const XT* X,
                                             int64_t ldv, int cv, bool on, double (&a)[VEC]) {
   using XV = typename XVec<XT, VEC>::T;
   constexpr int SP = 32 / BQ;
   const int sub = (threadIdx.x & 31) / BQ;
-  const XV* __restrict__ Xv = reinterpret_cast<const XV*>(X) + cv;
+  const XV* Xv = reinterpret_cast<const XV*>(X) + cv;
 #pragma unroll
   for (int c = 0; c < VEC; ++c) a[c] = 0.0;
   if (on) {
-    auto gx = [&](int j) { return __ldg(Xv + (int64_t)j * ldv); };
+    auto gx = [&](int j) { return Xv[(int64_t)j * ldv]; };
     // single entries up to 4-entry alignment, whole turns of U, then the rest
     int64_t e0 = (beg + 3) & ~int64_t(3);
     if (e0 > end) e0 = end;
