@@ -1,0 +1,146 @@
+"""Device memory that runs out, at every reservation of a call in turn (injected on the host: the n-th
+reservation of the calling thread reports a lack of memory; nothing runs out on the device).  The call
+either ends with the out-of-memory status or gets by without that buffer, with the same result; a second
+call, with memory to be had again, succeeds; and a destroyed context leaves nothing behind in the pool,
+however its calls ended.
+
+Results are compared exactly where the failed reservation cannot change the arithmetic (the matrix), to
+the eigensolver's stopping rule for eigenvalues (|dE| <= 1e-10 |E| a run, twice that between two) and to
+the rounding of sums in another order for the rest."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from test_resources import _pool_used
+
+pytestmark = pytest.mark.gpu
+
+
+def fail_alloc(first, count=1):
+    """Reservations first .. first + count - 1 of this thread fail from here on; returns how many there
+    were since the last call."""
+    from vhci_b200 import api
+    f = api.lib().vhci_test_fail_alloc
+    f.restype = ctypes.c_int64
+    f.argtypes = [ctypes.c_int64, ctypes.c_int64]
+    return f(first, count)
+
+
+def _context(n, k, precision=0, nm=9, pt2_chunk=0):
+    from vhci_b200 import VHCI
+    rng = np.random.default_rng(n)
+    freq = [float(f) for f in np.sort(rng.uniform(500, 3300, nm))]
+    fcs = [((i, j, l), float(40 * rng.standard_normal())) for i in range(nm) for j in range(i, nm)
+           for l in range(j, nm)]
+    fcs += [((i, i, i, i), 60.0) for i in range(nm)]
+    q = np.unique(rng.binomial(6, 0.2, (12 * n, nm)).astype(np.uint8), axis=0)
+    q = q[np.argsort(q @ np.array(freq), kind="stable")][:n]
+    assert len(q) == n
+    v = VHCI(problem=dict(freq=freq, cap=[8] * nm, ntot=1, fcs=fcs, eps1=0.0, nstate=k, pt2=1),
+             precision=precision, pt2_chunk=pt2_chunk)
+    v.set_basis(q)
+    return v
+
+
+def _set_vectors(v, k):
+    rng = np.random.default_rng(5)
+    C, _ = np.linalg.qr(rng.standard_normal((v.n, k)))
+    E = np.linspace(1000.0, 2000.0, k)
+    v.set_vectors(C, E)
+
+
+def _matrix(v):
+    H = v.h_csr()
+    return [H.indptr, H.indices, H.data]
+
+
+def _exact(a, b):
+    return all(np.array_equal(x, y) for x, y in zip(a, b))
+
+
+def _values(a, b):
+    return (np.abs(a - b) <= 2e-10 * np.abs(b)).all()
+
+
+def _sums(a, b):  # sums of up to 1e5 products in another order, or one more rounding
+    return np.abs(a - b).max() <= 1e5 * 2.0 ** -53 * np.abs(b).max()
+
+
+def _build(v):
+    v.build_h()
+
+
+def _append(v):
+    _set_vectors(v, 2)
+    v.build_h()
+    v.select(0.5, append=True)
+    assert v.n > 6001
+
+
+def _x(v, k):
+    return np.random.default_rng(3).standard_normal((v.n, k))
+
+
+CASES = {
+    # states, wanted, options, preparation, the call, what it returns, comparison
+    "build": (17001, 2, {}, None, _build, _matrix, _exact),
+    "build_small": (3001, 2, {}, None, _build, _matrix, _exact),
+    "build_f32": (17001, 2, dict(precision=1), None, _build, _matrix, _exact),
+    "build_appended": (6001, 2, {}, _append, _build, _matrix, _exact),
+    "eigs": (3333, 4, {}, _build, lambda v: v.eigs(4), lambda v: v.energies(), _values),
+    "eigs_f32": (3333, 4, dict(precision=1), _build, lambda v: v.eigs(4), lambda v: v.energies(), None),
+    "eigs_dense": (701, 20, {}, _build, lambda v: v.eigs(20), lambda v: v.energies(), _values),
+    "pt2": (6001, 4, {}, lambda v: _set_vectors(v, 4), lambda v: v.pt2(0.05), lambda v: v.energies(), _sums),
+    "pt2_chunks": (6001, 4, dict(pt2_chunk=1), lambda v: _set_vectors(v, 4), lambda v: v.pt2(0.05),
+                   lambda v: v.energies(), _sums),
+    "select": (6001, 4, {}, lambda v: _set_vectors(v, 4), lambda v: v.select(0.05),
+               lambda v: v.select(0.05), None),
+    "apply": (6001, 2, {}, _build, lambda v: v.apply_h(_x(v, 3)), lambda v: v.apply_h(_x(v, 3)), _sums),
+    "residuals": (6001, 2, {}, _build, lambda v: v.residual_norms(_x(v, 3), np.ones(3)),
+                  lambda v: v.residual_norms(_x(v, 3), np.ones(3)), _sums),
+    "vectors": (6001, 3, {}, lambda v: _set_vectors(v, 3), lambda v: v.vectors(), lambda v: v.vectors()[0],
+                _sums),
+}
+
+
+@pytest.mark.parametrize("name", CASES)
+def test_every_reservation_may_fail(name):
+    from vhci_b200 import api
+    n, k, opts, prep, call, result, same = CASES[name]
+
+    def run(first):
+        """(status, result after a second call when the first ran out, reservations of the call)"""
+        with _context(n, k, **opts) as v:
+            if prep:
+                prep(v)
+            fail_alloc(first)
+            code = api.OK
+            try:
+                call(v)
+            except api.VhciError as e:
+                code = e.code
+            seen = fail_alloc(0, 0)
+            if code != api.OK:
+                if name.startswith("pt2"):  # energies that PT2 has not touched
+                    _set_vectors(v, 4)
+                call(v)
+            return code, result(v), seen
+
+    code, ref, total = run(0)
+    assert code == api.OK and total >= {"pt2": 15, "pt2_chunks": 15, "select": 5}.get(name, 1)
+    run(0)
+    base = _pool_used()
+    out = []
+    for first in range(1, total + 1):
+        code, got, seen = run(first)
+        assert code in (api.OK, api.E_OOM), (first, code)
+        out.append(code)
+        if same is not None:
+            assert same(got, ref), first
+        elif name == "eigs_f32":
+            assert np.abs(got - ref).max() <= 1e-7 * np.abs(ref).max(), first
+        else:
+            assert {x.tobytes() for x in got} == {x.tobytes() for x in ref}, first
+        assert _pool_used() == base, (first, code)
+    print(name, total, "reservations,", out.count(api.OK), "done without")

@@ -25,6 +25,22 @@ int blas_fail(vhci_ctx* c, int st, const char* where) {
   return fail(c, VHCI_E_CUDA, std::string(where) + ": library status " + std::to_string(st));
 }
 
+// Host-side fault injection for the tests: of this thread's reservations from the call of
+// vhci_test_fail_alloc on, numbers first .. first + count - 1 report a lack of memory.
+namespace {
+struct AllocFault {
+  int64_t seen = 0, first = 0, count = 0;
+};
+thread_local AllocFault t_alloc;
+}  // namespace
+
+cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s) {
+  ++t_alloc.seen;
+  if (t_alloc.seen >= t_alloc.first && t_alloc.seen < t_alloc.first + t_alloc.count)
+    return cudaErrorMemoryAllocation;
+  return cudaMallocAsync(p, bytes, s);
+}
+
 HashView basis_view(vhci_ctx* c) { return HashView{c->hslots.p, c->hmask, c->keys.p}; }
 
 static void set_groups(ConnDev& d, const DevGroups& g) {
@@ -288,13 +304,13 @@ int promote_layout(vhci_ctx* c) {
   VCK(nk.reserve(std::max<int64_t>(c->keys.cap / A.W * B.W, (int64_t)c->n * B.W + 16), c->st));
   repack_keys(c->keys.p, A, nk.p, B, c->n, c->M.nm, c->st);
   c->keys.release(c->st);
-  c->keys = nk;
+  c->keys = std::move(nk);
   if (c->nsel > 0 && c->sel.p) {
     DBuf<uint64_t> ns;
     VCK(ns.reserve((size_t)c->nsel * B.W, c->st));
     repack_keys(c->sel.p, A, ns.p, B, c->nsel, c->M.nm, c->st);
     c->sel.release(c->st);
-    c->sel = ns;
+    c->sel = std::move(ns);
   }
   c->L = B;
   VTRY(upload_tables(c));
@@ -729,11 +745,10 @@ static int build_h_incremental(vhci_ctx* c) {
   VCK(cudaMemcpyAsync(diag_all.p + n_old, tdiag.p, nn * sizeof(double), cudaMemcpyDeviceToDevice, s));
   #undef VHCI_INC
   // the merged matrix replaces the stored one (the old arrays leave with the temporaries)
-  std::swap(c->rowptr.p, rp_all.p); std::swap(c->rowptr.cap, rp_all.cap);
-  std::swap(c->col.p, col_all.p); std::swap(c->col.cap, col_all.cap);
-  if (f) { std::swap(c->valf.p, valf_all.p); std::swap(c->valf.cap, valf_all.cap); }
-  else { std::swap(c->val.p, val_all.p); std::swap(c->val.cap, val_all.cap); }
-  std::swap(c->diag.p, diag_all.p); std::swap(c->diag.cap, diag_all.cap);
+  c->rowptr.swap(rp_all);
+  c->col.swap(col_all);
+  if (f) c->valf.swap(valf_all); else c->val.swap(val_all);
+  c->diag.swap(diag_all);
   release_all();
   c->nnz = nnz_all;
   c->row0 = 0;
@@ -946,6 +961,14 @@ vhci_status vhci_destroy(vhci_ctx* c) {
   release_handles(c);
   delete c;
   return VHCI_OK;
+}
+
+// For the tests, not part of the interface: see AllocFault.  Returns the reservations of this thread
+// since the call before.
+int64_t vhci_test_fail_alloc(int64_t first, int64_t count) {
+  const int64_t seen = t_alloc.seen;
+  t_alloc = AllocFault{0, first, count};
+  return seen;
 }
 
 vhci_status vhci_last_error(const vhci_ctx* c, char* buf, size_t n) {

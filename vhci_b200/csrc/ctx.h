@@ -6,6 +6,7 @@
 #include <cusolverDn.h>
 
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "model.h"
@@ -14,22 +15,36 @@
 
 namespace vhci {
 
-// Stream-ordered device buffer that grows on demand.
+// Device memory of the stream-ordered pool (cudaMallocAsync).
+cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s);
+
+// Stream-ordered device buffer that grows on demand; freed, in stream order, with its scope.
 template <class T>
 struct DBuf {
   T* p = nullptr;
   size_t cap = 0;  // elements
+  cudaStream_t st = nullptr;  // of the last reservation
+  DBuf() = default;
+  DBuf(DBuf&& o) noexcept { swap(o); }
+  DBuf& operator=(DBuf&& o) noexcept {
+    swap(o);
+    return *this;
+  }
+  ~DBuf() {
+    if (p) cudaFreeAsync(p, st);
+  }
   cudaError_t reserve(size_t n, cudaStream_t s, bool keep = false) {
     if (n <= cap && p) return cudaSuccess;
     size_t nc = n < 16 ? 16 : n;
     if (keep) nc = nc + nc / 2;
     T* q = nullptr;
-    cudaError_t e = cudaMallocAsync((void**)&q, nc * sizeof(T), s);
+    cudaError_t e = pool_alloc((void**)&q, nc * sizeof(T), s);
     if (e != cudaSuccess) return e;
     if (keep && p && cap) cudaMemcpyAsync(q, p, cap * sizeof(T), cudaMemcpyDeviceToDevice, s);
     if (p) cudaFreeAsync(p, s);
     p = q;
     cap = nc;
+    st = s;
     return cudaSuccess;
   }
   void release(cudaStream_t s) {
@@ -40,6 +55,7 @@ struct DBuf {
   void swap(DBuf& o) {
     std::swap(p, o.p);
     std::swap(cap, o.cap);
+    std::swap(st, o.st);
   }
 };
 
