@@ -144,3 +144,44 @@ def test_every_reservation_may_fail(name):
             assert {x.tobytes() for x in got} == {x.tobytes() for x in ref}, first
         assert _pool_used() == base, (first, code)
     print(name, total, "reservations,", out.count(api.OK), "done without")
+
+
+# What a build cannot do without: the row counts and pointers, the scan's scratch.  Everything else is
+# there to make it faster, or can be had once that is given back.
+@pytest.mark.parametrize("name", ["build", "build_small", "build_f32"])
+def test_build_gives_way(name):
+    from vhci_b200 import api
+    n, k, opts, _, call, result, same = CASES[name]
+    with _context(n, k, **opts) as v:
+        fail_alloc(0, 0)
+        call(v)
+        total, ref = fail_alloc(0, 0), result(v)
+    out = []
+    for first in range(1, total + 1):
+        with _context(n, k, **opts) as v:
+            fail_alloc(first)
+            try:
+                call(v)
+            except api.VhciError as e:
+                assert e.code == api.E_OOM
+                out.append(first)
+            fail_alloc(0, 0)
+            if first not in out:
+                assert same(result(v), ref), first
+    assert len(out) <= 3, (out, total)
+
+
+def test_matrix_that_cannot_be_had_is_refused_with_its_size():
+    """All reservations from the matrix's first on fail: the refusal states what was needed."""
+    from vhci_b200 import api
+    n, k, opts, _, call, _, _ = CASES["build_small"]
+    said = []
+    for first in range(1, 10):
+        with _context(n, k, **opts) as v:
+            fail_alloc(first, 100)
+            with pytest.raises(api.VhciError) as e:
+                call(v)
+            fail_alloc(0, 0)
+            assert e.value.code == api.E_OOM
+            said.append("GB for the eigensolver" in str(e.value))
+    assert any(said)

@@ -409,7 +409,8 @@ double device_available(vhci_ctx* c) {
 
 // Whether `need` bytes can be allocated.  The driver's free-memory query usually takes 65 us and at
 // times several ms, so it is asked last: not when the pool's idle reserve covers the need, and not
-// for less than 1/64 of the device, where the callers leave a shortage to the allocation itself.
+// for less than 1/64 of the device.  A yes is therefore no promise: the callers take the same way out
+// when the allocation itself fails as for a no.
 bool device_fits(vhci_ctx* c, double need) {
   if (need <= c->dev_bytes / 64) return true;
   cudaMemPool_t pool;
@@ -561,19 +562,24 @@ bool dense_path(int64_t n, int k) {
 // A sample of about 1,024 rows spread over all of them counts the connections (its mean is within 2 %
 // where the rows' counts spread by 60 %); 25 % and two batches per row of slack cover its spread and
 // the part-filled last batches.  Small row sets skip the sample for 8 batches (256 connections) a
-// row.  The room is limited to a quarter of the device, and a failed allocation is no error.
+// row.  The room is limited to a quarter of the device, and a failed allocation is no error: nothing is
+// kept then.
 int stage_reserve(vhci_ctx* c, Stage& st, HashView table, int64_t row0, int64_t n) {
   cudaStream_t s = c->st;
   st.view = StageView{};
   if (n <= 0 || n >= 0xFFFFFFFFll) return VHCI_OK;
   double batches = 8.0 * (double)n;
-  VCK(st.cursor.reserve(1, s));
+  auto have = [](cudaError_t e) {
+    if (e != cudaSuccess) cudaGetLastError();
+    return e == cudaSuccess;
+  };
+  if (!have(st.cursor.reserve(1, s))) return VHCI_OK;
   if (n > 4096) {
     const int64_t stride = n / 1024, ns = n / stride;
-    VCK(c->rowcnt.reserve(n, s));
-    VCK(c->scan_tmp.reserve(std::max<int64_t>(scan_tmp_elems(n), 1), s));
     DBuf<int64_t> sum;
-    VCK(sum.reserve(ns + 1, s));
+    if (!have(c->rowcnt.reserve(n, s)) ||
+        !have(c->scan_tmp.reserve(std::max<int64_t>(scan_tmp_elems(n), 1), s)) || !have(sum.reserve(ns + 1, s)))
+      return VHCI_OK;
     hbuild_count(c->keys.p, row0, stride, ns, c->L, table, conn_view(c), c->rowcnt.p, StageView{}, s);
     exclusive_scan_i32(c->rowcnt.p, sum.p, ns, c->scan_tmp.p, s);
     int64_t found = 0;
@@ -584,10 +590,8 @@ int stage_reserve(vhci_ctx* c, Stage& st, HashView table, int64_t row0, int64_t 
   }
   if (batches * 264.0 > 0.25 * (double)c->dev_bytes) return VHCI_OK;
   const int64_t cap = (int64_t)batches;
-  if (st.batch.reserve(cap, s) != cudaSuccess || st.pair.reserve(32 * (size_t)cap, s) != cudaSuccess) {
-    cudaGetLastError();
-    st.batch.release(s);
-    st.pair.release(s);
+  if (!have(st.batch.reserve(cap, s)) || !have(st.pair.reserve(32 * (size_t)cap, s))) {
+    st.release(s);
     return VHCI_OK;
   }
   VCK(cudaMemsetAsync(st.cursor.p, 0, sizeof(unsigned long long), s));
@@ -601,14 +605,13 @@ static int count_rows(vhci_ctx* c, Stage& st, int64_t row0, int64_t n, int32_t* 
                       int64_t* nnz, int64_t* nbatch) {
   cudaStream_t s = c->st;
   VTRY(stage_reserve(c, st, basis_view(c), row0, n));
-  if (hcount_filter_pays(n, c->n)) {
-    DBuf<uint32_t> bits;
-    VCK(bits.reserve(kBitsWords, s));
-    VCK(c->ull.reserve(2, s));
+  DBuf<uint32_t> bits;
+  if (hcount_filter_pays(n, c->n) && bits.reserve(kBitsWords, s) == cudaSuccess &&
+      c->ull.reserve(2, s) == cudaSuccess) {
     hcount_filtered(c->keys.p, row0, n, c->L, basis_view(c), c->n, conn_view(c), bits.p, cnt, st.view,
                     c->ull.p, s);
-    bits.release(s);
   } else {
+    cudaGetLastError();  // no memory for the bits: the count without them
     hbuild_count(c->keys.p, row0, 1, n, c->L, basis_view(c), conn_view(c), cnt, st.view, s);
   }
   exclusive_scan_i32(cnt, rowptr, n, c->scan_tmp.p, s);
@@ -802,33 +805,35 @@ int build_h(vhci_ctx* c, bool all_rows) {
   if ((int64_t)c->col.cap < nnz) c->col.release(c->st);
   if ((int64_t)c->val.cap < nnz) c->val.release(c->st);
   if ((int64_t)c->valf.cap < nnz) c->valf.release(c->st);
-  {  // admission: the matrix and the eigensolver's smallest working set must fit together
-    const double hbytes = (double)nnz * (4.0 + (c->o.precision == 1 ? 4.0 : 8.0)) + 8.0 * nr;
-    const double xb = 8.0 * (double)c->x_rows * c->ldx, eig = lanczos_min_bytes(c, c->M.nstate);
-    bool fits = device_fits(c, hbytes + eig - xb);
-    if (!fits && nbatch > 0) {  // the kept connections give way
-      stage.release(c->st);
-      nbatch = 0;
-      fits = device_fits(c, hbytes + eig - xb);
-    }
-    if (!fits) {
-      stage.release(c->st);
-      const double avail = device_available(c) + xb;
-      char msg[320];
-      std::snprintf(msg, sizeof msg,
-                    "Hamiltonian rows of %lld states and %lld off-diagonal entries need %.1f GB "
-                    "(plus %.1f GB for the eigensolver); %.1f GB of device memory is available",
-                    (long long)nr, (long long)nnz, hbytes / 1e9, eig / 1e9, avail / 1e9);
-      return fail(c, VHCI_E_OOM, msg);
-    }
+  // admission: the matrix and the eigensolver's smallest working set must fit together, and the matrix
+  // must be had; the kept connections give way to either
+  const double hbytes = (double)nnz * (4.0 + (c->o.precision == 1 ? 4.0 : 8.0)) + 8.0 * nr;
+  const double xb = 8.0 * (double)c->x_rows * c->ldx, eig = lanczos_min_bytes(c, c->M.nstate);
+  auto matrix = [&]() -> cudaError_t {
+    if (!device_fits(c, hbytes + eig - xb)) return cudaErrorMemoryAllocation;
+    const size_t ne = (size_t)std::max<int64_t>(nnz, 1);
+    cudaError_t e = c->col.reserve(ne, c->st);
+    if (!e) e = c->o.precision == 1 ? c->valf.reserve(ne, c->st) : c->val.reserve(ne, c->st);
+    return e ? e : c->diag.reserve(std::max<int64_t>(nr, 1), c->st);
+  };
+  cudaError_t e = matrix();
+  if (e == cudaErrorMemoryAllocation && stage.view.cap > 0) {
+    cudaGetLastError();
+    stage.release(c->st);
+    nbatch = 0;
+    e = matrix();
   }
-  VCK(c->col.reserve(std::max<int64_t>(nnz, 1), c->st));
-  if (c->o.precision == 1) {
-    VCK(c->valf.reserve(std::max<int64_t>(nnz, 1), c->st));
-  } else {
-    VCK(c->val.reserve(std::max<int64_t>(nnz, 1), c->st));
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    const double avail = device_available(c) + xb;
+    char msg[320];
+    std::snprintf(msg, sizeof msg,
+                  "Hamiltonian rows of %lld states and %lld off-diagonal entries need %.1f GB "
+                  "(plus %.1f GB for the eigensolver); %.1f GB of device memory is available",
+                  (long long)nr, (long long)nnz, hbytes / 1e9, eig / 1e9, avail / 1e9);
+    return fail(c, VHCI_E_OOM, msg);
   }
-  VCK(c->diag.reserve(std::max<int64_t>(nr, 1), c->st));
+  VCK(e);
   fill_rows(c, stage, nbatch, r0, nr, c->rowptr.p, c->col.p, c->o.precision == 1 ? nullptr : c->val.p,
             c->o.precision == 1 ? c->valf.p : nullptr, c->diag.p);
   c->nnz = nnz;
