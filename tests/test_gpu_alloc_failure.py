@@ -185,3 +185,39 @@ def test_matrix_that_cannot_be_had_is_refused_with_its_size():
             assert e.value.code == api.E_OOM
             said.append("GB for the eigensolver" in str(e.value))
     assert any(said)
+
+
+def _pt2_context(chunk):
+    v = _context(6001, 4, pt2_chunk=chunk)
+    _set_vectors(v, 4)
+    return v
+
+
+@pytest.mark.parametrize("chunk", [0, 1])
+def test_pt2_gives_way(chunk):
+    """PT2 with a reservation that fails, and from the first chunk's buffers on with several in a row: the
+    kept connections go, then the perturbers are taken in smaller chunks.  Only what comes before the
+    first chunk (the selection, the perturbers' table, the entry counts and the columns' sums) cannot be
+    done without."""
+    from vhci_b200 import api
+
+    def run(first, count):
+        with _pt2_context(chunk) as v:
+            fail_alloc(first, count)
+            try:
+                v.pt2(0.05)
+            except api.VhciError as e:
+                assert e.code == api.E_OOM
+                return None, fail_alloc(0, 0)
+            return v.energies(), fail_alloc(0, 0)
+
+    ref, total = run(0, 0)
+    with _pt2_context(chunk) as v:
+        v.pt2(0.05)
+        assert v.stats()["pt2_entries"] > 1 << 20  # more than the smallest chunk
+    needed = [first for first in range(1, total + 1) if run(first, 1)[0] is None]
+    assert total - needed[-1] >= 6, (needed, total)  # the chunk's buffers
+    for count in (1, 2, 5):
+        for first in range(needed[-1] + 1, total + 1):
+            got, _ = run(first, count)
+            assert got is not None and _sums(got, ref), (first, count)

@@ -85,47 +85,39 @@ int pt2(vhci_ctx* c, double eps2, double* dE_out, int64_t* n_pert) {
     auto chunk_entries = [&](int64_t a0, int64_t a1) {
       return arow_h.empty() ? total : arow_h[a1 - A0] - arow_h[a0 - A0];
     };
-    bool whole = c->o.pt2_chunk <= 0 && device_fits(c, (double)total * 40.0);
-    for (;;) {
-      bounds.assign(1, A0);
-      if (!whole) {
-        auto chunk_budget = [&] {
-          const int64_t e = c->o.pt2_chunk > 0 ? c->o.pt2_chunk : (int64_t)(device_available(c) * 0.4 / 16.0);
-          return std::max<int64_t>(e, 1 << 20);
-        };
-        int64_t budget = chunk_budget();
-        if (nbatch > 0 && total > budget && c->o.pt2_chunk <= 0) {  // the kept connections give way
-          stage.release(s);
-          nbatch = 0;
-          budget = chunk_budget();
-        }
-        if (total > budget) {
-          arow_h.resize(NA + 1);
-          VCK(d2h(c, arow_h.data(), arow.p, (NA + 1) * sizeof(int64_t)));
-          VCK(cudaStreamSynchronize(s));
-          while (bounds.back() < A1) {
-            const int64_t a0 = bounds.back();
-            const int64_t lim = arow_h[a0 - A0] + budget;
-            int64_t a1 = A0 + (std::upper_bound(arow_h.begin() + (a0 - A0) + 1, arow_h.end(), lim) -
-                               arow_h.begin()) - 1;
-            if (a1 <= a0) a1 = a0 + 1;
-            bounds.push_back(std::min(a1, A1));
-          }
+    auto host_offsets = [&]() -> int {
+      if (!arow_h.empty()) return VHCI_OK;
+      std::vector<int64_t> h(NA + 1);
+      VCK(d2h(c, h.data(), arow.p, (NA + 1) * sizeof(int64_t)));
+      VCK(cudaStreamSynchronize(s));
+      arow_h.swap(h);
+      return VHCI_OK;
+    };
+    bounds.assign(1, A0);
+    if (c->o.pt2_chunk > 0 || !device_fits(c, (double)total * 40.0)) {
+      auto chunk_budget = [&] {
+        const int64_t e = c->o.pt2_chunk > 0 ? c->o.pt2_chunk : (int64_t)(device_available(c) * 0.4 / 16.0);
+        return std::max<int64_t>(e, 1 << 20);
+      };
+      int64_t budget = chunk_budget();
+      if (nbatch > 0 && total > budget && c->o.pt2_chunk <= 0) {  // the kept connections give way
+        stage.release(s);
+        nbatch = 0;
+        budget = chunk_budget();
+      }
+      if (total > budget) {
+        VTRY(host_offsets());
+        while (bounds.back() < A1) {
+          const int64_t a0 = bounds.back();
+          const int64_t lim = arow_h[a0 - A0] + budget;
+          int64_t a1 = A0 + (std::upper_bound(arow_h.begin() + (a0 - A0) + 1, arow_h.end(), lim) -
+                             arow_h.begin()) - 1;
+          if (a1 <= a0) a1 = a0 + 1;
+          bounds.push_back(std::min(a1, A1));
         }
       }
-      if (arow_h.empty()) bounds.push_back(A1);
-      int64_t maxchunk = 1;
-      for (size_t q = 1; q < bounds.size(); ++q)
-        maxchunk = std::max(maxchunk, chunk_entries(bounds[q - 1], bounds[q]));
-      const cudaError_t e = ent.reserve(maxchunk, s);
-      if (e == cudaErrorMemoryAllocation && whole) {  // not to be had in one: by the budget
-        cudaGetLastError();
-        whole = false;
-        continue;
-      }
-      VCK(e);
-      break;
     }
+    if (arow_h.empty()) bounds.push_back(A1);
     const int nblk = pt2_en_blocks();
     VCK(part.reserve((size_t)nblk * nopt, s));
     VCK(cudaMemsetAsync(part.p, 0, (size_t)nblk * nopt * sizeof(double), s));
@@ -136,22 +128,52 @@ int pt2(vhci_ctx* c, double eps2, double* dE_out, int64_t* n_pert) {
     DBuf<int64_t> crow, lrow_d, loff_d;
     DBuf<unsigned long long> lcnt, apos;
     VCK(lcnt.reserve(2, s));
-    for (size_t q = 1; q < bounds.size(); ++q) {
-      const int64_t a0 = bounds[q - 1], a1 = bounds[q], na = a1 - a0;
-      // this chunk's row offsets, rebased on the device
-      VCK(crow.reserve(na + 1, s));
-      VCK(apos.reserve(na + 1, s));
+    unsigned long long lc[2] = {0, 0};  // a chunk's long rows and their entries
+    // A chunk's buffers, its row offsets rebased, and the list of its rows too long for one warp's
+    // ordering (only their count and entries come back, to size the scratch and the launch); most: the
+    // entries of the largest chunk still to come.
+    auto start_chunk = [&](int64_t a0, int64_t a1, int64_t most) -> cudaError_t {
+      const int64_t na = a1 - a0;
+      const int64_t maxlong = std::max<int64_t>(1, std::min(na, chunk_entries(a0, a1) / pt2_sort_long_min() + 1));
+      cudaError_t e = ent.reserve(most, s);
+      if (!e) e = crow.reserve(na + 1, s);
+      if (!e) e = apos.reserve(na + 1, s);
+      if (!e) e = ediag.reserve(std::max<int64_t>(na, 1), s);
+      if (!e) e = lrow_d.reserve(maxlong, s);
+      if (!e) e = loff_d.reserve(maxlong, s);
+      if (!e) e = cudaMemsetAsync(lcnt.p, 0, 2 * sizeof(unsigned long long), s);
+      if (e) return e;
       pt2_rebase_rows(arow.p + (a0 - A0), na, crow.p, apos.p, s);
-      // rows too long for one warp's ordering, listed on the device; only their count and
-      // entries come back, to size the scratch and the launch
-      const int64_t maxlong = std::min<int64_t>(na, chunk_entries(a0, a1) / pt2_sort_long_min() + 1);
-      VCK(lrow_d.reserve(std::max<int64_t>(maxlong, 1), s));
-      VCK(loff_d.reserve(std::max<int64_t>(maxlong, 1), s));
-      VCK(cudaMemsetAsync(lcnt.p, 0, 2 * sizeof(unsigned long long), s));
       pt2_list_long(crow.p, na, lrow_d.p, loff_d.p, lcnt.p, s);
-      unsigned long long lc[2] = {0, 0};
-      VCK(d2h(c, lc, lcnt.p, sizeof(lc)));
-      VCK(cudaStreamSynchronize(s));
+      e = d2h(c, lc, lcnt.p, sizeof(lc));
+      if (!e) e = cudaStreamSynchronize(s);
+      return e || lc[0] == 0 ? e : ltmp.reserve((int64_t)lc[1], s);
+    };
+    for (size_t q = 1; q < bounds.size(); ++q) {
+      const int64_t a0 = bounds[q - 1];
+      for (;;) {
+        int64_t most = 1;
+        for (size_t r = q; r < bounds.size(); ++r) most = std::max(most, chunk_entries(bounds[r - 1], bounds[r]));
+        const cudaError_t e = start_chunk(a0, bounds[q], most);
+        const bool smaller = stage.view.cap > 0 || bounds[q] - a0 > 1;
+        if (e != cudaErrorMemoryAllocation || !smaller) {
+          VCK(e);
+          break;
+        }
+        cudaGetLastError();  // not to be had: without the kept connections, then with half the entries
+        if (stage.view.cap > 0) {
+          stage.release(s);
+          nbatch = 0;
+          continue;
+        }
+        ent.release(s); crow.release(s); apos.release(s); ediag.release(s);
+        lrow_d.release(s); loff_d.release(s); ltmp.release(s);
+        VTRY(host_offsets());
+        const int64_t half = (arow_h[a0 - A0] + arow_h[bounds[q] - A0]) / 2;
+        const int64_t mid = A0 + (std::lower_bound(arow_h.begin(), arow_h.end(), half) - arow_h.begin());
+        bounds.insert(bounds.begin() + q, std::min(std::max(mid, a0 + 1), bounds[q] - 1));
+      }
+      const int64_t a1 = bounds[q], na = a1 - a0;
       if (nbatch > 0)
         pt2_fill_staged(c->keys.p, L, conn_view(c), stage.view, (int64_t)nbatch, a0, a1, apos.p, ent.p, s);
       else
@@ -161,12 +183,10 @@ int pt2(vhci_ctx* c, double eps2, double* dE_out, int64_t* n_pert) {
       // each, long rows by one block each
       pt2_sort_rows(crow.p, na, ent.p, s);
       if (lc[0] > 0) {
-        VCK(ltmp.reserve((int64_t)lc[1], s));
         for (int64_t q0 = 0; q0 < (int64_t)lc[0]; q0 += 65535)
           pt2_sort_long(crow.p, lrow_d.p + q0, loff_d.p + q0,
                         (int)std::min<int64_t>(65535, (int64_t)lc[0] - q0), ent.p, ltmp.p, s);
       }
-      VCK(ediag.reserve(std::max<int64_t>(na, 1), s));
       diag_energies(pkeys.p, a0, na, L, conn_view(c), ediag.p, s);
       EventPair ev_r0r1;
       VCK(ev_r0r1.create());
