@@ -221,3 +221,35 @@ def test_pt2_gives_way(chunk):
         for first in range(needed[-1] + 1, total + 1):
             got, _ = run(first, count)
             assert got is not None and _sums(got, ref), (first, count)
+
+
+@pytest.mark.parametrize("name,needed", [("eigs", 0), ("eigs_f32", 0), ("eigs_dense", 3)])
+def test_eigensolver_gives_way(name, needed):
+    """Any one buffer of the block Lanczos: the memory-lean variant has the eigenvalues.  The dense solver
+    cannot do without the matrix, the values and the vectors it returns, and leaves the rest to the
+    library's, which works in place."""
+    from vhci_b200 import api
+    n, k, opts, prep, call, result, same = CASES[name]
+
+    def run(first):
+        with _context(n, k, **opts) as v:
+            prep(v)
+            fail_alloc(first)
+            try:
+                call(v)
+            except api.VhciError as e:
+                assert e.code == api.E_OOM
+                return None, fail_alloc(0, 0)
+            seen = fail_alloc(0, 0)
+            return result(v), seen
+
+    ref, total = run(0)
+    out = []
+    for first in range(1, total + 1):
+        got, _ = run(first)
+        if got is None:
+            out.append(first)
+        else:
+            tol = 1e-7 * np.abs(ref).max() if same is None else 2e-10 * np.abs(ref)
+            assert (np.abs(got - ref) <= tol).all(), first
+    assert len(out) <= needed, (out, total)

@@ -49,7 +49,12 @@ int small_eigs_start(vhci_ctx* c, const double* T, int m, int ld, int nk, double
                      double* words, bool* started) {
   *started = false;
   if (m > kSmallEigMax) return VHCI_OK;
-  VCK(c->eig_work.reserve(small_eig_elems(m, nk), c->st));
+  const cudaError_t e = c->eig_work.reserve(small_eig_elems(m, nk), c->st);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    return VHCI_OK;
+  }
+  VCK(e);
   *started = small_eig(T, ld, m, nk, theta, Y, ld, c->eig_work.p,
                        reinterpret_cast<unsigned long long*>(words), c->st);
   return VHCI_OK;
@@ -62,7 +67,13 @@ bool small_eigs_verdict(const double* words) {
 }
 
 int small_eigs(vhci_ctx* c, const double* T, int m, int ld, int nk, double* theta, double* Y, bool* done) {
-  VCK(c->eig_dev.reserve(kSmallEigDev, c->st));
+  *done = false;
+  const cudaError_t e = c->eig_dev.reserve(kSmallEigDev, c->st);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    return VHCI_OK;
+  }
+  VCK(e);
   VTRY(small_eigs_start(c, T, m, ld, nk, theta, Y, c->eig_dev.p, done));
   if (!*done) return VHCI_OK;
   double w[kSmallEigDev];
@@ -106,8 +117,10 @@ int dense_eigs(vhci_ctx* c, int keep) {
   DBuf<double> Y;  // the vectors, column-major
   bool done = false;
   if (n <= kSmallEigMax) {
-    VCK(Y.reserve((size_t)n * keep, c->st));
-    VTRY(small_eigs(c, A.p, (int)n, (int)n, keep, w.p, Y.p, &done));
+    const cudaError_t e = Y.reserve((size_t)n * keep, c->st);
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();  // syevd works in place
+    else VCK(e);
+    if (!e) VTRY(small_eigs(c, A.p, (int)n, (int)n, keep, w.p, Y.p, &done));
   }
   if (!done) VTRY(syevd(c, A.p, (int)n, (int)n, w.p));
   VCK(c->X.reserve((size_t)n * keep, c->st));

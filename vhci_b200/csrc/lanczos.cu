@@ -482,6 +482,8 @@ int block_lanczos_impl(vhci_ctx* c, int k, bool dev_svqb) {
   const int plevel = prof ? std::atoi(prof) : 0;
   LWork w;
   const int nblk = residual_blocks(nl);
+  // all of them before the first product, so that a lack of memory shows while the lean variant can
+  // still be taken
   auto reserve_all = [&]() -> cudaError_t {
     cudaError_t e = w.Q.reserve((size_t)nl * ld, s);
     if (!e && mixed) e = w.HQ.reserve((size_t)nl * ld, s);  // H Q, rotated for the explicit residuals
@@ -494,6 +496,18 @@ int block_lanczos_impl(vhci_ctx* c, int k, bool dev_svqb) {
     if (!e) e = w.W.reserve((size_t)nl * b, s);
     if (!e) e = w.part.reserve((size_t)nblk * kk, s);
     if (!e) e = w.rn2.reserve(kk, s);
+    const int bw = std::max(b, 16);  // the final FP64 sweep takes 16 columns at a time
+    if (!e) e = w.Xc.reserve((size_t)rb * bw, s);
+    if (!e && mixed) e = w.Xf.reserve((size_t)rb * b, s);
+    if (!e) e = w.S.reserve((size_t)std::max(mmax, bw) * bw, s);
+    if (!e) e = w.M.reserve((size_t)b * b, s);
+    if (!e) e = w.G.reserve((size_t)b * b, s);
+    if (!e) e = w.gpart.reserve((size_t)proj_gram_scratch(mmax, bw), s);
+    if (!e && is_sharded(c)) {
+      e = w.Xg.reserve((size_t)c->comm.nranks * rb * bw, s);
+      if (!e && mixed) e = w.Xgf.reserve((size_t)c->comm.nranks * rb * b, s);
+      if (!e) e = w.gtmp.reserve((size_t)mmax * bw, s);
+    }
     return e;
   };
   if (const cudaError_t e = reserve_all()) {
