@@ -442,6 +442,19 @@ double lanczos_min_bytes(vhci_ctx* c, int k) {
 
 int block_lanczos_lean(vhci_ctx* c, int k);
 
+// *yes = whether any rank of a sharded solve says so (they share the answer; alone: unchanged).
+static int any_rank(vhci_ctx* c, bool* yes) {
+  if (!is_sharded(c)) return VHCI_OK;
+  VCK(c->eig_dev.reserve(kSmallEigDev, c->st));
+  double v = *yes ? 1.0 : 0.0;
+  VCK(h2d(c, c->eig_dev.p, &v, sizeof(v)));
+  VTRY(comm_sum(c, c->eig_dev.p, 1));
+  VCK(d2h(c, &v, c->eig_dev.p, sizeof(v)));
+  VCK(cudaStreamSynchronize(c->st));
+  *yes = v > 0.0;
+  return VHCI_OK;
+}
+
 // Relative residual tolerance of the FP32-gather eigensolve in mixed precision.
 constexpr double kMixedTol = 1e-7;
 
@@ -467,8 +480,6 @@ int block_lanczos_impl(vhci_ctx* c, int k, bool dev_svqb) {
   if (const char* e = std::getenv("VHCI_LANCZOS_LEAN"))
     if (std::atoi(e) == 1) return block_lanczos_lean(c, k);
   if (const char* e = std::getenv("VHCI_LANCZOS_SPAN")) span = std::max(2, std::min(8, std::atoi(e)));
-  if (!device_fits(c, lanczos_bytes(n, nl, k, span, b, c->o.precision == 1) + 1e9))
-    return block_lanczos_lean(c, k);
   const int mmax = (int)std::min<int64_t>(n, (int64_t)span * kk + 2 * b);
   const bool dev = dev_svqb && n >= 8 * (int64_t)mmax;
   // row stride padded to whole 128-byte lines so every b-column gather touches whole L2 lines
@@ -510,10 +521,17 @@ int block_lanczos_impl(vhci_ctx* c, int k, bool dev_svqb) {
     }
     return e;
   };
-  if (const cudaError_t e = reserve_all()) {
+  // one variant for every rank: the two issue different collectives
+  bool lean = !device_fits(c, lanczos_bytes(n, nl, k, span, b, mixed) + 1e9);
+  if (!lean) {
+    const cudaError_t e = reserve_all();
+    if (e != cudaSuccess && e != cudaErrorMemoryAllocation) return cuda_fail(c, e, "eigensolver buffers");
+    if (e) cudaGetLastError();  // too little memory after all
+    lean = e != cudaSuccess;
+  }
+  VTRY(any_rank(c, &lean));
+  if (lean) {
     w.release(s);
-    if (e != cudaErrorMemoryAllocation) return cuda_fail(c, e, "eigensolver buffers");
-    cudaGetLastError();  // too little memory after all
     return block_lanczos_lean(c, k);
   }
   const int nout = ld + kk + kSmallEigDev + 1;
