@@ -253,3 +253,37 @@ def test_eigensolver_gives_way(name, needed):
             tol = 1e-7 * np.abs(ref).max() if same is None else 2e-10 * np.abs(ref)
             assert (np.abs(got - ref) <= tol).all(), first
     assert len(out) <= needed, (out, total)
+
+
+@pytest.mark.parametrize("name,needed", [("apply", 2), ("residuals", 4), ("vectors", 0), ("set_vectors", 1)])
+def test_transfers_give_way(name, needed):
+    """Vectors between host and device need the device's copy of them (and residuals their sums), no more."""
+    from vhci_b200 import api
+    n, k, opts, prep, call, result, same = CASES["vectors" if name == "set_vectors" else name]
+    if name == "set_vectors":
+        prep, call = None, lambda v: _set_vectors(v, 3)
+
+    def run(first):
+        with _context(n, k, **opts) as v:
+            if prep:
+                prep(v)
+            fail_alloc(first)
+            try:
+                got = call(v)
+            except api.VhciError as e:
+                assert e.code == api.E_OOM
+                return None, fail_alloc(0, 0)
+            seen = fail_alloc(0, 0)
+            return result(v) if name == "set_vectors" else (got[0] if name == "vectors" else got), seen
+
+    ref, total = run(0)
+    out = []
+    for first in range(1, total + 1):
+        got, _ = run(first)
+        if got is None:
+            out.append(first)
+        elif "vectors" in name:
+            assert np.array_equal(got, ref), first  # copies
+        else:
+            assert _sums(got, ref), first
+    assert len(out) <= needed and total > needed, (out, total)

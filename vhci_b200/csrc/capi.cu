@@ -1023,10 +1023,30 @@ static int transfer_cols(int64_t n, int k) {
   return (int)std::min<int64_t>(k, w);
 }
 
+// The transfers' buffer; false when there is no memory for it, and the host transposes.
+static int transfer_buffer(vhci_ctx* c, DBuf<double>& t, size_t elems, bool* have) {
+  const cudaError_t e = t.reserve(elems, c->st);
+  *have = e == cudaSuccess;
+  if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+  else VCK(e);
+  return VHCI_OK;
+}
+
 int upload_cols(vhci_ctx* c, const double* host, int64_t n, int k, double* dev, int ldd) {
   const int w = transfer_cols(n, k);
   DBuf<double> t;
-  VCK(t.reserve((size_t)n * w, c->st));
+  bool have = false;
+  VTRY(transfer_buffer(c, t, (size_t)n * w, &have));
+  if (!have) {
+    std::vector<double> h((size_t)n * k);
+    for (int64_t i = 0; i < n; ++i)
+      for (int j = 0; j < k; ++j) h[(size_t)i * k + j] = host[(size_t)j * n + i];
+    c->stats.h2d_bytes += (int64_t)(h.size() * sizeof(double));
+    VCK(cudaMemcpy2DAsync(dev, ldd * sizeof(double), h.data(), k * sizeof(double), k * sizeof(double), n,
+                          cudaMemcpyHostToDevice, c->st));
+    VCK(cudaStreamSynchronize(c->st));
+    return VHCI_OK;
+  }
   for (int j = 0; j < k; j += w) {
     const int m = std::min(w, k - j);
     VCK(h2d(c, t.p, host + (size_t)j * n, (size_t)n * m * sizeof(double)));
@@ -1039,7 +1059,18 @@ int upload_cols(vhci_ctx* c, const double* host, int64_t n, int k, double* dev, 
 int download_cols(vhci_ctx* c, const double* dev, int lds, int64_t n, int k, double* host) {
   const int w = transfer_cols(n, k);
   DBuf<double> t;
-  VCK(t.reserve((size_t)n * w, c->st));
+  bool have = false;
+  VTRY(transfer_buffer(c, t, (size_t)n * w, &have));
+  if (!have) {
+    std::vector<double> h((size_t)n * k);
+    c->stats.d2h_bytes += (int64_t)(h.size() * sizeof(double));
+    VCK(cudaMemcpy2DAsync(h.data(), k * sizeof(double), dev, lds * sizeof(double), k * sizeof(double), n,
+                          cudaMemcpyDeviceToHost, c->st));
+    VCK(cudaStreamSynchronize(c->st));
+    for (int64_t i = 0; i < n; ++i)
+      for (int j = 0; j < k; ++j) host[(size_t)j * n + i] = h[(size_t)i * k + j];
+    return VHCI_OK;
+  }
   for (int j = 0; j < k; j += w) {
     const int m = std::min(w, k - j);
     rows_to_cols(dev + j, lds, n, m, t.p, c->st);

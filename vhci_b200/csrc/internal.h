@@ -70,7 +70,8 @@ struct EventPair {
 };
 
 // Blocks of k column-major host vectors (n x k, leading dimension n) to a row-major device block and
-// back, a few columns at a time through a device buffer of limited size.
+// back, a few columns at a time through a device buffer of limited size (transposed on the host when there
+// is no memory for it).
 int upload_cols(vhci_ctx* c, const double* host, int64_t n, int k, double* dev, int ldd);
 int download_cols(vhci_ctx* c, const double* dev, int lds, int64_t n, int k, double* host);
 // Device buffers of a walk's kept connections.
