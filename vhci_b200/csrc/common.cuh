@@ -64,12 +64,16 @@ __host__ __device__ __forceinline__ uint64_t mix64(uint64_t x) {
 
 // Key hash in two parts: a sum that is linear in the key words (mod 2^64), so the sum of a target
 // key k + delta is that of k plus a constant of delta (stored per connection group), and a
-// finaliser.
+// finaliser.  The multipliers: the golden ratio's first 64 bits, and a spacing that must be even, so that
+// all of them are odd (an even one would drop the word's top bit): the first constant of P. Evensen's
+// rrxmrrxmsx_0 mixer less one.
 constexpr int kMaxKeyWords = 8;
+constexpr uint64_t kHashFirst = 0x9E3779B97F4A7C15ull, kHashStep = 0xA24BAED4963EE406ull;
+static_assert(kHashFirst % 2 == 1 && kHashStep % 2 == 0, "every multiplier is odd");
 __host__ __device__ __forceinline__ uint64_t hash_word(uint64_t k, int w) {
-  // odd multipliers, spaced by an odd constant
-  return k * (0x9E3779B97F4A7C15ull + 0xA24BAED4963EE406ull * (uint64_t)w);
+  return k * (kHashFirst + kHashStep * (uint64_t)w);
 }
+// degski's 64-bit mixer (xor-shift, multiply, twice) with the second multiplication left out
 __host__ __device__ __forceinline__ uint64_t hash_final(uint64_t x) {
   x ^= x >> 32;
   x *= 0xD6E8FEB86659FD93ull;
