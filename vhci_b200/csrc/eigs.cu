@@ -60,9 +60,21 @@ int small_eigs_start(vhci_ctx* c, const double* T, int m, int ld, int nk, double
   return VHCI_OK;
 }
 
+static thread_local int t_waits_lost = 0;
+
+// For the tests, not part of the interface: small_eig_polls; returns how many of this thread's solves
+// reported a wait that ran out since the call before.
+extern "C" int vhci_test_grid_polls(int polls) {
+  const int lost = t_waits_lost;
+  t_waits_lost = 0;
+  small_eig_polls(polls);
+  return lost;
+}
+
 bool small_eigs_verdict(const double* words) {
   unsigned long long err;
   std::memcpy(&err, words + 3, sizeof(err));
+  if (err) ++t_waits_lost;
   return small_eig_good(words[0], words[1], err);
 }
 

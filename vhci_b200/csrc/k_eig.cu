@@ -305,7 +305,7 @@ __device__ __forceinline__ double grid_block_sum(double v, double (&red)[2][kGri
 __global__ void __launch_bounds__(kGridThreads, 1) k_tridiag_grid(
     const double* __restrict__ T, int ldt, int m, double* __restrict__ d, double* __restrict__ e,
     double* __restrict__ tau, double* __restrict__ V, double* xch, unsigned long long* ctr,
-    unsigned long long* err, double* __restrict__ tail) {
+    unsigned long long* err, double* __restrict__ tail, int max_polls) {
   extern __shared__ double sm[];
   __shared__ double red[2][kGridWarps], s_v[kGridRows], s_p[kGridRows], s_x[2];
   __shared__ double s_part[kGridWarps][kGridRows];
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(kGridThreads, 1) k_tridiag_grid(
         int polls = 0;
         do {
           asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(seen) : "l"(ctr) : "memory");
-        } while (seen < want && ++polls < (1 << 21));
+        } while (seen < want && ++polls < max_polls);
         if (seen < want) {
           s_stop = 1;
           *err = 1;
@@ -975,6 +975,11 @@ TriKernel tri_kernel(int m) {
   return m <= 192 ? k_tridiag<6> : m <= 256 ? k_tridiag<8> : m <= 384 ? k_tridiag<12> : k_tridiag<20>;
 }
 
+// Polls of k_tridiag_grid's counter before a block gives up (over a second); the tests lower it for their
+// thread, to see the wait run out.
+constexpr int kGridPolls = 1 << 21;
+thread_local int t_grid_polls = kGridPolls;
+
 // Shared-memory and cluster limits of the kernels, set once per device.
 constexpr int kMaxDevices = 64;
 std::once_flag g_eig_once[kMaxDevices];
@@ -999,6 +1004,8 @@ bool eig_attributes() {
 }
 
 }  // namespace
+
+void small_eig_polls(int polls) { t_grid_polls = polls > 0 ? polls : kGridPolls; }
 
 size_t small_eig_elems(int m, int nk) {
   // d, e, tau; the exchange; V; two vector blocks; S; the last rows
@@ -1044,7 +1051,7 @@ bool small_eig(const double* T, int ldt, int m, int nk, double* theta, double* Y
       cfg.dynamicSmemBytes = grid_smem(m);
       at.id = cudaLaunchAttributeCooperative;
       at.val.cooperative = 1;
-      err = cudaLaunchKernelEx(&cfg, k_tridiag_grid, T, ldt, m, d, e, tau, V, rowx, dev + 2, dev + 3, tail);
+      err = cudaLaunchKernelEx(&cfg, k_tridiag_grid, T, ldt, m, d, e, tau, V, rowx, dev + 2, dev + 3, tail, t_grid_polls);
     }
     if (err != cudaSuccess) {
       cudaGetLastError();

@@ -247,6 +247,8 @@ constexpr int kClusterEigMax = 640, kSmallEigMax = 1800, kSmallEigDev = 4;
 size_t small_eig_elems(int m, int nk);
 bool small_eig(const double* T, int ldt, int m, int nk, double* theta, double* Y, int ldy, double* work,
                unsigned long long* dev, cudaStream_t s);
+// Limit of the waits between the grid's blocks for this thread's calls (0: the usual one).
+void small_eig_polls(int polls);
 // Each correction squares the deviation (times 3/4 of the number of vectors at worst): from these
 // bounds the second leaves less than 1e-15 of it.
 inline bool small_eig_good(double dev0, double dev1, unsigned long long err) {
