@@ -246,12 +246,16 @@ __global__ void __launch_bounds__(256, 4) k_spmm_f32x(int64_t n, const int64_t* 
   const bool on = cc < bq;
   const int64_t stride = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += stride) {
-    double a[4];
+    double a[4], xd[4], d = 0.0;
+    const bool put = on && lane < BQ;
+    if (put) {  // asked for before the row's gathers
+      d = diag[i];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) xd[c] = Xd[i * ldd + 4 * cc + c];
+    }
     row_product<kSpmmUnrollF, BQ, 4>(__ldg(rowptr + i), __ldg(rowptr + i + 1), col, val, X,
                                      ldx / 4, cc, on, a);
-    if (!on || lane >= BQ) continue;
-    const double d = diag[i];
-    const double* xd = Xd + i * ldd + 4 * cc;
+    if (!put) continue;
     double* y = Y + i * ldy + 4 * cc;
 #pragma unroll
     for (int c = 0; c < 4; ++c) y[c] = fma(d, xd[c], a[c]);
