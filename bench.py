@@ -61,13 +61,13 @@ def bench_config(workload: int, batch: int) -> dict:
 
 # Basis size after each heat-bath iteration and |P| of the workload-1 solve (FP64 path).
 WORKLOAD_COUNTS = {"sizes": [38934, 215006, 336950, 372333, 380418], "n_pert": 6583465}
-# DRAM traffic of one product over its algorithmic bytes, from an ncu capture of its earlier form
-# (dram__bytes_read.sum + dram__bytes_write.sum = 4.186e9 + 0.051e9 bytes) of a 16-column product
+# DRAM traffic of one product over its algorithmic bytes, from an ncu capture of k_spmm<8, 2, double>
+# (dram__bytes_read.sum + dram__bytes_write.sum = 3.85e9 + 0.049e9 bytes) of a 16-column product
 # on the final workload-1 basis (380,418 rows, 255,052,558 entries; algorithmic 3.164e9 bytes) by
-# `python bench.py --spmm-sweep --sweep-eigs --sweep-reps 2 --checkpoint <file>` on B200.  The
+# `python bench.py --spmm-sweep --sweep-reps 2 --checkpoint <file>` on B200.  The
 # bench's launches run on every basis of the solve, so their traffic is this ratio times their
 # algorithmic bytes (the excess is vector-block gathers that miss L2, which scales with the entries).
-NCU_SPMM_TRAFFIC_RATIO = (4.186275e9 + 0.051259e9) / 3.1641044e9
+NCU_SPMM_TRAFFIC_RATIO = (3.85e9 + 0.049e9) / 3.1641044e9
 
 
 def _dist():

@@ -96,7 +96,8 @@ typedef struct {
   double ms_spmm;                 /* part of ms_eigs spent in the SpMM kernel                  */
   int64_t spmm_calls, spmm_cols;  /* SpMM launches and total vector columns multiplied         */
   int64_t spmm_bytes;             /* algorithmic bytes of all SpMM launches                    */
-  int64_t hbuild_probes;          /* hash probes issued by the Hamiltonian build               */
+  int64_t hbuild_probes;          /* twice the (row, connection group) pairs of the rows built:
+                                     an upper bound of what the build's walks look up          */
   int64_t select_candidates;      /* candidate states generated by heat-bath selection         */
   int64_t pt2_entries;            /* perturber-Hamiltonian entries (a, i, H_ai)                */
   int64_t pt2_perturbers;         /* |P|                                                       */
